@@ -37,6 +37,11 @@ SIGNATURES = {
     "dilution_backward_scratch_bytes": (_Z, [_L, _L, _I]),
     "dilution_backward": (_I, [_P, _P, _P, _I, _I, _L, _L, _I, _F, _F,
                                _P, _I, _P, _P, _P, _P, _I, _P, _P, _P, _P, _P, _P, _P, _P]),
+    "dilution_split_operands": (_I, [_P, _P, _P, _L, _I, _P, _P, _P, _P]),
+    "dilution_wide_forward": (_I, [_P, _P, _P, _I, _L, _L, _I, _F, _F, _P, _P, _P, _P, _P, _P, _P, _P]),
+    "dilution_wide_scratch_bytes": (_Z, [_I, _L, _L, _I]),
+    "dilution_wide_backward": (_I, [_P, _P, _P, _I, _L, _L, _I, _F, _F, _P, _I, _P, _P, _P, _P, _P, _P, _P, _P,
+                                    _P, _P, _P, _P]),
     "dilution_decode_scratch_bytes": (_Z, [_L, _L, _I]),
     "dilution_decode": (_I, [_P, _P, _P, _I, _L, _L, _L, _I, _F, _F, _P, _P, _P, _P]),
     "dilution_decode_append": (_I, [_P, _P, _P, _P, _P, _I, _L, _L, _L, _I, _F, _F, _P, _P, _P, _P]),
@@ -113,3 +118,11 @@ def carry_rows(dtype_code: int, precision_code: int, head_dim: int, training: bo
 def tensor_core_path(dtype_code: int, precision_code: int, head_dim: int) -> bool:
     """True when a call with these parameters runs on the tcgen05 kernels."""
     return dtype_code == BF16 and precision_code == PREC["bf16"] and head_dim == 64
+
+
+def wide_path(dtype_code: int, precision_code: int, head_dim: int) -> bool:
+    """True for the cases of the tcgen05 kernels' 256-byte rows (dilution_wide_forward): bf16 heads of 128
+    under "bf16", fp32 heads of up to 64 under "tf32"."""
+    if dtype_code == BF16:
+        return precision_code == PREC["bf16"] and head_dim == 128
+    return precision_code == PREC["tf32"] and head_dim in (16, 32, 64)

@@ -17,6 +17,7 @@
 #include "tc_kernels.cuh"
 #include "tc_rowpass_kernels.cuh"
 #include "tc_fused_forward.cuh"
+#include "tc_wide_kernels.cuh"
 #define DILUTION_TENSOR_PATH 1
 #endif
 
@@ -107,7 +108,7 @@ int check_carry_rows(const char* fn, int dtype, int precision, int d, int64_t q_
 
 dil::Geom make_geom(int64_t n, int64_t tq, int64_t tk, int64_t q_offset, float scale, float eps,
                     int carry_rows = dil::kCarryRows, int bid = dil::kBidSoftmax,
-                    int share = dil::kShareInclusive, float shift = 1.f) {
+                    int share = dil::kShareInclusive, float shift = 1.f, int d = 64) {
   dil::Geom g;
   g.carry_rows = carry_rows;
   g.bid = dil::bid_form(bid);
@@ -115,6 +116,7 @@ dil::Geom make_geom(int64_t n, int64_t tq, int64_t tk, int64_t q_offset, float s
   g.normalised = bid == dil::kBidSoftmax || dil::row_sum_bid(bid);
   g.lshift = (bid == dil::kBidExpshift || bid == dil::kBidSigshift) ? log2f(shift) : 0.f;
   g.ghat_pass = 0;
+  g.d = d;
   g.n = n;
   g.tq = (int)tq;
   g.tk = (int)tk;
@@ -623,6 +625,78 @@ int dilution_backward(const void* q, const void* k, const void* v, int dtype, in
   DIL_DISPATCH(dtype, d, DIL_DISPATCH_MMA(precision, return (launch_backward<T, D, MMA>(
       q, k, v, g, (const float*)dout, out, rmax, rden, carry, ssum, pk, s, dq, dk, dv, st))))
   return DILUTION_OK;
+}
+
+// ---- rows of 256 bytes: bf16 heads of 128, fp32 heads of up to 64 as hi | lo planes -----------------
+static int check_wide(const char* fn, int dtype, int64_t n, int64_t t, int d) {
+  if (int rc = check_common(fn, dtype, dtype == DILUTION_F32 ? DILUTION_PREC_TF32 : DILUTION_PREC_BF16, n, t, t, 0, d)) return rc;
+  if (dtype == DILUTION_BF16 ? d != 128 : d > 64)
+    return fail(DILUTION_ERR_UNSUPPORTED, "%s: bf16 heads of 128 or fp32 heads of at most 64 (got %d)", fn, d);
+  return DILUTION_OK;
+}
+
+int dilution_split_operands(const float* q, const float* k, const float* v, int64_t rows, int d, void* qs, void* ks,
+                            void* vs, void* stream) {
+  if (!q || !k || !v || !qs || !ks || !vs) return fail(DILUTION_ERR_ARG, "dilution_split_operands: null pointer");
+  if (rows < 1 || rows > ((int64_t)1 << 34) || !valid_d(d) || d > 64)
+    return fail(DILUTION_ERR_ARG, "dilution_split_operands: rows must be positive and d one of 16, 32, 64");
+  if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)qs | (uintptr_t)ks | (uintptr_t)vs) & 15)
+    return fail(DILUTION_ERR_ARG, "dilution_split_operands: tensors must be 16-byte aligned");
+#ifdef DILUTION_TENSOR_PATH
+  cudaStream_t st = (cudaStream_t)stream;
+  using bf = __nv_bfloat16;
+  const dil::tc::SplitArgs a{{q, k, v}, {(bf*)qs, (bf*)ks, (bf*)vs}};
+  Prof prof("tc_split_operands", st);
+  return dil::tc::split_operands(a, 3, rows, d, st, g_err, sizeof(g_err));
+#else
+  return fail(DILUTION_ERR_UNSUPPORTED, "built without the tensor-core path");
+#endif
+}
+
+int dilution_wide_forward(const void* q, const void* k, const void* v, int dtype, int64_t n, int64_t t, int d,
+                          float scale, float eps, float* rmax, float* rden, float* carry, float* total, float* out,
+                          float* ssum, float* pk, void* stream) {
+  if (int rc = check_wide("dilution_wide_forward", dtype, n, t, d)) return rc;
+  if (!q || !k || !v || !rmax || !rden || !carry || !total || !out || !ssum)
+    return fail(DILUTION_ERR_ARG, "dilution_wide_forward: null pointer");
+#ifdef DILUTION_TENSOR_PATH
+  const dil::Geom g = make_geom(n, t, t, 0, scale, eps, dil::kCarryRows, dil::kBidSoftmax, dil::kShareInclusive, 1.f, d);
+  auto fwd = dtype == DILUTION_F32 ? dil::tc::wide_forward<dil::tc::kSplit> : dil::tc::wide_forward<dil::tc::kWide128>;
+  return fwd(q, k, v, g, rmax, rden, carry, total, out, ssum, pk, (cudaStream_t)stream, g_err, sizeof(g_err), mark_scope);
+#else
+  return fail(DILUTION_ERR_UNSUPPORTED, "built without the tensor-core path");
+#endif
+}
+
+size_t dilution_wide_scratch_bytes(int dtype, int64_t n, int64_t t, int d) {
+  if (n < 1 || t < 1 || d < 1) return 0;
+  const size_t rows = (size_t)(n * t);
+  return rows * (2 * sizeof(float) * (dtype == DILUTION_F32 ? 64 : 128) + 2 * 128 + 2 * sizeof(float));
+}
+
+int dilution_wide_backward(const void* q, const void* k, const void* v, int dtype, int64_t n, int64_t t, int d,
+                           float scale, float eps, const void* dout, int dout_dtype, const float* out,
+                           const float* rmax, const float* rden, const float* carry, const float* total,
+                           const float* ssum, const float* pk, void* scratch, void* dq, void* dk, void* dv,
+                           void* stream) {
+  if (int rc = check_wide("dilution_wide_backward", dtype, n, t, d)) return rc;
+  if (!q || !k || !v || !dout || !out || !rmax || !rden || !carry || !total || !ssum || !pk || !scratch || !dq || !dk || !dv)
+    return fail(DILUTION_ERR_ARG, "dilution_wide_backward: null pointer");
+  if (dout_dtype != DILUTION_F32 && dout_dtype != DILUTION_BF16)
+    return fail(DILUTION_ERR_ARG, "dilution_wide_backward: dout_dtype must be DILUTION_F32 or DILUTION_BF16");
+#ifdef DILUTION_TENSOR_PATH
+  const dil::Geom g = make_geom(n, t, t, 0, scale, eps, dil::kCarryRows, dil::kBidSoftmax, dil::kShareInclusive, 1.f, d);
+  const int64_t rows = n * t, head = dtype == DILUTION_F32 ? 64 : 128;
+  float* dq_main = (float*)scratch;
+  float* dk_main = dq_main + rows * head;
+  char* dop = (char*)(dk_main + rows * head);         // a TMA source: in front of the two (n, t) vectors
+  float* ghat = (float*)(dop + 2 * 128 * rows);
+  auto bwd = dtype == DILUTION_F32 ? dil::tc::wide_backward<dil::tc::kSplit> : dil::tc::wide_backward<dil::tc::kWide128>;
+  return bwd(q, k, v, g, dout, dout_dtype, out, rmax, rden, carry, total, ssum, pk, dq_main, dk_main, dop, ghat,
+             ghat + rows, dq, dk, dv, (cudaStream_t)stream, g_err, sizeof(g_err), mark_scope);
+#else
+  return fail(DILUTION_ERR_UNSUPPORTED, "built without the tensor-core path");
+#endif
 }
 
 size_t dilution_decode_scratch_bytes(int64_t n, int64_t length, int d) {

@@ -120,6 +120,7 @@ struct Geom {
                   // row statistics and the backward has the Jacobian correction ghat; otherwise
                   // l = lshift for every row
   float lshift;   // log2 of the shift of expshift / sigshift (kernels_bid.py:19-26); 0 for the sigmoid
+  int d;          // head size of q, k, v and of every output row
   int ghat_pass;  // reverse pass of an f(a) / rowsum(f) bid, whose Jacobian factor is unbounded (1 / row mass):
                   // 1 = accumulate ghat only, 2 = ghat is known and is subtracted BEFORE the factor
                   // multiplies (kernels_bid.py:718); 0 = one pass, correction afterwards (softmax: jac = p <= 1)

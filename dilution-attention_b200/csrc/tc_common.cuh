@@ -28,6 +28,26 @@ constexpr int kHeadDim = 64;
 constexpr uint32_t kTileBytes = kTileRows * kHeadDim * 2;   // 16 KB
 constexpr long long kWaitCycles = 4000000000LL;             // ~2 s: a live wait is microseconds
 
+// How many [rows][64 bf16] sub-tiles one row of q, k, v or dout takes, and what they hold.
+//   kNarrow : heads of 64 in bf16, one sub-tile;
+//   kWide128: heads of 128 in bf16, two sub-tiles of 64 features;
+//   kSplit  : heads of up to 64 in fp32, each value as hi + lo with hi = bf16(x), lo = bf16(x - hi):
+//             sub-tile 0 holds the hi parts, sub-tile 1 the lo parts (zeros behind the head size).  A product of
+//             two such operands keeps 16 bits of each (2^-17 relative), where tf32 keeps 11.
+// Sub-tile s of a [128 rows] tile lies kTileBytes * s behind its start.
+enum : int { kNarrow = 0, kWide128 = 1, kSplit = 2 };
+template <int W> struct Rows {
+  static constexpr int kSub = W == kNarrow ? 1 : 2;
+  static constexpr int kPlanes = W == kSplit ? 2 : 1;              // bf16 parts of a value the kernels form
+  static constexpr int kCols = 64 * kSub;                          // accumulator columns of a product with k, v, q or dout
+  static constexpr int kHead = W == kWide128 ? 128 : 64;           // head size (kSplit: padded)
+  static constexpr uint32_t kBytes = kSub * kTileBytes;            // one [128 rows] tile
+  // score products: sub-tile pairs (a, b) that are multiplied.  kSplit leaves out lo * lo (2^-18 of the score).
+  static constexpr int kPairs = W == kNarrow ? 1 : W == kWide128 ? 2 : 3;
+  static __device__ constexpr int pair_a(int i) { return W == kSplit ? (i == 2) : i; }
+  static __device__ constexpr int pair_b(int i) { return W == kSplit ? (i == 1) : i; }
+};
+
 enum : int { kErrWaitTma = 101, kErrWaitMma = 102, kErrWaitDrain = 103, kErrAlign = 104, kErrWaitTile = 105, kErrSelfTest = 199 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -107,15 +127,23 @@ __device__ __forceinline__ void fence_async_smem() {
 }
 
 // ---- TMA ----------------------------------------------------------------------
-// One [box rows][64 bf16] tile of a (n, t, 64) tensor: coordinates (0, row, n).
+// One [box rows][64 bf16] tile of a (n, t, 64 or 128) tensor: coordinates (col, row, n).
 __device__ __forceinline__ void tma_load_tile(uint32_t dst, const CUtensorMap* map, int row, int n,
-                                              uint32_t bar) {
+                                              uint32_t bar, int col = 0) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
       " [%0], [%1, {%3, %4, %5}], [%2];"
       :
-      : "r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(0), "r"(row), "r"(n)
+      : "r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(col), "r"(row), "r"(n)
       : "memory");
+}
+
+// All sub-tiles of one tile, `sub_bytes` apart (kTileBytes for 128 rows).
+template <int W>
+__device__ __forceinline__ void tma_load_rows(uint32_t dst, const CUtensorMap* map, int row, int n, uint32_t bar,
+                                              uint32_t sub_bytes = kTileBytes) {
+#pragma unroll
+  for (int s = 0; s < Rows<W>::kSub; ++s) tma_load_tile(dst + sub_bytes * s, map, row, n, bar, 64 * s);
 }
 
 // Element-wise add of a shared-memory tile into global memory (performed at L2), one
@@ -292,12 +320,22 @@ __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, Desc b,
       : "memory");
 }
 
-// S[128 x n_cols] = A[128 x 64] * B[n_cols x 64]^T, both K-major tiles: 4 instructions.
-__device__ __forceinline__ void mma_scores(uint32_t d_tmem, uint32_t a_smem, uint32_t b_smem, int n_cols) {
-  const uint32_t idesc = instr_desc(128, n_cols, 0, 0);
-  const Desc a = make_desc(a_smem, 16, 1024), b = make_desc(b_smem, 16, 1024);
+// S[128 x n_cols] = A[128 rows] * B[n_cols rows]^T over the features of a row, both K-major: four instructions per
+// pair of sub-tiles, which lie a_sub and b_sub bytes apart.
+template <int W>
+__device__ __forceinline__ void mma_scores_wide(uint32_t d_tmem, Desc a, uint32_t a_sub, Desc b, uint32_t b_sub,
+                                                uint32_t idesc) {
 #pragma unroll
-  for (int kk = 0; kk < 4; ++kk) mma_ss(d_tmem, a, 2 * kk, b, 2 * kk, idesc, kk > 0);
+  for (int i = 0; i < Rows<W>::kPairs; ++i)
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk)
+      mma_ss(d_tmem, a, (a_sub >> 4) * Rows<W>::pair_a(i) + 2 * kk, b, (b_sub >> 4) * Rows<W>::pair_b(i) + 2 * kk, idesc,
+             i > 0 || kk > 0);
+}
+template <int W>
+__device__ __forceinline__ void mma_scores_w(uint32_t d_tmem, uint32_t a_smem, uint32_t b_smem, int n_cols) {
+  mma_scores_wide<W>(d_tmem, make_desc(a_smem, 16, 1024), kTileBytes, make_desc(b_smem, 16, 1024), kTileBytes,
+                     instr_desc(128, n_cols, 0, 0));
 }
 
 // Dynamic shared memory base rounded up to 1024 bytes.

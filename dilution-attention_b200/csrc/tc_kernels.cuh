@@ -67,10 +67,11 @@ inline void ensure_context() {
 struct MapKey {
   const void* base;
   int64_t n, t;
-  int kind;      // 0: bf16 box {64, rows, 1}; 1: fp32 box {32, 128, 1}
+  int kind;      // 0: bf16 box {64, rows, 1}; 1: fp32 box {32, rows, 1}, swizzled; 2: the same, not swizzled
   int box_rows;
+  int feat;      // row length of the tensor in elements
   bool operator==(const MapKey& o) const {
-    return base == o.base && n == o.n && t == o.t && kind == o.kind && box_rows == o.box_rows;
+    return base == o.base && n == o.n && t == o.t && kind == o.kind && box_rows == o.box_rows && feat == o.feat;
   }
 };
 struct MapCache {
@@ -97,11 +98,11 @@ inline MapCache& map_cache() {
   return c;
 }
 
-// (n, t, 64) bf16 row-major -> 3-D map {64, t, n}, box {64, 128, 1}, 128-byte swizzle.
+// (n, t, feat) bf16 row-major -> 3-D map {feat, t, n}, box {64, rows, 1}, 128-byte swizzle.
 // Rows past t read as zero, and a box never crosses into the next (batch, head) row.
 inline int make_map(CUtensorMap* map, const void* base, int64_t n, int64_t t, char* err, size_t errlen,
-                    int box_rows = kTileRows) {
-  const MapKey key{base, n, t, 0, box_rows};
+                    int feat = kHeadDim, int box_rows = kTileRows) {
+  const MapKey key{base, n, t, 0, box_rows, feat};
   if (map_cache().find(key, map)) return 0;
   ensure_context();
   EncodeTiledFn fn = encode_fn();
@@ -113,8 +114,8 @@ inline int make_map(CUtensorMap* map, const void* base, int64_t n, int64_t t, ch
     snprintf(err, errlen, "bf16 tensor-core path needs 16-byte aligned q/k/v");
     return 1;
   }
-  const cuuint64_t dims[3] = {(cuuint64_t)kHeadDim, (cuuint64_t)t, (cuuint64_t)n};
-  const cuuint64_t strides[2] = {(cuuint64_t)kHeadDim * 2, (cuuint64_t)t * kHeadDim * 2};
+  const cuuint64_t dims[3] = {(cuuint64_t)feat, (cuuint64_t)t, (cuuint64_t)n};
+  const cuuint64_t strides[2] = {(cuuint64_t)feat * 2, (cuuint64_t)t * feat * 2};
   const cuuint32_t box[3] = {(cuuint32_t)kHeadDim, (cuuint32_t)box_rows, 1};
   const cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides,
@@ -128,10 +129,11 @@ inline int make_map(CUtensorMap* map, const void* base, int64_t n, int64_t t, ch
   return 0;
 }
 
-// (n, t, 64) fp32 row-major -> 3-D map {64, t, n}, box {32, 128, 1} (128 bytes wide),
-// 128-byte swizzle: the target of the dQ tile reductions.
-inline int make_map_f32(CUtensorMap* map, const void* base, int64_t n, int64_t t, char* err, size_t errlen) {
-  const MapKey key{base, n, t, 1, kTileRows};
+// (n, t, feat) fp32 row-major -> 3-D map {feat, t, n}, box {32, rows, 1} (128 bytes wide), with the
+// 128-byte swizzle or (swizzle = false) plain rows: the target of the O and dQ tile reductions.
+inline int make_map_f32(CUtensorMap* map, const void* base, int64_t n, int64_t t, char* err, size_t errlen,
+                        int feat = kHeadDim, int box_rows = kTileRows, bool swizzle = true) {
+  const MapKey key{base, n, t, swizzle ? 1 : 2, box_rows, feat};
   if (map_cache().find(key, map)) return 0;
   ensure_context();
   EncodeTiledFn fn = encode_fn();
@@ -139,12 +141,13 @@ inline int make_map_f32(CUtensorMap* map, const void* base, int64_t n, int64_t t
     snprintf(err, errlen, "cuTensorMapEncodeTiled is not available from the driver");
     return 3;
   }
-  const cuuint64_t dims[3] = {(cuuint64_t)kHeadDim, (cuuint64_t)t, (cuuint64_t)n};
-  const cuuint64_t strides[2] = {(cuuint64_t)kHeadDim * 4, (cuuint64_t)t * kHeadDim * 4};
-  const cuuint32_t box[3] = {32, (cuuint32_t)kTileRows, 1};
+  const cuuint64_t dims[3] = {(cuuint64_t)feat, (cuuint64_t)t, (cuuint64_t)n};
+  const cuuint64_t strides[2] = {(cuuint64_t)feat * 4, (cuuint64_t)t * feat * 4};
+  const cuuint32_t box[3] = {32, (cuuint32_t)box_rows, 1};
   const cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides, box,
-                        estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     snprintf(err, errlen, "cuTensorMapEncodeTiled (fp32) failed (%d)", (int)r);
@@ -165,6 +168,26 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   uint32_t r;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
   return r;
+}
+
+// bf16 pair of what `hi` (a packed pair of the rounded values) leaves of (a, b): the lo plane of a split value.
+__device__ __forceinline__ uint32_t pack_bf16_rest(float a, float b, uint32_t hi) {
+  return pack_bf16(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xffff0000u));
+}
+
+// 32 columns of one output row; kSplit rows end after `left` columns (a multiple of 16).
+template <int W>
+__device__ __forceinline__ void store_row32(float* dst, const float* m, int left) {
+#pragma unroll
+  for (int e = 0; e < 32; e += 4)
+    if (W != kSplit || e < left) *reinterpret_cast<float4*>(dst + e) = make_float4(m[e], m[e + 1], m[e + 2], m[e + 3]);
+}
+template <int W>
+__device__ __forceinline__ void store_row32(__nv_bfloat16* dst, const float* m, int) {
+#pragma unroll
+  for (int e = 0; e < 32; e += 8)
+    *reinterpret_cast<uint4*>(dst + e) = make_uint4(pack_bf16(m[e], m[e + 1]), pack_bf16(m[e + 2], m[e + 3]),
+                                                    pack_bf16(m[e + 4], m[e + 5]), pack_bf16(m[e + 6], m[e + 7]));
 }
 
 // Byte offset of the 16-byte chunk holding queries [q, q+8) of `key` in an
@@ -197,17 +220,19 @@ __device__ __forceinline__ float bid_p(float s, float zscale, float l) {
 // grid = n * ceil(tq/128), longest rows first.  S = Q K^T, lane = query: each
 // thread reduces its 64 key columns of the tile with an online max / sum; the two
 // halves of a row are merged once at the end.  TMEM: 128 columns; 4 CTAs per SM.
-constexpr int kRowstatsSmem = 3 * kTileBytes + 1024 + 1024 + 256;
+template <int W> constexpr int kRowstatsSmem = 3 * (int)Rows<W>::kBytes + 1024 + 1024 + 256;
 
-__global__ void __launch_bounds__(256, 4) rowstats_kernel(const __grid_constant__ CUtensorMap map_q,
+template <int W = kNarrow>
+__global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) rowstats_kernel(const __grid_constant__ CUtensorMap map_q,
                                                           const __grid_constant__ CUtensorMap map_k,
                                                           Geom g, float* __restrict__ rmax,
                                                           float* __restrict__ rden) {
+  constexpr uint32_t TB = Rows<W>::kBytes;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
-  const uint32_t sQ = smem_u32(smem), sK0 = sQ + kTileBytes;
-  float2* sMerge = reinterpret_cast<float2*>(smem + 3 * kTileBytes);          // [128]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 3 * kTileBytes + 1024);
+  const uint32_t sQ = smem_u32(smem), sK0 = sQ + TB;
+  float2* sMerge = reinterpret_cast<float2*>(smem + 3 * TB);          // [128]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 3 * TB + 1024);
   Ctl* ctl = reinterpret_cast<Ctl*>(bars + 8);
   const uint32_t kfull = smem_u32(bars), sdone = smem_u32(bars + 2);
 
@@ -231,12 +256,12 @@ __global__ void __launch_bounds__(256, 4) rowstats_kernel(const __grid_constant_
   const uint32_t tmem = ctl->tmem;
 
   if (tid == 0) {
-    mbar_expect_tx(kfull, 2 * kTileBytes);
-    tma_load_tile(sQ, &map_q, ib * kTileRows, n, kfull);
-    tma_load_tile(sK0, &map_k, 0, n, kfull);
+    mbar_expect_tx(kfull, 2 * TB);
+    tma_load_rows<W>(sQ, &map_q, ib * kTileRows, n, kfull);
+    tma_load_rows<W>(sK0, &map_k, 0, n, kfull);
     if (njb > 1) {
-      mbar_expect_tx(kfull + 8, kTileBytes);
-      tma_load_tile(sK0 + kTileBytes, &map_k, kTileRows, n, kfull + 8);
+      mbar_expect_tx(kfull + 8, TB);
+      tma_load_rows<W>(sK0 + TB, &map_k, kTileRows, n, kfull + 8);
     }
   }
   float m = -INFINITY, s = 0.f;
@@ -247,15 +272,15 @@ __global__ void __launch_bounds__(256, 4) rowstats_kernel(const __grid_constant_
     if (tid == 0) {
       mbar_wait(kfull + 8 * b, (jb >> 1) & 1, ctl, &g_status, kErrWaitTma);
       tc_fence_after();
-      mma_scores(tmem, sQ, sK0 + kTileBytes * b, 128);
+      mma_scores_w<W>(tmem, sQ, sK0 + TB * b, 128);
       mma_commit(sdone);
     }
     __syncwarp();
     mbar_wait(sdone, jb & 1, ctl, &g_status, kErrWaitMma);
     tc_fence_after();
     if (tid == 0 && jb + 2 < njb) {     // this K stage is free again
-      mbar_expect_tx(kfull + 8 * b, kTileBytes);
-      tma_load_tile(sK0 + kTileBytes * b, &map_k, (jb + 2) * kTileRows, n, kfull + 8 * b);
+      mbar_expect_tx(kfull + 8 * b, TB);
+      tma_load_rows<W>(sK0 + TB * b, &map_k, (jb + 2) * kTileRows, n, kfull + 8 * b);
     }
     __syncwarp();
     const bool edge = (jb * kTileRows + kTileRows - 1 > q0) || ((jb + 1) * kTileRows > g.tk);
@@ -320,21 +345,22 @@ __global__ void __launch_bounds__(256, 4) rowstats_kernel(const __grid_constant_
 // a backward will read the checkpoints (two threads per key there, 32 queries each),
 // 64 for forward-only calls (the main forward pass starts its two warpgroups at queries
 // 0 and 64 of a tile): half the scratch and half the checkpoint stores.
-constexpr int kColsumSmem = 3 * kTileBytes + 1024 + 2048 + 1024 + 256;
+template <int W> constexpr int kColsumSmem = 3 * (int)Rows<W>::kBytes + 1024 + 2048 + 1024 + 256;
 
-template <int CR, int BID = kBidSoftmax>
-__global__ void __launch_bounds__(256, 4) colsum_scan_kernel(
+template <int CR, int BID = kBidSoftmax, int W = kNarrow>
+__global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) colsum_scan_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, Geom g,
     const float* __restrict__ rmax, const float* __restrict__ rden,
     const float* __restrict__ carry_base, float* __restrict__ carry, float* __restrict__ total) {
   static_assert(CR == 32 || CR == 64, "checkpoints every 32 or 64 query rows");
   constexpr int kPerTile = kTileRows / CR;                                      // 4 or 2
+  constexpr uint32_t TB = Rows<W>::kBytes;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
-  const uint32_t sK = smem_u32(smem), sQ0 = sK + kTileBytes;
-  float* sL = reinterpret_cast<float*>(smem + 3 * kTileBytes);                 // [2][128]
-  float2* sCs = reinterpret_cast<float2*>(smem + 3 * kTileBytes + 1024);       // [2][128] the two sums of warpgroup 1
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 3 * kTileBytes + 3072);
+  const uint32_t sK = smem_u32(smem), sQ0 = sK + TB;
+  float* sL = reinterpret_cast<float*>(smem + 3 * TB);                 // [2][128]
+  float2* sCs = reinterpret_cast<float2*>(smem + 3 * TB + 1024);       // [2][128] the two sums of warpgroup 1
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 3 * TB + 3072);
   Ctl* ctl = reinterpret_cast<Ctl*>(bars + 8);
   const uint32_t qfull = smem_u32(bars), sdone = smem_u32(bars + 2);
 
@@ -362,12 +388,12 @@ __global__ void __launch_bounds__(256, 4) colsum_scan_kernel(
   const uint32_t tmem = ctl->tmem;
 
   if (tid == 0 && nib > 0) {
-    mbar_expect_tx(qfull, 2 * kTileBytes);
-    tma_load_tile(sK, &map_k, k0, n, qfull);
-    tma_load_tile(sQ0, &map_q, ib0 * kTileRows, n, qfull);
+    mbar_expect_tx(qfull, 2 * TB);
+    tma_load_rows<W>(sK, &map_k, k0, n, qfull);
+    tma_load_rows<W>(sQ0, &map_q, ib0 * kTileRows, n, qfull);
     if (nib > 1) {
-      mbar_expect_tx(qfull + 8, kTileBytes);
-      tma_load_tile(sQ0 + kTileBytes, &map_q, (ib0 + 1) * kTileRows, n, qfull + 8);
+      mbar_expect_tx(qfull + 8, TB);
+      tma_load_rows<W>(sQ0 + TB, &map_q, (ib0 + 1) * kTileRows, n, qfull + 8);
     }
   }
   const int ja = k0 + row;
@@ -399,7 +425,7 @@ __global__ void __launch_bounds__(256, 4) colsum_scan_kernel(
     if (tid == 0) {
       mbar_wait(qfull + 8 * b, (it >> 1) & 1, ctl, &g_status, kErrWaitTma);
       tc_fence_after();
-      mma_scores(tmem, sK, sQ0 + kTileBytes * b, 128);
+      mma_scores_w<W>(tmem, sK, sQ0 + TB * b, 128);
       mma_commit(sdone);
     }
     __syncwarp();
@@ -410,8 +436,8 @@ __global__ void __launch_bounds__(256, 4) colsum_scan_kernel(
     mbar_wait(sdone, it & 1, ctl, &g_status, kErrWaitMma);
     tc_fence_after();
     if (tid == 0 && it + 2 < nib) {
-      mbar_expect_tx(qfull + 8 * b, kTileBytes);
-      tma_load_tile(sQ0 + kTileBytes * b, &map_q, (ib + 2) * kTileRows, n, qfull + 8 * b);
+      mbar_expect_tx(qfull + 8 * b, TB);
+      tma_load_rows<W>(sQ0 + TB * b, &map_q, (ib + 2) * kTileRows, n, qfull + 8 * b);
     }
     __syncwarp();
     const int i0 = g.q_off + ib * kTileRows + 64 * wg;   // absolute position of this half's first query
@@ -473,29 +499,34 @@ __global__ void __launch_bounds__(256, 4) colsum_scan_kernel(
 //   rs  [query x 16] += share * ones   (row sums of the SAME bf16 shares)
 // so the final divide out = O / (rs + eps) normalises exactly what was summed.
 // TMEM: S^T 128 columns, O 64, rs 16 (256 allocated; two CTAs per SM).
-constexpr int kMainSmem = 7 * kTileBytes + 512 + 128;   // exact: the base must already be 1024-aligned
+// Q, K[2], V, ones, shares (two 64-query sub-tiles per plane); exact: the base must already be 1024-aligned
+template <int W> constexpr int kMainSmem =
+    4 * (int)Rows<W>::kBytes + (1 + 2 * Rows<W>::kPlanes) * (int)kTileBytes + 512 + 128;
 
 // BID / SHARE select the ablations of kernels_bid.py (sigmoid bid; exclusive or absent share step,
 // :254-262); the default instantiation is the operator.
-template <int BID = kBidSoftmax, int SHARE = kShareInclusive>
-__global__ void __launch_bounds__(256, 2) forward_main_kernel(
+template <int BID = kBidSoftmax, int SHARE = kShareInclusive, int W = kNarrow>
+__global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) forward_main_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, Geom g, const float* __restrict__ rmax,
     const float* __restrict__ rden, const float* __restrict__ carry,
     const float* __restrict__ carry_base, float* __restrict__ out, float* __restrict__ ssum) {
+  constexpr uint32_t TB = Rows<W>::kBytes;
+  constexpr int kOCols = Rows<W>::kCols + 16;        // O and the row sums: one tile
+  constexpr int kTmem = W == kNarrow ? 256 : 512;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   if (smem_u32(smem) & 1023u) {                      // no slack is requested: refuse instead of overrunning
     if (threadIdx.x == 0) atomicCAS(&g_status, 0, kErrAlign);
     return;
   }
-  const uint32_t sQ = smem_u32(smem), sK0 = sQ + kTileBytes, sV = sQ + 3 * kTileBytes;
-  // a [128 keys][64] bf16 tile of ones right behind V: the second 64-column group of the B
-  // operand of share @ [V | ones] (N = 80), so the row sums come out of the same MMA
-  const uint32_t sOnes = sQ + 4 * kTileBytes, sSh = sQ + 5 * kTileBytes;
-  uint8_t* ones_ptr = smem + 4 * kTileBytes;
-  float* sL = reinterpret_cast<float*>(smem + 7 * kTileBytes);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 7 * kTileBytes + 512);
+  const uint32_t sQ = smem_u32(smem), sK0 = sQ + TB, sV = sQ + 3 * TB;
+  // a [128 keys][64] bf16 tile of ones right behind V: the last 64-column group of the B
+  // operand of share @ [V | ones] (N = 80 or 144), so the row sums come out of the same MMA
+  const uint32_t sOnes = sQ + 4 * TB, sSh = sOnes + kTileBytes;
+  uint8_t* ones_ptr = smem + 4 * TB;
+  float* sL = reinterpret_cast<float*>(smem + 4 * TB + (1 + 2 * Rows<W>::kPlanes) * kTileBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(sL) + 512);
   Ctl* ctl = reinterpret_cast<Ctl*>(bars + 8);
   const uint32_t kfull = smem_u32(bars), vfull = smem_u32(bars + 2), sdone = smem_u32(bars + 3);
 
@@ -513,7 +544,7 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
     fence_barrier_init();
   }
   __syncwarp();
-  if (warp == 0) tmem_alloc(smem_u32(&ctl->tmem), 256);
+  if (warp == 0) tmem_alloc(smem_u32(&ctl->tmem), kTmem);
   if (wg == 0) sL[row] = load_lse<BID>(rmax, rden, (int64_t)n * g.tq, ib * kTileRows + row, g.tq, g.lshift);
   else {
 #pragma unroll
@@ -525,21 +556,21 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = ctl->tmem;
-  const uint32_t tS = tmem, tO = tmem + 128, tR = tmem + 192;   // O (64) and row sums (16): one N = 80 tile
+  const uint32_t tS = tmem, tO = tmem + 128, tR = tO + Rows<W>::kCols;
 
   if (tid == 0) {
-    mbar_expect_tx(kfull, 2 * kTileBytes);
-    tma_load_tile(sQ, &map_q, ib * kTileRows, n, kfull);
-    tma_load_tile(sK0, &map_k, 0, n, kfull);
-    mbar_expect_tx(vfull, kTileBytes);
-    tma_load_tile(sV, &map_v, 0, n, vfull);
+    mbar_expect_tx(kfull, 2 * TB);
+    tma_load_rows<W>(sQ, &map_q, ib * kTileRows, n, kfull);
+    tma_load_rows<W>(sK0, &map_k, 0, n, kfull);
+    mbar_expect_tx(vfull, TB);
+    tma_load_rows<W>(sV, &map_v, 0, n, vfull);
     if (njb > 1) {
-      mbar_expect_tx(kfull + 8, kTileBytes);
-      tma_load_tile(sK0 + kTileBytes, &map_k, kTileRows, n, kfull + 8);
+      mbar_expect_tx(kfull + 8, TB);
+      tma_load_rows<W>(sK0 + TB, &map_k, kTileRows, n, kfull + 8);
     }
     mbar_wait(kfull, 0, ctl, &g_status, kErrWaitTma);
     tc_fence_after();
-    mma_scores(tS, sK0, sQ, 128);
+    mma_scores_w<W>(tS, sK0, sQ, 128);
     mma_commit(sdone);
   }
   __syncwarp();
@@ -569,12 +600,12 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
     tc_fence_after();
     if (tid == 0) {
       if (jb >= 1) {                      // the V buffer is free: the previous share*V finished
-        mbar_expect_tx(vfull, kTileBytes);
-        tma_load_tile(sV, &map_v, jb * kTileRows, n, vfull);
+        mbar_expect_tx(vfull, TB);
+        tma_load_rows<W>(sV, &map_v, jb * kTileRows, n, vfull);
       }
       if (jb >= 1 && jb + 1 < njb) {      // K stage of tile jb-1 is free
-        mbar_expect_tx(kfull + 8 * (b ^ 1), kTileBytes);
-        tma_load_tile(sK0 + kTileBytes * (b ^ 1), &map_k, (jb + 1) * kTileRows, n, kfull + 8 * (b ^ 1));
+        mbar_expect_tx(kfull + 8 * (b ^ 1), TB);
+        tma_load_rows<W>(sK0 + TB * (b ^ 1), &map_k, (jb + 1) * kTileRows, n, kfull + 8 * (b ^ 1));
       }
     }
     __syncwarp();
@@ -593,7 +624,7 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
       float4 lnext[2] = {L4[c * 8], L4[c * 8 + 1]};
 #pragma unroll
       for (int e8 = 0; e8 < 4; ++e8) {
-        uint32_t packed[4];
+        uint32_t packed[4], rest[4];
         const float4 lcur[2] = {lnext[0], lnext[1]};
         if (e8 < 3) {
           lnext[0] = L4[c * 8 + e8 * 2 + 2];
@@ -622,11 +653,19 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
           }
           packed[h * 2 + 0] = pack_bf16(sh[0], sh[1]);
           packed[h * 2 + 1] = pack_bf16(sh[2], sh[3]);
+          if (W == kSplit) {
+            rest[h * 2 + 0] = pack_bf16_rest(sh[0], sh[1], packed[h * 2 + 0]);
+            rest[h * 2 + 1] = pack_bf16_rest(sh[2], sh[3], packed[h * 2 + 1]);
+          }
         }
         const uint32_t dst = sSh + share_chunk_offset(row, wg * 64 + c * 32 + e8 * 8);
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(packed[0]),
                      "r"(packed[1]), "r"(packed[2]), "r"(packed[3])
                      : "memory");
+        if (W == kSplit)
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + 2 * kTileBytes), "r"(rest[0]),
+                       "r"(rest[1]), "r"(rest[2]), "r"(rest[3])
+                       : "memory");
       }
     }
     };
@@ -638,15 +677,18 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
       tc_fence_after();
       mbar_wait(vfull, jb & 1, ctl, &g_status, kErrWaitTma);
       tc_fence_after();
-      constexpr uint32_t id_o = instr_desc(128, 80, 1, 1);
+      constexpr uint32_t id_o = instr_desc(128, kOCols, 1, 1);
       // descriptors are built once per tile; a k-step is a constant 2048 B (128 units) further
-      const Desc dSh = make_desc(sSh, kTileBytes, 1024), dVm = make_desc(sV, sOnes - sV, 1024);
+      const Desc dSh = make_desc(sSh, kTileBytes, 1024), dVm = make_desc(sV, kTileBytes, 1024);
 #pragma unroll
-      for (int kk = 0; kk < 8; ++kk) mma_ss(tO, dSh, 128 * kk, dVm, 128 * kk, id_o, (jb > 0 || kk > 0));
+      for (int pl = 0; pl < Rows<W>::kPlanes; ++pl)
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)
+          mma_ss(tO, dSh, 2048 * pl + 128 * kk, dVm, 128 * kk, id_o, (jb > 0 || pl > 0 || kk > 0));
       if (jb + 1 < njb) {
         mbar_wait(kfull + 8 * (b ^ 1), ((jb + 1) >> 1) & 1, ctl, &g_status, kErrWaitTma);
         tc_fence_after();
-        mma_scores(tS, sK0 + kTileBytes * (b ^ 1), sQ, 128);
+        mma_scores_w<W>(tS, sK0 + TB * (b ^ 1), sQ, 128);
       }
       mma_commit(sdone);
     }
@@ -655,27 +697,42 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
   mbar_wait(sdone, njb & 1, ctl, &g_status, kErrWaitMma);
   tc_fence_after();
   {
-    // lane = query now: each warpgroup stores 32 of the 64 output columns of row `row`
+    // lane = query now: each warpgroup stores half of the output columns of row `row`, 32 at a time
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-    float o[32], r[32];
-    tmem_ld32(tO + lane_base + 32 * wg, o);
-    tmem_ld32(tR + lane_base, r);
-    tmem_ld_wait(o);
-    tmem_ld_wait(r);
+    constexpr int kHalf = Rows<W>::kHead / 2;
     const int i = ib * kTileRows + row;
-    if (i < g.tq) {
-      const float inv = 1.f / (r[0] + g.eps);
-      float4* dst = reinterpret_cast<float4*>(out + ((int64_t)n * g.tq + i) * kHeadDim + 32 * wg);
+    float rs;
+    tmem_ld1(tR + lane_base, &rs);
+    tmem_ld_wait();
+    const float inv = 1.f / (rs + g.eps);
+    const int d = W == kSplit ? g.d : Rows<W>::kHead;
 #pragma unroll
-      for (int c = 0; c < 8; ++c)
-        dst[c] = make_float4(o[4 * c] * inv, o[4 * c + 1] * inv, o[4 * c + 2] * inv, o[4 * c + 3] * inv);
-      if (wg == 0) ssum[(int64_t)n * g.tq + i] = r[0];
+    for (int c0 = 0; c0 < kHalf; c0 += 32) {
+      const int col = kHalf * wg + c0;
+      float o[32];
+      tmem_ld32(tO + lane_base + col, o);
+      tmem_ld_wait(o);
+      if (W == kSplit) {                              // share V_hi + share V_lo
+        float lo[32];
+        tmem_ld32(tO + lane_base + 64 + col, lo);
+        tmem_ld_wait(lo);
+#pragma unroll
+        for (int e = 0; e < 32; ++e) o[e] += lo[e];
+      }
+      if (i < g.tq) {
+        float4* dst = reinterpret_cast<float4*>(out + ((int64_t)n * g.tq + i) * d + col);
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          if (W != kSplit || col + 4 * c < d)
+            dst[c] = make_float4(o[4 * c] * inv, o[4 * c + 1] * inv, o[4 * c + 2] * inv, o[4 * c + 3] * inv);
+      }
     }
+    if (i < g.tq && wg == 0) ssum[(int64_t)n * g.tq + i] = rs;
   }
   drain_if_aborted(ctl);
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_free(tmem, 256);
+  if (warp == 0) tmem_free(tmem, kTmem);
 }
 
 // ---------------------------------------------------------------- pass 4: backward
@@ -706,6 +763,95 @@ __global__ void backward_prep_kernel(const TD* __restrict__ dout, const float* _
   if (lane == 0) {
     dbarp[row] = dot * sinv;
     ghat[row] = 0.f;
+  }
+}
+
+// One thread's 32 queries of the main reverse pass: vs holds their raw scores against the thread's key, vd
+// dO' . v; incle is the key's demand (+ eps) in front of them, R the suffix of dk_share behind them, and query
+// e sees the key when e >= first_q.  Afterwards shp holds the shares as bf16 pairs (SPLIT: their lo plane
+// behind them), vs the Jacobian factor, vd that factor times dp, and R the suffix in front of the queries.
+// Two sweeps.  Forwards: p and 1/(committed+p+eps), the demand
+// accumulated from the checkpoint in front exactly as the forward pass did.  Backwards: the
+// suffix of dk_share (kernels.py:763-764), accumulated from the last query to the first as
+// the reference does — its terms grow towards a key's first bidders, so the other order
+// loses the small ones.
+template <int BID, int SHARE, bool MASK, bool SPLIT>
+__device__ __forceinline__ void reverse_sweeps(float (&vs)[32], float (&vd)[32], uint32_t* shp, float& R, float incle,
+                                               const float4* Lse4, const float4* Dbar4, const Geom& g, bool dead,
+                                               int first_q) {
+  float inv[32];
+#pragma unroll
+  for (int e4 = 0; e4 < 8; ++e4) {
+    const float4 l4 = Lse4[e4];
+    const float lse[4] = {l4.x, l4.y, l4.z, l4.w};
+    // softmax: z = s*zscale - lse, p = 2^z;  sigmoid: z = lse - s*zscale, p = 1/(1 + 2^z)
+    const float zsign = BID == kBidSigmoid ? -g.zscale : g.zscale;
+    const float lsign = BID == kBidSigmoid ? 1.f : -1.f;
+    const float2 zs = make_float2(zsign, zsign);
+    const float2 z01 = fma2(make_float2(vs[e4 * 4], vs[e4 * 4 + 1]), zs, make_float2(lsign * lse[0], lsign * lse[1]));
+    const float2 z23 = fma2(make_float2(vs[e4 * 4 + 2], vs[e4 * 4 + 3]), zs, make_float2(lsign * lse[2], lsign * lse[3]));
+    const float z[4] = {z01.x, z01.y, z23.x, z23.y};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int e = e4 * 4 + u;
+      float p = fast_exp2(z[u]);
+      if (BID == kBidSigmoid) p = fast_rcp(1.f + p);
+      if (MASK) {
+        if (dead || first_q > e) p = 0.f;
+      }
+      if (SHARE == kShareInclusive) {
+        incle += p;
+        inv[e] = fast_rcp(incle);
+      } else if (SHARE == kShareExclusive) {     // the demand of earlier queries only
+        inv[e] = fast_rcp(incle);
+        incle += p;
+      } else {
+        inv[e] = 1.f;
+      }
+      vs[e] = p;
+    }
+  }
+#pragma unroll
+  for (int e4 = 7; e4 >= 0; --e4) {
+    const float4 d4 = Dbar4[e4];
+    const float dbr[4] = {d4.x, d4.y, d4.z, d4.w};
+    // with inv = 1/(committed+p+eps), share = p*inv and w = ds*inv:
+    //   ds*(committed+eps)*inv^2 = w*(1-share),  dk_share = -w*share,
+    //   dp = w - w*share + (suffix before this query) = w + (suffix after it)
+    // (element-wise parts two queries per instruction; the suffix itself is serial).
+    // Exclusive share step (inv = 1/(committed+eps)): the direct term is w itself, so
+    // dp = w + (suffix BEFORE this query); no share step: dp = ds, no suffix at all.
+    // The Jacobian factor is p for the softmax bid and p(1-p) for the sigmoid
+    // (kernels_bid.py:196-204, 735-754); vs keeps it for the later suffix fix-up.
+#pragma unroll
+    for (int h = 1; h >= 0; --h) {
+      const int e = e4 * 4 + 2 * h;
+      const float2 p2 = make_float2(vs[e], vs[e + 1]), i2 = make_float2(inv[e], inv[e + 1]);
+      const float2 w2 = mul2(sub2(make_float2(vd[e], vd[e + 1]), make_float2(dbr[2 * h], dbr[2 * h + 1])), i2);
+      const float2 s2 = mul2(p2, i2);
+      float2 jac2 = p2;
+      if (BID == kBidSigmoid) jac2 = mul2(p2, sub2(make_float2(1.f, 1.f), p2));
+      float2 pd2;
+      if (SHARE == kShareInclusive) {
+        const float r1 = fmaf(-w2.y, s2.y, R);
+        R = fmaf(-w2.x, s2.x, r1);
+        pd2 = mul2(jac2, add2(w2, make_float2(R, r1)));
+      } else if (SHARE == kShareExclusive) {
+        const float r1 = fmaf(-w2.y, s2.y, R);
+        pd2 = mul2(jac2, add2(w2, make_float2(r1, R)));
+        R = fmaf(-w2.x, s2.x, r1);
+      } else {
+        pd2 = mul2(jac2, w2);
+      }
+      vd[e] = pd2.x;
+      vd[e + 1] = pd2.y;
+      if (BID == kBidSigmoid) {
+        vs[e] = jac2.x;
+        vs[e + 1] = jac2.y;
+      }
+      shp[e4 * 2 + h] = pack_bf16(s2.x, s2.y);
+      if (SPLIT) shp[16 + e4 * 2 + h] = pack_bf16_rest(s2.x, s2.y, shp[e4 * 2 + h]);
+    }
   }
 }
 
@@ -1035,88 +1181,9 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
       // warpgroup 0 (queries 32..63) knows the suffix of dk_share behind its queries; warpgroup 1
       // starts from zero and adds p * (the suffix warpgroup 0 ends with) afterwards: dp is linear in it
       float R = wg == 0 ? sigma : 0.f;
-      float incle = incl + g.eps;                      // demand + eps at the walk's position
-
-      // Two sweeps over the thread's 32 queries.  Forwards: p and 1/(committed+p+eps), the demand
-      // accumulated from the checkpoint in front exactly as the forward pass did.  Backwards: the
-      // suffix of dk_share (kernels.py:763-764), accumulated from the last query to the first as
-      // the reference does — its terms grow towards a key's first bidders, so the other order
-      // loses the small ones.  Afterwards vs holds p and vd holds p * dp.
       auto chunk = [&](auto mask_tag) {
-        constexpr bool MASK = decltype(mask_tag)::value;
-        float inv[32];
-#pragma unroll
-        for (int e4 = 0; e4 < 8; ++e4) {
-          const float4 l4 = Lse4[e4];
-          const float lse[4] = {l4.x, l4.y, l4.z, l4.w};
-          // softmax: z = s*zscale - lse, p = 2^z;  sigmoid: z = lse - s*zscale, p = 1/(1 + 2^z)
-          const float zsign = BID == kBidSigmoid ? -g.zscale : g.zscale;
-          const float lsign = BID == kBidSigmoid ? 1.f : -1.f;
-          const float2 zs = make_float2(zsign, zsign);
-          const float2 z01 = fma2(make_float2(vs[e4 * 4], vs[e4 * 4 + 1]), zs, make_float2(lsign * lse[0], lsign * lse[1]));
-          const float2 z23 = fma2(make_float2(vs[e4 * 4 + 2], vs[e4 * 4 + 3]), zs, make_float2(lsign * lse[2], lsign * lse[3]));
-          const float z[4] = {z01.x, z01.y, z23.x, z23.y};
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int e = e4 * 4 + u;
-            float p = fast_exp2(z[u]);
-            if (BID == kBidSigmoid) p = fast_rcp(1.f + p);
-            if (MASK) {
-              if (dead || ja > iq0 + e) p = 0.f;
-            }
-            if (SHARE == kShareInclusive) {
-              incle += p;
-              inv[e] = fast_rcp(incle);
-            } else if (SHARE == kShareExclusive) {     // the demand of earlier queries only
-              inv[e] = fast_rcp(incle);
-              incle += p;
-            } else {
-              inv[e] = 1.f;
-            }
-            vs[e] = p;
-          }
-        }
-#pragma unroll
-        for (int e4 = 7; e4 >= 0; --e4) {
-          const float4 d4 = Dbar4[e4];
-          const float dbr[4] = {d4.x, d4.y, d4.z, d4.w};
-          // with inv = 1/(committed+p+eps), share = p*inv and w = ds*inv:
-          //   ds*(committed+eps)*inv^2 = w*(1-share),  dk_share = -w*share,
-          //   dp = w - w*share + (suffix before this query) = w + (suffix after it)
-          // (element-wise parts two queries per instruction; the suffix itself is serial).
-          // Exclusive share step (inv = 1/(committed+eps)): the direct term is w itself, so
-          // dp = w + (suffix BEFORE this query); no share step: dp = ds, no suffix at all.
-          // The Jacobian factor is p for the softmax bid and p(1-p) for the sigmoid
-          // (kernels_bid.py:196-204, 735-754); vs keeps it for the later suffix fix-up.
-#pragma unroll
-          for (int h = 1; h >= 0; --h) {
-            const int e = e4 * 4 + 2 * h;
-            const float2 p2 = make_float2(vs[e], vs[e + 1]), i2 = make_float2(inv[e], inv[e + 1]);
-            const float2 w2 = mul2(sub2(make_float2(vd[e], vd[e + 1]), make_float2(dbr[2 * h], dbr[2 * h + 1])), i2);
-            const float2 s2 = mul2(p2, i2);
-            float2 jac2 = p2;
-            if (BID == kBidSigmoid) jac2 = mul2(p2, sub2(make_float2(1.f, 1.f), p2));
-            float2 pd2;
-            if (SHARE == kShareInclusive) {
-              const float r1 = fmaf(-w2.y, s2.y, R);
-              R = fmaf(-w2.x, s2.x, r1);
-              pd2 = mul2(jac2, add2(w2, make_float2(R, r1)));
-            } else if (SHARE == kShareExclusive) {
-              const float r1 = fmaf(-w2.y, s2.y, R);
-              pd2 = mul2(jac2, add2(w2, make_float2(r1, R)));
-              R = fmaf(-w2.x, s2.x, r1);
-            } else {
-              pd2 = mul2(jac2, w2);
-            }
-            vd[e] = pd2.x;
-            vd[e + 1] = pd2.y;
-            if (BID == kBidSigmoid) {
-              vs[e] = jac2.x;
-              vs[e + 1] = jac2.y;
-            }
-            shp[e4 * 2 + h] = pack_bf16(s2.x, s2.y);
-          }
-        }
+        reverse_sweeps<BID, SHARE, decltype(mask_tag)::value, false>(vs, vd, shp, R, incl + g.eps, Lse4, Dbar4, g, dead,
+                                                                     ja - iq0);
       };
       if (masked_tile) chunk(std::true_type{}); else chunk(std::false_type{});
       // warpgroup 0: the suffix behind query 32; warpgroup 1: minus its own sum of -dk_share
@@ -1260,7 +1327,7 @@ __global__ void __launch_bounds__(256, 2) backward_correction_kernel(
     }
     mbar_wait(qfull, 0, ctl, &g_status, kErrWaitTma);
     tc_fence_after();
-    mma_scores(tS, sK, sQ0, 128);
+    mma_scores_w<kNarrow>(tS, sK, sQ0, 128);
     mma_commit(sdone);
   }
   __syncwarp();
@@ -1362,7 +1429,7 @@ __global__ void __launch_bounds__(256, 2) backward_correction_kernel(
       if (t + 1 < nsteps) {
         mbar_wait(qfull + 8 * (b ^ 1), ((t + 1) >> 1) & 1, ctl, &g_status, kErrWaitTma);
         tc_fence_after();
-        mma_scores(tS, sK, sQ0 + kTileBytes * (b ^ 1), 128);
+        mma_scores_w<kNarrow>(tS, sK, sQ0 + kTileBytes * (b ^ 1), 128);
       }
       mma_commit(sdone);
     }
@@ -1438,7 +1505,7 @@ __global__ void cast_dq_kernel(const float* __restrict__ src, __nv_bfloat16* __r
 // The opt-in to more than 48 KB of dynamic shared memory is per kernel and per device: it is
 // made on the first launch of that kernel on that device and remembered.
 inline int set_smem_attr(const void* fn, int bytes, char* err, size_t errlen) {
-  constexpr int kKernels = 16, kDevices = 64;
+  constexpr int kKernels = 64, kDevices = 64;
   static std::mutex mu;
   static const void* fns[kKernels];
   static bool done[kKernels][kDevices];
@@ -1477,7 +1544,7 @@ inline int launch_status(const char* what, char* err, size_t errlen) {
 // Shared memory of the 256-column kernels is padded so that at most two CTAs share
 // an SM (an SM has 512 TMEM columns); the 128-column kernels fit four by themselves.
 constexpr int kTwoPerSm = 100 * 1024;
-static_assert(5 * (kRowstatsSmem + 1024) > 233472 && 5 * (kColsumSmem + 1024) > 233472,
+static_assert(5 * (kRowstatsSmem<kNarrow> + 1024) > 233472 && 5 * (kColsumSmem<kNarrow> + 1024) > 233472,
               "at most four CTAs of a 128-column kernel may share an SM");
 
 // Compile-time bid / share of a launch from the run-time fields of its geometry.
@@ -1494,10 +1561,10 @@ inline int rowstats(const void* q, const void* k, const Geom& g, float* rmax, fl
   CUtensorMap mq, mk;
   if (int rc = make_map(&mq, q, g.n, g.tq, err, errlen)) return rc;
   if (int rc = make_map(&mk, k, g.n, g.tk, err, errlen)) return rc;
-  constexpr int smem = kRowstatsSmem;
-  if (int rc = set_smem_attr((const void*)rowstats_kernel, smem, err, errlen)) return rc;
+  constexpr int smem = kRowstatsSmem<kNarrow>;
+  if (int rc = set_smem_attr((const void*)rowstats_kernel<>, smem, err, errlen)) return rc;
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
-  rowstats_kernel<<<(unsigned)(g.n * nqb), 256, smem, st>>>(mq, mk, g, rmax, rden);
+  rowstats_kernel<><<<(unsigned)(g.n * nqb), 256, smem, st>>>(mq, mk, g, rmax, rden);
   return launch_status("tc rowstats", err, errlen);
 }
 
@@ -1507,7 +1574,7 @@ inline int colsum_scan(const void* q, const void* k, const Geom& g, const float*
   CUtensorMap mq, mk;
   if (int rc = make_map(&mq, q, g.n, g.tq, err, errlen)) return rc;
   if (int rc = make_map(&mk, k, g.n, g.tk, err, errlen)) return rc;
-  constexpr int smem = kColsumSmem;
+  constexpr int smem = kColsumSmem<kNarrow>;
   const int nkb = (g.tk + kTileRows - 1) / kTileRows;
   const unsigned grid = (unsigned)(g.n * nkb);
   if (g.carry_rows == 32) {
@@ -1531,7 +1598,7 @@ inline int forward_main(const void* q, const void* k, const void* v, const Geom&
   if (int rc = make_map(&mq, q, g.n, g.tq, err, errlen)) return rc;
   if (int rc = make_map(&mk, k, g.n, g.tk, err, errlen)) return rc;
   if (int rc = make_map(&mv, v, g.n, g.tk, err, errlen)) return rc;
-  constexpr int smem = kMainSmem;
+  constexpr int smem = kMainSmem<kNarrow>;
   static_assert(2 * (smem + 1024) <= 233472 && 3 * (smem + 1024) > 233472, "exactly two CTAs of the main pass fit one SM");
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
   const unsigned grid = (unsigned)(g.n * nqb);

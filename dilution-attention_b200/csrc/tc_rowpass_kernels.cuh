@@ -31,31 +31,34 @@ namespace dil {
 namespace tc {
 
 constexpr float kRefLimit = 1099511627776.f;         // 2^40: a tile whose P~ sum to more moves the reference
-template <int MODE> struct RowpassSmem {
+template <int MODE, int W = kNarrow> struct RowpassSmem {
   // Q | K[stages] | (V[stages]) | stats [2][128] float4 | barriers + control.  Three stages when
   // K is the only streamed operand; two of K and two of V otherwise, so that two CTAs fit an SM.
   static constexpr int kStages = MODE == 2 ? 2 : 3;
   static constexpr int kTiles = 1 + kStages * (MODE == 2 ? 2 : 1);
-  static constexpr int kBytes = kTiles * (int)kTileBytes + 4096 + 256 + 1024;
+  static constexpr int kBytes = kTiles * (int)Rows<W>::kBytes + 4096 + 256 + 1024;
 };
 
-template <int MODE, typename TOut>
-__global__ void __launch_bounds__(256, 2) rowpass_product_kernel(
+template <int MODE, typename TOut, int W = kNarrow>
+__global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) rowpass_product_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, Geom g, float* __restrict__ rmax, float* __restrict__ rden,
     TOut* __restrict__ out) {
   static_assert(MODE == 1 || MODE == 2, "1: B = K (pk); 2: B = V (softmax attention)");
+  constexpr uint32_t TB = Rows<W>::kBytes;
+  constexpr int kAcc = Rows<W>::kCols;               // accumulator columns of one warpgroup
+  constexpr int kTmem = W == kNarrow ? 256 : 512;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
-  const uint32_t sQ = smem_u32(smem), sK0 = sQ + kTileBytes;
-  constexpr int kRowpassStages = RowpassSmem<MODE>::kStages;
-  const uint32_t sB0 = MODE == 2 ? sK0 + kRowpassStages * kTileBytes : sK0;
-  constexpr int kTiles = RowpassSmem<MODE>::kTiles;
-  float4* sStat = reinterpret_cast<float4*>(smem + kTiles * kTileBytes);            // [2][128]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kTiles * kTileBytes + 4096);
+  const uint32_t sQ = smem_u32(smem), sK0 = sQ + TB;
+  constexpr int kRowpassStages = RowpassSmem<MODE, W>::kStages;
+  const uint32_t sB0 = MODE == 2 ? sK0 + kRowpassStages * TB : sK0;
+  constexpr int kTiles = RowpassSmem<MODE, W>::kTiles;
+  float4* sStat = reinterpret_cast<float4*>(smem + kTiles * TB);            // [2][128]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kTiles * TB + 4096);
   Ctl* ctl = reinterpret_cast<Ctl*>(bars + 8);
   const uint32_t kfull = smem_u32(bars), sdone = smem_u32(bars + 4);
-  float* sX = reinterpret_cast<float*>(smem + kTileBytes);    // merge area over the K stages: [2][128][32]
+  float* sX = reinterpret_cast<float*>(smem + TB);    // merge area over the K stages: [2][128][half a row]
 
   const int tid = threadIdx.x, warp = tid >> 5, wg = tid >> 7, row = tid & 127;
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
@@ -63,7 +66,7 @@ __global__ void __launch_bounds__(256, 2) rowpass_product_kernel(
   const int ib = nqb - 1 - (int)(blockIdx.x / g.n);
   const int q0 = g.q_off + ib * kTileRows;
   const int njb = min(g.tk - 1, q0 + kTileRows - 1) / kTileRows + 1;
-  constexpr uint32_t kStageTx = (MODE == 2 ? 2u : 1u) * kTileBytes;
+  constexpr uint32_t kStageTx = (MODE == 2 ? 2u : 1u) * TB;
 
   if (tid == 0) {
     ctl->abort = 0;
@@ -72,32 +75,32 @@ __global__ void __launch_bounds__(256, 2) rowpass_product_kernel(
     fence_barrier_init();
   }
   __syncwarp();
-  if (warp == 0) tmem_alloc(smem_u32(&ctl->tmem), 256);
+  if (warp == 0) tmem_alloc(smem_u32(&ctl->tmem), kTmem);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = ctl->tmem;
   const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-  const uint32_t tS = tmem, tO = tmem + 128 + 64 * wg;      // this warpgroup's accumulator
+  const uint32_t tS = tmem, tO = tmem + 128 + kAcc * wg;      // this warpgroup's accumulator
   {
     uint32_t z[16];
 #pragma unroll
     for (int c = 0; c < 16; ++c) z[c] = 0u;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) tmem_st16(tO + lane_base + 16 * c, z);
+    for (int c = 0; c < kAcc / 16; ++c) tmem_st16(tO + lane_base + 16 * c, z);
     tmem_st_wait();
   }
   auto load_stage = [&](int jb) {          // thread 0: K (and V) tile jb into its ring slot
     const int st = jb % kRowpassStages;
     mbar_expect_tx(kfull + 8 * st, kStageTx);
-    tma_load_tile(sK0 + kTileBytes * st, &map_k, jb * kTileRows, n, kfull + 8 * st);
-    if (MODE == 2) tma_load_tile(sB0 + kTileBytes * st, &map_v, jb * kTileRows, n, kfull + 8 * st);
+    tma_load_rows<W>(sK0 + TB * st, &map_k, jb * kTileRows, n, kfull + 8 * st);
+    if (MODE == 2) tma_load_rows<W>(sB0 + TB * st, &map_v, jb * kTileRows, n, kfull + 8 * st);
   };
   if (tid == 0) {
-    mbar_expect_tx(kfull, kStageTx + kTileBytes);
-    tma_load_tile(sQ, &map_q, ib * kTileRows, n, kfull);
-    tma_load_tile(sK0, &map_k, 0, n, kfull);
-    if (MODE == 2) tma_load_tile(sB0, &map_v, 0, n, kfull);
+    mbar_expect_tx(kfull, kStageTx + TB);
+    tma_load_rows<W>(sQ, &map_q, ib * kTileRows, n, kfull);
+    tma_load_rows<W>(sK0, &map_k, 0, n, kfull);
+    if (MODE == 2) tma_load_rows<W>(sB0, &map_v, 0, n, kfull);
     for (int jb = 1; jb < kRowpassStages && jb < njb; ++jb) load_stage(jb);
   }
   tc_fence_before();
@@ -106,7 +109,7 @@ __global__ void __launch_bounds__(256, 2) rowpass_product_kernel(
   if (tid == 0) {
     mbar_wait(kfull, 0, ctl, &g_status, kErrWaitTma);
     tc_fence_after();
-    mma_scores(tS, sQ, sK0, 128);
+    mma_scores_w<W>(tS, sQ, sK0, 128);
     mma_commit(sdone);
   }
   __syncwarp();
@@ -127,7 +130,7 @@ __global__ void __launch_bounds__(256, 2) rowpass_product_kernel(
     tmem_ld32(taddr + 32, v + 32);
     tmem_ld_wait(v);
     tmem_ld_wait(v + 32);
-    uint32_t pw[32];
+    uint32_t pw[32], pr[W == kSplit ? 32 : 1];
     float ps = 0.f;
     // P~ = 2^(z - reference) for the thread's 64 scores, two per instruction; their sum in ps
     auto exponentials = [&]() {
@@ -144,6 +147,10 @@ __global__ void __launch_bounds__(256, 2) rowpass_product_kernel(
         acc1 = add2(acc1, p1);
         pw[e >> 1] = pack_bf16(p0.x, p0.y);
         pw[(e >> 1) + 1] = pack_bf16(p1.x, p1.y);
+        if (W == kSplit) {
+          pr[e >> 1] = pack_bf16_rest(p0.x, p0.y, pw[e >> 1]);
+          pr[(e >> 1) + 1] = pack_bf16_rest(p1.x, p1.y, pw[(e >> 1) + 1]);
+        }
       }
       const float2 acc = add2(acc0, acc1);
       ps = acc.x + acc.y;
@@ -184,7 +191,7 @@ __global__ void __launch_bounds__(256, 2) rowpass_product_kernel(
         const float f = m_new == -INFINITY ? 1.f : fast_exp2(m_ref - m_new);
         if (!fresh) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
+          for (int c = 0; c < kAcc / 16; ++c) {
             float o[16];
             tmem_ld16(tO + lane_base + 16 * c, o);
             tmem_ld_wait16(o);
@@ -201,26 +208,32 @@ __global__ void __launch_bounds__(256, 2) rowpass_product_kernel(
     }
     s += ps;
     // P~ goes over the first 32 of this thread's 64 consumed score columns: keys 2c, 2c+1 of the
-    // warpgroup's half in column c
+    // warpgroup's half in column c (kSplit: the lo plane over the other 32)
     tmem_st16(taddr, pw);
     tmem_st16(taddr + 16, pw + 16);
+    if (W == kSplit) {
+      tmem_st16(taddr + 32, pr);
+      tmem_st16(taddr + 48, pr + 16);
+    }
     tmem_st_wait();
     tc_fence_before();
     __syncthreads();
     if (tid == 0) {
       tc_fence_after();
-      constexpr uint32_t id_pv = instr_desc(128, 64, 0, 1);   // A from TMEM (M = queries), B MN-major
-      const Desc dB = make_desc(sB0 + kTileBytes * st, kTileBytes, 1024);
+      constexpr uint32_t id_pv = instr_desc(128, kAcc, 0, 1);   // A from TMEM (M = queries), B MN-major
+      const Desc dB = make_desc(sB0 + TB * st, kTileBytes, 1024);
 #pragma unroll
       for (int w = 0; w < 2; ++w)
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)      // 16 keys per instruction: 16 rows of 128 B = 128 units
-          mma_ts(tmem + 128 + 64 * w, tS + 64 * w + 8 * kk, dB, 128 * (4 * w + kk), id_pv, 1);
+        for (int pl = 0; pl < Rows<W>::kPlanes; ++pl)
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)      // 16 keys per instruction: 16 rows of 128 B = 128 units
+            mma_ts(tmem + 128 + kAcc * w, tS + 64 * w + 32 * pl + 8 * kk, dB, 128 * (4 * w + kk), id_pv, 1);
       if (jb + 1 < njb) {
         const int sn = (jb + 1) % kRowpassStages;
         mbar_wait(kfull + 8 * sn, ((jb + 1) / kRowpassStages) & 1, ctl, &g_status, kErrWaitTma);
         tc_fence_after();
-        mma_scores(tS, sQ, sK0 + kTileBytes * sn, 128);
+        mma_scores_w<W>(tS, sQ, sK0 + TB * sn, 128);
       }
       mma_commit(sdone);
     }
@@ -228,22 +241,32 @@ __global__ void __launch_bounds__(256, 2) rowpass_product_kernel(
   }
   mbar_wait(sdone, njb & 1, ctl, &g_status, kErrWaitMma);
   tc_fence_after();
-  // merge the two halves of every row.  Each warpgroup finishes 32 of the 64 output columns:
-  // it hands the other 32 of its accumulator, with its statistics, to the other warpgroup.
+  // merge the two halves of every row.  Each warpgroup finishes half of the output columns:
+  // it hands the other half of its accumulator, with its statistics, to the other warpgroup.
   auto merge = [&](auto wg_c) {
     constexpr int WG = decltype(wg_c)::value;
-    float o[64];
-    tmem_ld32(tO + lane_base, o);
-    tmem_ld32(tO + lane_base + 32, o + 32);
-    tmem_ld_wait(o);
-    tmem_ld_wait(o + 32);
-    sStat[WG * 128 + row] = make_float4(m_ref, s, 0.f, 0.f);
-    float* give = sX + ((1 - WG) * 128 + row) * 32;         // read by the other warpgroup
+    constexpr int kHalf = Rows<W>::kHead / 2;
+    // columns [base, base + 32) of this warpgroup's accumulator (kSplit: P K_hi + P K_lo)
+    auto fetch = [&](int base, float* o) {
+      tmem_ld32(tO + lane_base + base, o);
+      tmem_ld_wait(o);
+      if (W == kSplit) {
+        float lo[32];
+        tmem_ld32(tO + lane_base + 64 + base, lo);
+        tmem_ld_wait(lo);
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      constexpr int base = 32 * (1 - WG);
-      reinterpret_cast<float4*>(give)[c ^ (row & 7)] =
-          make_float4(o[base + 4 * c], o[base + 4 * c + 1], o[base + 4 * c + 2], o[base + 4 * c + 3]);
+        for (int e = 0; e < 32; ++e) o[e] += lo[e];
+      }
+    };
+    sStat[WG * 128 + row] = make_float4(m_ref, s, 0.f, 0.f);
+    float* give = sX + ((1 - WG) * 128 + row) * kHalf;      // read by the other warpgroup
+#pragma unroll
+    for (int c0 = 0; c0 < kHalf; c0 += 32) {
+      float o[32];
+      fetch(kHalf * (1 - WG) + c0, o);
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        reinterpret_cast<float4*>(give + c0)[c ^ (row & 7)] = make_float4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
     }
     __syncthreads();
     const float4 other = sStat[(1 - WG) * 128 + row];
@@ -253,23 +276,28 @@ __global__ void __launch_bounds__(256, 2) rowpass_product_kernel(
     const float den = s * f_own + other.y * f_oth;
     const float inv = (MODE == 1 ? g.scale : 1.f) / den;
     const float a_own = f_own * inv, a_oth = f_oth * inv;
-    const float* take = sX + (WG * 128 + row) * 32;
+    const float* take = sX + (WG * 128 + row) * kHalf;
     const int i = ib * kTileRows + row;
-    if (i < g.tq) {
+    const int d = W == kSplit ? g.d : Rows<W>::kHead;
+#pragma unroll
+    for (int c0 = 0; c0 < kHalf; c0 += 32) {
       float r[32];
+      fetch(kHalf * WG + c0, r);
+      if (i >= g.tq) continue;
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
-        const float4 x = reinterpret_cast<const float4*>(take)[c ^ (row & 7)];
-        r[4 * c] = o[32 * WG + 4 * c] * a_own + x.x * a_oth;
-        r[4 * c + 1] = o[32 * WG + 4 * c + 1] * a_own + x.y * a_oth;
-        r[4 * c + 2] = o[32 * WG + 4 * c + 2] * a_own + x.z * a_oth;
-        r[4 * c + 3] = o[32 * WG + 4 * c + 3] * a_own + x.w * a_oth;
+        const float4 x = reinterpret_cast<const float4*>(take + c0)[c ^ (row & 7)];
+        r[4 * c] = r[4 * c] * a_own + x.x * a_oth;
+        r[4 * c + 1] = r[4 * c + 1] * a_own + x.y * a_oth;
+        r[4 * c + 2] = r[4 * c + 2] * a_own + x.z * a_oth;
+        r[4 * c + 3] = r[4 * c + 3] * a_own + x.w * a_oth;
       }
-      TOut* dst = out + ((int64_t)n * g.tq + i) * kHeadDim + 32 * WG;
+      TOut* dst = out + ((int64_t)n * g.tq + i) * d + kHalf * WG + c0;
       if (std::is_same<TOut, float>::value) {
 #pragma unroll
         for (int c = 0; c < 8; ++c)
-          reinterpret_cast<float4*>(dst)[c] = make_float4(r[4 * c], r[4 * c + 1], r[4 * c + 2], r[4 * c + 3]);
+          if (W != kSplit || kHalf * WG + c0 + 4 * c < d)
+            reinterpret_cast<float4*>(dst)[c] = make_float4(r[4 * c], r[4 * c + 1], r[4 * c + 2], r[4 * c + 3]);
       } else {
 #pragma unroll
         for (int c = 0; c < 4; ++c)
@@ -277,19 +305,19 @@ __global__ void __launch_bounds__(256, 2) rowpass_product_kernel(
               make_uint4(pack_bf16(r[8 * c], r[8 * c + 1]), pack_bf16(r[8 * c + 2], r[8 * c + 3]),
                          pack_bf16(r[8 * c + 4], r[8 * c + 5]), pack_bf16(r[8 * c + 6], r[8 * c + 7]));
       }
-      if (WG == 0 && rmax != nullptr) {
-        // the merged reference, not necessarily the row maximum (it lags behind it by design);
-        // every consumer uses the pair only as the log-sum-exp rmax + log2(rden)
-        rmax[(int64_t)n * g.tq + i] = m;
-        rden[(int64_t)n * g.tq + i] = den;
-      }
+    }
+    if (WG == 0 && i < g.tq && rmax != nullptr) {
+      // the merged reference, not necessarily the row maximum (it lags behind it by design);
+      // every consumer uses the pair only as the log-sum-exp rmax + log2(rden)
+      rmax[(int64_t)n * g.tq + i] = m;
+      rden[(int64_t)n * g.tq + i] = den;
     }
   };
   if (wg == 0) merge(std::integral_constant<int, 0>{}); else merge(std::integral_constant<int, 1>{});
   drain_if_aborted(ctl);
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_free(tmem, 256);
+  if (warp == 0) tmem_free(tmem, kTmem);
 }
 
 // Key half of the softmax-Jacobian correction alone (the reference's BC, kernels.py:777-809),
@@ -301,18 +329,22 @@ __global__ void __launch_bounds__(256, 2) rowpass_product_kernel(
 // a CTA allocates 128 (S^T 64 + dKc 64) and four CTAs share an SM (32 warps to hide each other's
 // MMA round trips, as in the column-sum pass; a version with 128-query steps and two CTAs per SM
 // measured 5% slower).  The two warpgroups split a half-step's 64 query columns.
-constexpr int kCorrKey64Smem = 3 * kTileBytes + 2048 + 1024 + 256;
-static_assert(5 * (kCorrKey64Smem + 1024) > 233472, "at most four CTAs of the half-step correction pass share an SM");
+template <int W> constexpr int kCorrKey64Smem = 3 * (int)Rows<W>::kBytes + 2048 + 1024 + 256;
+static_assert(5 * (kCorrKey64Smem<kNarrow> + 1024) > 233472, "at most four CTAs of the half-step correction pass share an SM");
 
-__global__ void __launch_bounds__(256, 4) backward_key_correction64_kernel(
+// TOut: element type of dk (bf16, or float for kSplit).
+template <int W = kNarrow, typename TOut = __nv_bfloat16>
+__global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) backward_key_correction64_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, Geom g,
     const float* __restrict__ rmax, const float* __restrict__ rden, const float* __restrict__ ghat,
-    const float* __restrict__ dk_main, __nv_bfloat16* __restrict__ dk) {
+    const float* __restrict__ dk_main, TOut* __restrict__ dk) {
+  constexpr uint32_t TB = Rows<W>::kBytes;
+  constexpr int kAcc = Rows<W>::kCols, kTmem = W == kNarrow ? 128 : 256;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
-  const uint32_t sK = smem_u32(smem), sQ0 = sK + kTileBytes;
-  float2* sStat = reinterpret_cast<float2*>(smem + 3 * kTileBytes);           // [2][128] (lse, ghat)
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 3 * kTileBytes + 2048);
+  const uint32_t sK = smem_u32(smem), sQ0 = sK + TB;
+  float2* sStat = reinterpret_cast<float2*>(smem + 3 * TB);           // [2][128] (lse, ghat)
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 3 * TB + 2048);
   Ctl* ctl = reinterpret_cast<Ctl*>(bars + 8);
   const uint32_t qfull = smem_u32(bars), sdone = smem_u32(bars + 2);
 
@@ -330,7 +362,7 @@ __global__ void __launch_bounds__(256, 4) backward_key_correction64_kernel(
     fence_barrier_init();
   }
   __syncwarp();
-  if (warp == 0) tmem_alloc(smem_u32(&ctl->tmem), 128);
+  if (warp == 0) tmem_alloc(smem_u32(&ctl->tmem), kTmem);
   if (wg == 1) {
     const int i = jb * kTileRows + row;
     float2 st = make_float2(INFINITY, 0.f);
@@ -342,22 +374,21 @@ __global__ void __launch_bounds__(256, 4) backward_key_correction64_kernel(
   tc_fence_after();
   const uint32_t tmem = ctl->tmem;
   const uint32_t tS = tmem, tDK = tmem + 64;
-  constexpr uint32_t id_s = instr_desc(128, 64, 0, 0), id_kd = instr_desc(128, 64, 0, 1);
+  constexpr uint32_t id_s = instr_desc(128, 64, 0, 0), id_kd = instr_desc(128, kAcc, 0, 1);
   // scores of half-step (stage, odd): queries 64*odd.. of the Q tile in that stage (K-major: a
-  // row is 128 B = 8 units)
+  // row is 128 B)
   auto issue_scores = [&](int stage, int odd) {
-    const Desc dKk = make_desc(sK, 16, 1024), dQk = make_desc(sQ0 + kTileBytes * stage, 16, 1024);
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk) mma_ss(tS, dKk, 2 * kk, dQk, 512 * odd + 2 * kk, id_s, kk > 0);
+    mma_scores_wide<W>(tS, make_desc(sK, 16, 1024), kTileBytes,
+                       make_desc(sQ0 + TB * stage + 8192 * odd, 16, 1024), kTileBytes, id_s);
   };
 
   if (tid == 0) {
-    mbar_expect_tx(qfull, 2 * kTileBytes);
-    tma_load_tile(sK, &map_k, k0, n, qfull);
-    tma_load_tile(sQ0, &map_q, jb * kTileRows, n, qfull);
+    mbar_expect_tx(qfull, 2 * TB);
+    tma_load_rows<W>(sK, &map_k, k0, n, qfull);
+    tma_load_rows<W>(sQ0, &map_q, jb * kTileRows, n, qfull);
     if (nsteps > 1) {
-      mbar_expect_tx(qfull + 8, kTileBytes);
-      tma_load_tile(sQ0 + kTileBytes, &map_q, (jb + 1) * kTileRows, n, qfull + 8);
+      mbar_expect_tx(qfull + 8, TB);
+      tma_load_rows<W>(sQ0 + TB, &map_q, (jb + 1) * kTileRows, n, qfull + 8);
     }
     mbar_wait(qfull, 0, ctl, &g_status, kErrWaitTma);
     tc_fence_after();
@@ -384,15 +415,15 @@ __global__ void __launch_bounds__(256, 4) backward_key_correction64_kernel(
     mbar_wait(sdone, h & 1, ctl, &g_status, kErrWaitMma);
     tc_fence_after();
     if (tid == 0 && odd == 0 && t >= 1 && t + 1 < nsteps) {      // the Q stage of step t-1 is free
-      mbar_expect_tx(qfull + 8 * (b ^ 1), kTileBytes);
-      tma_load_tile(sQ0 + kTileBytes * (b ^ 1), &map_q, (ib + 1) * kTileRows, n, qfull + 8 * (b ^ 1));
+      mbar_expect_tx(qfull + 8 * (b ^ 1), TB);
+      tma_load_rows<W>(sQ0 + TB * (b ^ 1), &map_q, (ib + 1) * kTileRows, n, qfull + 8 * (b ^ 1));
     }
     __syncwarp();
     const int i0 = ib * kTileRows + 64 * odd + 32 * wg;           // first query of this thread's 32
     const bool masked = dead || t == 0;
     const float4* St4 = reinterpret_cast<const float4*>(sStat + b * 128 + 64 * odd + 32 * wg);
     float vs[32];
-    uint32_t wt[16];
+    uint32_t wt[16], wr[W == kSplit ? 16 : 1];
     tmem_ld32(tcol, vs);
     tmem_ld_wait(vs);
     auto tile = [&](auto mask_tag) {
@@ -407,20 +438,25 @@ __global__ void __launch_bounds__(256, 4) backward_key_correction64_kernel(
           if (dead || ja > i0 + 2 * e2 + 1) p1 = 0.f;
         }
         wt[e2] = pack_bf16(p0 * st.y, p1 * st.w);
+        if (W == kSplit) wr[e2] = pack_bf16_rest(p0 * st.y, p1 * st.w, wt[e2]);
       }
     };
     if (masked) tile(std::true_type{}); else tile(std::false_type{});
-    tmem_st16(tcol, wt);            // W over the first 16 of the 32 consumed columns
+    tmem_st16(tcol, wt);            // W over the first 16 of the 32 consumed columns (its lo plane over the others)
+    if (W == kSplit) tmem_st16(tcol + 16, wr);
     if (fetch) sStat[(b ^ 1) * 128 + row] = make_float2(nx_max + log2f(nx_den), nx_gh);
     tmem_st_wait();
     tc_fence_before();
     __syncthreads();
     if (tid == 0) {
       tc_fence_after();
-      const Desc dQm = make_desc(sQ0 + kTileBytes * b, kTileBytes, 1024);
+      const Desc dQm = make_desc(sQ0 + TB * b, kTileBytes, 1024);
 #pragma unroll
-      for (int kq = 0; kq < 4; ++kq)        // 16 queries per instruction: 16 rows of 128 B = 128 units
-        mma_ts(tDK, tS + 32 * (kq >> 1) + 8 * (kq & 1), dQm, 128 * (4 * odd + kq), id_kd, (h > 0 || kq > 0));
+      for (int pl = 0; pl < Rows<W>::kPlanes; ++pl)
+#pragma unroll
+        for (int kq = 0; kq < 4; ++kq)        // 16 queries per instruction: 16 rows of 128 B = 128 units
+          mma_ts(tDK, tS + 32 * (kq >> 1) + 16 * pl + 8 * (kq & 1), dQm, 128 * (4 * odd + kq), id_kd,
+                 (h > 0 || pl > 0 || kq > 0));
       if (h + 1 < nhalf) {
         if (odd) {                          // the next half-step opens step t+1
           mbar_wait(qfull + 8 * (b ^ 1), ((t + 1) >> 1) & 1, ctl, &g_status, kErrWaitTma);
@@ -436,43 +472,52 @@ __global__ void __launch_bounds__(256, 4) backward_key_correction64_kernel(
   }
   mbar_wait(sdone, nhalf & 1, ctl, &g_status, kErrWaitMma);
   tc_fence_after();
-  {
+  // lane = key: each warpgroup finishes half of the columns of dk, 32 at a time
+  constexpr int kHead = Rows<W>::kHead, kHalf = kHead / 2;
+#pragma unroll
+  for (int c0 = kHalf * wg; c0 < kHalf * (wg + 1); c0 += 32) {
     float a[32];
-    const int64_t o = ((int64_t)n * g.tk + ja) * kHeadDim + 32 * wg;
-    tmem_ld32(tDK + lane_base + 32 * wg, a);
+    tmem_ld32(tDK + lane_base + c0, a);
     tmem_ld_wait(a);
+    if (W == kSplit) {                                          // W Q_hi + W Q_lo
+      float lo[32];
+      tmem_ld32(tDK + lane_base + 64 + c0, lo);
+      tmem_ld_wait(lo);
+#pragma unroll
+      for (int e = 0; e < 32; ++e) a[e] += lo[e];
+    }
     if (!dead) {
+      const float* src = dk_main + ((int64_t)n * g.tk + ja) * kHead + c0;
+      const int d = W == kSplit ? g.d : kHead;
+      TOut* dst = dk + ((int64_t)n * g.tk + ja) * d + c0;
       float m[32];
 #pragma unroll
       for (int e = 0; e < 32; e += 4) {
-        const float4 x = *reinterpret_cast<const float4*>(dk_main + o + e);
+        const float4 x = *reinterpret_cast<const float4*>(src + e);
         m[e] = x.x - g.scale * a[e];
         m[e + 1] = x.y - g.scale * a[e + 1];
         m[e + 2] = x.z - g.scale * a[e + 2];
         m[e + 3] = x.w - g.scale * a[e + 3];
       }
-#pragma unroll
-      for (int e = 0; e < 32; e += 8)
-        *reinterpret_cast<uint4*>(dk + o + e) =
-            make_uint4(pack_bf16(m[e], m[e + 1]), pack_bf16(m[e + 2], m[e + 3]),
-                       pack_bf16(m[e + 4], m[e + 5]), pack_bf16(m[e + 6], m[e + 7]));
+      store_row32<W>(dst, m, d - c0);
     }
   }
   drain_if_aborted(ctl);
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_free(tmem, 128);
+  if (warp == 0) tmem_free(tmem, kTmem);
 }
 
 // dq = bf16(dq_main - ghat * pk): the query half of the correction from the saved pk
 // (the reference's dq epilogue, kernels.py:814-826; pk already carries the scale).
+template <int HEAD = kHeadDim>
 __global__ void dq_from_pk_kernel(const float* __restrict__ dq_main, const float* __restrict__ pk,
                                   const float* __restrict__ ghat, __nv_bfloat16* __restrict__ dq, int64_t n4) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n4) return;
   const float4 a = reinterpret_cast<const float4*>(dq_main)[i];
   const float4 b = reinterpret_cast<const float4*>(pk)[i];
-  const float gh = ghat[i / (kHeadDim / 4)];
+  const float gh = ghat[i / (HEAD / 4)];
   reinterpret_cast<uint2*>(dq)[i] = make_uint2(pack_bf16(fmaf(-gh, b.x, a.x), fmaf(-gh, b.y, a.y)),
                                                pack_bf16(fmaf(-gh, b.z, a.z), fmaf(-gh, b.w, a.w)));
 }
@@ -515,16 +560,16 @@ inline int backward_tail_with_pk(const CUtensorMap& mq, const CUtensorMap& mk, c
                                  const float* dq_main, const float* pk, void* dq, void* dk, cudaStream_t st,
                                  char* err, size_t errlen, void (*mark)(const char*, cudaStream_t, int)) {
   const int nkb = (g.tk + kTileRows - 1) / kTileRows;
-  constexpr int smem = kCorrKey64Smem;
-  if (int rc = set_smem_attr((const void*)backward_key_correction64_kernel, smem, err, errlen)) return rc;
+  constexpr int smem = kCorrKey64Smem<kNarrow>;
+  if (int rc = set_smem_attr((const void*)backward_key_correction64_kernel<>, smem, err, errlen)) return rc;
   mark("tc_backward_key_correction", st, 0);
-  backward_key_correction64_kernel<<<(unsigned)(g.n * nkb), 256, smem, st>>>(mq, mk, g, rmax, rden, ghat,
+  backward_key_correction64_kernel<><<<(unsigned)(g.n * nkb), 256, smem, st>>>(mq, mk, g, rmax, rden, ghat,
                                                                            dk_main, (__nv_bfloat16*)dk);
   mark("tc_backward_key_correction", st, 1);
   if (int rc = launch_status("tc backward_key_correction", err, errlen)) return rc;
   const int64_t n4 = g.n * g.tq * kHeadDim / 4;
   mark("tc_dq_from_pk", st, 0);
-  dq_from_pk_kernel<<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(dq_main, pk, ghat, (__nv_bfloat16*)dq, n4);
+  dq_from_pk_kernel<><<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(dq_main, pk, ghat, (__nv_bfloat16*)dq, n4);
   mark("tc_dq_from_pk", st, 1);
   return launch_status("tc dq_from_pk", err, errlen);
 }

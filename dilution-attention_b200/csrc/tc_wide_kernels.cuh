@@ -1,0 +1,569 @@
+// Rows of 256 bytes on the tcgen05 kernels: bf16 heads of 128 (kWide128) and fp32 heads of up to 64 under
+// "tf32", every value held as a bf16 pair hi + lo (kSplit; Rows in tc_common.cuh).  Both have the same
+// tiles — two [rows][64 bf16] sub-tiles — and the same accumulators: 128 columns, which are the 128
+// features of a head, or X_hi and X_lo products of 64 features that the epilogue adds.
+//
+// The forward is row pass + column-sum scan + query-stationary main pass, the wide instantiations of the
+// kernels in tc_kernels.cuh and tc_rowpass_kernels.cuh; the reverse main pass has a kernel of its own, since the
+// narrow one's accumulators would need 656 of the 512 TMEM columns.
+//
+// Forward + backward at B4 H8 T4096 on one B200, before (tile kernels with tf32 products) and after:
+//   bf16 d = 128  14.8 ms -> 1.64 ms  (reverse pass 7.24 -> 0.70, main pass 3.82 -> 0.33)
+//   fp32 d = 64    7.1 ms -> 2.10 ms  (reverse pass 3.51 -> 0.93, main pass 1.61 -> 0.39)
+// and against exact products the fp32 outputs move from 2.8e-4 to about 1e-5 (2-norm).
+#pragma once
+
+#include "tc_kernels.cuh"
+#include "tc_rowpass_kernels.cuh"
+
+namespace dil {
+namespace tc {
+
+// fp32 (rows, d) -> bf16 (rows, 128): [hi 64 | lo 64], zeros behind d.  One thread per 4 features of a row; grid.y
+// picks the tensor.  Bound by memory: 16 bytes read and 16 written per 4 values of d = 64.
+struct SplitArgs {
+  const float* src[3];
+  __nv_bfloat16* dst[3];
+};
+__global__ void split_operands_kernel(SplitArgs a, int64_t rows, int d) {
+  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= rows * 16) return;
+  const int64_t r = idx >> 4;
+  const int c = (int)(idx & 15) * 4;
+  float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (c < d) x = *reinterpret_cast<const float4*>(a.src[blockIdx.y] + r * d + c);
+  const uint32_t h0 = pack_bf16(x.x, x.y), h1 = pack_bf16(x.z, x.w);
+  uint2* dst = reinterpret_cast<uint2*>(a.dst[blockIdx.y] + r * 128 + c);
+  dst[0] = make_uint2(h0, h1);
+  dst[16] = make_uint2(pack_bf16_rest(x.x, x.y, h0), pack_bf16_rest(x.z, x.w, h1));
+}
+
+__device__ __forceinline__ void load_vec(const float* p, float (&x)[2]) {
+  const float2 v = *reinterpret_cast<const float2*>(p);
+  x[0] = v.x; x[1] = v.y;
+}
+__device__ __forceinline__ void load_vec(const float* p, float (&x)[4]) {
+  const float4 v = *reinterpret_cast<const float4*>(p);
+  x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+}
+template <int E> __device__ __forceinline__ void load_vec(const __nv_bfloat16* p, float (&x)[E]) {
+#pragma unroll
+  for (int e = 0; e < E; e += 2) {
+    const uint32_t v = *reinterpret_cast<const uint32_t*>(p + e);
+    x[e] = __uint_as_float(v << 16);
+    x[e + 1] = __uint_as_float(v & 0xffff0000u);
+  }
+}
+
+// backward_prep_kernel for wide rows: dbar' and do' = sinv * dout, as bf16 (kWide128) or as hi | lo (kSplit).
+template <typename TD, int W>
+__global__ void wide_backward_prep_kernel(const TD* __restrict__ dout, const float* __restrict__ out,
+                                          const float* __restrict__ ssum, float eps, int64_t rows, int d,
+                                          float* __restrict__ dbarp, __nv_bfloat16* __restrict__ dop,
+                                          float* __restrict__ ghat, float* __restrict__ dq_main) {
+  const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const int lane = threadIdx.x & 31;
+  constexpr int E = Rows<W>::kHead / 32;                 // features per lane: 4 or 2
+  const int c = lane * E;
+  float a[E], b[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) a[e] = b[e] = 0.f;
+  if (c < d) {
+    load_vec(dout + row * d + c, a);
+    load_vec(out + row * d + c, b);
+  }
+  const float sinv = 1.f / (ssum[row] + eps);
+  float dot = 0.f;
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    dot = fmaf(a[e], b[e], dot);
+    a[e] *= sinv;
+  }
+  dot = warp_sum(dot);
+  if (W == kWide128) {
+    reinterpret_cast<uint2*>(dop + row * 128)[lane] = make_uint2(pack_bf16(a[0], a[1]), pack_bf16(a[E - 2], a[E - 1]));
+    reinterpret_cast<float4*>(dq_main + row * 128)[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+  } else {
+    const uint32_t hi = pack_bf16(a[0], a[1]);
+    reinterpret_cast<uint32_t*>(dop + row * 128)[lane] = hi;
+    reinterpret_cast<uint32_t*>(dop + row * 128 + 64)[lane] = pack_bf16_rest(a[0], a[1], hi);
+    reinterpret_cast<float2*>(dq_main + row * 64)[lane] = make_float2(0.f, 0.f);
+  }
+  if (lane == 0) {
+    dbarp[row] = dot * sinv;
+    ghat[row] = 0.f;
+  }
+}
+
+// dq = dq_main - ghat * pk in fp32, rows of d out of padded rows of 64.
+__global__ void split_dq_from_pk_kernel(const float* __restrict__ dq_main, const float* __restrict__ pk,
+                                        const float* __restrict__ ghat, float* __restrict__ dq, int64_t rows, int d) {
+  const int per = d / 4;
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= rows * per) return;
+  const int64_t r = i / per;
+  const float4 a = reinterpret_cast<const float4*>(dq_main + r * 64)[i - r * per];
+  const float4 b = reinterpret_cast<const float4*>(pk)[i];
+  const float gh = ghat[r];
+  reinterpret_cast<float4*>(dq)[i] =
+      make_float4(fmaf(-gh, b.x, a.x), fmaf(-gh, b.y, a.y), fmaf(-gh, b.z, a.z), fmaf(-gh, b.w, a.w));
+}
+
+// Main reverse pass over wide rows: the arithmetic of backward_main_kernel (two compute warpgroups, lane =
+// key, two threads per key and half-step of 64 queries, reverse_sweeps), 384 threads, one CTA per SM.
+//   TMEM, all 512 columns: S^T 64 | dOV^T 64 | dV 128 | dK 128 | dQ^T 64 | ghat^T 64.
+// What differs from the narrow kernel, and why:
+//  * one stage of scores instead of two (dV and dK take 256 columns): the scores of half-step h + 1 are issued right
+//    behind the dV and dK products of h, which read the share and pdp values stored over the scores of h;
+//  * dQ comes out transposed, dQ^T [128 features x 64 queries] = K^T pdp, M = the 128 columns of a K row: pdp is
+//    then the B operand [keys][64 queries], 16 KB per half-step instead of 32 KB per 128 queries, and a
+//    thread of the read-out (lane = feature) writes one fp32 column of the [query][32 features] staging
+//    tile of its warp, 128 consecutive bytes per warp and store;
+//  * V stays in shared memory (as a TMEM operand it would take 64 columns);
+//  * ghat^T = 1^T pdp is a product of its own against a 4 KB tile of ones.
+// kSplit multiplies hi and lo planes of share and pdp (two A operands side by side in TMEM, two pdp tiles),
+// and dQ^T rows 64..127 (K_lo) are reduced into the same columns of dq_main as rows 0..63.
+template <int W> constexpr int kBwdWideSmem =
+    4 * (int)Rows<W>::kBytes + (Rows<W>::kPlanes + 2) * (int)kTileBytes + 4096 + 1024 + 2048 + 256 + 256 + 1024;
+
+template <int W, typename TOut>
+__global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
+    const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+    const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
+    const __grid_constant__ CUtensorMap map_dq, Geom g, const float* __restrict__ rmax,
+    const float* __restrict__ rden, const float* __restrict__ dbarp, const float* __restrict__ carry,
+    const float* __restrict__ total, float* __restrict__ dk_main, TOut* __restrict__ dv, float* __restrict__ ghat) {
+  constexpr uint32_t TB = Rows<W>::kBytes;                 // [128] rows of k or v: 32 KB
+  constexpr uint32_t HB = TB / 2, HSub = kTileBytes / 2;   // [64] rows of q or do', and one of their sub-tiles
+  constexpr int P = Rows<W>::kPlanes;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = align1024(smem_raw);
+  const uint32_t sK = smem_u32(smem), sV = sK + TB;
+  const uint32_t sQ0 = sK + 2 * TB, sD0 = sQ0 + 2 * HB;        // [2] stages each
+  const uint32_t sPd = sD0 + 2 * HB;                           // [P][128 keys][64 queries] bf16
+  const uint32_t sDq = sPd + P * kTileBytes;                   // [4 warps][64 queries][32 features] fp32
+  const uint32_t sOnes = sDq + 2 * kTileBytes;
+  uint8_t* tail = smem + 4 * TB + (P + 2) * kTileBytes;        // the ones tile
+  float* sLse = reinterpret_cast<float*>(tail + 4096);         // [2][64]
+  float* sDbar = sLse + 128;                                   // [2][64]
+  float* sG = sDbar + 128;                                     // [2][2][128] sums of dk_share
+  float* sGh = sG + 512;                                       // [64]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sGh + 64);
+  Ctl* ctl = reinterpret_cast<Ctl*>(bars + 12);
+  const uint32_t kfull = smem_u32(bars), qfull = smem_u32(bars + 1);           // qfull[2]
+  const uint32_t sdone = smem_u32(bars + 3), tiles = smem_u32(bars + 4), dqdone = smem_u32(bars + 5);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wg = tid >> 7, row = tid & 127;
+  const int nqb = (g.tq + kTileRows - 1) / kTileRows;
+  const int ncb = (g.tq + kCarryRows - 1) / kCarryRows;
+  const int n = (int)(blockIdx.x % g.n);
+  const int jb = (int)(blockIdx.x / g.n);
+  const int k0 = jb * kTileRows;
+  const int nhalf = 2 * (nqb - jb);                // 64-query blocks 2 nqb - 1 .. 2 jb, visited in this order
+  const int64_t row_base = (int64_t)n * g.tq;
+  const int ja = k0 + row;
+  const bool dead = ja >= g.tk;
+
+  auto load_stats = [&](int hb, float* lse, float* dbar) {      // of query 64 hb + row, row < 64
+    const int i = hb * 64 + row;
+    *lse = load_lse(rmax, rden, row_base, i, g.tq);
+    *dbar = i < g.tq ? dbarp[row_base + i] : 0.f;
+  };
+
+  if (tid == 0) {
+    ctl->abort = 0;
+    for (int i = 0; i < 4; ++i) mbar_init(kfull + 8 * i, 1);      // kfull, qfull[2], sdone
+    mbar_init(tiles, 8);
+    mbar_init(dqdone, 1);
+    fence_barrier_init();
+  }
+  __syncwarp();
+  if (warp == 0) tmem_alloc(smem_u32(&ctl->tmem), 512);
+  if (wg == 0) {
+    if (row < 64) {
+      float l, db;
+      load_stats(2 * nqb - 1, &l, &db);
+      sLse[row] = l;
+      sDbar[row] = db;
+    }
+  } else if (wg == 1) {
+    const uint4 one = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
+    reinterpret_cast<uint4*>(tail)[row] = one;
+    reinterpret_cast<uint4*>(tail)[row + 128] = one;
+  }
+  fence_async_smem();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = ctl->tmem;
+  const uint32_t tS = tmem, tDOV = tmem + 64, tDV = tmem + 128, tDK = tmem + 256, tDQ = tmem + 384, tG = tmem + 448;
+  const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+  if (wg < 2) {
+    // dV and dK start from zero, so that every MMA into them accumulates
+    uint32_t z[16];
+#pragma unroll
+    for (int c = 0; c < 16; ++c) z[c] = 0u;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) tmem_st16((wg == 0 ? tDV : tDK) + lane_base + 16 * c, z);
+    tmem_st_wait();
+  }
+  auto load_stage = [&](int h) {                     // thread 256: q and do' of half-step h
+    const int st = h & 1, r0 = (2 * nqb - 1 - h) * 64;
+    mbar_expect_tx(qfull + 8 * st, 2 * HB);
+    tma_load_rows<W>(sQ0 + HB * st, &map_q, r0, n, qfull + 8 * st, HSub);
+    tma_load_rows<W>(sD0 + HB * st, &map_do, r0, n, qfull + 8 * st, HSub);
+  };
+  if (tid == 256) {
+    mbar_expect_tx(kfull, 2 * TB);
+    tma_load_rows<W>(sK, &map_k, k0, n, kfull);
+    tma_load_rows<W>(sV, &map_v, k0, n, kfull);
+    load_stage(0);
+    load_stage(1);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+
+  if (wg == 2) {
+    // ------------------------------------------------------------ issue, and the dQ read-out
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");
+    constexpr uint32_t id_s = instr_desc(128, 64, 0, 0);     // scores: both operands K-major
+    constexpr uint32_t id_kd = instr_desc(128, 128, 0, 1);   // dV, dK: A from TMEM (M = keys), B MN-major
+    constexpr uint32_t id_qd = instr_desc(128, 64, 1, 1);    // dQ^T, ghat^T: A and B MN-major
+    const Desc dKk = make_desc(sK, 16, 1024), dVk = make_desc(sV, 16, 1024);
+    const Desc dKm = make_desc(sK, kTileBytes, 1024), dOnes = make_desc(sOnes, 2048, 1024);
+    const Desc dPm = make_desc(sPd, kTileBytes, 1024);
+    auto issue_scores = [&](int h) {
+      const int st = h & 1;
+      mma_scores_wide<W>(tS, dKk, kTileBytes, make_desc(sQ0 + HB * st, 16, 1024), HSub, id_s);
+      mma_scores_wide<W>(tDOV, dVk, kTileBytes, make_desc(sD0 + HB * st, 16, 1024), HSub, id_s);
+    };
+    if (tid == 256) {
+      mbar_wait(kfull, 0, ctl, &g_status, kErrWaitTma);
+      mbar_wait(qfull, 0, ctl, &g_status, kErrWaitTma);
+      tc_fence_after();
+      issue_scores(0);
+      mma_commit(sdone);
+    }
+    __syncwarp();
+    for (int h = 0; h < nhalf; ++h) {
+      const int st = h & 1;
+      if (tid == 256) {
+        mbar_wait(tiles, h & 1, ctl, &g_status, kErrWaitTile);
+        tc_fence_after();
+        const Desc dQm = make_desc(sQ0 + HB * st, HSub, 1024), dDm = make_desc(sD0 + HB * st, HSub, 1024);
+#pragma unroll
+        for (int pl = 0; pl < P; ++pl)
+#pragma unroll
+          for (int kq = 0; kq < 4; ++kq) {                    // contraction over the 64 queries, 16 each
+            const uint32_t col = 32 * (kq >> 1) + 16 * pl + 8 * (kq & 1);
+            mma_ts(tDV, tS + col, dDm, 128 * kq, id_kd, 1);
+            mma_ts(tDK, tDOV + col, dQm, 128 * kq, id_kd, 1);
+          }
+        if (h + 1 < nhalf) {
+          mbar_wait(qfull + 8 * (st ^ 1), ((h + 1) >> 1) & 1, ctl, &g_status, kErrWaitTma);
+          tc_fence_after();
+          issue_scores(h + 1);
+        }
+        mma_commit(sdone);
+#pragma unroll
+        for (int pl = 0; pl < P; ++pl)
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk) {                    // contraction over the 128 keys
+            mma_ss(tDQ, dKm, 128 * kk, dPm, 1024 * pl + 128 * kk, id_qd, (pl > 0 || kk > 0));
+            mma_ss(tG, dOnes, 0, dPm, 1024 * pl + 128 * kk, id_qd, (pl > 0 || kk > 0));
+          }
+        mma_commit(dqdone);
+        if (h + 2 < nhalf) {
+          // the products that read this stage come before the scores of h + 1, whose commit covers them
+          mbar_wait(sdone, (h + 1) & 1, ctl, &g_status, kErrWaitMma);
+          load_stage(h + 2);
+        }
+      }
+      __syncwarp();
+      // dQ^T and ghat^T of the half-step's 64 queries: lane = feature.  Each warp stages its 32 features and
+      // adds them to dq_main with one tensor reduction.
+      if (lane == 0) mbar_wait(dqdone, h & 1, ctl, &g_status, kErrWaitMma);
+      __syncwarp();
+      tc_fence_after();
+      const int q0 = (2 * nqb - 1 - h) * 64, w4 = warp & 3;
+      if (lane == 0) tma_wait_read_all();               // the previous reduction has read this warp's staging
+      __syncwarp();
+      const uint32_t stage = sDq + w4 * 8192 + lane * 4;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        float x[32];
+        tmem_ld32(tDQ + lane_base + 32 * c, x);
+        tmem_ld_wait(x);
+#pragma unroll
+        for (int e = 0; e < 32; ++e)
+          asm volatile("st.shared.f32 [%0], %1;" ::"r"(stage + (32 * c + e) * 128), "f"(x[e] * g.scale) : "memory");
+      }
+      if (w4 == 0) {                                    // every lane of ghat^T holds the same 64 sums
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          float x[32];
+          tmem_ld32(tG + lane_base + 32 * c, x);
+          tmem_ld_wait(x);
+          if (lane == 0) {
+#pragma unroll
+            for (int e = 0; e < 32; e += 4)
+              *reinterpret_cast<float4*>(sGh + 32 * c + e) = make_float4(x[e], x[e + 1], x[e + 2], x[e + 3]);
+          }
+        }
+        __syncwarp();
+        for (int q = lane; q < 64; q += 32)
+          if (q0 + q < g.tq) atomicAdd(ghat + row_base + q0 + q, sGh[q]);
+      }
+      fence_async_smem();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0 && q0 < g.tq)                       // a reduction never starts behind the last row
+        tma_reduce_add_tile(&map_dq, sDq + w4 * 8192, W == kSplit ? 32 * (w4 & 1) : 32 * w4, q0, n);
+      asm volatile("bar.sync 2, 128;" ::: "memory");    // every warp has read the tile: the next one may be issued
+      tc_fence_after();
+    }
+    if (lane == 0) tma_wait_read_all();
+    __syncwarp();
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");
+    // ------------------------------------------------------------ the compute warps
+    const int cw = 32 * (1 - wg);                    // this warpgroup's queries of a half-step
+    auto load_edge = [&](int h) {                    // demand in front of this thread's 32 queries of half-step h
+      if (dead) return 0.f;
+      const int rb = 2 * (2 * nqb - 1 - h) + (wg == 0 ? 1 : 0);
+      return rb < ncb ? carry[((int64_t)n * ncb + rb) * g.tk + ja] : total[(int64_t)n * g.tk + ja];
+    };
+    float sigma = 0.f;                               // suffix of dk_share behind the half-step
+    float incl = load_edge(0);
+    float incl_next = load_edge(1);                  // nhalf >= 2
+    const uint32_t tcol = lane_base + cw;
+    for (int h = 0; h < nhalf; ++h) {
+      const int b = h & 1, hb = 2 * nqb - 1 - h;
+      float incl_next2 = 0.f, nx_lse = INFINITY, nx_dbar = 0.f;
+      if (h + 2 < nhalf) incl_next2 = load_edge(h + 2);
+      const bool fetch = wg == 0 && row < 64 && h + 1 < nhalf;
+      if (fetch) load_stats(hb - 1, &nx_lse, &nx_dbar);
+      mbar_wait(sdone, h & 1, ctl, &g_status, kErrWaitMma);
+      tc_fence_after();
+      float vs[32], vd[32];
+      tmem_ld32(tS + tcol, vs);
+      tmem_ld32(tDOV + tcol, vd);
+      tmem_ld_wait(vs);
+      tmem_ld_wait(vd);
+      const int iq0 = hb * 64 + cw;                   // position of this thread's first query
+      const bool masked = dead || hb * 64 < k0 + kTileRows - 1;
+      const float4* Lse4 = reinterpret_cast<const float4*>(sLse + b * 64 + cw);
+      const float4* Dbar4 = reinterpret_cast<const float4*>(sDbar + b * 64 + cw);
+      uint32_t shp[16 * P];
+      // warpgroup 0 (queries 32..63) knows the suffix of dk_share behind its queries; warpgroup 1 starts
+      // from zero and adds p * (the suffix warpgroup 0 ends with) afterwards: dp is linear in it
+      float R = wg == 0 ? sigma : 0.f;
+      auto chunk = [&](auto mask_tag) {
+        reverse_sweeps<kBidSoftmax, kShareInclusive, decltype(mask_tag)::value, W == kSplit>(
+            vs, vd, shp, R, incl + g.eps, Lse4, Dbar4, g, dead, ja - iq0);
+      };
+      if (masked) chunk(std::true_type{}); else chunk(std::false_type{});
+      sG[(b * 2 + wg) * 128 + row] = R;
+      tmem_st16(tS + tcol, shp);                       // the shares, over score columns this thread has consumed
+      if (W == kSplit) tmem_st16(tS + tcol + 16, shp + 16 * (P - 1));
+      asm volatile("bar.sync 1, 256;" ::: "memory");   // the compute warps
+      const float rother = sG[(b * 2 + (1 - wg)) * 128 + row];
+      const float fix = wg == 1 ? rother : 0.f;
+      sigma = R + rother;                              // the suffix behind the next half-step
+      // the dQ products of the previous half-step read the pdp buffer that is written next
+      if (h >= 1) mbar_wait(dqdone, (h - 1) & 1, ctl, &g_status, kErrWaitMma);
+      {
+        uint32_t pdt[16 * P];
+#pragma unroll
+        for (int e8 = 0; e8 < 4; ++e8) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int e = e8 * 8 + 2 * u;
+            const float2 f2 = fma2(make_float2(vs[e], vs[e + 1]), make_float2(fix, fix), make_float2(vd[e], vd[e + 1]));
+            pdt[e8 * 4 + u] = pack_bf16(f2.x, f2.y);
+            if (W == kSplit) pdt[16 * (P - 1) + e8 * 4 + u] = pack_bf16_rest(f2.x, f2.y, pdt[e8 * 4 + u]);
+          }
+#pragma unroll
+          for (int pl = 0; pl < P; ++pl) {              // [key][query]: the MN-major B operand of dQ^T and ghat^T
+            const uint32_t* w = pdt + 16 * pl + 4 * e8;
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sPd + kTileBytes * pl + share_chunk_offset(row, cw + e8 * 8)),
+                         "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
+                         : "memory");
+          }
+        }
+        tmem_st16(tDOV + tcol, pdt);                    // the A operand of dK (M = keys)
+        if (W == kSplit) tmem_st16(tDOV + tcol + 16, pdt + 16 * (P - 1));
+      }
+      if (fetch) {
+        sLse[(b ^ 1) * 64 + row] = nx_lse;
+        sDbar[(b ^ 1) * 64 + row] = nx_dbar;
+      }
+      incl = incl_next;
+      incl_next = incl_next2;
+      tmem_st_wait();
+      fence_async_smem();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(tiles);
+    }
+  }
+  mbar_wait(sdone, nhalf & 1, ctl, &g_status, kErrWaitMma);
+  tc_fence_after();
+  if (warp < 8) {
+    // lane = key: each warpgroup stores half of the columns of dk_main and dv, 32 at a time
+    constexpr int kHead = Rows<W>::kHead, kHalf = kHead / 2;
+    const int d = W == kSplit ? g.d : kHead;
+    auto fetch32 = [&](uint32_t t, float* a) {
+      tmem_ld32(t + lane_base, a);
+      tmem_ld_wait(a);
+      if (W == kSplit) {                              // A X_hi + A X_lo
+        float lo[32];
+        tmem_ld32(t + lane_base + 64, lo);
+        tmem_ld_wait(lo);
+#pragma unroll
+        for (int e = 0; e < 32; ++e) a[e] += lo[e];
+      }
+    };
+#pragma unroll
+    for (int c0 = 0; c0 < kHalf; c0 += 32) {
+      const int col = kHalf * wg + c0;
+      float a[32];
+      fetch32(tDK + col, a);
+      if (!dead) {
+#pragma unroll
+        for (int e = 0; e < 32; e += 4)
+          *reinterpret_cast<float4*>(dk_main + ((int64_t)n * g.tk + ja) * kHead + col + e) =
+              make_float4(a[e] * g.scale, a[e + 1] * g.scale, a[e + 2] * g.scale, a[e + 3] * g.scale);
+      }
+      fetch32(tDV + col, a);
+      if (!dead) store_row32<W>(dv + ((int64_t)n * g.tk + ja) * d + col, a, d - col);
+    }
+  }
+  drain_if_aborted(ctl);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_free(tmem, 512);
+}
+
+// ---------------------------------------------------------------- host launchers
+inline int split_operands(const SplitArgs& a, int count, int64_t rows, int d, cudaStream_t st, char* err, size_t errlen) {
+  split_operands_kernel<<<dim3((unsigned)((rows * 16 + 255) / 256), (unsigned)count), 256, 0, st>>>(a, rows, d);
+  return launch_status("split_operands", err, errlen);
+}
+
+struct WideMaps {
+  CUtensorMap q, k, v;
+};
+inline int wide_maps(WideMaps* m, const void* q, const void* k, const void* v, const Geom& g, char* err, size_t errlen) {
+  if (int rc = make_map(&m->q, q, g.n, g.tq, err, errlen, 128)) return rc;
+  if (int rc = make_map(&m->k, k, g.n, g.tk, err, errlen, 128)) return rc;
+  return make_map(&m->v, v, g.n, g.tk, err, errlen, 128);
+}
+
+// Passes 1-3 on wide rows; pk (n, t, d) fp32 is written when it is not null.
+template <int W>
+inline int wide_forward(const void* q, const void* k, const void* v, const Geom& g, float* rmax, float* rden,
+                        float* carry, float* total, float* out, float* ssum, float* pk, cudaStream_t st, char* err,
+                        size_t errlen, void (*mark)(const char*, cudaStream_t, int)) {
+  WideMaps m;
+  if (int rc = wide_maps(&m, q, k, v, g, err, errlen)) return rc;
+  const unsigned grid = (unsigned)(g.n * ((g.tq + kTileRows - 1) / kTileRows));
+  if (pk != nullptr) {
+    auto kern = rowpass_product_kernel<1, float, W>;
+    constexpr int smem = RowpassSmem<1, W>::kBytes;
+    static_assert(smem <= 232448 && 2 * smem > 233472, "one CTA (512 TMEM columns) per SM");
+    if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
+    mark("tc_wide_rowstats_pk", st, 0);
+    kern<<<grid, 256, smem, st>>>(m.q, m.k, m.k, g, rmax, rden, pk);
+    mark("tc_wide_rowstats_pk", st, 1);
+  } else {
+    constexpr int smem = kRowstatsSmem<W>;
+    if (int rc = set_smem_attr((const void*)rowstats_kernel<W>, smem, err, errlen)) return rc;
+    mark("tc_wide_rowstats", st, 0);
+    rowstats_kernel<W><<<grid, 256, smem, st>>>(m.q, m.k, g, rmax, rden);
+    mark("tc_wide_rowstats", st, 1);
+  }
+  if (int rc = launch_status("tc wide rowstats", err, errlen)) return rc;
+  {
+    constexpr int smem = kColsumSmem<W>;
+    auto kern = colsum_scan_kernel<32, kBidSoftmax, W>;
+    if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
+    mark("tc_wide_colsum_scan", st, 0);
+    kern<<<grid, 256, smem, st>>>(m.q, m.k, g, rmax, rden, nullptr, carry, total);
+    mark("tc_wide_colsum_scan", st, 1);
+  }
+  if (int rc = launch_status("tc wide colsum_scan", err, errlen)) return rc;
+  {
+    constexpr int smem = kMainSmem<W>;
+    static_assert(smem <= 232448 && 2 * smem > 233472, "one CTA (512 TMEM columns) per SM");
+    auto kern = forward_main_kernel<kBidSoftmax, kShareInclusive, W>;
+    if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
+    mark("tc_wide_forward_main", st, 0);
+    kern<<<grid, 256, smem, st>>>(m.q, m.k, m.v, g, rmax, rden, carry, nullptr, out, ssum);
+    mark("tc_wide_forward_main", st, 1);
+  }
+  return launch_status("tc wide forward_main", err, errlen);
+}
+
+// dq_main and dk_main: (n, t, 128), kSplit (n, t, 64); dop: (n, t, 128) bf16; ghat, dbarp: (n, t).
+template <int W>
+inline int wide_backward(const void* q, const void* k, const void* v, const Geom& g, const void* dout, int dout_dtype,
+                         const float* out, const float* rmax, const float* rden, const float* carry,
+                         const float* total, const float* ssum, const float* pk, float* dq_main, float* dk_main,
+                         void* dop, float* ghat, float* dbarp, void* dq, void* dk, void* dv, cudaStream_t st,
+                         char* err, size_t errlen, void (*mark)(const char*, cudaStream_t, int)) {
+  using TOut = std::conditional_t<W == kSplit, float, __nv_bfloat16>;
+  constexpr int kHead = Rows<W>::kHead;
+  WideMaps m;
+  if (int rc = wide_maps(&m, q, k, v, g, err, errlen)) return rc;
+  CUtensorMap mq64, md64, mdq;
+  if (int rc = make_map(&mq64, q, g.n, g.tq, err, errlen, 128, 64)) return rc;
+  if (int rc = make_map(&md64, dop, g.n, g.tq, err, errlen, 128, 64)) return rc;
+  if (int rc = make_map_f32(&mdq, dq_main, g.n, g.tq, err, errlen, kHead, 64, false)) return rc;
+  const int64_t rows = g.n * g.tq;
+  const unsigned grid = (unsigned)(g.n * ((g.tk + kTileRows - 1) / kTileRows));
+  mark("tc_wide_backward_prep", st, 0);
+  if (dout_dtype == 0)
+    wide_backward_prep_kernel<float, W><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(
+        (const float*)dout, out, ssum, g.eps, rows, g.d, dbarp, (__nv_bfloat16*)dop, ghat, dq_main);
+  else
+    wide_backward_prep_kernel<__nv_bfloat16, W><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(
+        (const __nv_bfloat16*)dout, out, ssum, g.eps, rows, g.d, dbarp, (__nv_bfloat16*)dop, ghat, dq_main);
+  mark("tc_wide_backward_prep", st, 1);
+  if (int rc = launch_status("tc wide backward_prep", err, errlen)) return rc;
+  {
+    constexpr int smem = kBwdWideSmem<W>;
+    static_assert(smem <= 232448 && 2 * smem > 233472, "the wide reverse pass runs one CTA per SM");
+    auto kern = wide_backward_main_kernel<W, TOut>;
+    if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
+    mark("tc_wide_backward_main", st, 0);
+    kern<<<grid, kBwdThreads, smem, st>>>(mq64, m.k, m.v, md64, mdq, g, rmax, rden, dbarp, carry, total, dk_main,
+                                          (TOut*)dv, ghat);
+    mark("tc_wide_backward_main", st, 1);
+  }
+  if (int rc = launch_status("tc wide backward_main", err, errlen)) return rc;
+  {
+    constexpr int smem = kCorrKey64Smem<W>;
+    auto kern = backward_key_correction64_kernel<W, TOut>;
+    if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
+    mark("tc_wide_backward_key_correction", st, 0);
+    kern<<<grid, 256, smem, st>>>(m.q, m.k, g, rmax, rden, ghat, dk_main, (TOut*)dk);
+    mark("tc_wide_backward_key_correction", st, 1);
+  }
+  if (int rc = launch_status("tc wide backward_key_correction", err, errlen)) return rc;
+  mark("tc_wide_dq_from_pk", st, 0);
+  if (W == kSplit) {
+    const int64_t n4 = rows * (g.d / 4);
+    split_dq_from_pk_kernel<<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(dq_main, pk, ghat, (float*)dq, rows, g.d);
+  } else {
+    const int64_t n4 = rows * (kHead / 4);
+    dq_from_pk_kernel<kHead><<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(dq_main, pk, ghat, (__nv_bfloat16*)dq, n4);
+  }
+  mark("tc_wide_dq_from_pk", st, 1);
+  return launch_status("tc wide dq_from_pk", err, errlen);
+}
+
+}  // namespace tc
+}  // namespace dil

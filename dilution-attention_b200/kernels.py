@@ -125,6 +125,18 @@ def _forward_rows(lib, qf, kf, vf, code, prec, scale, out, ssum, rmax, rden, car
                "dilution_forward_main")
 
 
+def _wide_operands(lib, qf, kf, vf, code):
+    """What dilution_wide_forward takes: bf16 tensors as they are, fp32 tensors as hi | lo planes."""
+    if code == _lib.BF16:
+        return qf, kf, vf
+    n, t, d = qf.shape
+    planes = tuple(torch.empty(n, t, 128, device=qf.device, dtype=torch.bfloat16) for _ in range(3))
+    _lib.check(lib.dilution_split_operands(qf.data_ptr(), kf.data_ptr(), vf.data_ptr(), n * t, d,
+                                           *(x.data_ptr() for x in planes), _stream(qf.device)),
+               "dilution_split_operands")
+    return planes
+
+
 def dilution_attention_forward(
     q: torch.Tensor,
     k: torch.Tensor,
@@ -155,12 +167,24 @@ def dilution_attention_forward(
     quadratic carry scratch stays under scratch_budget_gib; rows are independent,
     so this changes nothing numerically.
     """
+    result, aux, _ = _attention_forward(q, k, v, dot_precision, return_aux, _save_pk, scratch_budget_gib, _training)
+    if return_aux:
+        aux.update(block_m=block_m, block_n=block_n, dot_precision=dot_precision, num_warps=num_warps)
+        return result, aux
+    return result
+
+
+def _attention_forward(q, k, v, dot_precision, return_aux, _save_pk, scratch_budget_gib=16.0, _training=None):
+    """(out, aux, operands): aux without the caller's tuning arguments, operands as the kernels took q, k and v."""
     lib = _lib.load()
     (qf, kf, vf), code, prec, n = _prepare(q, k, v, dot_precision)
     batch, heads, seq, head_dim = q.shape
     dev = q.device
     scale = 1.0 / math.sqrt(head_dim)
     training = _save_pk if _training is None else _training
+    wide = _lib.wide_path(code, prec, head_dim)
+    if wide:
+        qf, kf, vf = _wide_operands(lib, qf, kf, vf, code)
     carry_rows = _lib.carry_rows(code, prec, head_dim, training)
     ncb = (seq + carry_rows - 1) // carry_rows
 
@@ -179,18 +203,20 @@ def dilution_attention_forward(
     carry = torch.empty(rows, ncb, seq, **f32)
     for a in range(0, n, rows):
         b = min(a + rows, n)
+        if wide:
+            _lib.check(lib.dilution_wide_forward(
+                qf[a:b].data_ptr(), kf[a:b].data_ptr(), vf[a:b].data_ptr(), code, b - a, seq, head_dim, scale, EPS,
+                rmax[a:b].data_ptr(), rden[a:b].data_ptr(), carry.data_ptr(), total[a:b].data_ptr(),
+                out[a:b].data_ptr(), ssum[a:b].data_ptr(), None if pk is None else pk[a:b].data_ptr(), _stream(dev)),
+                "dilution_wide_forward")
+            continue
         _forward_rows(lib, qf[a:b], kf[a:b], vf[a:b], code, prec, scale, out[a:b], ssum[a:b],
                       rmax[a:b], rden[a:b], carry[: b - a], total[a:b],
                       None if pk is None else pk[a:b], carry_rows)
 
-    result = out.reshape(batch, heads, seq, head_dim)
-    if return_aux:
-        aux = dict(pk=pk, rmax=rmax, rden=rden, carry=carry, ssum=ssum, bwd_block_m=carry_rows,
-                   block_m=block_m, block_n=block_n, dot_precision=dot_precision,
-                   num_warps=num_warps,
-                   committed_total=total.reshape(batch, heads, seq))
-        return result, aux
-    return result
+    aux = dict(pk=pk, rmax=rmax, rden=rden, carry=carry, ssum=ssum, bwd_block_m=carry_rows,
+               committed_total=total.reshape(batch, heads, seq))
+    return out.reshape(batch, heads, seq, head_dim), aux, (qf, kf, vf)
 
 
 class _DilutionAttentionFn(torch.autograd.Function):
@@ -202,47 +228,56 @@ class _DilutionAttentionFn(torch.autograd.Function):
         lowp, _ = _resolve_precision(dot_precision)
         on_tc = _lib.tensor_core_path(_lib.BF16 if (lowp or q.dtype == torch.bfloat16) else _lib.F32,
                                       _lib.PREC[dot_precision], q.shape[-1])
-        out, aux = dilution_attention_forward(
-            q, k, v, dot_precision=dot_precision, return_aux=True,
-            _save_pk=any(ctx.needs_input_grad[:3]) and (TC_SAVE_PK or not on_tc),
+        out, aux, operands = _attention_forward(
+            q, k, v, dot_precision, True, any(ctx.needs_input_grad[:3]) and (TC_SAVE_PK or not on_tc),
             _training=any(ctx.needs_input_grad[:3]))
         ctx.carry_rows = aux["bwd_block_m"]
-        ctx.save_for_backward(q, k, v, out, aux["rmax"], aux["rden"], aux["carry"], aux["ssum"], aux["pk"],
+        # what the backward's kernels read: the operands as the forward took them (casts, copies of strided views
+        # and hi | lo planes are made once)
+        ctx.save_for_backward(*operands, out, aux["rmax"], aux["rden"], aux["carry"], aux["ssum"], aux["pk"],
                               aux["committed_total"])
         ctx.dot_precision = dot_precision
+        ctx.dtypes = (q.dtype, k.dtype, v.dtype)
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        q, k, v, out, rmax, rden, carry, ssum, pk, total = ctx.saved_tensors
+        qf, kf, vf, out, rmax, rden, carry, ssum, pk, total = ctx.saved_tensors
         lib = _lib.load()
-        batch, heads, seq, head_dim = q.shape
-        (qf, kf, vf), code, prec, n = _prepare(q, k, v, ctx.dot_precision)
-        dev = q.device
-        # the tensor-core path reads a bf16 upstream gradient as it is (its first kernel makes a
+        batch, heads, seq, head_dim = out.shape
+        lowp, _ = _resolve_precision(ctx.dot_precision)
+        code = _lib.BF16 if (lowp or ctx.dtypes[0] == torch.bfloat16) else _lib.F32
+        prec = _lib.PREC[ctx.dot_precision]
+        n, dev = batch * heads, out.device
+        # the tensor-core paths read a bf16 upstream gradient as it is (their first kernel makes a
         # scaled bf16 copy anyway); everything else is widened to fp32 as the reference does
-        on_tc = _lib.tensor_core_path(code, prec, head_dim)
+        wide = _lib.wide_path(code, prec, head_dim)
+        on_tc = wide or _lib.tensor_core_path(code, prec, head_dim)
         dof = dout.reshape(n, seq, head_dim)
         if not (on_tc and dof.dtype == torch.bfloat16):
             dof = dof.float()
         dof = dof.contiguous()
         do_code = _lib.BF16 if dof.dtype == torch.bfloat16 else _lib.F32
-        of = out.reshape(n, seq, head_dim)
-        gdt = qf.dtype
-        dq = torch.empty(n, seq, head_dim, device=dev, dtype=gdt)
-        dk = torch.empty_like(dq)
-        dv = torch.empty_like(dq)
-        nbytes = lib.dilution_backward_scratch_bytes(n, seq, head_dim)
+        gdt = torch.bfloat16 if code == _lib.BF16 else torch.float32
+        dq, dk, dv = (torch.empty(batch, heads, seq, head_dim, device=dev, dtype=gdt) for _ in range(3))
+        nbytes = (lib.dilution_wide_scratch_bytes(code, n, seq, head_dim) if wide
+                  else lib.dilution_backward_scratch_bytes(n, seq, head_dim))
         scratch = torch.empty(nbytes, device=dev, dtype=torch.uint8)
-        _lib.check(lib.dilution_backward(
-            qf.data_ptr(), kf.data_ptr(), vf.data_ptr(), code, prec, n, seq, head_dim,
-            1.0 / math.sqrt(head_dim), EPS, dof.data_ptr(), do_code, of.data_ptr(),
-            rmax.data_ptr(), rden.data_ptr(), carry.data_ptr(), ctx.carry_rows, total.data_ptr(), ssum.data_ptr(),
-            _ptr(pk), scratch.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), _stream(dev)),
-            "dilution_backward")
-        shape4 = (batch, heads, seq, head_dim)
-        return (dq.reshape(shape4).to(q.dtype), dk.reshape(shape4).to(k.dtype),
-                dv.reshape(shape4).to(v.dtype), None)
+        scale = 1.0 / math.sqrt(head_dim)
+        if wide:
+            _lib.check(lib.dilution_wide_backward(
+                qf.data_ptr(), kf.data_ptr(), vf.data_ptr(), code, n, seq, head_dim, scale, EPS, dof.data_ptr(), do_code,
+                out.data_ptr(), rmax.data_ptr(), rden.data_ptr(), carry.data_ptr(), total.data_ptr(), ssum.data_ptr(),
+                pk.data_ptr(), scratch.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), _stream(dev)),
+                "dilution_wide_backward")
+        else:
+            _lib.check(lib.dilution_backward(
+                qf.data_ptr(), kf.data_ptr(), vf.data_ptr(), code, prec, n, seq, head_dim,
+                scale, EPS, dof.data_ptr(), do_code, out.data_ptr(),
+                rmax.data_ptr(), rden.data_ptr(), carry.data_ptr(), ctx.carry_rows, total.data_ptr(), ssum.data_ptr(),
+                _ptr(pk), scratch.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), _stream(dev)),
+                "dilution_backward")
+        return (*(x.to(dt) for x, dt in zip((dq, dk, dv), ctx.dtypes)), None)
 
 
 def dilution_attention(

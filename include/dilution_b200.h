@@ -193,6 +193,28 @@ int dilution_backward(const void* q, const void* k, const void* v, int dtype, in
                       const float* total, const float* ssum, const float* pk,
                       void* scratch, void* dq, void* dk, void* dv, void* stream);
 
+/* Rows of 256 bytes on the tcgen05 kernels: the whole forward (passes 1-3, checkpoints every 32 rows) and
+ * backward of bf16 heads of 128 under BF16 (dtype DILUTION_BF16: q, k, v are (n, t, 128) bf16) and of fp32
+ * heads of 16, 32 or 64 under TF32 (dtype DILUTION_F32: q, k, v are the planes dilution_split_operands makes
+ * of them).  Replaces the same entry points of the reference as dilution_rowstats .. dilution_backward
+ * (kernels.py:328-455, 829-903) for those cases.
+ *
+ * dilution_split_operands: fp32 (rows, d) -> bf16 (rows, 128), [hi 64 | lo 64] with hi = bf16(x),
+ * lo = bf16(x - hi), zeros behind d.  A product of two such operands keeps 16 bits of each, tf32 keeps 11.
+ * out, pk: (n, t, d) fp32; pk may be NULL when no backward follows.  dq, dk, dv: (n, t, d) of `dtype`.
+ * scratch: dilution_wide_scratch_bytes. */
+int dilution_split_operands(const float* q, const float* k, const float* v, int64_t rows, int d, void* qs,
+                            void* ks, void* vs, void* stream);
+int dilution_wide_forward(const void* q, const void* k, const void* v, int dtype, int64_t n, int64_t t, int d,
+                          float scale, float eps, float* rmax, float* rden, float* carry, float* total,
+                          float* out, float* ssum, float* pk, void* stream);
+size_t dilution_wide_scratch_bytes(int dtype, int64_t n, int64_t t, int d);
+int dilution_wide_backward(const void* q, const void* k, const void* v, int dtype, int64_t n, int64_t t, int d,
+                           float scale, float eps, const void* dout, int dout_dtype, const float* out,
+                           const float* rmax, const float* rden, const float* carry, const float* total,
+                           const float* ssum, const float* pk, void* scratch, void* dq, void* dk, void* dv,
+                           void* stream);
+
 /* Bytes of scratch dilution_decode needs for n rows at this `length`. */
 size_t dilution_decode_scratch_bytes(int64_t n, int64_t length, int d);
 
