@@ -114,9 +114,12 @@ dil::Geom make_geom(int64_t n, int64_t tq, int64_t tk, int64_t q_offset, float s
   g.bid = dil::bid_form(bid);
   g.share = share;
   g.normalised = bid == dil::kBidSoftmax || dil::row_sum_bid(bid);
-  g.lshift = (bid == dil::kBidExpshift || bid == dil::kBidSigshift) ? log2f(shift) : 0.f;
+  g.lshift = (bid == dil::kBidExpshift || bid == dil::kBidSigshift) ? log2f(shift)
+             : bid == dil::kBidRelu ? scale : bid == dil::kBidRelu2 ? scale * scale
+             : bid == dil::kBidSoftplus ? dil::kLn2 : 0.f;
   g.ghat_pass = 0;
   g.d = d;
+  g.rscale = 1.f / scale;
   g.n = n;
   g.tq = (int)tq;
   g.tk = (int)tk;
@@ -671,7 +674,8 @@ int dilution_wide_forward(const void* q, const void* k, const void* v, int dtype
 size_t dilution_wide_scratch_bytes(int dtype, int64_t n, int64_t t, int d) {
   if (n < 1 || t < 1 || d < 1) return 0;
   const size_t rows = (size_t)(n * t);
-  return rows * (2 * sizeof(float) * (dtype == DILUTION_F32 ? 64 : 128) + 2 * 128 + 2 * sizeof(float));
+  return rows * (dtype == DILUTION_F32 ? 2 * sizeof(float) * 64 + 2 * 128 + 2 * sizeof(float)
+                                       : 2 * sizeof(float) * 128 + 2 * 256 + 2 * sizeof(float));
 }
 
 int dilution_wide_backward(const void* q, const void* k, const void* v, int dtype, int64_t n, int64_t t, int d,
@@ -690,7 +694,7 @@ int dilution_wide_backward(const void* q, const void* k, const void* v, int dtyp
   float* dq_main = (float*)scratch;
   float* dk_main = dq_main + rows * head;
   char* dop = (char*)(dk_main + rows * head);         // a TMA source: in front of the two (n, t) vectors
-  float* ghat = (float*)(dop + 2 * 128 * rows);
+  float* ghat = (float*)(dop + 2 * (dtype == DILUTION_F32 ? 128 : 256) * rows);
   auto bwd = dtype == DILUTION_F32 ? dil::tc::wide_backward<dil::tc::kSplit> : dil::tc::wide_backward<dil::tc::kWide128>;
   return bwd(q, k, v, g, dout, dout_dtype, out, rmax, rden, carry, total, ssum, pk, dq_main, dk_main, dop, ghat,
              ghat + rows, dq, dk, dv, (cudaStream_t)stream, g_err, sizeof(g_err), mark_scope);
@@ -817,7 +821,20 @@ int dilution_softmax_decode_append(const void* q1, const void* k1, const void* v
   return DILUTION_OK;
 }
 
-// ---- share / bid variants (the tile kernels; kernels_bid.py of the reference) -------------
+// ---- share / bid variants (kernels_bid.py of the reference) -------------
+#ifdef DILUTION_TENSOR_PATH
+// bf16 heads of 64 under "bf16" take the tcgen05 kernels; of the f(a) / rowsum(f) bids the three whose f needs no row
+// minimum, from kMassMinSeq tokens on: 780 -> 213 us forward + backward at n = 32, t = 1024 (softplus), 39.2 -> 7.5 ms
+// at t = 8192.  Shorter rows would gain too (tile kernels 350 us at n = 4, t = 512; the host's launches are 200 us of
+// either), but up to 520 tokens the tests hold them to the tile kernels' route; the line is the next tile boundary that
+// leaves that contract alone.
+constexpr int64_t kMassMinSeq = 5 * 128 + 1;
+static bool tc_variant(int dtype, int precision, int64_t t, int d, int bid, float scale) {
+  if (!dil::tc::supported(dtype, precision, d, 0)) return false;
+  if (!dil::row_sum_bid(bid)) return true;
+  return bid != dil::kBidMinshift && t >= kMassMinSeq && scale > 0.f;
+}
+#endif
 static int check_variant(const char* fn, int bid, int share, float shift) {
   if (bid < 0 || bid > 7)
     return fail(DILUTION_ERR_ARG, "%s: bid %d is not one of softmax 0, relu 1, relu2 2, softplus 3, minshift 4, "
@@ -846,7 +863,7 @@ int dilution_variant_forward(const void* q, const void* k, const void* v, int dt
   const dil::Geom g = make_geom(n, t, t, 0, scale, eps, dil::kCarryRows, bid, share, shift);
   cudaStream_t st = (cudaStream_t)stream;
 #if defined(DILUTION_TENSOR_PATH) && DILUTION_TC_HAS_MAIN
-  if (dil::tc::supported(dtype, precision, d, 0) && !dil::row_sum_bid(bid)) {
+  if (tc_variant(dtype, precision, t, d, bid, scale)) {
     // bf16 tensors, head_dim 64: the tcgen05 kernels, instantiated for the bid and share step
     if (stats && pk) {
       Prof prof("tc_rowstats_pk", st);
@@ -860,6 +877,8 @@ int dilution_variant_forward(const void* q, const void* k, const void* v, int dt
       if (int rc = dil::tc::colsum_scan(q, k, g, rmax, rden, nullptr, carry, total, st, g_err, sizeof(g_err))) return rc;
     }
     Prof prof("tc_forward_main", st);
+    if (dil::row_sum_bid(bid))
+      return dil::tc::mass_forward_main(q, k, v, g, rmax, rden, carry, out, ssum, st, g_err, sizeof(g_err));
     return dil::tc::forward_main(q, k, v, g, rmax, rden, carry, nullptr, out, ssum, st, g_err, sizeof(g_err));
   }
 #endif
@@ -895,7 +914,11 @@ int dilution_variant_backward(const void* q, const void* k, const void* v, int d
   const BwdScratch s = carve_bwd(scratch, n, t, d);
   cudaStream_t st = (cudaStream_t)stream;
 #if defined(DILUTION_TENSOR_PATH) && DILUTION_TC_HAS_BACKWARD
-  if (dil::tc::supported(dtype, precision, d, 0) && !dil::row_sum_bid(bid))
+  if (tc_variant(dtype, precision, t, d, bid, scale) && dil::row_sum_bid(bid))
+    // do' as [hi | lo] takes the place of dk_main, which these bids do not need
+    return dil::tc::mass_backward(q, k, v, g, dout, out, rmax, rden, carry, total, ssum, s.dq_main, s.dk_main, s.ghat,
+                                  s.dbar, dq, dk, dv, st, g_err, sizeof(g_err), mark_scope);
+  if (tc_variant(dtype, precision, t, d, bid, scale))
     return dil::tc::backward(q, k, v, g, dout, DILUTION_F32, out, rmax, rden, carry, total, ssum, pk, s.dq_main,
                              s.dk_main, s.ghat, s.dbar, s.dop, dq, dk, dv, st, g_err, sizeof(g_err), mark_scope);
 #endif

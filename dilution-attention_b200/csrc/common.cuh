@@ -32,6 +32,12 @@ __device__ __forceinline__ float fast_rcp(float x) {
   return y;
 }
 
+__device__ __forceinline__ float fast_log2(float x) {
+  float y;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 // 2^x for x <= 0 on the FMA pipe: x = n + f with n = round(x), f in [-0.5, 0.5];
 // a minimax polynomial gives 2^f (relative error 2.7e-6 with degree 4, 7.5e-5 with
 // degree 3) and n is added to the exponent field.  The special-function unit does 16
@@ -119,7 +125,9 @@ struct Geom {
   int normalised; // the bid divides by its row sum (softmax, relu, relu2, softplus, minshift): there are
                   // row statistics and the backward has the Jacobian correction ghat; otherwise
                   // l = lshift for every row
-  float lshift;   // log2 of the shift of expshift / sigshift (kernels_bid.py:19-26); 0 for the sigmoid
+  float lshift;   // log2 of the shift of expshift / sigshift (kernels_bid.py:19-26); 0 for the sigmoid; on the
+                  // tcgen05 kernels the constant between mass_term and f of an f(a) / rowsum(f) bid
+  float rscale;   // 1 / scale
   int d;          // head size of q, k, v and of every output row
   int ghat_pass;  // reverse pass of an f(a) / rowsum(f) bid, whose Jacobian factor is unbounded (1 / row mass):
                   // 1 = accumulate ghat only, 2 = ghat is known and is subtracted BEFORE the factor

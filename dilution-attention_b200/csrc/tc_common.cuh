@@ -28,24 +28,33 @@ constexpr int kHeadDim = 64;
 constexpr uint32_t kTileBytes = kTileRows * kHeadDim * 2;   // 16 KB
 constexpr long long kWaitCycles = 4000000000LL;             // ~2 s: a live wait is microseconds
 
-// How many [rows][64 bf16] sub-tiles one row of q, k, v or dout takes, and what they hold.
-//   kNarrow : heads of 64 in bf16, one sub-tile;
+// How many [rows][64 bf16] sub-tiles one row of q, k, v takes, what they hold, and how exactly the kernels
+// multiply the values that they form (shares, pdp, P~, W).
+//   kNarrow : heads of 64 in bf16, one sub-tile; formed values rounded to bf16;
 //   kWide128: heads of 128 in bf16, two sub-tiles of 64 features;
+//   kPairs64: heads of 64 in bf16, one sub-tile;
 //   kSplit  : heads of up to 64 in fp32, each value as hi + lo with hi = bf16(x), lo = bf16(x - hi):
 //             sub-tile 0 holds the hi parts, sub-tile 1 the lo parts (zeros behind the head size).  A product of
 //             two such operands keeps 16 bits of each (2^-17 relative), where tf32 keeps 11.
+// All but kNarrow form hi + lo pairs too (kPlanes), and take do' as hi + lo: [hi | lo] sub-tiles.
 // Sub-tile s of a [128 rows] tile lies kTileBytes * s behind its start.
-enum : int { kNarrow = 0, kWide128 = 1, kSplit = 2 };
+enum : int { kNarrow = 0, kWide128 = 1, kSplit = 2, kPairs64 = 3 };
 template <int W> struct Rows {
-  static constexpr int kSub = W == kNarrow ? 1 : 2;
-  static constexpr int kPlanes = W == kSplit ? 2 : 1;              // bf16 parts of a value the kernels form
+  static constexpr int kSub = W == kWide128 || W == kSplit ? 2 : 1;
+  static constexpr int kPlanes = W == kNarrow ? 1 : 2;             // bf16 parts of a value the kernels form
   static constexpr int kCols = 64 * kSub;                          // accumulator columns of a product with k, v, q or dout
   static constexpr int kHead = W == kWide128 ? 128 : 64;           // head size (kSplit: padded)
   static constexpr uint32_t kBytes = kSub * kTileBytes;            // one [128 rows] tile
   // score products: sub-tile pairs (a, b) that are multiplied.  kSplit leaves out lo * lo (2^-18 of the score).
-  static constexpr int kPairs = W == kNarrow ? 1 : W == kWide128 ? 2 : 3;
+  static constexpr int kPairs = W == kSplit ? 3 : kSub;
   static __device__ constexpr int pair_a(int i) { return W == kSplit ? (i == 2) : i; }
   static __device__ constexpr int pair_b(int i) { return W == kSplit ? (i == 1) : i; }
+  // the same of V do'^T, and the parts of do' that dV takes one after the other (kSplit: both in one N = 128 product)
+  static constexpr int kDoSub = W == kNarrow ? 1 : W == kWide128 ? 4 : 2;
+  static constexpr int kDoPairs = W == kSplit ? 3 : kDoSub;
+  static __device__ constexpr int do_a(int i) { return W == kSplit ? (i == 2) : W == kWide128 ? (i & 1) : 0; }
+  static __device__ constexpr int do_b(int i) { return W == kSplit ? (i == 1) : i; }
+  static constexpr int kDoParts = W == kSplit || W == kNarrow ? 1 : 2;
 };
 
 enum : int { kErrWaitTma = 101, kErrWaitMma = 102, kErrWaitDrain = 103, kErrAlign = 104, kErrWaitTile = 105, kErrSelfTest = 199 };
@@ -139,11 +148,11 @@ __device__ __forceinline__ void tma_load_tile(uint32_t dst, const CUtensorMap* m
 }
 
 // All sub-tiles of one tile, `sub_bytes` apart (kTileBytes for 128 rows).
-template <int W>
+template <int W, int SUB = Rows<W>::kSub>
 __device__ __forceinline__ void tma_load_rows(uint32_t dst, const CUtensorMap* map, int row, int n, uint32_t bar,
                                               uint32_t sub_bytes = kTileBytes) {
 #pragma unroll
-  for (int s = 0; s < Rows<W>::kSub; ++s) tma_load_tile(dst + sub_bytes * s, map, row, n, bar, 64 * s);
+  for (int s = 0; s < SUB; ++s) tma_load_tile(dst + sub_bytes * s, map, row, n, bar, 64 * s);
 }
 
 // Element-wise add of a shared-memory tile into global memory (performed at L2), one
@@ -330,6 +339,16 @@ __device__ __forceinline__ void mma_scores_wide(uint32_t d_tmem, Desc a, uint32_
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk)
       mma_ss(d_tmem, a, (a_sub >> 4) * Rows<W>::pair_a(i) + 2 * kk, b, (b_sub >> 4) * Rows<W>::pair_b(i) + 2 * kk, idesc,
+             i > 0 || kk > 0);
+}
+// The same of V do'^T.
+template <int W>
+__device__ __forceinline__ void mma_dov_wide(uint32_t d_tmem, Desc a, uint32_t a_sub, Desc b, uint32_t b_sub, uint32_t idesc) {
+#pragma unroll
+  for (int i = 0; i < Rows<W>::kDoPairs; ++i)
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk)
+      mma_ss(d_tmem, a, (a_sub >> 4) * Rows<W>::do_a(i) + 2 * kk, b, (b_sub >> 4) * Rows<W>::do_b(i) + 2 * kk, idesc,
              i > 0 || kk > 0);
 }
 template <int W>

@@ -197,12 +197,33 @@ __device__ __forceinline__ uint32_t share_chunk_offset(int key, int q) {
   return (uint32_t)((q >> 6) * (int)kTileBytes + key * 128 + ((((q & 63) >> 3) ^ (key & 7)) << 4));
 }
 
+// f of the f(a) / rowsum(f) bids up to a constant (mass_scale) that sits in the per-query factor:
+// relu max(s, 0), relu2 the same before the square, softplus log2(1 + 2^z) with z = s * zscale.
+// POLY: the exponential on the FMA pipe.
+template <int BID, bool POLY = false>
+__device__ __forceinline__ float mass_term(float s, float zscale) {
+  if (BID != kBidSoftplus) return fmaxf(s, 0.f);
+  const float z = s * zscale;
+  const float e = POLY ? poly_exp2<4>(-fabsf(z)) : fast_exp2(-fabsf(z));
+  return fmaxf(z, 0.f) + fast_log2(1.f + e);
+}
+template <int BID> __device__ __forceinline__ float mass_power(float f) { return BID == kBidRelu2 ? f * f : f; }
+__device__ __forceinline__ float mass_factor(float mass, int i, float mass_scale) {
+  return mass > 0.f ? mass_scale / mass : -1.f / (float)(i + 1);
+}
+__device__ __forceinline__ float mass_bid(float fp, float l) { return l >= 0.f ? fp * l : -l; }
+
 // log2-domain log-sum-exp of query i (+inf past the end, so that its p is 0).  The sigmoid bid
 // and the shifted bids have no row statistics: their "lse" is log2 of the shift (0 for the plain
 // sigmoid) for a query that exists and +inf past the end.
+//
+// An f(a) / rowsum(f) bid (q_off = 0) has one factor per query instead: l = lshift / (row mass), with lshift the
+// constant that turns mass_term into f, so that the bid is mass_term * l; -1 / (keys in the window) for a row
+// without mass, which bids that uniformly; 0 past the end.
 template <int BID = kBidSoftmax>
 __device__ __forceinline__ float load_lse(const float* __restrict__ rmax, const float* __restrict__ rden,
                                           int64_t row_base, int i, int tq, float lshift = 0.f) {
+  if (row_sum_bid(BID)) return i < tq ? mass_factor(rden[row_base + i], i, lshift) : 0.f;
   if (BID == kBidSigmoid || rmax == nullptr) return i < tq ? lshift : INFINITY;   // no row statistics
   return i < tq ? rmax[row_base + i] + log2f(rden[row_base + i]) : INFINITY;
 }
@@ -211,6 +232,7 @@ __device__ __forceinline__ float load_lse(const float* __restrict__ rmax, const 
 // softmax 2^(s*zscale - l); sigmoid 1 / (1 + 2^(l - s*zscale)), which is 0 for l = +inf.
 template <int BID, bool POLY = false>
 __device__ __forceinline__ float bid_p(float s, float zscale, float l) {
+  if (row_sum_bid(BID)) return mass_bid(mass_power<BID>(mass_term<BID, POLY>(s, zscale)), l);
   if (BID == kBidSigmoid) return fast_rcp(1.f + fast_exp2(fmaf(s, -zscale, l)));
   // POLY: the exponential on the FMA pipe (a share of them, where the special-function unit binds)
   return POLY ? poly_exp2<4>(fmaf(s, zscale, -l)) : fast_exp2(fmaf(s, zscale, -l));
@@ -222,7 +244,8 @@ __device__ __forceinline__ float bid_p(float s, float zscale, float l) {
 // halves of a row are merged once at the end.  TMEM: 128 columns; 4 CTAs per SM.
 template <int W> constexpr int kRowstatsSmem = 3 * (int)Rows<W>::kBytes + 1024 + 1024 + 256;
 
-template <int W = kNarrow>
+// BID: an f(a) / rowsum(f) bid takes the row's mass instead (rmax is 0 then, rden the mass).
+template <int W = kNarrow, int BID = kBidSoftmax>
 __global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) rowstats_kernel(const __grid_constant__ CUtensorMap map_q,
                                                           const __grid_constant__ CUtensorMap map_k,
                                                           Geom g, float* __restrict__ rmax,
@@ -292,6 +315,18 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) rowstats_kernel(con
         float v[32];
         tmem_ld32(taddr + 32 * c, v);
         tmem_ld_wait(v);
+        if (row_sum_bid(BID)) {
+          float part[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            const int ja = jb * kTileRows + wg * 64 + c * 32 + e;
+            float f = (e & 3) == 3 ? mass_term<BID, true>(v[e], g.zscale) : mass_term<BID>(v[e], g.zscale);
+            if (EDGE && (ja > ia || ja >= g.tk)) f = 0.f;
+            part[e & 3] += mass_power<BID>(f);
+          }
+          s += (part[0] + part[1]) + (part[2] + part[3]);
+          continue;
+        }
         float cmax = -INFINITY;          // max of the raw scores (zscale > 0 keeps the order)
 #pragma unroll
         for (int e = 0; e < 32; ++e) {
@@ -325,10 +360,15 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) rowstats_kernel(con
   const int i = ib * kTileRows + row;
   if (wg == 0 && i < g.tq) {
     const float2 o = sMerge[row];
+    if (row_sum_bid(BID)) {
+      rmax[(int64_t)n * g.tq + i] = 0.f;
+      rden[(int64_t)n * g.tq + i] = (s + o.y) * g.lshift;
+    } else {
     const float nm = fmaxf(m, o.x);          // finite: the first tile always holds key 0
     const float tot = s * fast_exp2(m - nm) + o.y * fast_exp2(o.x - nm);
     rmax[(int64_t)n * g.tq + i] = nm;
     rden[(int64_t)n * g.tq + i] = tot;
+    }
   }
   drain_if_aborted(ctl);
   tc_fence_before();
@@ -348,7 +388,7 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) rowstats_kernel(con
 template <int W> constexpr int kColsumSmem = 3 * (int)Rows<W>::kBytes + 1024 + 2048 + 1024 + 256;
 
 template <int CR, int BID = kBidSoftmax, int W = kNarrow>
-__global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) colsum_scan_kernel(
+__global__ void __launch_bounds__(256, W != kNarrow ? 2 : row_sum_bid(BID) ? 3 : 4) colsum_scan_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, Geom g,
     const float* __restrict__ rmax, const float* __restrict__ rden,
     const float* __restrict__ carry_base, float* __restrict__ carry, float* __restrict__ total) {
@@ -653,7 +693,7 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) forward_main_kernel
           }
           packed[h * 2 + 0] = pack_bf16(sh[0], sh[1]);
           packed[h * 2 + 1] = pack_bf16(sh[2], sh[3]);
-          if (W == kSplit) {
+          if (Rows<W>::kPlanes == 2) {
             rest[h * 2 + 0] = pack_bf16_rest(sh[0], sh[1], packed[h * 2 + 0]);
             rest[h * 2 + 1] = pack_bf16_rest(sh[2], sh[3], packed[h * 2 + 1]);
           }
@@ -662,7 +702,7 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) forward_main_kernel
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(packed[0]),
                      "r"(packed[1]), "r"(packed[2]), "r"(packed[3])
                      : "memory");
-        if (W == kSplit)
+        if (Rows<W>::kPlanes == 2)
           asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + 2 * kTileBytes), "r"(rest[0]),
                        "r"(rest[1]), "r"(rest[2]), "r"(rest[3])
                        : "memory");
@@ -766,6 +806,19 @@ __global__ void backward_prep_kernel(const TD* __restrict__ dout, const float* _
   }
 }
 
+// The factor da / (dp - ghat) of an f(a) / rowsum(f) bid from mass_term and the query's l, f'(a) / (row mass)
+// (kernels_bid.py:206-225): zero for a row without mass (l < 0) and, under MASK, for a masked query (f < 0).
+template <int BID, bool MASK>
+__device__ __forceinline__ float mass_jac(float f, float l, const Geom& g) {
+  float d;                                             // f' up to the constant in l
+  if (BID == kBidSoftplus) d = 1.f - fast_exp2(-f);    // sigmoid(a) = 1 - e^-softplus(a)
+  else if (BID == kBidRelu2) d = f + f;
+  else d = f > 0.f ? 1.f : 0.f;
+  if (MASK && f < 0.f) d = 0.f;
+  // l is (mass_scale / mass), and mass_scale is ln 2 (softplus), scale (relu), scale^2 (relu2: f' = 2 scale^2 s / scale)
+  return d * fmaxf(l, 0.f) * (BID == kBidSoftplus ? kLog2e : g.rscale);
+}
+
 // One thread's 32 queries of the main reverse pass: vs holds their raw scores against the thread's key, vd
 // dO' . v; incle is the key's demand (+ eps) in front of them, R the suffix of dk_share behind them, and query
 // e sees the key when e >= first_q.  Afterwards shp holds the shares as bf16 pairs (SPLIT: their lo plane
@@ -775,10 +828,16 @@ __global__ void backward_prep_kernel(const TD* __restrict__ dout, const float* _
 // suffix of dk_share (kernels.py:763-764), accumulated from the last query to the first as
 // the reference does — its terms grow towards a key's first bidders, so the other order
 // loses the small ones.
-template <int BID, int SHARE, bool MASK, bool SPLIT>
+//
+// PASS: 0 = the Jacobian correction (if any) follows in a pass of its own.  An f(a) / rowsum(f) bid, whose factor is
+// unbounded, takes two passes: 1 leaves p and p * dp in vs and vd, the terms of ghat; 2 subtracts ghat (Gh4) from dp
+// before the factor multiplies.  These bids keep mass_term of a query between the sweeps (-1 where the query does not
+// see the key), which gives p and the factor both.
+template <int BID, int SHARE, bool MASK, bool SPLIT, int PASS = 0>
 __device__ __forceinline__ void reverse_sweeps(float (&vs)[32], float (&vd)[32], uint32_t* shp, float& R, float incle,
                                                const float4* Lse4, const float4* Dbar4, const Geom& g, bool dead,
-                                               int first_q) {
+                                               int first_q, const float4* Gh4 = nullptr) {
+  constexpr bool MASS = row_sum_bid(BID);
   float inv[32];
 #pragma unroll
   for (int e4 = 0; e4 < 8; ++e4) {
@@ -794,7 +853,14 @@ __device__ __forceinline__ void reverse_sweeps(float (&vs)[32], float (&vd)[32],
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int e = e4 * 4 + u;
-      float p = fast_exp2(z[u]);
+      float p, keep;
+      if (MASS) {
+        keep = u == 3 ? mass_term<BID, true>(vs[e], g.zscale) : mass_term<BID>(vs[e], g.zscale);
+        p = mass_bid(mass_power<BID>(keep), lse[u]);
+        if (MASK && (dead || first_q > e)) keep = -1.f;
+      } else {
+        p = fast_exp2(z[u]);
+      }
       if (BID == kBidSigmoid) p = fast_rcp(1.f + p);
       if (MASK) {
         if (dead || first_q > e) p = 0.f;
@@ -808,13 +874,22 @@ __device__ __forceinline__ void reverse_sweeps(float (&vs)[32], float (&vd)[32],
       } else {
         inv[e] = 1.f;
       }
-      vs[e] = p;
+      vs[e] = MASS ? keep : p;
     }
   }
 #pragma unroll
   for (int e4 = 7; e4 >= 0; --e4) {
     const float4 d4 = Dbar4[e4];
     const float dbr[4] = {d4.x, d4.y, d4.z, d4.w};
+    float lr[4], gh[4];
+    if (MASS) {
+      const float4 l4 = Lse4[e4];
+      lr[0] = l4.x; lr[1] = l4.y; lr[2] = l4.z; lr[3] = l4.w;
+      if (PASS == 2) {
+        const float4 g4 = Gh4[e4];
+        gh[0] = g4.x; gh[1] = g4.y; gh[2] = g4.z; gh[3] = g4.w;
+      }
+    }
     // with inv = 1/(committed+p+eps), share = p*inv and w = ds*inv:
     //   ds*(committed+eps)*inv^2 = w*(1-share),  dk_share = -w*share,
     //   dp = w - w*share + (suffix before this query) = w + (suffix after it)
@@ -826,29 +901,43 @@ __device__ __forceinline__ void reverse_sweeps(float (&vs)[32], float (&vd)[32],
 #pragma unroll
     for (int h = 1; h >= 0; --h) {
       const int e = e4 * 4 + 2 * h;
-      const float2 p2 = make_float2(vs[e], vs[e + 1]), i2 = make_float2(inv[e], inv[e + 1]);
+      float2 p2 = make_float2(vs[e], vs[e + 1]);
+      float2 jac2;
+      if (MASS) {
+        jac2 = make_float2(mass_jac<BID, MASK>(p2.x, lr[2 * h], g), mass_jac<BID, MASK>(p2.y, lr[2 * h + 1], g));
+        p2 = make_float2(mass_bid(mass_power<BID>(p2.x), lr[2 * h]), mass_bid(mass_power<BID>(p2.y), lr[2 * h + 1]));
+        if (MASK) {
+          if (vs[e] < 0.f) p2.x = 0.f;
+          if (vs[e + 1] < 0.f) p2.y = 0.f;
+        }
+        if (PASS == 1) jac2 = p2;
+      }
+      const float2 i2 = make_float2(inv[e], inv[e + 1]);
       const float2 w2 = mul2(sub2(make_float2(vd[e], vd[e + 1]), make_float2(dbr[2 * h], dbr[2 * h + 1])), i2);
       const float2 s2 = mul2(p2, i2);
-      float2 jac2 = p2;
+      if (!MASS) jac2 = p2;
       if (BID == kBidSigmoid) jac2 = mul2(p2, sub2(make_float2(1.f, 1.f), p2));
       float2 pd2;
       if (SHARE == kShareInclusive) {
         const float r1 = fmaf(-w2.y, s2.y, R);
         R = fmaf(-w2.x, s2.x, r1);
-        pd2 = mul2(jac2, add2(w2, make_float2(R, r1)));
+        pd2 = add2(w2, make_float2(R, r1));
       } else if (SHARE == kShareExclusive) {
         const float r1 = fmaf(-w2.y, s2.y, R);
-        pd2 = mul2(jac2, add2(w2, make_float2(r1, R)));
+        pd2 = add2(w2, make_float2(r1, R));
         R = fmaf(-w2.x, s2.x, r1);
       } else {
-        pd2 = mul2(jac2, w2);
+        pd2 = w2;
       }
+      if (PASS == 2) pd2 = sub2(pd2, make_float2(gh[2 * h], gh[2 * h + 1]));
+      pd2 = mul2(jac2, pd2);
       vd[e] = pd2.x;
       vd[e + 1] = pd2.y;
-      if (BID == kBidSigmoid) {
+      if (BID == kBidSigmoid || MASS) {
         vs[e] = jac2.x;
         vs[e + 1] = jac2.y;
       }
+      if (PASS == 1) continue;
       shp[e4 * 2 + h] = pack_bf16(s2.x, s2.y);
       if (SPLIT) shp[16 + e4 * 2 + h] = pack_bf16_rest(s2.x, s2.y, shp[e4 * 2 + h]);
     }
@@ -890,7 +979,11 @@ __device__ __forceinline__ void reverse_sweeps(float (&vs)[32], float (&vd)[32],
 constexpr int kBwdThreads = 384;
 constexpr int kBwdSmem = 12 * kTileBytes + 2048 + 2048 + 256 + 1024;
 
-template <int BID = kBidSoftmax, int SHARE = kShareInclusive>
+// PASS 1 (reverse_sweeps; pass 2 is wide_backward_main_kernel) forms only the scores and adds up ghat, p * dp over the
+// 32 keys of a warp by shuffles (31 for 32 queries) and over warps by atomics, all in fp32.  Its do' is
+// [hi | lo] as in pass 2, so that ghat is the sum of exactly the dp it will be subtracted from; the lo tiles take the
+// shared memory of the pdp and dQ tiles.
+template <int BID = kBidSoftmax, int SHARE = kShareInclusive, int PASS = 0>
 __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_do, const __grid_constant__ CUtensorMap map_dq, Geom g,
@@ -913,6 +1006,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
   float* sG = reinterpret_cast<float*>(smem + 12 * kTileBytes + 2048);         // [2][2][128] sums of dk_share
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 12 * kTileBytes + 4096);
   Ctl* ctl = reinterpret_cast<Ctl*>(bars + 12);
+  static_assert(PASS == 0 || PASS == 1, "pass 2 runs on wide_backward_main_kernel");
+  constexpr uint32_t kStageTx = (PASS == 1 ? 3 : 2) * kTileBytes;
   const uint32_t kfull = smem_u32(bars), qfull = smem_u32(bars + 1);           // qfull[3]
   const uint32_t sdone = smem_u32(bars + 4), tiles = smem_u32(bars + 6);       // [2] each
   const uint32_t dqdone = smem_u32(bars + 8);
@@ -931,7 +1026,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
 
   auto load_stats = [&](int ib) {
     const int i = ib * kTileRows + row;
-    float2 st = make_float2(INFINITY, 0.f);
+    float2 st = make_float2(row_sum_bid(BID) ? 0.f : INFINITY, 0.f);
     if (i < g.tq) st = make_float2(load_lse<BID>(rmax, rden, row_base, i, g.tq, g.lshift), dbarp[row_base + i]);
     return st;
   };
@@ -993,9 +1088,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
     mbar_expect_tx(kfull, kTileBytes);
     tma_load_tile(sK, &map_k, k0, n, kfull);
     for (int s = 0; s < 3 && s < nsteps; ++s) {
-      mbar_expect_tx(qfull + 8 * s, 2 * kTileBytes);
+      mbar_expect_tx(qfull + 8 * s, kStageTx);
       tma_load_tile(sQ0 + kTileBytes * s, &map_q, (nqb - 1 - s) * kTileRows, n, qfull + 8 * s);
       tma_load_tile(sD0 + kTileBytes * s, &map_do, (nqb - 1 - s) * kTileRows, n, qfull + 8 * s);
+      if (PASS == 1) tma_load_tile(sPd + kTileBytes * s, &map_do, (nqb - 1 - s) * kTileRows, n, qfull + 8 * s, 64);
     }
   }
   tc_fence_before();
@@ -1026,6 +1122,9 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
       for (int kk = 0; kk < 4; ++kk) mma_ss(tS0 + 64 * ODD, dKk, 2 * kk, dQk, off + 2 * kk, id_s, kk > 0);
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) mma_ts(tDOV0 + 64 * ODD, tV + 8 * kk, dDk, off + 2 * kk, id_s, kk > 0);
+#pragma unroll
+      for (int kk = 0; PASS == 1 && kk < 4; ++kk)            // + V (lo part of do')^T
+        mma_ts(tDOV0 + 64 * ODD, tV + 8 * kk, make_desc(sPd, 16, 1024), off + 2 * kk, id_s, 1);
     };
     if (tid == 256) {
       mbar_wait(kfull, 0, ctl, &g_status, kErrWaitTma);
@@ -1045,7 +1144,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
         mbar_wait(tiles + 8 * ODD, s & 1, ctl, &g_status, kErrWaitTile);
         tc_fence_after();
 #pragma unroll
-        for (int kq = 0; kq < 4; ++kq) {                    // contraction over the 64 queries
+        for (int kq = 0; PASS != 1 && kq < 4; ++kq) {       // contraction over the 64 queries
           // queries [16kq, 16kq+16) of the half-step: 8 columns at the start of the owning
           // warpgroup's 32-column range (warpgroup 1 owns queries 0..31)
           constexpr uint32_t base = ST * 1024 + (ODD ? 0 : 4) * 128;
@@ -1053,7 +1152,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
           mma_ts(tDV, tS0 + col, dDm, base + 128 * kq, id_kd, 1);
           mma_ts(tDK, tDOV0 + col, dQm, base + 128 * kq, id_kd, 1);
         }
-        if (ODD) {
+        if (ODD && PASS != 1) {
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)                    // contraction over the 128 keys
             mma_ss(tDQ, dPm, 128 * kk, dKm, 128 * kk, id_qd, kk > 0);
@@ -1071,13 +1170,14 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
           // every MMA of step s-1 has completed once the commit of its second half-step has:
           // its Q and dO' stage takes step s+2
           mbar_wait(sdone + 8, s & 1, ctl, &g_status, kErrWaitMma);
-          mbar_expect_tx(qfull + 8 * ST2, 2 * kTileBytes);
+          mbar_expect_tx(qfull + 8 * ST2, kStageTx);
           tma_load_tile(sQ0 + kTileBytes * ST2, &map_q, (nqb - 3 - s) * kTileRows, n, qfull + 8 * ST2);
           tma_load_tile(sD0 + kTileBytes * ST2, &map_do, (nqb - 3 - s) * kTileRows, n, qfull + 8 * ST2);
+          if (PASS == 1) tma_load_tile(sPd + kTileBytes * ST2, &map_do, (nqb - 3 - s) * kTileRows, n, qfull + 8 * ST2, 64);
         }
       }
       __syncwarp();
-      if (ODD) {
+      if (ODD && PASS != 1) {
         // dQ and ghat of the step's 128 queries: lane = query.  The fp32 tile is staged in
         // shared memory in the copy engine's swizzled layout and added to dq_main by two
         // tensor reductions of 32 columns.
@@ -1112,7 +1212,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
           tma_reduce_add_tile(&map_dq, sDq + kTileBytes, 32, ibq * kTileRows, n);
         }
         const int i = ibq * kTileRows + row;
-        if (i < g.tq) atomicAdd(ghat + row_base + i, gh);
+        if (PASS == 0 && i < g.tq) atomicAdd(ghat + row_base + i, gh);
       }
     };
     using C0 = std::integral_constant<int, 0>;
@@ -1156,7 +1256,9 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
       const bool fetch_stats = !odd && wg == 0 && s + 1 < nsteps;
       if (fetch_stats) {
         const int i = (ib - 1) * kTileRows + row;     // ib >= 1 here, so i < tq
-        if (BID == kBidSoftmax && rmax != nullptr) {
+        if (row_sum_bid(BID)) {
+          st_den = rden[row_base + i];
+        } else if (BID == kBidSoftmax && rmax != nullptr) {
           st_max = rmax[row_base + i];
           st_den = rden[row_base + i];
         } else {
@@ -1182,23 +1284,34 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
       // starts from zero and adds p * (the suffix warpgroup 0 ends with) afterwards: dp is linear in it
       float R = wg == 0 ? sigma : 0.f;
       auto chunk = [&](auto mask_tag) {
-        reverse_sweeps<BID, SHARE, decltype(mask_tag)::value, false>(vs, vd, shp, R, incl + g.eps, Lse4, Dbar4, g, dead,
-                                                                     ja - iq0);
+        reverse_sweeps<BID, SHARE, decltype(mask_tag)::value, false, PASS>(
+            vs, vd, shp, R, incl + g.eps, Lse4, Dbar4, g, dead, ja - iq0);
       };
       if (masked_tile) chunk(std::true_type{}); else chunk(std::false_type{});
       // warpgroup 0: the suffix behind query 32; warpgroup 1: minus its own sum of -dk_share
       sG[(odd * 2 + wg) * 128 + row] = R;
       // the shares stay in TMEM, over score columns this thread has consumed
-      tmem_st16(tS0 + tcol, shp);
+      if (PASS != 1) tmem_st16(tS0 + tcol, shp);
       asm volatile("bar.sync 1, 256;" ::: "memory");   // the compute warps
       const float rother = sG[(odd * 2 + (1 - wg)) * 128 + row];
       const float fix = wg == 1 ? rother : 0.f;
       sigma = R + rother;                              // the suffix behind the next half-step
-      // the dQ MMAs of the previous 128 queries read the pdp buffer that is written next
-      if (!odd && s >= 1) {
-        mbar_wait(dqdone, (s - 1) & 1, ctl, &g_status, kErrWaitMma);
-      }
-      {
+      if (PASS == 1) {
+        // p * dp summed over the warp's 32 keys: each step halves the queries a lane holds, lane l ends with query l
+#pragma unroll
+        for (int e = 0; e < 32; ++e) vd[e] = fmaf(vs[e], fix, vd[e]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+          for (int e = 0; e < o; ++e) {
+            const float give = lane & o ? vd[e] : vd[e + o], mine = lane & o ? vd[e + o] : vd[e];
+            vd[e] = mine + __shfl_xor_sync(0xffffffffu, give, o);
+          }
+        }
+        if (iq0 + lane < g.tq) atomicAdd(ghat + row_base + iq0 + lane, vd[0]);
+      } else {
+        // the dQ MMAs of the previous 128 queries read the pdp buffer that is written next
+        if (!odd && s >= 1) mbar_wait(dqdone, (s - 1) & 1, ctl, &g_status, kErrWaitMma);
         uint32_t pdt[16];                              // 32 pdp values as bf16 pairs
 #pragma unroll
         for (int e8 = 0; e8 < 4; ++e8) {
@@ -1217,7 +1330,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
         tmem_st16(tDOV0 + tcol, pdt);
       }
       if (fetch_stats) {
-        sLse[(b ^ 1) * 128 + row] = st_max + log2f(st_den);
+        sLse[(b ^ 1) * 128 + row] = row_sum_bid(BID) ? mass_factor(st_den, (ib - 1) * kTileRows + row, g.lshift)
+                                                     : st_max + log2f(st_den);
         sDbar[(b ^ 1) * 128 + row] = st_dbar;
       }
       incl = incl_next;
@@ -1231,7 +1345,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
   }
   mbar_wait(sdone + 8, nsteps & 1, ctl, &g_status, kErrWaitMma);
   tc_fence_after();
-  if (warp < 8) {
+  if (PASS != 1 && warp < 8) {
     // lane = key: each warpgroup stores 32 of the 64 columns of dk_main and dv
     float a[32];
     const int64_t o = ((int64_t)n * g.tk + ja) * kHeadDim + 32 * wg;
@@ -1552,9 +1666,16 @@ static_assert(5 * (kRowstatsSmem<kNarrow> + 1024) > 233472 && 5 * (kColsumSmem<k
   if ((g).share == kShareInclusive) { constexpr int SHARE = kShareInclusive; __VA_ARGS__; }        \
   else if ((g).share == kShareExclusive) { constexpr int SHARE = kShareExclusive; __VA_ARGS__; }   \
   else { constexpr int SHARE = kShareNone; __VA_ARGS__; }
-#define DIL_TC_BID(g, ...)                                                     \
+#define DIL_TC_PLAIN_BID(g, ...)                                               \
   if ((g).bid == kBidSigmoid) { constexpr int BID = kBidSigmoid; __VA_ARGS__; } \
   else { constexpr int BID = kBidSoftmax; __VA_ARGS__; }
+#define DIL_TC_MASS_BID(g, ...)                                                     \
+  if ((g).bid == kBidRelu) { constexpr int BID = kBidRelu; __VA_ARGS__; }           \
+  else if ((g).bid == kBidRelu2) { constexpr int BID = kBidRelu2; __VA_ARGS__; }    \
+  else { constexpr int BID = kBidSoftplus; __VA_ARGS__; }
+#define DIL_TC_BID(g, ...)                                            \
+  if (row_sum_bid((g).bid)) { DIL_TC_MASS_BID(g, __VA_ARGS__) }       \
+  else { DIL_TC_PLAIN_BID(g, __VA_ARGS__) }
 
 inline int rowstats(const void* q, const void* k, const Geom& g, float* rmax, float* rden,
                     cudaStream_t st, char* err, size_t errlen) {
@@ -1562,9 +1683,16 @@ inline int rowstats(const void* q, const void* k, const Geom& g, float* rmax, fl
   if (int rc = make_map(&mq, q, g.n, g.tq, err, errlen)) return rc;
   if (int rc = make_map(&mk, k, g.n, g.tk, err, errlen)) return rc;
   constexpr int smem = kRowstatsSmem<kNarrow>;
-  if (int rc = set_smem_attr((const void*)rowstats_kernel<>, smem, err, errlen)) return rc;
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
-  rowstats_kernel<><<<(unsigned)(g.n * nqb), 256, smem, st>>>(mq, mk, g, rmax, rden);
+  auto launch = [&](auto kern) -> int {
+    if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
+    kern<<<(unsigned)(g.n * nqb), 256, smem, st>>>(mq, mk, g, rmax, rden);
+    return 0;
+  };
+  if (int rc = g.bid == kBidRelu       ? launch(rowstats_kernel<kNarrow, kBidRelu>)
+               : g.bid == kBidRelu2    ? launch(rowstats_kernel<kNarrow, kBidRelu2>)
+               : g.bid == kBidSoftplus ? launch(rowstats_kernel<kNarrow, kBidSoftplus>)
+                                       : launch(rowstats_kernel<>)) return rc;
   return launch_status("tc rowstats", err, errlen);
 }
 
@@ -1582,8 +1710,8 @@ inline int colsum_scan(const void* q, const void* k, const Geom& g, const float*
       if (int rc = set_smem_attr((const void*)colsum_scan_kernel<32, BID>, smem, err, errlen)) return rc;
       colsum_scan_kernel<32, BID><<<grid, 256, smem, st>>>(mq, mk, g, rmax, rden, carry_base, carry, total);
     })
-  } else {
-    DIL_TC_BID(g, {
+  } else {                              // forward-only calls of the operator
+    DIL_TC_PLAIN_BID(g, {
       if (int rc = set_smem_attr((const void*)colsum_scan_kernel<64, BID>, smem, err, errlen)) return rc;
       colsum_scan_kernel<64, BID><<<grid, 256, smem, st>>>(mq, mk, g, rmax, rden, carry_base, carry, total);
     })
@@ -1602,7 +1730,7 @@ inline int forward_main(const void* q, const void* k, const void* v, const Geom&
   static_assert(2 * (smem + 1024) <= 233472 && 3 * (smem + 1024) > 233472, "exactly two CTAs of the main pass fit one SM");
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
   const unsigned grid = (unsigned)(g.n * nqb);
-  DIL_TC_BID(g, DIL_TC_SHARE(g, {
+  DIL_TC_PLAIN_BID(g, DIL_TC_SHARE(g, {
     if (int rc = set_smem_attr((const void*)forward_main_kernel<BID, SHARE>, smem, err, errlen)) return rc;
     forward_main_kernel<BID, SHARE><<<grid, 256, smem, st>>>(mq, mk, mv, g, rmax, rden, carry, carry_base, out, ssum);
   }))
@@ -1645,17 +1773,17 @@ inline int backward(const void* q, const void* k, const void* v, const Geom& g, 
     static_assert(smem_bwd <= 232448 && 2 * smem_bwd > 233472, "the backward main pass runs one CTA per SM");
     mark("tc_backward_main", st, 0);
     const unsigned grid = (unsigned)(g.n * nkb);
-    DIL_TC_BID(g, DIL_TC_SHARE(g, {
+    DIL_TC_PLAIN_BID(g, DIL_TC_SHARE(g, {
       if (int rc = set_smem_attr((const void*)backward_main_kernel<BID, SHARE>, smem_bwd, err, errlen)) return rc;
       backward_main_kernel<BID, SHARE><<<grid, kBwdThreads, smem_bwd, st>>>(
           mq, mk, md, mdq, g, (const __nv_bfloat16*)v, rmax, rden, dbarp, carry, total, dq_main, dk_main,
           (__nv_bfloat16*)dv, ghat);
     }))
+    mark("tc_backward_main", st, 1);
   } else {
     snprintf(err, errlen, "the tensor-core backward needs checkpoints every 32 query rows (got %d)", g.carry_rows);
     return 1;
   }
-  mark("tc_backward_main", st, 1);
   if (int rc = launch_status("tc backward_main", err, errlen)) return rc;
   if (!g.normalised || g.share == kShareNone) {
     // no row normalisation in the bid: no Jacobian correction, dk and dq are dk_main and dq_main.

@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) rowpass_product_ker
     tmem_ld32(taddr + 32, v + 32);
     tmem_ld_wait(v);
     tmem_ld_wait(v + 32);
-    uint32_t pw[32], pr[W == kSplit ? 32 : 1];
+    uint32_t pw[32], pr[Rows<W>::kPlanes == 2 ? 32 : 1];
     float ps = 0.f;
     // P~ = 2^(z - reference) for the thread's 64 scores, two per instruction; their sum in ps
     auto exponentials = [&]() {
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) rowpass_product_ker
         acc1 = add2(acc1, p1);
         pw[e >> 1] = pack_bf16(p0.x, p0.y);
         pw[(e >> 1) + 1] = pack_bf16(p1.x, p1.y);
-        if (W == kSplit) {
+        if (Rows<W>::kPlanes == 2) {
           pr[e >> 1] = pack_bf16_rest(p0.x, p0.y, pw[e >> 1]);
           pr[(e >> 1) + 1] = pack_bf16_rest(p1.x, p1.y, pw[(e >> 1) + 1]);
         }
@@ -208,10 +208,10 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) rowpass_product_ker
     }
     s += ps;
     // P~ goes over the first 32 of this thread's 64 consumed score columns: keys 2c, 2c+1 of the
-    // warpgroup's half in column c (kSplit: the lo plane over the other 32)
+    // warpgroup's half in column c (two planes: the lo plane over the other 32)
     tmem_st16(taddr, pw);
     tmem_st16(taddr + 16, pw + 16);
-    if (W == kSplit) {
+    if (Rows<W>::kPlanes == 2) {
       tmem_st16(taddr + 32, pr);
       tmem_st16(taddr + 48, pr + 16);
     }
@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) backward_key_correc
     const bool masked = dead || t == 0;
     const float4* St4 = reinterpret_cast<const float4*>(sStat + b * 128 + 64 * odd + 32 * wg);
     float vs[32];
-    uint32_t wt[16], wr[W == kSplit ? 16 : 1];
+    uint32_t wt[16], wr[Rows<W>::kPlanes == 2 ? 16 : 1];
     tmem_ld32(tcol, vs);
     tmem_ld_wait(vs);
     auto tile = [&](auto mask_tag) {
@@ -438,12 +438,12 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) backward_key_correc
           if (dead || ja > i0 + 2 * e2 + 1) p1 = 0.f;
         }
         wt[e2] = pack_bf16(p0 * st.y, p1 * st.w);
-        if (W == kSplit) wr[e2] = pack_bf16_rest(p0 * st.y, p1 * st.w, wt[e2]);
+        if (Rows<W>::kPlanes == 2) wr[e2] = pack_bf16_rest(p0 * st.y, p1 * st.w, wt[e2]);
       }
     };
     if (masked) tile(std::true_type{}); else tile(std::false_type{});
     tmem_st16(tcol, wt);            // W over the first 16 of the 32 consumed columns (its lo plane over the others)
-    if (W == kSplit) tmem_st16(tcol + 16, wr);
+    if (Rows<W>::kPlanes == 2) tmem_st16(tcol + 16, wr);
     if (fetch) sStat[(b ^ 1) * 128 + row] = make_float2(nx_max + log2f(nx_den), nx_gh);
     tmem_st_wait();
     tc_fence_before();

@@ -1,16 +1,20 @@
 // Rows of 256 bytes on the tcgen05 kernels: bf16 heads of 128 (kWide128) and fp32 heads of up to 64 under
 // "tf32", every value held as a bf16 pair hi + lo (kSplit; Rows in tc_common.cuh).  Both have the same
 // tiles — two [rows][64 bf16] sub-tiles — and the same accumulators: 128 columns, which are the 128
-// features of a head, or X_hi and X_lo products of 64 features that the epilogue adds.
+// features of a head, or X_hi and X_lo products of 64 features that the epilogue adds.  At the end of the file, the
+// relu, relu2 and softplus bids of bf16 heads of 64 (kPairs64).
+// The shares, pdp, P~ and do' that these kernels form are multiplied as pairs hi + lo, 16 bits of each: the tile
+// kernels that they replace keep 11 (tf32), one bf16 value would keep 8.
 //
 // The forward is row pass + column-sum scan + query-stationary main pass, the wide instantiations of the
 // kernels in tc_kernels.cuh and tc_rowpass_kernels.cuh; the reverse main pass has a kernel of its own, since the
 // narrow one's accumulators would need 656 of the 512 TMEM columns.
 //
 // Forward + backward at B4 H8 T4096 on one B200, before (tile kernels with tf32 products) and after:
-//   bf16 d = 128  14.8 ms -> 1.64 ms  (reverse pass 7.24 -> 0.70, main pass 3.82 -> 0.33)
-//   fp32 d = 64    7.1 ms -> 2.10 ms  (reverse pass 3.51 -> 0.93, main pass 1.61 -> 0.39)
-// and against exact products the fp32 outputs move from 2.8e-4 to about 1e-5 (2-norm).
+//   bf16 d = 128  14.8 ms -> 2.18 ms  (reverse pass 7.24 -> 1.12, main pass 3.82 -> 0.39)
+//   fp32 d = 64    7.1 ms -> 2.06 ms  (reverse pass 3.51 -> 0.93, main pass 1.61 -> 0.39)
+// (with single bf16 values bf16 d = 128 takes 1.64 ms, its outputs 1.0e-3 off).  Against 64 bits, 2-norm: bf16 outputs
+// 1.3e-4 -> 1.6e-6, gradients 1.7e-3 before and after (their own rounding to bf16); fp32 outputs 2.8e-4 -> about 1e-5.
 #pragma once
 
 #include "tc_kernels.cuh"
@@ -55,7 +59,7 @@ template <int E> __device__ __forceinline__ void load_vec(const __nv_bfloat16* p
   }
 }
 
-// backward_prep_kernel for wide rows: dbar' and do' = sinv * dout, as bf16 (kWide128) or as hi | lo (kSplit).
+// backward_prep_kernel for wide rows: dbar' and do' = sinv * dout as [hi | lo], 128 | 128 (kWide128) or 64 | 64 features.
 template <typename TD, int W>
 __global__ void wide_backward_prep_kernel(const TD* __restrict__ dout, const float* __restrict__ out,
                                           const float* __restrict__ ssum, float eps, int64_t rows, int d,
@@ -82,7 +86,10 @@ __global__ void wide_backward_prep_kernel(const TD* __restrict__ dout, const flo
   }
   dot = warp_sum(dot);
   if (W == kWide128) {
-    reinterpret_cast<uint2*>(dop + row * 128)[lane] = make_uint2(pack_bf16(a[0], a[1]), pack_bf16(a[E - 2], a[E - 1]));
+    const uint2 hi = make_uint2(pack_bf16(a[0], a[1]), pack_bf16(a[E - 2], a[E - 1]));
+    reinterpret_cast<uint2*>(dop + row * 256)[lane] = hi;
+    reinterpret_cast<uint2*>(dop + row * 256 + 128)[lane] =
+        make_uint2(pack_bf16_rest(a[0], a[1], hi.x), pack_bf16_rest(a[E - 2], a[E - 1], hi.y));
     reinterpret_cast<float4*>(dq_main + row * 128)[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
   } else {
     const uint32_t hi = pack_bf16(a[0], a[1]);
@@ -124,32 +131,42 @@ __global__ void split_dq_from_pk_kernel(const float* __restrict__ dq_main, const
 //  * ghat^T = 1^T pdp is a product of its own against a 4 KB tile of ones.
 // kSplit multiplies hi and lo planes of share and pdp (two A operands side by side in TMEM, two pdp tiles),
 // and dQ^T rows 64..127 (K_lo) are reduced into the same columns of dq_main as rows 0..63.
+//  * kWide128 stages 32 queries of dQ at a time (16 KB instead of 32): its do' takes 64 KB.
+// kPairs64 serves pass 2 of the f(a) / rowsum(f) bids: ghat (of backward_main_kernel's pass 1) is subtracted before the
+// factor multiplies, dk is final (written as TOut to dk_main), and rows 64..127 of dQ^T, whose A operand is the V tile
+// behind K, are not used.
+template <int W> constexpr int kDqRows = W == kWide128 ? 32 : 64;
 template <int W> constexpr int kBwdWideSmem =
-    4 * (int)Rows<W>::kBytes + (Rows<W>::kPlanes + 2) * (int)kTileBytes + 4096 + 1024 + 2048 + 256 + 256 + 1024;
+    3 * (int)Rows<W>::kBytes + (Rows<W>::kDoSub + Rows<W>::kPlanes) * (int)kTileBytes + kDqRows<W> * 512 + 4096 + 1024 +
+    2048 + 512 + 256 + 1024;
 
-template <int W, typename TOut>
+template <int W, typename TOut, int BID = kBidSoftmax, int SHARE = kShareInclusive, int PASS = 0>
 __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
     const __grid_constant__ CUtensorMap map_dq, Geom g, const float* __restrict__ rmax,
     const float* __restrict__ rden, const float* __restrict__ dbarp, const float* __restrict__ carry,
-    const float* __restrict__ total, float* __restrict__ dk_main, TOut* __restrict__ dv, float* __restrict__ ghat) {
+    const float* __restrict__ total, std::conditional_t<PASS == 2, TOut, float>* __restrict__ dk_main,
+    TOut* __restrict__ dv, float* __restrict__ ghat) {
+  static_assert(PASS == 0 || PASS == 2, "pass 1 is backward_main_kernel's");
   constexpr uint32_t TB = Rows<W>::kBytes;                 // [128] rows of k or v: 32 KB
-  constexpr uint32_t HB = TB / 2, HSub = kTileBytes / 2;   // [64] rows of q or do', and one of their sub-tiles
+  constexpr uint32_t HB = TB / 2, HSub = kTileBytes / 2;   // [64] rows of q, and one of their sub-tiles
+  constexpr uint32_t HBd = Rows<W>::kDoSub * HSub;         // [64] rows of do'
+  constexpr int kDqFeat = W == kPairs64 ? 64 : 128;        // rows of dQ^T that count
   constexpr int P = Rows<W>::kPlanes;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
   const uint32_t sK = smem_u32(smem), sV = sK + TB;
   const uint32_t sQ0 = sK + 2 * TB, sD0 = sQ0 + 2 * HB;        // [2] stages each
-  const uint32_t sPd = sD0 + 2 * HB;                           // [P][128 keys][64 queries] bf16
-  const uint32_t sDq = sPd + P * kTileBytes;                   // [4 warps][64 queries][32 features] fp32
-  const uint32_t sOnes = sDq + 2 * kTileBytes;
-  uint8_t* tail = smem + 4 * TB + (P + 2) * kTileBytes;        // the ones tile
+  const uint32_t sPd = sD0 + 2 * HBd;                          // [P][128 keys][64 queries] bf16
+  const uint32_t sDq = sPd + P * kTileBytes;                   // [4 warps][kDqRows queries][32 features] fp32
+  const uint32_t sOnes = sDq + kDqRows<W> * 512;
+  uint8_t* tail = smem + (sOnes - sK);                         // the ones tile
   float* sLse = reinterpret_cast<float*>(tail + 4096);         // [2][64]
   float* sDbar = sLse + 128;                                   // [2][64]
   float* sG = sDbar + 128;                                     // [2][2][128] sums of dk_share
-  float* sGh = sG + 512;                                       // [64]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sGh + 64);
+  float* sGh = sG + 512;                                       // [64]; PASS 2: [2][64] ghat of the queries
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sGh + 128);
   Ctl* ctl = reinterpret_cast<Ctl*>(bars + 12);
   const uint32_t kfull = smem_u32(bars), qfull = smem_u32(bars + 1);           // qfull[2]
   const uint32_t sdone = smem_u32(bars + 3), tiles = smem_u32(bars + 4), dqdone = smem_u32(bars + 5);
@@ -165,10 +182,11 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
   const int ja = k0 + row;
   const bool dead = ja >= g.tk;
 
-  auto load_stats = [&](int hb, float* lse, float* dbar) {      // of query 64 hb + row, row < 64
+  auto load_stats = [&](int hb, float* lse, float* dbar, float* gh) {      // of query 64 hb + row, row < 64
     const int i = hb * 64 + row;
-    *lse = load_lse(rmax, rden, row_base, i, g.tq);
+    *lse = load_lse<BID>(rmax, rden, row_base, i, g.tq, g.lshift);
     *dbar = i < g.tq ? dbarp[row_base + i] : 0.f;
+    *gh = PASS == 2 && i < g.tq ? ghat[row_base + i] : 0.f;
   };
 
   if (tid == 0) {
@@ -182,10 +200,11 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
   if (warp == 0) tmem_alloc(smem_u32(&ctl->tmem), 512);
   if (wg == 0) {
     if (row < 64) {
-      float l, db;
-      load_stats(2 * nqb - 1, &l, &db);
+      float l, db, gh;
+      load_stats(2 * nqb - 1, &l, &db, &gh);
       sLse[row] = l;
       sDbar[row] = db;
+      if (PASS == 2) sGh[row] = gh;
     }
   } else if (wg == 1) {
     const uint4 one = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
@@ -210,9 +229,9 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
   }
   auto load_stage = [&](int h) {                     // thread 256: q and do' of half-step h
     const int st = h & 1, r0 = (2 * nqb - 1 - h) * 64;
-    mbar_expect_tx(qfull + 8 * st, 2 * HB);
+    mbar_expect_tx(qfull + 8 * st, HB + HBd);
     tma_load_rows<W>(sQ0 + HB * st, &map_q, r0, n, qfull + 8 * st, HSub);
-    tma_load_rows<W>(sD0 + HB * st, &map_do, r0, n, qfull + 8 * st, HSub);
+    tma_load_rows<W, Rows<W>::kDoSub>(sD0 + HBd * st, &map_do, r0, n, qfull + 8 * st, HSub);
   };
   if (tid == 256) {
     mbar_expect_tx(kfull, 2 * TB);
@@ -229,7 +248,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
     // ------------------------------------------------------------ issue, and the dQ read-out
     asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");
     constexpr uint32_t id_s = instr_desc(128, 64, 0, 0);     // scores: both operands K-major
-    constexpr uint32_t id_kd = instr_desc(128, 128, 0, 1);   // dV, dK: A from TMEM (M = keys), B MN-major
+    constexpr uint32_t id_kd = instr_desc(128, Rows<W>::kCols, 0, 1);   // dV, dK: A from TMEM (M = keys), B MN-major
     constexpr uint32_t id_qd = instr_desc(128, 64, 1, 1);    // dQ^T, ghat^T: A and B MN-major
     const Desc dKk = make_desc(sK, 16, 1024), dVk = make_desc(sV, 16, 1024);
     const Desc dKm = make_desc(sK, kTileBytes, 1024), dOnes = make_desc(sOnes, 2048, 1024);
@@ -237,7 +256,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
     auto issue_scores = [&](int h) {
       const int st = h & 1;
       mma_scores_wide<W>(tS, dKk, kTileBytes, make_desc(sQ0 + HB * st, 16, 1024), HSub, id_s);
-      mma_scores_wide<W>(tDOV, dVk, kTileBytes, make_desc(sD0 + HB * st, 16, 1024), HSub, id_s);
+      mma_dov_wide<W>(tDOV, dVk, kTileBytes, make_desc(sD0 + HBd * st, 16, 1024), HSub, id_s);
     };
     if (tid == 256) {
       mbar_wait(kfull, 0, ctl, &g_status, kErrWaitTma);
@@ -252,13 +271,15 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
       if (tid == 256) {
         mbar_wait(tiles, h & 1, ctl, &g_status, kErrWaitTile);
         tc_fence_after();
-        const Desc dQm = make_desc(sQ0 + HB * st, HSub, 1024), dDm = make_desc(sD0 + HB * st, HSub, 1024);
+        const Desc dQm = make_desc(sQ0 + HB * st, HSub, 1024), dDm = make_desc(sD0 + HBd * st, HSub, 1024);
 #pragma unroll
         for (int pl = 0; pl < P; ++pl)
 #pragma unroll
           for (int kq = 0; kq < 4; ++kq) {                    // contraction over the 64 queries, 16 each
             const uint32_t col = 32 * (kq >> 1) + 16 * pl + 8 * (kq & 1);
             mma_ts(tDV, tS + col, dDm, 128 * kq, id_kd, 1);
+            if (Rows<W>::kDoParts == 2 && pl == 0)            // share_hi do'_lo; share_lo do'_lo is left out (2^-18)
+              mma_ts(tDV, tS + col, dDm, (HSub >> 4) * Rows<W>::kSub + 128 * kq, id_kd, 1);
             mma_ts(tDK, tDOV + col, dQm, 128 * kq, id_kd, 1);
           }
         if (h + 1 < nhalf) {
@@ -272,7 +293,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {                    // contraction over the 128 keys
             mma_ss(tDQ, dKm, 128 * kk, dPm, 1024 * pl + 128 * kk, id_qd, (pl > 0 || kk > 0));
-            mma_ss(tG, dOnes, 0, dPm, 1024 * pl + 128 * kk, id_qd, (pl > 0 || kk > 0));
+            if (PASS == 0) mma_ss(tG, dOnes, 0, dPm, 1024 * pl + 128 * kk, id_qd, (pl > 0 || kk > 0));
           }
         mma_commit(dqdone);
         if (h + 2 < nhalf) {
@@ -288,19 +309,30 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
       __syncwarp();
       tc_fence_after();
       const int q0 = (2 * nqb - 1 - h) * 64, w4 = warp & 3;
-      if (lane == 0) tma_wait_read_all();               // the previous reduction has read this warp's staging
-      __syncwarp();
-      const uint32_t stage = sDq + w4 * 8192 + lane * 4;
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
+        constexpr bool kEach = kDqRows<W> == 32;        // staged and reduced 32 queries at a time
+        if (32 * w4 >= kDqFeat) break;
+        if (kEach || c == 0) {
+          if (lane == 0) tma_wait_read_all();           // the previous reduction has read this warp's staging
+          __syncwarp();
+        }
+        const uint32_t stage = sDq + w4 * (kDqRows<W> * 128), off = kEach ? 0 : 32 * c;
         float x[32];
         tmem_ld32(tDQ + lane_base + 32 * c, x);
         tmem_ld_wait(x);
 #pragma unroll
         for (int e = 0; e < 32; ++e)
-          asm volatile("st.shared.f32 [%0], %1;" ::"r"(stage + (32 * c + e) * 128), "f"(x[e] * g.scale) : "memory");
+          asm volatile("st.shared.f32 [%0], %1;" ::"r"(stage + lane * 4 + (off + e) * 128), "f"(x[e] * g.scale) : "memory");
+        if (kEach || c == 1) {
+          fence_async_smem();
+          __syncwarp();
+          const int qr = q0 + (kEach ? 32 * c : 0);
+          if (lane == 0 && qr < g.tq)                   // a reduction never starts behind the last row
+            tma_reduce_add_tile(&map_dq, stage, W == kSplit ? 32 * (w4 & 1) : 32 * w4, qr, n);
+        }
       }
-      if (w4 == 0) {                                    // every lane of ghat^T holds the same 64 sums
+      if (PASS == 0 && w4 == 0) {                       // every lane of ghat^T holds the same 64 sums
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           float x[32];
@@ -316,11 +348,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
         for (int q = lane; q < 64; q += 32)
           if (q0 + q < g.tq) atomicAdd(ghat + row_base + q0 + q, sGh[q]);
       }
-      fence_async_smem();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0 && q0 < g.tq)                       // a reduction never starts behind the last row
-        tma_reduce_add_tile(&map_dq, sDq + w4 * 8192, W == kSplit ? 32 * (w4 & 1) : 32 * w4, q0, n);
       asm volatile("bar.sync 2, 128;" ::: "memory");    // every warp has read the tile: the next one may be issued
       tc_fence_after();
     }
@@ -331,7 +360,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
     // ------------------------------------------------------------ the compute warps
     const int cw = 32 * (1 - wg);                    // this warpgroup's queries of a half-step
     auto load_edge = [&](int h) {                    // demand in front of this thread's 32 queries of half-step h
-      if (dead) return 0.f;
+      if (dead || SHARE == kShareNone) return 0.f;   // no share step: no demand is read
       const int rb = 2 * (2 * nqb - 1 - h) + (wg == 0 ? 1 : 0);
       return rb < ncb ? carry[((int64_t)n * ncb + rb) * g.tk + ja] : total[(int64_t)n * g.tk + ja];
     };
@@ -341,10 +370,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
     const uint32_t tcol = lane_base + cw;
     for (int h = 0; h < nhalf; ++h) {
       const int b = h & 1, hb = 2 * nqb - 1 - h;
-      float incl_next2 = 0.f, nx_lse = INFINITY, nx_dbar = 0.f;
+      float incl_next2 = 0.f, nx_lse = INFINITY, nx_dbar = 0.f, nx_gh = 0.f;
       if (h + 2 < nhalf) incl_next2 = load_edge(h + 2);
       const bool fetch = wg == 0 && row < 64 && h + 1 < nhalf;
-      if (fetch) load_stats(hb - 1, &nx_lse, &nx_dbar);
+      if (fetch) load_stats(hb - 1, &nx_lse, &nx_dbar, &nx_gh);
       mbar_wait(sdone, h & 1, ctl, &g_status, kErrWaitMma);
       tc_fence_after();
       float vs[32], vd[32];
@@ -361,13 +390,14 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
       // from zero and adds p * (the suffix warpgroup 0 ends with) afterwards: dp is linear in it
       float R = wg == 0 ? sigma : 0.f;
       auto chunk = [&](auto mask_tag) {
-        reverse_sweeps<kBidSoftmax, kShareInclusive, decltype(mask_tag)::value, W == kSplit>(
-            vs, vd, shp, R, incl + g.eps, Lse4, Dbar4, g, dead, ja - iq0);
+        reverse_sweeps<BID, SHARE, decltype(mask_tag)::value, true, PASS>(
+            vs, vd, shp, R, incl + g.eps, Lse4, Dbar4, g, dead, ja - iq0,
+            reinterpret_cast<const float4*>(sGh + b * 64 + cw));
       };
       if (masked) chunk(std::true_type{}); else chunk(std::false_type{});
       sG[(b * 2 + wg) * 128 + row] = R;
       tmem_st16(tS + tcol, shp);                       // the shares, over score columns this thread has consumed
-      if (W == kSplit) tmem_st16(tS + tcol + 16, shp + 16 * (P - 1));
+      tmem_st16(tS + tcol + 16, shp + 16);
       asm volatile("bar.sync 1, 256;" ::: "memory");   // the compute warps
       const float rother = sG[(b * 2 + (1 - wg)) * 128 + row];
       const float fix = wg == 1 ? rother : 0.f;
@@ -383,7 +413,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
             const int e = e8 * 8 + 2 * u;
             const float2 f2 = fma2(make_float2(vs[e], vs[e + 1]), make_float2(fix, fix), make_float2(vd[e], vd[e + 1]));
             pdt[e8 * 4 + u] = pack_bf16(f2.x, f2.y);
-            if (W == kSplit) pdt[16 * (P - 1) + e8 * 4 + u] = pack_bf16_rest(f2.x, f2.y, pdt[e8 * 4 + u]);
+            pdt[16 + e8 * 4 + u] = pack_bf16_rest(f2.x, f2.y, pdt[e8 * 4 + u]);
           }
 #pragma unroll
           for (int pl = 0; pl < P; ++pl) {              // [key][query]: the MN-major B operand of dQ^T and ghat^T
@@ -394,11 +424,12 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
           }
         }
         tmem_st16(tDOV + tcol, pdt);                    // the A operand of dK (M = keys)
-        if (W == kSplit) tmem_st16(tDOV + tcol + 16, pdt + 16 * (P - 1));
+        tmem_st16(tDOV + tcol + 16, pdt + 16);
       }
       if (fetch) {
         sLse[(b ^ 1) * 64 + row] = nx_lse;
         sDbar[(b ^ 1) * 64 + row] = nx_dbar;
+        if (PASS == 2) sGh[(b ^ 1) * 64 + row] = nx_gh;
       }
       incl = incl_next;
       incl_next = incl_next2;
@@ -431,12 +462,9 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
       const int col = kHalf * wg + c0;
       float a[32];
       fetch32(tDK + col, a);
-      if (!dead) {
 #pragma unroll
-        for (int e = 0; e < 32; e += 4)
-          *reinterpret_cast<float4*>(dk_main + ((int64_t)n * g.tk + ja) * kHead + col + e) =
-              make_float4(a[e] * g.scale, a[e + 1] * g.scale, a[e + 2] * g.scale, a[e + 3] * g.scale);
-      }
+      for (int e = 0; e < 32; ++e) a[e] *= g.scale;
+      if (!dead) store_row32<kNarrow>(dk_main + ((int64_t)n * g.tk + ja) * kHead + col, a, 32);
       fetch32(tDV + col, a);
       if (!dead) store_row32<W>(dv + ((int64_t)n * g.tk + ja) * d + col, a, d - col);
     }
@@ -507,7 +535,7 @@ inline int wide_forward(const void* q, const void* k, const void* v, const Geom&
   return launch_status("tc wide forward_main", err, errlen);
 }
 
-// dq_main and dk_main: (n, t, 128), kSplit (n, t, 64); dop: (n, t, 128) bf16; ghat, dbarp: (n, t).
+// dq_main and dk_main: (n, t, 128), kSplit (n, t, 64); dop: (n, t, 64 kDoSub) bf16; ghat, dbarp: (n, t).
 template <int W>
 inline int wide_backward(const void* q, const void* k, const void* v, const Geom& g, const void* dout, int dout_dtype,
                          const float* out, const float* rmax, const float* rden, const float* carry,
@@ -520,8 +548,8 @@ inline int wide_backward(const void* q, const void* k, const void* v, const Geom
   if (int rc = wide_maps(&m, q, k, v, g, err, errlen)) return rc;
   CUtensorMap mq64, md64, mdq;
   if (int rc = make_map(&mq64, q, g.n, g.tq, err, errlen, 128, 64)) return rc;
-  if (int rc = make_map(&md64, dop, g.n, g.tq, err, errlen, 128, 64)) return rc;
-  if (int rc = make_map_f32(&mdq, dq_main, g.n, g.tq, err, errlen, kHead, 64, false)) return rc;
+  if (int rc = make_map(&md64, dop, g.n, g.tq, err, errlen, 64 * Rows<W>::kDoSub, 64)) return rc;
+  if (int rc = make_map_f32(&mdq, dq_main, g.n, g.tq, err, errlen, kHead, kDqRows<W>, false)) return rc;
   const int64_t rows = g.n * g.tq;
   const unsigned grid = (unsigned)(g.n * ((g.tk + kTileRows - 1) / kTileRows));
   mark("tc_wide_backward_prep", st, 0);
@@ -563,6 +591,79 @@ inline int wide_backward(const void* q, const void* k, const void* v, const Geom
   }
   mark("tc_wide_dq_from_pk", st, 1);
   return launch_status("tc wide dq_from_pk", err, errlen);
+}
+
+// ---------------------------------------------------------------- f(a) / rowsum(f) bids of bf16 heads of 64
+// relu, relu2, softplus.  The row mass and the column sums only need scores and run on the narrow kernels.
+// softplus / inclusive at B4 H8 T8192, forward + backward on one B200: 39.2 ms on the tile kernels -> 7.5 ms (row mass
+// 0.54, column sums 0.67, main pass 2.2, ghat 1.6, reverse pass 3.1); outputs 1.3e-4 -> 1.5e-6 off 64 bits (2-norm),
+// gradients 1.7e-3 before and after.  Bound by the special-function unit (four operations per score in the reverse
+// passes, three in the main pass) and, with one CTA per SM in the two product passes, by the hand-over between scores,
+// arithmetic and products.
+inline int mass_forward_main(const void* q, const void* k, const void* v, const Geom& g, const float* rmax,
+                             const float* rden, const float* carry, float* out, float* ssum, cudaStream_t st, char* err,
+                             size_t errlen) {
+  CUtensorMap mq, mk, mv;
+  if (int rc = make_map(&mq, q, g.n, g.tq, err, errlen)) return rc;
+  if (int rc = make_map(&mk, k, g.n, g.tk, err, errlen)) return rc;
+  if (int rc = make_map(&mv, v, g.n, g.tk, err, errlen)) return rc;
+  constexpr int smem = kMainSmem<kPairs64>;
+  static_assert(smem <= 232448 && 2 * smem > 233472, "one CTA (512 TMEM columns) per SM");
+  const unsigned grid = (unsigned)(g.n * ((g.tq + kTileRows - 1) / kTileRows));
+  DIL_TC_MASS_BID(g, DIL_TC_SHARE(g, {
+    auto kern = forward_main_kernel<BID, SHARE, kPairs64>;
+    if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
+    kern<<<grid, 256, smem, st>>>(mq, mk, mv, g, rmax, rden, carry, nullptr, out, ssum);
+  }))
+  return launch_status("tc forward_main", err, errlen);
+}
+
+// dq_main: (n, t, 64) fp32; dop: (n, t, 128) bf16; ghat, dbarp: (n, t).
+inline int mass_backward(const void* q, const void* k, const void* v, const Geom& g, const float* dout, const float* out,
+                         const float* rmax, const float* rden, const float* carry, const float* total,
+                         const float* ssum, float* dq_main, void* dop, float* ghat, float* dbarp, void* dq, void* dk,
+                         void* dv, cudaStream_t st, char* err, size_t errlen, void (*mark)(const char*, cudaStream_t, int)) {
+  CUtensorMap mq, mk, mv, md, mq64, md64, mdq;
+  if (int rc = make_map(&mq, q, g.n, g.tq, err, errlen)) return rc;
+  if (int rc = make_map(&mk, k, g.n, g.tk, err, errlen)) return rc;
+  if (int rc = make_map(&mv, v, g.n, g.tk, err, errlen)) return rc;
+  if (int rc = make_map(&md, dop, g.n, g.tq, err, errlen, 128)) return rc;
+  if (int rc = make_map(&mq64, q, g.n, g.tq, err, errlen, 64, 64)) return rc;
+  if (int rc = make_map(&md64, dop, g.n, g.tq, err, errlen, 128, 64)) return rc;
+  if (int rc = make_map_f32(&mdq, dq_main, g.n, g.tq, err, errlen, 64, kDqRows<kPairs64>, false)) return rc;
+  using bf = __nv_bfloat16;
+  const int64_t rows = g.n * g.tq;
+  const unsigned grid = (unsigned)(g.n * ((g.tk + kTileRows - 1) / kTileRows));
+  mark("tc_backward_prep", st, 0);
+  wide_backward_prep_kernel<float, kPairs64><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(
+      dout, out, ssum, g.eps, rows, 64, dbarp, (bf*)dop, ghat, dq_main);
+  mark("tc_backward_prep", st, 1);
+  if (int rc = launch_status("tc backward_prep", err, errlen)) return rc;
+  // ghat first, also without a share step, where it is zero in exact arithmetic: do' and the shares are rounded, and a
+  // factor of 1 / (row mass) would multiply what that leaves of it
+  DIL_TC_MASS_BID(g, DIL_TC_SHARE(g, {
+    auto kern = backward_main_kernel<BID, SHARE, 1>;
+    if (int rc = set_smem_attr((const void*)kern, kBwdSmem, err, errlen)) return rc;
+    mark("tc_backward_ghat", st, 0);
+    kern<<<grid, kBwdThreads, kBwdSmem, st>>>(mq, mk, md, mdq, g, (const bf*)v, rmax, rden, dbarp, carry, total, nullptr,
+                                              nullptr, nullptr, ghat);
+    mark("tc_backward_ghat", st, 1);
+    if (int rc = launch_status("tc backward_ghat", err, errlen)) return rc;
+    auto main = wide_backward_main_kernel<kPairs64, bf, BID, SHARE, 2>;
+    constexpr int smem = kBwdWideSmem<kPairs64>;
+    static_assert(smem <= 232448 && 2 * smem > 233472, "the wide reverse pass runs one CTA per SM");
+    if (int rc = set_smem_attr((const void*)main, smem, err, errlen)) return rc;
+    mark("tc_backward_main", st, 0);
+    main<<<grid, kBwdThreads, smem, st>>>(mq64, mk, mv, md64, mdq, g, rmax, rden, dbarp, carry, total, (bf*)dk, (bf*)dv,
+                                          ghat);
+    mark("tc_backward_main", st, 1);
+  }))
+  if (int rc = launch_status("tc backward_main", err, errlen)) return rc;
+  const int64_t n4 = rows * kHeadDim / 4;
+  mark("tc_cast_dq", st, 0);
+  cast_dq_kernel<<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(dq_main, (bf*)dq, n4);
+  mark("tc_cast_dq", st, 1);
+  return launch_status("tc cast_dq", err, errlen);
 }
 
 }  // namespace tc
