@@ -545,15 +545,16 @@ template <int W> constexpr int kMainSmem =
 
 // BID / SHARE select the ablations of kernels_bid.py (sigmoid bid; exclusive or absent share step,
 // :254-262); the default instantiation is the operator.
-template <int BID = kBidSoftmax, int SHARE = kShareInclusive, int W = kNarrow>
-__global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) forward_main_kernel(
+template <int BID = kBidSoftmax, int SHARE = kShareInclusive>
+__global__ void __launch_bounds__(256, 2) forward_main_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, Geom g, const float* __restrict__ rmax,
     const float* __restrict__ rden, const float* __restrict__ carry,
     const float* __restrict__ carry_base, float* __restrict__ out, float* __restrict__ ssum) {
+  constexpr int W = kNarrow;
   constexpr uint32_t TB = Rows<W>::kBytes;
   constexpr int kOCols = Rows<W>::kCols + 16;        // O and the row sums: one tile
-  constexpr int kTmem = W == kNarrow ? 256 : 512;
+  constexpr int kTmem = 256;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   if (smem_u32(smem) & 1023u) {                      // no slack is requested: refuse instead of overrunning
@@ -562,10 +563,10 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) forward_main_kernel
   }
   const uint32_t sQ = smem_u32(smem), sK0 = sQ + TB, sV = sQ + 3 * TB;
   // a [128 keys][64] bf16 tile of ones right behind V: the last 64-column group of the B
-  // operand of share @ [V | ones] (N = 80 or 144), so the row sums come out of the same MMA
+  // operand of share @ [V | ones] (N = 80), so the row sums come out of the same MMA
   const uint32_t sOnes = sQ + 4 * TB, sSh = sOnes + kTileBytes;
   uint8_t* ones_ptr = smem + 4 * TB;
-  float* sL = reinterpret_cast<float*>(smem + 4 * TB + (1 + 2 * Rows<W>::kPlanes) * kTileBytes);
+  float* sL = reinterpret_cast<float*>(smem + 4 * TB + 3 * kTileBytes);
   uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(sL) + 512);
   Ctl* ctl = reinterpret_cast<Ctl*>(bars + 8);
   const uint32_t kfull = smem_u32(bars), vfull = smem_u32(bars + 2), sdone = smem_u32(bars + 3);
@@ -664,7 +665,7 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) forward_main_kernel
       float4 lnext[2] = {L4[c * 8], L4[c * 8 + 1]};
 #pragma unroll
       for (int e8 = 0; e8 < 4; ++e8) {
-        uint32_t packed[4], rest[4];
+        uint32_t packed[4];
         const float4 lcur[2] = {lnext[0], lnext[1]};
         if (e8 < 3) {
           lnext[0] = L4[c * 8 + e8 * 2 + 2];
@@ -693,19 +694,11 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) forward_main_kernel
           }
           packed[h * 2 + 0] = pack_bf16(sh[0], sh[1]);
           packed[h * 2 + 1] = pack_bf16(sh[2], sh[3]);
-          if (Rows<W>::kPlanes == 2) {
-            rest[h * 2 + 0] = pack_bf16_rest(sh[0], sh[1], packed[h * 2 + 0]);
-            rest[h * 2 + 1] = pack_bf16_rest(sh[2], sh[3], packed[h * 2 + 1]);
-          }
         }
         const uint32_t dst = sSh + share_chunk_offset(row, wg * 64 + c * 32 + e8 * 8);
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(packed[0]),
                      "r"(packed[1]), "r"(packed[2]), "r"(packed[3])
                      : "memory");
-        if (Rows<W>::kPlanes == 2)
-          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + 2 * kTileBytes), "r"(rest[0]),
-                       "r"(rest[1]), "r"(rest[2]), "r"(rest[3])
-                       : "memory");
       }
     }
     };
@@ -721,10 +714,7 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) forward_main_kernel
       // descriptors are built once per tile; a k-step is a constant 2048 B (128 units) further
       const Desc dSh = make_desc(sSh, kTileBytes, 1024), dVm = make_desc(sV, kTileBytes, 1024);
 #pragma unroll
-      for (int pl = 0; pl < Rows<W>::kPlanes; ++pl)
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          mma_ss(tO, dSh, 2048 * pl + 128 * kk, dVm, 128 * kk, id_o, (jb > 0 || pl > 0 || kk > 0));
+      for (int kk = 0; kk < 8; ++kk) mma_ss(tO, dSh, 128 * kk, dVm, 128 * kk, id_o, (jb > 0 || kk > 0));
       if (jb + 1 < njb) {
         mbar_wait(kfull + 8 * (b ^ 1), ((jb + 1) >> 1) & 1, ctl, &g_status, kErrWaitTma);
         tc_fence_after();
@@ -735,6 +725,248 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) forward_main_kernel
     __syncwarp();
   }
   mbar_wait(sdone, njb & 1, ctl, &g_status, kErrWaitMma);
+  tc_fence_after();
+  {
+    // lane = query now: each warpgroup stores half of the output columns of row `row`, 32 at a time
+    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+    constexpr int kHalf = kHeadDim / 2;
+    const int i = ib * kTileRows + row;
+    float rs;
+    tmem_ld1(tR + lane_base, &rs);
+    tmem_ld_wait();
+    const float inv = 1.f / (rs + g.eps);
+    float o[32];
+    tmem_ld32(tO + lane_base + kHalf * wg, o);
+    tmem_ld_wait(o);
+    if (i < g.tq) {
+      float4* dst = reinterpret_cast<float4*>(out + ((int64_t)n * g.tq + i) * kHeadDim + kHalf * wg);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) dst[c] = make_float4(o[4 * c] * inv, o[4 * c + 1] * inv, o[4 * c + 2] * inv, o[4 * c + 3] * inv);
+    }
+    if (i < g.tq && wg == 0) ssum[(int64_t)n * g.tq + i] = rs;
+  }
+  drain_if_aborted(ctl);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_free(tmem, kTmem);
+}
+
+// The main pass with its own issuing warp, for rows that leave room for one CTA per SM (W != kNarrow) and the
+// element-wise bids.  The arithmetic is forward_main_kernel's.  A ninth warp issues every copy and product, so that
+// no compute warp waits for another one's turn at the tensor pipe: the scores of tile jb + 1 are issued as soon as
+// all warps have read those of tile jb (half of the arithmetic still ahead of them), and share V of tile jb runs under
+// the arithmetic of tile jb + 1, whose first 32 shares per thread wait in registers until it has read the share tile.
+// Where one CTA fills an SM nothing else hides those round trips: bf16 heads of 128 0.39 -> 0.30 ms (n = 32, T = 4096),
+// softplus bid 1.55 -> 1.26 ms (n = 32, T = 8192); with two CTAs: sigmoid bid 0.98 -> 0.89 ms.  The softmax bid of heads
+// of 64 stays on forward_main_kernel: its long rows run at the card's power limit, where this form is 1 to 3% slower
+// (145.2 -> 148 ms for the passes of a 128K prompt, 16 heads).
+constexpr int kMainThreads = 288;
+template <int BID = kBidSoftmax, int SHARE = kShareInclusive, int W = kNarrow>
+__global__ void __launch_bounds__(kMainThreads, W == kNarrow ? 2 : 1) forward_main_async_kernel(
+    const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+    const __grid_constant__ CUtensorMap map_v, Geom g, const float* __restrict__ rmax,
+    const float* __restrict__ rden, const float* __restrict__ carry,
+    const float* __restrict__ carry_base, float* __restrict__ out, float* __restrict__ ssum) {
+  constexpr uint32_t TB = Rows<W>::kBytes;
+  constexpr int P = Rows<W>::kPlanes;
+  constexpr int kOCols = Rows<W>::kCols + 16;        // O and the row sums: one tile
+  constexpr int kTmem = W == kNarrow ? 256 : 512;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = smem_raw;
+  if (smem_u32(smem) & 1023u) {                      // no slack is requested: refuse instead of overrunning
+    if (threadIdx.x == 0) atomicCAS(&g_status, 0, kErrAlign);
+    return;
+  }
+  const uint32_t sQ = smem_u32(smem), sK0 = sQ + TB, sV = sQ + 3 * TB;
+  // a [128 keys][64] bf16 tile of ones right behind V: the last 64-column group of the B
+  // operand of share @ [V | ones] (N = 80 or 144), so the row sums come out of the same MMA
+  const uint32_t sOnes = sQ + 4 * TB, sSh = sOnes + kTileBytes;
+  uint8_t* ones_ptr = smem + 4 * TB;
+  float* sL = reinterpret_cast<float*>(smem + 4 * TB + (1 + 2 * P) * kTileBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(sL) + 512);
+  Ctl* ctl = reinterpret_cast<Ctl*>(bars + 8);
+  const uint32_t kfull = smem_u32(bars), vfull = smem_u32(bars + 2), sdone = smem_u32(bars + 3);
+  const uint32_t odone = smem_u32(bars + 4), sfree = smem_u32(bars + 5), shready = smem_u32(bars + 6);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wg = tid >> 7, row = tid & 127;
+  const int nqb = (g.tq + kTileRows - 1) / kTileRows;
+  const int ncb = (g.tq + g.carry_rows - 1) / g.carry_rows;
+  const int n = (int)(blockIdx.x % g.n);
+  const int ib = nqb - 1 - (int)(blockIdx.x / g.n);
+  const int q0 = g.q_off + ib * kTileRows;
+  const int njb = min(g.tk - 1, q0 + kTileRows - 1) / kTileRows + 1;
+
+  if (tid == 0) {
+    ctl->abort = 0;
+    for (int i = 0; i < 5; ++i) mbar_init(kfull + 8 * i, 1);      // kfull[2], vfull, sdone, odone
+    mbar_init(sfree, 8);
+    mbar_init(shready, 8);
+    fence_barrier_init();
+  }
+  __syncwarp();
+  if (warp == 0) tmem_alloc(smem_u32(&ctl->tmem), kTmem);
+  if (wg == 0) sL[row] = load_lse<BID>(rmax, rden, (int64_t)n * g.tq, ib * kTileRows + row, g.tq, g.lshift);
+  else if (wg == 1) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      reinterpret_cast<uint4*>(ones_ptr)[row * 8 + c] = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
+  }
+  fence_async_smem();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = ctl->tmem;
+  const uint32_t tS = tmem, tO = tmem + 128, tR = tO + Rows<W>::kCols;
+
+  if (warp == 8) {
+    if (lane == 0) {
+      mbar_expect_tx(kfull, 2 * TB);
+      tma_load_rows<W>(sQ, &map_q, ib * kTileRows, n, kfull);
+      tma_load_rows<W>(sK0, &map_k, 0, n, kfull);
+      mbar_expect_tx(vfull, TB);
+      tma_load_rows<W>(sV, &map_v, 0, n, vfull);
+      if (njb > 1) {
+        mbar_expect_tx(kfull + 8, TB);
+        tma_load_rows<W>(sK0 + TB, &map_k, kTileRows, n, kfull + 8);
+      }
+      constexpr uint32_t id_s = instr_desc(128, 128, 0, 0), id_o = instr_desc(128, kOCols, 1, 1);
+      // descriptors are built once; a k-step of O is a constant 2048 B (128 units) further
+      const Desc dK0 = make_desc(sK0, 16, 1024), dK1 = make_desc(sK0 + TB, 16, 1024), dQ = make_desc(sQ, 16, 1024);
+      const Desc dSh = make_desc(sSh, kTileBytes, 1024), dVm = make_desc(sV, kTileBytes, 1024);
+      mbar_wait(kfull, 0, ctl, &g_status, kErrWaitTma);
+      tc_fence_after();
+      mma_scores_wide<W>(tS, dK0, kTileBytes, dQ, kTileBytes, id_s);
+      mma_commit(sdone);
+      for (int jb = 0; jb < njb; ++jb) {
+        const int b = jb & 1;
+        if (jb + 1 < njb) {
+          mbar_wait(kfull + 8 * (b ^ 1), ((jb + 1) >> 1) & 1, ctl, &g_status, kErrWaitTma);
+          mbar_wait(sfree, jb & 1, ctl, &g_status, kErrWaitTile);
+          tc_fence_after();
+          mma_scores_wide<W>(tS, b ? dK0 : dK1, kTileBytes, dQ, kTileBytes, id_s);
+          mma_commit(sdone);
+          if (jb + 2 < njb) {             // the scores of jb have been read, so its K stage is free
+            mbar_expect_tx(kfull + 8 * b, TB);
+            tma_load_rows<W>(sK0 + TB * b, &map_k, (jb + 2) * kTileRows, n, kfull + 8 * b);
+          }
+        }
+        if (jb >= 1) {                    // V is free once the previous share V has completed
+          mbar_wait(odone, (jb - 1) & 1, ctl, &g_status, kErrWaitMma);
+          mbar_expect_tx(vfull, TB);
+          tma_load_rows<W>(sV, &map_v, jb * kTileRows, n, vfull);
+        }
+        mbar_wait(shready, jb & 1, ctl, &g_status, kErrWaitTile);
+        mbar_wait(vfull, jb & 1, ctl, &g_status, kErrWaitTma);
+        tc_fence_after();
+#pragma unroll
+        for (int pl = 0; pl < P; ++pl)
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)
+            mma_ss(tO, dSh, 2048 * pl + 128 * kk, dVm, 128 * kk, id_o, (jb > 0 || pl > 0 || kk > 0));
+        mma_commit(odone);
+      }
+    }
+    __syncwarp();
+  } else {
+  // the checkpoint row this warpgroup starts from: the one in front of query 0 / query 64 of the block
+  const int rb = (ib * kTileRows + 64 * wg) / g.carry_rows;
+  const bool have_rows = rb < ncb;                 // false only for a ragged last half block
+  const int64_t carry_row = ((int64_t)n * ncb + (have_rows ? rb : 0)) * g.tk;
+  const float4* L4 = reinterpret_cast<const float4*>(sL + 64 * wg);
+  const uint32_t taddr = tS + ((uint32_t)((warp & 3) * 32) << 16) + 64 * wg;
+  const int qh = q0 + 64 * wg;                     // absolute position of this half's first query
+  auto load_den = [&](int jbx) {
+    const int jx = jbx * kTileRows + row;
+    float d = g.eps;
+    if (SHARE != kShareNone && jx < g.tk && have_rows) {      // no share step: no demand is read
+      d += carry[carry_row + jx];
+      if (carry_base != nullptr) d += carry_base[(int64_t)n * g.tk + jx];
+    }
+    return d;
+  };
+  float den_next = load_den(0);
+  for (int jb = 0; jb < njb; ++jb) {
+    const int ja = jb * kTileRows + row;
+    float den = den_next;
+    if (jb + 1 < njb) den_next = load_den(jb + 1);   // lands while this tile is processed
+    const bool dead = ja >= g.tk;
+    const bool masked = dead || jb * kTileRows + kTileRows - 1 > qh;
+    mbar_wait(sdone, jb & 1, ctl, &g_status, kErrWaitMma);
+    tc_fence_after();
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      float v[32];
+      uint32_t packed[16], rest[P == 2 ? 16 : 1];
+      tmem_ld32(taddr + 32 * c, v);
+      tmem_ld_wait(v);
+      if (c == 1) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(sfree);
+      }
+      auto chunk = [&](auto mask_tag) {
+        constexpr bool MASK = decltype(mask_tag)::value;
+#pragma unroll
+        for (int e8 = 0; e8 < 4; ++e8) {
+          const float4 la = L4[c * 8 + 2 * e8], lb = L4[c * 8 + 2 * e8 + 1];
+          const float ls[8] = {la.x, la.y, la.z, la.w, lb.x, lb.y, lb.z, lb.w};
+          float p[8], r[8];
+          if (BID == kBidSoftmax) {
+            const float2 zs = make_float2(g.zscale, g.zscale);
+            float2 z[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              z[i] = fma2(make_float2(v[e8 * 8 + 2 * i], v[e8 * 8 + 2 * i + 1]), zs, make_float2(-ls[2 * i], -ls[2 * i + 1]));
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              p[2 * i] = fast_exp2(z[i].x);
+              p[2 * i + 1] = (i & 1) ? poly_exp2<4>(z[i].y) : fast_exp2(z[i].y);
+            }
+          } else {
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+              p[u] = (u & 3) == 3 ? bid_p<BID, true>(v[e8 * 8 + u], g.zscale, ls[u]) : bid_p<BID>(v[e8 * 8 + u], g.zscale, ls[u]);
+          }
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            if (MASK && (dead || ja > qh + c * 32 + e8 * 8 + u)) p[u] = 0.f;
+            if (SHARE == kShareExclusive) {            // earlier queries' demand only
+              r[u] = fast_rcp(den);
+              den += p[u];
+            } else if (SHARE == kShareInclusive) {
+              den += p[u];
+              r[u] = fast_rcp(den);
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            float2 s2 = make_float2(p[2 * i], p[2 * i + 1]);
+            if (SHARE != kShareNone) s2 = mul2(s2, make_float2(r[2 * i], r[2 * i + 1]));
+            const int o = 4 * e8 + i;
+            packed[o] = pack_bf16(s2.x, s2.y);
+            if (P == 2) rest[P == 2 ? o : 0] = pack_bf16_rest(s2.x, s2.y, packed[o]);
+          }
+        }
+      };
+      if (masked) chunk(std::true_type{}); else chunk(std::false_type{});
+      if (c == 0 && jb >= 1) mbar_wait(odone, (jb - 1) & 1, ctl, &g_status, kErrWaitMma);
+#pragma unroll
+      for (int e8 = 0; e8 < 4; ++e8) {
+        const uint32_t dst = sSh + share_chunk_offset(row, wg * 64 + c * 32 + e8 * 8);
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(packed[4 * e8]),
+                     "r"(packed[4 * e8 + 1]), "r"(packed[4 * e8 + 2]), "r"(packed[4 * e8 + 3])
+                     : "memory");
+        if (P == 2)
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + 2 * kTileBytes), "r"(rest[P == 2 ? 4 * e8 : 0]),
+                       "r"(rest[P == 2 ? 4 * e8 + 1 : 0]), "r"(rest[P == 2 ? 4 * e8 + 2 : 0]), "r"(rest[P == 2 ? 4 * e8 + 3 : 0])
+                       : "memory");
+      }
+    }
+    fence_async_smem();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(shready);
+  }
+  mbar_wait(odone, (njb - 1) & 1, ctl, &g_status, kErrWaitMma);
   tc_fence_after();
   {
     // lane = query now: each warpgroup stores half of the output columns of row `row`, 32 at a time
@@ -768,6 +1000,7 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) forward_main_kernel
       }
     }
     if (i < g.tq && wg == 0) ssum[(int64_t)n * g.tq + i] = rs;
+  }
   }
   drain_if_aborted(ctl);
   tc_fence_before();
@@ -1730,10 +1963,15 @@ inline int forward_main(const void* q, const void* k, const void* v, const Geom&
   static_assert(2 * (smem + 1024) <= 233472 && 3 * (smem + 1024) > 233472, "exactly two CTAs of the main pass fit one SM");
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
   const unsigned grid = (unsigned)(g.n * nqb);
-  DIL_TC_PLAIN_BID(g, DIL_TC_SHARE(g, {
-    if (int rc = set_smem_attr((const void*)forward_main_kernel<BID, SHARE>, smem, err, errlen)) return rc;
-    forward_main_kernel<BID, SHARE><<<grid, 256, smem, st>>>(mq, mk, mv, g, rmax, rden, carry, carry_base, out, ssum);
-  }))
+  auto launch = [&](auto kern, int threads) -> int {
+    if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
+    kern<<<grid, threads, smem, st>>>(mq, mk, mv, g, rmax, rden, carry, carry_base, out, ssum);
+    return 0;
+  };
+  DIL_TC_SHARE(g, {
+    if (int rc = g.bid == kBidSigmoid ? launch(forward_main_async_kernel<kBidSigmoid, SHARE>, kMainThreads)
+                                      : launch(forward_main_kernel<kBidSoftmax, SHARE>, 256)) return rc;
+  })
   return launch_status("tc forward_main", err, errlen);
 }
 

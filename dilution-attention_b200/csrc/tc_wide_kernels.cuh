@@ -526,10 +526,10 @@ inline int wide_forward(const void* q, const void* k, const void* v, const Geom&
   {
     constexpr int smem = kMainSmem<W>;
     static_assert(smem <= 232448 && 2 * smem > 233472, "one CTA (512 TMEM columns) per SM");
-    auto kern = forward_main_kernel<kBidSoftmax, kShareInclusive, W>;
+    auto kern = forward_main_async_kernel<kBidSoftmax, kShareInclusive, W>;
     if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
     mark("tc_wide_forward_main", st, 0);
-    kern<<<grid, 256, smem, st>>>(m.q, m.k, m.v, g, rmax, rden, carry, nullptr, out, ssum);
+    kern<<<grid, kMainThreads, smem, st>>>(m.q, m.k, m.v, g, rmax, rden, carry, nullptr, out, ssum);
     mark("tc_wide_forward_main", st, 1);
   }
   return launch_status("tc wide forward_main", err, errlen);
@@ -611,9 +611,9 @@ inline int mass_forward_main(const void* q, const void* k, const void* v, const 
   static_assert(smem <= 232448 && 2 * smem > 233472, "one CTA (512 TMEM columns) per SM");
   const unsigned grid = (unsigned)(g.n * ((g.tq + kTileRows - 1) / kTileRows));
   DIL_TC_MASS_BID(g, DIL_TC_SHARE(g, {
-    auto kern = forward_main_kernel<BID, SHARE, kPairs64>;
+    auto kern = forward_main_async_kernel<BID, SHARE, kPairs64>;
     if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
-    kern<<<grid, 256, smem, st>>>(mq, mk, mv, g, rmax, rden, carry, nullptr, out, ssum);
+    kern<<<grid, kMainThreads, smem, st>>>(mq, mk, mv, g, rmax, rden, carry, nullptr, out, ssum);
   }))
   return launch_status("tc forward_main", err, errlen);
 }
