@@ -49,7 +49,8 @@ HAS_CUDA_LIB = _lib.available()
 # correction pass recomputes the query half.
 TC_SAVE_PK = os.environ.get("DILUTION_SAVE_PK", "1") != "0"
 # Training forward on the tensor-core path: one key-stationary sweep for passes 2 and 3
-# (dilution_forward_fused) instead of the column-sum pass plus the query-stationary main pass.
+# (dilution_forward_fused) instead of the column-sum pass plus the query-stationary main pass, which short rows keep
+# (_short_rows).
 TC_FUSED_FORWARD = os.environ.get("DILUTION_FUSED_FORWARD", "1") != "0"
 
 
@@ -93,6 +94,16 @@ def _prepare(q, k, v, dot_precision):
     return ops, code, _lib.PREC[dot_precision], n
 
 
+def _short_rows(n, seq):
+    """Training forwards that take the column-sum and main passes instead of the fused sweep.  The sweep owns
+    256 keys per block: a short row is mostly diagonal blocks, and the output that it adds up in memory is zeroed,
+    reduced into and divided once per row of few tiles.  Passes 2 and 3 of a call, fused sweep with its division against
+    two passes: n = 384, T = 1024 327 / 295 us, n = 16, T = 1777 79 / 69, n = 256, T = 2048 639 / 607; n = 64, T = 4096
+    521 / 528; n = 64, T = 16384 7.66 / 8.06 ms.  With fewer than 74 super-blocks (half of the SMs) the host's launches
+    outlast either."""
+    return seq <= 2048 and n * -(-seq // 256) >= 74
+
+
 def _forward_rows(lib, qf, kf, vf, code, prec, scale, out, ssum, rmax, rden, carry, total, pk,
                   carry_rows, q_offset=0, carry_base=None):
     """Passes 1-3 on a slab of (batch*head) rows.  On the tensor-core path a requested pk comes
@@ -109,7 +120,7 @@ def _forward_rows(lib, qf, kf, vf, code, prec, scale, out, ssum, rmax, rden, car
         _lib.check(lib.dilution_rowstats(qf.data_ptr(), kf.data_ptr(), code, prec, n, tq, tk, q_offset,
                                          d, scale, rmax.data_ptr(), rden.data_ptr(), st), "dilution_rowstats")
     if (TC_FUSED_FORWARD and carry_rows == 32 and carry_base is None and q_offset == 0 and tq == tk
-            and _lib.tensor_core_path(code, prec, d)):
+            and _lib.tensor_core_path(code, prec, d) and not _short_rows(n, tq)):
         _lib.check(lib.dilution_forward_fused(qf.data_ptr(), kf.data_ptr(), vf.data_ptr(), code, prec, n, tq, d,
                                               scale, EPS, rmax.data_ptr(), rden.data_ptr(), carry.data_ptr(),
                                               total.data_ptr(), out.data_ptr(), ssum.data_ptr(), st),
