@@ -1177,6 +1177,20 @@ __device__ __forceinline__ void reverse_sweeps(float (&vs)[32], float (&vd)[32],
   }
 }
 
+// x[l] summed over the warp, in lane l: each of the five steps halves the values that a lane holds (31 shuffles for 32
+// sums).  Overwrites x.
+__device__ __forceinline__ float sum_over_lanes(float (&x)[32], int lane) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+    for (int e = 0; e < o; ++e) {
+      const float give = lane & o ? x[e] : x[e + o], mine = lane & o ? x[e + o] : x[e];
+      x[e] = mine + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  return x[0];
+}
+
 // Main reverse pass (the reference's BA, kernels.py:677-775).  grid = n * ceil(t/128),
 // key blocks with the most query blocks first; one CTA per SM, three warpgroups: two of
 // compute warps and one whose first thread issues every TMA copy and every MMA and whose
@@ -1530,18 +1544,11 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
       const float fix = wg == 1 ? rother : 0.f;
       sigma = R + rother;                              // the suffix behind the next half-step
       if (PASS == 1) {
-        // p * dp summed over the warp's 32 keys: each step halves the queries a lane holds, lane l ends with query l
+        // p * dp summed over the warp's 32 keys
 #pragma unroll
         for (int e = 0; e < 32; ++e) vd[e] = fmaf(vs[e], fix, vd[e]);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-          for (int e = 0; e < o; ++e) {
-            const float give = lane & o ? vd[e] : vd[e + o], mine = lane & o ? vd[e + o] : vd[e];
-            vd[e] = mine + __shfl_xor_sync(0xffffffffu, give, o);
-          }
-        }
-        if (iq0 + lane < g.tq) atomicAdd(ghat + row_base + iq0 + lane, vd[0]);
+        const float sum = sum_over_lanes(vd, lane);
+        if (iq0 + lane < g.tq) atomicAdd(ghat + row_base + iq0 + lane, sum);
       } else {
         // the dQ MMAs of the previous 128 queries read the pdp buffer that is written next
         if (!odd && s >= 1) mbar_wait(dqdone, (s - 1) & 1, ctl, &g_status, kErrWaitMma);

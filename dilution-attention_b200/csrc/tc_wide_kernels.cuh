@@ -11,8 +11,8 @@
 // narrow one's accumulators would need 656 of the 512 TMEM columns.
 //
 // Forward + backward at B4 H8 T4096 on one B200, before (tile kernels with tf32 products) and after:
-//   bf16 d = 128  14.8 ms -> 2.18 ms  (reverse pass 7.24 -> 1.12, main pass 3.82 -> 0.39)
-//   fp32 d = 64    7.1 ms -> 2.06 ms  (reverse pass 3.51 -> 0.93, main pass 1.61 -> 0.39)
+//   bf16 d = 128  14.8 ms -> 1.93 ms  (reverse pass 7.24 -> 0.94, main pass 3.82 -> 0.31)
+//   fp32 d = 64    7.1 ms -> 1.84 ms  (reverse pass 3.51 -> 0.81, main pass 1.61 -> 0.31)
 // (with single bf16 values bf16 d = 128 takes 1.64 ms, its outputs 1.0e-3 off).  Against 64 bits, 2-norm: bf16 outputs
 // 1.3e-4 -> 1.6e-6, gradients 1.7e-3 before and after (their own rounding to bf16); fp32 outputs 2.8e-4 -> about 1e-5.
 #pragma once
@@ -119,7 +119,7 @@ __global__ void split_dq_from_pk_kernel(const float* __restrict__ dq_main, const
 
 // Main reverse pass over wide rows: the arithmetic of backward_main_kernel (two compute warpgroups, lane =
 // key, two threads per key and half-step of 64 queries, reverse_sweeps), 384 threads, one CTA per SM.
-//   TMEM, all 512 columns: S^T 64 | dOV^T 64 | dV 128 | dK 128 | dQ^T 64 | ghat^T 64.
+//   TMEM: S^T 64 | dOV^T 64 | dV 128 | dK 128 | dQ^T 64.
 // What differs from the narrow kernel, and why:
 //  * one stage of scores instead of two (dV and dK take 256 columns): the scores of half-step h + 1 are issued right
 //    behind the dV and dK products of h, which read the share and pdp values stored over the scores of h;
@@ -128,7 +128,10 @@ __global__ void split_dq_from_pk_kernel(const float* __restrict__ dq_main, const
 //    thread of the read-out (lane = feature) writes one fp32 column of the [query][32 features] staging
 //    tile of its warp, 128 consecutive bytes per warp and store;
 //  * V stays in shared memory (as a TMEM operand it would take 64 columns);
-//  * ghat^T = 1^T pdp is a product of its own against a 4 KB tile of ones.
+//  * ghat, the sum of pdp over keys, is formed by shuffles in fp32 once the half-step's tiles are handed over, while
+//    the compute warps would wait for the next scores (as a product of its own against a tile of ones it was 16 of
+//    the 76 MMAs of a kWide128 half-step, each about 50 cycles of the issuing thread: 1.11 -> 0.94 ms, kSplit 0.92 ->
+//    0.81 ms, n = 32, T = 4096).
 // kSplit multiplies hi and lo planes of share and pdp (two A operands side by side in TMEM, two pdp tiles),
 // and dQ^T rows 64..127 (K_lo) are reduced into the same columns of dq_main as rows 0..63.
 //  * kWide128 stages 32 queries of dQ at a time (16 KB instead of 32): its do' takes 64 KB.
@@ -137,7 +140,7 @@ __global__ void split_dq_from_pk_kernel(const float* __restrict__ dq_main, const
 // behind K, are not used.
 template <int W> constexpr int kDqRows = W == kWide128 ? 32 : 64;
 template <int W> constexpr int kBwdWideSmem =
-    3 * (int)Rows<W>::kBytes + (Rows<W>::kDoSub + Rows<W>::kPlanes) * (int)kTileBytes + kDqRows<W> * 512 + 4096 + 1024 +
+    3 * (int)Rows<W>::kBytes + (Rows<W>::kDoSub + Rows<W>::kPlanes) * (int)kTileBytes + kDqRows<W> * 512 + 1024 +
     2048 + 512 + 256 + 1024;
 
 template <int W, typename TOut, int BID = kBidSoftmax, int SHARE = kShareInclusive, int PASS = 0>
@@ -160,12 +163,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
   const uint32_t sQ0 = sK + 2 * TB, sD0 = sQ0 + 2 * HB;        // [2] stages each
   const uint32_t sPd = sD0 + 2 * HBd;                          // [P][128 keys][64 queries] bf16
   const uint32_t sDq = sPd + P * kTileBytes;                   // [4 warps][kDqRows queries][32 features] fp32
-  const uint32_t sOnes = sDq + kDqRows<W> * 512;
-  uint8_t* tail = smem + (sOnes - sK);                         // the ones tile
-  float* sLse = reinterpret_cast<float*>(tail + 4096);         // [2][64]
+  float* sLse = reinterpret_cast<float*>(smem + (sDq - sK) + kDqRows<W> * 512);   // [2][64]
   float* sDbar = sLse + 128;                                   // [2][64]
   float* sG = sDbar + 128;                                     // [2][2][128] sums of dk_share
-  float* sGh = sG + 512;                                       // [64]; PASS 2: [2][64] ghat of the queries
+  float* sGh = sG + 512;                                       // PASS 2: [2][64] ghat of the queries
   uint64_t* bars = reinterpret_cast<uint64_t*>(sGh + 128);
   Ctl* ctl = reinterpret_cast<Ctl*>(bars + 12);
   const uint32_t kfull = smem_u32(bars), qfull = smem_u32(bars + 1);           // qfull[2]
@@ -206,17 +207,12 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
       sDbar[row] = db;
       if (PASS == 2) sGh[row] = gh;
     }
-  } else if (wg == 1) {
-    const uint4 one = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
-    reinterpret_cast<uint4*>(tail)[row] = one;
-    reinterpret_cast<uint4*>(tail)[row + 128] = one;
   }
-  fence_async_smem();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = ctl->tmem;
-  const uint32_t tS = tmem, tDOV = tmem + 64, tDV = tmem + 128, tDK = tmem + 256, tDQ = tmem + 384, tG = tmem + 448;
+  const uint32_t tS = tmem, tDOV = tmem + 64, tDV = tmem + 128, tDK = tmem + 256, tDQ = tmem + 384;
   const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
   if (wg < 2) {
     // dV and dK start from zero, so that every MMA into them accumulates
@@ -249,9 +245,9 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
     asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");
     constexpr uint32_t id_s = instr_desc(128, 64, 0, 0);     // scores: both operands K-major
     constexpr uint32_t id_kd = instr_desc(128, Rows<W>::kCols, 0, 1);   // dV, dK: A from TMEM (M = keys), B MN-major
-    constexpr uint32_t id_qd = instr_desc(128, 64, 1, 1);    // dQ^T, ghat^T: A and B MN-major
+    constexpr uint32_t id_qd = instr_desc(128, 64, 1, 1);    // dQ^T: A and B MN-major
     const Desc dKk = make_desc(sK, 16, 1024), dVk = make_desc(sV, 16, 1024);
-    const Desc dKm = make_desc(sK, kTileBytes, 1024), dOnes = make_desc(sOnes, 2048, 1024);
+    const Desc dKm = make_desc(sK, kTileBytes, 1024);
     const Desc dPm = make_desc(sPd, kTileBytes, 1024);
     auto issue_scores = [&](int h) {
       const int st = h & 1;
@@ -291,10 +287,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
 #pragma unroll
         for (int pl = 0; pl < P; ++pl)
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk) {                    // contraction over the 128 keys
+          for (int kk = 0; kk < 8; ++kk)                      // contraction over the 128 keys
             mma_ss(tDQ, dKm, 128 * kk, dPm, 1024 * pl + 128 * kk, id_qd, (pl > 0 || kk > 0));
-            if (PASS == 0) mma_ss(tG, dOnes, 0, dPm, 1024 * pl + 128 * kk, id_qd, (pl > 0 || kk > 0));
-          }
         mma_commit(dqdone);
         if (h + 2 < nhalf) {
           // the products that read this stage come before the scores of h + 1, whose commit covers them
@@ -303,7 +297,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
         }
       }
       __syncwarp();
-      // dQ^T and ghat^T of the half-step's 64 queries: lane = feature.  Each warp stages its 32 features and
+      // dQ^T of the half-step's 64 queries: lane = feature.  Each warp stages its 32 features and
       // adds them to dq_main with one tensor reduction.
       if (lane == 0) mbar_wait(dqdone, h & 1, ctl, &g_status, kErrWaitMma);
       __syncwarp();
@@ -331,22 +325,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
           if (lane == 0 && qr < g.tq)                   // a reduction never starts behind the last row
             tma_reduce_add_tile(&map_dq, stage, W == kSplit ? 32 * (w4 & 1) : 32 * w4, qr, n);
         }
-      }
-      if (PASS == 0 && w4 == 0) {                       // every lane of ghat^T holds the same 64 sums
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          float x[32];
-          tmem_ld32(tG + lane_base + 32 * c, x);
-          tmem_ld_wait(x);
-          if (lane == 0) {
-#pragma unroll
-            for (int e = 0; e < 32; e += 4)
-              *reinterpret_cast<float4*>(sGh + 32 * c + e) = make_float4(x[e], x[e + 1], x[e + 2], x[e + 3]);
-          }
-        }
-        __syncwarp();
-        for (int q = lane; q < 64; q += 32)
-          if (q0 + q < g.tq) atomicAdd(ghat + row_base + q0 + q, sGh[q]);
       }
       tc_fence_before();
       __syncwarp();
@@ -412,11 +390,13 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
           for (int u = 0; u < 4; ++u) {
             const int e = e8 * 8 + 2 * u;
             const float2 f2 = fma2(make_float2(vs[e], vs[e + 1]), make_float2(fix, fix), make_float2(vd[e], vd[e + 1]));
+            vd[e] = f2.x;
+            vd[e + 1] = f2.y;
             pdt[e8 * 4 + u] = pack_bf16(f2.x, f2.y);
             pdt[16 + e8 * 4 + u] = pack_bf16_rest(f2.x, f2.y, pdt[e8 * 4 + u]);
           }
 #pragma unroll
-          for (int pl = 0; pl < P; ++pl) {              // [key][query]: the MN-major B operand of dQ^T and ghat^T
+          for (int pl = 0; pl < P; ++pl) {              // [key][query]: the MN-major B operand of dQ^T
             const uint32_t* w = pdt + 16 * pl + 4 * e8;
             asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sPd + kTileBytes * pl + share_chunk_offset(row, cw + e8 * 8)),
                          "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
@@ -438,6 +418,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(tiles);
+      if (PASS == 0) {
+        const float sum = sum_over_lanes(vd, lane);
+        if (iq0 + lane < g.tq) atomicAdd(ghat + row_base + iq0 + lane, sum);
+      }
     }
   }
   mbar_wait(sdone, nhalf & 1, ctl, &g_status, kErrWaitMma);
@@ -595,8 +579,8 @@ inline int wide_backward(const void* q, const void* k, const void* v, const Geom
 
 // ---------------------------------------------------------------- f(a) / rowsum(f) bids of bf16 heads of 64
 // relu, relu2, softplus.  The row mass and the column sums only need scores and run on the narrow kernels.
-// softplus / inclusive at B4 H8 T8192, forward + backward on one B200: 39.2 ms on the tile kernels -> 7.5 ms (row mass
-// 0.54, column sums 0.67, main pass 2.2, ghat 1.6, reverse pass 3.1); outputs 1.3e-4 -> 1.5e-6 off 64 bits (2-norm),
+// softplus / inclusive at B4 H8 T8192, forward + backward on one B200: 39.2 ms on the tile kernels -> 7.2 ms (row mass
+// 0.54, column sums 0.67, main pass 1.26, ghat 1.6, reverse pass 3.1); outputs 1.3e-4 -> 1.5e-6 off 64 bits (2-norm),
 // gradients 1.7e-3 before and after.  Bound by the special-function unit (four operations per score in the reverse
 // passes, three in the main pass) and, with one CTA per SM in the two product passes, by the hand-over between scores,
 // arithmetic and products.
