@@ -7,6 +7,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <algorithm>
 #include <vector>
 
 #include "../../include/dilution_b200.h"
@@ -294,6 +295,16 @@ int decode_chunk(int64_t n, int64_t len) {
   while ((len + chunk - 1) / chunk > dil::decode::MAX_CHUNKS) chunk *= 2;
   return (int)chunk;
 }
+// How many CTAs per row a step of n rows and `len` keys takes as one launch of clusters (cluster_step_kernel), 0 for the
+// three launches.  A CTA per 256 keys, at most eight; up to two CTAs per SM and 128 KB of either cache per CTA.
+// GPU time of a step in a CUDA graph, one launch against three: 16 rows of 3001 keys (bf16, 64) 7.2 / 9.3 us, 64 x 1024
+// 6.4 / 8.8, 1 x 32 5.1 / 6.7, 16 x 4096 (bf16, 128) 10.8 / 11.1; behind the line 64 x 2048 13.5 / 10.8, 256 x 2048
+// 42.5 / 33.9, 1 x 8192 (bf16, 128) 13.5 / 10.4: more CTAs wait for each other's clusters, longer chunks for memory.
+int cluster_ctas(int64_t n, int64_t len, int64_t row_bytes) {
+  const int64_t c = std::min<int64_t>(dil::decode::kClusterMax, (len + dil::decode::ROUND - 1) / dil::decode::ROUND);
+  const int64_t keys = (len + c - 1) / c;
+  return n * c <= 2 * 148 && keys <= dil::decode::kClusterKeys && keys * row_bytes <= 128 * 1024 ? (int)c : 0;
+}
 int64_t decode_stride(int64_t len) { return (len + 31) / 32 * 32; }
 
 dil::decode::Scratch carve_decode(void* scratch, int64_t n, int64_t len, int d) {
@@ -319,6 +330,28 @@ int launch_decode(const void* q1, const void* kc, const void* vc, int64_t n, int
   // with the length on the device (pos_dev) the launch geometry cannot follow it: the grid, the
   // chunking and the scratch layout are those of a full cache
   const int64_t geo = pos_dev != nullptr ? cap : len;
+  if constexpr (MODE != kSweepVariant) {
+    if (const int C = cluster_ctas(n, geo, sizeof(T) * D)) {
+      const int keys = (int)((geo + C - 1) / C + 31) / 32 * 32;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)C, (unsigned)n);
+      cfg.blockDim = dim3(NT);
+      cfg.stream = st;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = (unsigned)C;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      Prof prof("decode_scores", st, timing);      // the name that a step has always begun with
+      const cudaError_t e = cudaLaunchKernelEx(
+          &cfg, cluster_step_kernel<T, D, MODE>, (const T*)q1, (const T*)kc, (const T*)vc, cap, (int)len, keys,
+          scale * dil::kLog2e, eps, committed, (const T*)knew, (const T*)vnew, (T*)const_cast<void*>(kc),
+          (T*)const_cast<void*>(vc), (T*)out, pos_dev);
+      if (e != cudaSuccess) return fail(DILUTION_ERR_CUDA, "decode step: %s", cudaGetErrorString(e));
+      return check_launch("decode step");
+    }
+  }
   const int chunk = decode_chunk(n, geo);
   const int nch = (int)((geo + chunk - 1) / chunk);
   const Scratch s = carve_decode(scratch, n, geo, D);
