@@ -181,6 +181,32 @@ int launch_colsum(const void* q, const void* k, const dil::Geom& g, const float*
   return check_launch("colsum_scan");
 }
 
+// CTAs per block of the FFMA passes (Part in simt_kernels.cuh): the largest power of two up to 8 that keeps the
+// grid within two CTAs per SM and leaves every rank a tile of the longest block.
+int split_of(unsigned grid, int tiles) {
+  int s = 8;
+  while (s > 1 && (grid * (unsigned)s > 2 * 148 || s > tiles)) s /= 2;
+  return s;
+}
+template <typename K, typename... A>
+int launch_split(K kern, unsigned grid, int split, size_t smem, cudaStream_t st, A... args) {
+  if (int rc = set_smem(kern, smem)) return rc;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid * (unsigned)split);
+  cfg.blockDim = dim3(dil::simt::NT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)split;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
+  if (e != cudaSuccess) return fail(DILUTION_ERR_CUDA, "cluster launch: %s", cudaGetErrorString(e));
+  return check_launch("cluster launch");
+}
+
 template <typename T, int D, bool MMA>
 int launch_main(const void* q, const void* k, const void* v, const dil::Geom& g, const float* rmax,
                 const float* rden, const float* carry, const float* base, float* out, float* ssum,
@@ -189,17 +215,14 @@ int launch_main(const void* q, const void* k, const void* v, const dil::Geom& g,
   const int nqb = (g.tq + TS - 1) / TS;
   const unsigned grid = (unsigned)(g.n * nqb);
   Prof prof("simt_forward_main", st);
-  if (pk) {
-    auto kern = main_kernel<T, D, true, MMA>;
-    if (int rc = set_smem(kern, smem_main<D>())) return rc;
-    kern<<<grid, NT, smem_main<D>(), st>>>((const T*)q, (const T*)k, (const T*)v, g, rmax, rden,
-                                            carry, base, out, ssum, pk);
-  } else {
-    auto kern = main_kernel<T, D, false, MMA>;
-    if (int rc = set_smem(kern, smem_main<D>())) return rc;
-    kern<<<grid, NT, smem_main<D>(), st>>>((const T*)q, (const T*)k, (const T*)v, g, rmax, rden,
-                                            carry, base, out, ssum, nullptr);
+  if (const int split = MMA ? 1 : split_of(grid, nqb); split > 1) {
+    auto kern = pk ? main_kernel<T, D, true, false, true> : main_kernel<T, D, false, false, true>;
+    return launch_split(kern, grid, split, smem_main<D>(), st, (const T*)q, (const T*)k, (const T*)v, g, rmax, rden, carry,
+                        base, out, ssum, pk, split);
   }
+  auto kern = pk ? main_kernel<T, D, true, MMA> : main_kernel<T, D, false, MMA>;
+  if (int rc = set_smem(kern, smem_main<D>())) return rc;
+  kern<<<grid, NT, smem_main<D>(), st>>>((const T*)q, (const T*)k, (const T*)v, g, rmax, rden, carry, base, out, ssum, pk, 1);
   return check_launch("forward_main");
 }
 
@@ -244,6 +267,7 @@ int launch_backward(const void* q, const void* k, const void* v, const dil::Geom
   if (int rc = check_launch("dbar")) return rc;
   const int nkb = (g.tk + TS - 1) / TS;
   const unsigned grid = (unsigned)(g.n * nkb);
+  const int split = MMA ? 1 : split_of(grid, nkb);
   // an f(a) / rowsum(f) bid under a share step: its Jacobian factor 1 / (row mass) is unbounded, so
   // ghat is found first and subtracted before the factor multiplies (two sweeps, as the reference's
   // B1-B2 then B4, kernels_bid.py:513-612, 659-728); everything else: one sweep, correction afterwards
@@ -255,9 +279,15 @@ int launch_backward(const void* q, const void* k, const void* v, const dil::Geom
     if (int rc = set_smem(kern, smem_bwd_main<D>())) return rc;
     {
       Prof prof(sweep == 1 ? "simt_backward_ghat" : "simt_backward_main", st);
-      kern<<<grid, NT, smem_bwd_main<D>(), st>>>((const T*)q, (const T*)k, (const T*)v, gs, dout, s.dbar,
-                                                  ssum, rmax, rden, carry, s.dq_main, s.dk_main,
-                                                  (T*)dv, s.ghat);
+      if (split > 1) {
+        if (int rc = launch_split(backward_main_kernel<T, D, false, true>, grid, split, smem_bwd_main<D>(), st, (const T*)q,
+                                  (const T*)k, (const T*)v, gs, dout, s.dbar, ssum, rmax, rden, carry, s.dq_main, s.dk_main,
+                                  (T*)dv, s.ghat, split)) return rc;
+      } else {
+        kern<<<grid, NT, smem_bwd_main<D>(), st>>>((const T*)q, (const T*)k, (const T*)v, gs, dout, s.dbar,
+                                                    ssum, rmax, rden, carry, s.dq_main, s.dk_main,
+                                                    (T*)dv, s.ghat, 1);
+      }
     }
     if (int rc = check_launch("backward_main")) return rc;
   }
@@ -269,8 +299,13 @@ int launch_backward(const void* q, const void* k, const void* v, const dil::Geom
     if (int rc = set_smem(kern, smem_bwd_dk<D>())) return rc;
     {
       Prof prof("simt_backward_dk_correction", st);
-      kern<<<grid, NT, smem_bwd_dk<D>(), st>>>((const T*)q, (const T*)k, g, rmax, rden, s.ghat,
-                                                s.dk_main, (T*)dk);
+      if (split > 1) {
+        if (int rc = launch_split(backward_dk_correction_kernel<T, D, false, true>, grid, split, smem_bwd_dk<D>(), st,
+                                  (const T*)q, (const T*)k, g, rmax, rden, s.ghat, s.dk_main, (T*)dk, split)) return rc;
+      } else {
+        kern<<<grid, NT, smem_bwd_dk<D>(), st>>>((const T*)q, (const T*)k, g, rmax, rden, s.ghat,
+                                                  s.dk_main, (T*)dk, 1);
+      }
     }
     if (int rc = check_launch("backward_dk_correction")) return rc;
   } else {

@@ -98,6 +98,20 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   return r;
 }
 
+// Barrier of every thread of the cluster; what was written before it is visible behind it.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// A float of CTA `rank`'s shared memory, by its address in this CTA's.
+__device__ __forceinline__ float ld_cluster(const float* p, int rank) {
+  uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(r) : "memory");
+  return v;
+}
+
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));

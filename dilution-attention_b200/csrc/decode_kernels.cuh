@@ -361,18 +361,6 @@ __global__ void __launch_bounds__(NT) sweep_kernel(const T* __restrict__ vc, int
 constexpr int kClusterMax = 8;
 constexpr int kClusterKeys = 1024;           // keys of one CTA: its scores and their V rows' shares
 
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// A float of CTA `rank`'s shared memory, by its address in this CTA's.
-__device__ __forceinline__ float ld_cluster(const float* p, int rank) {
-  uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
-  float v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(r) : "memory");
-  return v;
-}
 
 // grid = (C, n), clusters of (C, 1); `chunk` = keys of a CTA, at most kClusterKeys.
 template <typename T, int D, int MODE>
