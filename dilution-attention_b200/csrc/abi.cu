@@ -892,7 +892,7 @@ int dilution_softmax_decode_append(const void* q1, const void* k1, const void* v
 // ---- share / bid variants (kernels_bid.py of the reference) -------------
 #ifdef DILUTION_TENSOR_PATH
 // bf16 heads of 64 under "bf16" take the tcgen05 kernels; of the f(a) / rowsum(f) bids the three whose f needs no row
-// minimum, from kMassMinSeq tokens on: 780 -> 213 us forward + backward at n = 32, t = 1024 (softplus), 39.2 -> 7.5 ms
+// minimum, from kMassMinSeq tokens on: 780 -> 213 us forward + backward at n = 32, t = 1024 (softplus), 39.2 -> 7.1 ms
 // at t = 8192.  Shorter rows would gain too (tile kernels 350 us at n = 4, t = 512; the host's launches are 200 us of
 // either), but up to 520 tokens the tests hold them to the tile kernels' route; the line is the next tile boundary that
 // leaves that contract alone.

@@ -132,16 +132,20 @@ __global__ void split_dq_from_pk_kernel(const float* __restrict__ dq_main, const
 //    the compute warps would wait for the next scores (as a product of its own against a tile of ones it was 16 of
 //    the 76 MMAs of a kWide128 half-step, each about 50 cycles of the issuing thread: 1.11 -> 0.94 ms, kSplit 0.92 ->
 //    0.81 ms, n = 32, T = 4096).
-// kSplit multiplies hi and lo planes of share and pdp (two A operands side by side in TMEM, two pdp tiles),
-// and dQ^T rows 64..127 (K_lo) are reduced into the same columns of dq_main as rows 0..63.
+//  * share and pdp are multiplied as hi and lo planes (two A operands side by side in TMEM, two pdp tiles); for kSplit
+//    dQ^T rows 64..127 (K_lo) are reduced into the same columns of dq_main as rows 0..63;
 //  * kWide128 stages 32 queries of dQ at a time (16 KB instead of 32): its do' takes 64 KB.
 // kPairs64 serves pass 2 of the f(a) / rowsum(f) bids: ghat (of backward_main_kernel's pass 1) is subtracted before the
 // factor multiplies, dk is final (written as TOut to dk_main), and rows 64..127 of dQ^T, whose A operand is the V tile
 // behind K, are not used.
 template <int W> constexpr int kDqRows = W == kWide128 ? 32 : 64;
+// Its accumulators leave TMEM for two stages of scores, so the products of a half-step and the scores of the next but one
+// run under the arithmetic of the next (with one stage the softplus pass at n = 32, T = 8192 took 3.12 ms, now 2.99).
+template <int W> constexpr int kScoreStages = W == kPairs64 ? 2 : 1;
+template <int W> constexpr int kRowStages = 2 * kScoreStages<W>;          // half-steps of q and do' in shared memory
 template <int W> constexpr int kBwdWideSmem =
-    3 * (int)Rows<W>::kBytes + (Rows<W>::kDoSub + Rows<W>::kPlanes) * (int)kTileBytes + kDqRows<W> * 512 + 1024 +
-    2048 + 512 + 256 + 1024;
+    2 * (int)Rows<W>::kBytes + kRowStages<W> * (Rows<W>::kSub + Rows<W>::kDoSub) * (int)kTileBytes / 2 +
+    Rows<W>::kPlanes * (int)kTileBytes + kDqRows<W> * 512 + 2048 + 2048 + 1024 + 256 + 1024;
 
 template <int W, typename TOut, int BID = kBidSoftmax, int SHARE = kShareInclusive, int PASS = 0>
 __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
@@ -160,17 +164,18 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
   const uint32_t sK = smem_u32(smem), sV = sK + TB;
-  const uint32_t sQ0 = sK + 2 * TB, sD0 = sQ0 + 2 * HB;        // [2] stages each
-  const uint32_t sPd = sD0 + 2 * HBd;                          // [P][128 keys][64 queries] bf16
+  constexpr int NS = kScoreStages<W>, NR = kRowStages<W>;
+  const uint32_t sQ0 = sK + 2 * TB, sD0 = sQ0 + NR * HB;       // [NR] stages each
+  const uint32_t sPd = sD0 + NR * HBd;                         // [P][128 keys][64 queries] bf16
   const uint32_t sDq = sPd + P * kTileBytes;                   // [4 warps][kDqRows queries][32 features] fp32
-  float* sLse = reinterpret_cast<float*>(smem + (sDq - sK) + kDqRows<W> * 512);   // [2][64]
-  float* sDbar = sLse + 128;                                   // [2][64]
-  float* sG = sDbar + 128;                                     // [2][2][128] sums of dk_share
-  float* sGh = sG + 512;                                       // PASS 2: [2][64] ghat of the queries
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sGh + 128);
+  float* sLse = reinterpret_cast<float*>(smem + (sDq - sK) + kDqRows<W> * 512);   // [4][64]
+  float* sDbar = sLse + 256;                                   // [4][64]
+  float* sG = sDbar + 256;                                     // [2][2][128] sums of dk_share
+  float* sGh = sG + 512;                                       // PASS 2: [4][64] ghat of the queries
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sGh + 256);
   Ctl* ctl = reinterpret_cast<Ctl*>(bars + 12);
-  const uint32_t kfull = smem_u32(bars), qfull = smem_u32(bars + 1);           // qfull[2]
-  const uint32_t sdone = smem_u32(bars + 3), tiles = smem_u32(bars + 4), dqdone = smem_u32(bars + 5);
+  const uint32_t kfull = smem_u32(bars), qfull = smem_u32(bars + 1);           // qfull[4]
+  const uint32_t sdone = smem_u32(bars + 5), tiles = smem_u32(bars + 7), dqdone = smem_u32(bars + 9);   // [2], [2]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wg = tid >> 7, row = tid & 127;
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
@@ -183,8 +188,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
   const int ja = k0 + row;
   const bool dead = ja >= g.tk;
 
-  auto load_stats = [&](int hb, float* lse, float* dbar, float* gh) {      // of query 64 hb + row, row < 64
-    const int i = hb * 64 + row;
+  auto load_stats = [&](int hb, float* lse, float* dbar, float* gh) {      // of query 64 hb + row % 64
+    const int i = hb * 64 + (row & 63);
     *lse = load_lse<BID>(rmax, rden, row_base, i, g.tq, g.lshift);
     *dbar = i < g.tq ? dbarp[row_base + i] : 0.f;
     *gh = PASS == 2 && i < g.tq ? ghat[row_base + i] : 0.f;
@@ -192,27 +197,27 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
 
   if (tid == 0) {
     ctl->abort = 0;
-    for (int i = 0; i < 4; ++i) mbar_init(kfull + 8 * i, 1);      // kfull, qfull[2], sdone
+    for (int i = 0; i < 7; ++i) mbar_init(kfull + 8 * i, 1);      // kfull, qfull[4], sdone[2]
     mbar_init(tiles, 8);
+    mbar_init(tiles + 8, 8);
     mbar_init(dqdone, 1);
     fence_barrier_init();
   }
   __syncwarp();
   if (warp == 0) tmem_alloc(smem_u32(&ctl->tmem), 512);
-  if (wg == 0) {
-    if (row < 64) {
-      float l, db, gh;
-      load_stats(2 * nqb - 1, &l, &db, &gh);
-      sLse[row] = l;
-      sDbar[row] = db;
-      if (PASS == 2) sGh[row] = gh;
-    }
+  if (wg == 0) {                                     // of the first two half-steps (nhalf >= 2)
+    float l, db, gh;
+    load_stats(2 * nqb - 1 - (row >> 6), &l, &db, &gh);
+    sLse[row] = l;
+    sDbar[row] = db;
+    if (PASS == 2) sGh[row] = gh;
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = ctl->tmem;
-  const uint32_t tS = tmem, tDOV = tmem + 64, tDV = tmem + 128, tDK = tmem + 256, tDQ = tmem + 384;
+  // score stage s at tS + 128 s and tDOV + 128 s
+  const uint32_t tS = tmem, tDOV = tmem + 64, tDV = tmem + 128 * NS, tDK = tDV + Rows<W>::kCols, tDQ = tDK + Rows<W>::kCols;
   const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
   if (wg < 2) {
     // dV and dK start from zero, so that every MMA into them accumulates
@@ -220,11 +225,11 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
 #pragma unroll
     for (int c = 0; c < 16; ++c) z[c] = 0u;
 #pragma unroll
-    for (int c = 0; c < 8; ++c) tmem_st16((wg == 0 ? tDV : tDK) + lane_base + 16 * c, z);
+    for (int c = 0; c < Rows<W>::kCols / 16; ++c) tmem_st16((wg == 0 ? tDV : tDK) + lane_base + 16 * c, z);
     tmem_st_wait();
   }
   auto load_stage = [&](int h) {                     // thread 256: q and do' of half-step h
-    const int st = h & 1, r0 = (2 * nqb - 1 - h) * 64;
+    const int st = h % NR, r0 = (2 * nqb - 1 - h) * 64;
     mbar_expect_tx(qfull + 8 * st, HB + HBd);
     tma_load_rows<W>(sQ0 + HB * st, &map_q, r0, n, qfull + 8 * st, HSub);
     tma_load_rows<W, Rows<W>::kDoSub>(sD0 + HBd * st, &map_do, r0, n, qfull + 8 * st, HSub);
@@ -233,8 +238,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
     mbar_expect_tx(kfull, 2 * TB);
     tma_load_rows<W>(sK, &map_k, k0, n, kfull);
     tma_load_rows<W>(sV, &map_v, k0, n, kfull);
-    load_stage(0);
-    load_stage(1);
+    for (int h = 0; h < NR && h < nhalf; ++h) load_stage(h);
   }
   tc_fence_before();
   __syncthreads();
@@ -250,50 +254,55 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
     const Desc dKm = make_desc(sK, kTileBytes, 1024);
     const Desc dPm = make_desc(sPd, kTileBytes, 1024);
     auto issue_scores = [&](int h) {
-      const int st = h & 1;
-      mma_scores_wide<W>(tS, dKk, kTileBytes, make_desc(sQ0 + HB * st, 16, 1024), HSub, id_s);
-      mma_dov_wide<W>(tDOV, dVk, kTileBytes, make_desc(sD0 + HBd * st, 16, 1024), HSub, id_s);
+      const int st = h % NR;
+      const uint32_t col = NS == 2 ? 128 * (h & 1) : 0;
+      mbar_wait(qfull + 8 * st, (h / NR) & 1, ctl, &g_status, kErrWaitTma);
+      tc_fence_after();
+      mma_scores_wide<W>(tS + col, dKk, kTileBytes, make_desc(sQ0 + HB * st, 16, 1024), HSub, id_s);
+      mma_dov_wide<W>(tDOV + col, dVk, kTileBytes, make_desc(sD0 + HBd * st, 16, 1024), HSub, id_s);
     };
     if (tid == 256) {
       mbar_wait(kfull, 0, ctl, &g_status, kErrWaitTma);
-      mbar_wait(qfull, 0, ctl, &g_status, kErrWaitTma);
-      tc_fence_after();
-      issue_scores(0);
-      mma_commit(sdone);
+      for (int h = 0; h < NS; ++h) {
+        issue_scores(h);
+        mma_commit(sdone + 8 * h);
+      }
     }
     __syncwarp();
     for (int h = 0; h < nhalf; ++h) {
-      const int st = h & 1;
+      const int st = h % NR, sc = NS == 2 ? h & 1 : 0;      // stage of q and do', stage of the scores
       if (tid == 256) {
-        mbar_wait(tiles, h & 1, ctl, &g_status, kErrWaitTile);
+        mbar_wait(tiles + 8 * sc, (h / NS) & 1, ctl, &g_status, kErrWaitTile);
         tc_fence_after();
         const Desc dQm = make_desc(sQ0 + HB * st, HSub, 1024), dDm = make_desc(sD0 + HBd * st, HSub, 1024);
 #pragma unroll
         for (int pl = 0; pl < P; ++pl)
 #pragma unroll
           for (int kq = 0; kq < 4; ++kq) {                    // contraction over the 64 queries, 16 each
-            const uint32_t col = 32 * (kq >> 1) + 16 * pl + 8 * (kq & 1);
+            const uint32_t col = 128 * sc + 32 * (kq >> 1) + 16 * pl + 8 * (kq & 1);
             mma_ts(tDV, tS + col, dDm, 128 * kq, id_kd, 1);
             if (Rows<W>::kDoParts == 2 && pl == 0)            // share_hi do'_lo; share_lo do'_lo is left out (2^-18)
               mma_ts(tDV, tS + col, dDm, (HSub >> 4) * Rows<W>::kSub + 128 * kq, id_kd, 1);
             mma_ts(tDK, tDOV + col, dQm, 128 * kq, id_kd, 1);
           }
-        if (h + 1 < nhalf) {
-          mbar_wait(qfull + 8 * (st ^ 1), ((h + 1) >> 1) & 1, ctl, &g_status, kErrWaitTma);
-          tc_fence_after();
-          issue_scores(h + 1);
-        }
-        mma_commit(sdone);
+        if (h + NS < nhalf) issue_scores(h + NS);
+        mma_commit(sdone + 8 * sc);
 #pragma unroll
         for (int pl = 0; pl < P; ++pl)
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)                      // contraction over the 128 keys
             mma_ss(tDQ, dKm, 128 * kk, dPm, 1024 * pl + 128 * kk, id_qd, (pl > 0 || kk > 0));
         mma_commit(dqdone);
-        if (h + 2 < nhalf) {
-          // the products that read this stage come before the scores of h + 1, whose commit covers them
-          mbar_wait(sdone, (h + 1) & 1, ctl, &g_status, kErrWaitMma);
-          load_stage(h + 2);
+        if (NS == 1) {
+          if (h + 2 < nhalf) {
+            // the products that read this stage come before the scores of h + 1, whose commit covers them
+            mbar_wait(sdone, (h + 1) & 1, ctl, &g_status, kErrWaitMma);
+            load_stage(h + 2);
+          }
+        } else if (h >= 1 && h + 3 < nhalf) {
+          // the products of h - 1 have completed once the commit behind them has: their stage takes h + 3
+          mbar_wait(sdone + 8 * ((h - 1) & 1), ((h - 1) / 2 + 1) & 1, ctl, &g_status, kErrWaitMma);
+          load_stage(h + 3);
         }
       }
       __syncwarp();
@@ -348,21 +357,23 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
     const uint32_t tcol = lane_base + cw;
     for (int h = 0; h < nhalf; ++h) {
       const int b = h & 1, hb = 2 * nqb - 1 - h;
+      const uint32_t sc = NS == 2 ? 128 * b : 0;       // columns of the score stage
       float incl_next2 = 0.f, nx_lse = INFINITY, nx_dbar = 0.f, nx_gh = 0.f;
       if (h + 2 < nhalf) incl_next2 = load_edge(h + 2);
-      const bool fetch = wg == 0 && row < 64 && h + 1 < nhalf;
-      if (fetch) load_stats(hb - 1, &nx_lse, &nx_dbar, &nx_gh);
-      mbar_wait(sdone, h & 1, ctl, &g_status, kErrWaitMma);
+      // statistics go two half-steps ahead: one barrier of the compute warps lies between their store and their use
+      const bool fetch = wg == 0 && row < 64 && h + 2 < nhalf;
+      if (fetch) load_stats(hb - 2, &nx_lse, &nx_dbar, &nx_gh);
+      mbar_wait(sdone + (NS == 2 ? 8 * b : 0), (h / NS) & 1, ctl, &g_status, kErrWaitMma);
       tc_fence_after();
       float vs[32], vd[32];
-      tmem_ld32(tS + tcol, vs);
-      tmem_ld32(tDOV + tcol, vd);
+      tmem_ld32(tS + sc + tcol, vs);
+      tmem_ld32(tDOV + sc + tcol, vd);
       tmem_ld_wait(vs);
       tmem_ld_wait(vd);
       const int iq0 = hb * 64 + cw;                   // position of this thread's first query
       const bool masked = dead || hb * 64 < k0 + kTileRows - 1;
-      const float4* Lse4 = reinterpret_cast<const float4*>(sLse + b * 64 + cw);
-      const float4* Dbar4 = reinterpret_cast<const float4*>(sDbar + b * 64 + cw);
+      const float4* Lse4 = reinterpret_cast<const float4*>(sLse + (h & 3) * 64 + cw);
+      const float4* Dbar4 = reinterpret_cast<const float4*>(sDbar + (h & 3) * 64 + cw);
       uint32_t shp[16 * P];
       // warpgroup 0 (queries 32..63) knows the suffix of dk_share behind its queries; warpgroup 1 starts
       // from zero and adds p * (the suffix warpgroup 0 ends with) afterwards: dp is linear in it
@@ -370,12 +381,12 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
       auto chunk = [&](auto mask_tag) {
         reverse_sweeps<BID, SHARE, decltype(mask_tag)::value, true, PASS>(
             vs, vd, shp, R, incl + g.eps, Lse4, Dbar4, g, dead, ja - iq0,
-            reinterpret_cast<const float4*>(sGh + b * 64 + cw));
+            reinterpret_cast<const float4*>(sGh + (h & 3) * 64 + cw));
       };
       if (masked) chunk(std::true_type{}); else chunk(std::false_type{});
       sG[(b * 2 + wg) * 128 + row] = R;
-      tmem_st16(tS + tcol, shp);                       // the shares, over score columns this thread has consumed
-      tmem_st16(tS + tcol + 16, shp + 16);
+      tmem_st16(tS + sc + tcol, shp);                  // the shares, over score columns this thread has consumed
+      tmem_st16(tS + sc + tcol + 16, shp + 16);
       asm volatile("bar.sync 1, 256;" ::: "memory");   // the compute warps
       const float rother = sG[(b * 2 + (1 - wg)) * 128 + row];
       const float fix = wg == 1 ? rother : 0.f;
@@ -403,13 +414,13 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
                          : "memory");
           }
         }
-        tmem_st16(tDOV + tcol, pdt);                    // the A operand of dK (M = keys)
-        tmem_st16(tDOV + tcol + 16, pdt + 16);
+        tmem_st16(tDOV + sc + tcol, pdt);                  // the A operand of dK (M = keys)
+        tmem_st16(tDOV + sc + tcol + 16, pdt + 16);
       }
       if (fetch) {
-        sLse[(b ^ 1) * 64 + row] = nx_lse;
-        sDbar[(b ^ 1) * 64 + row] = nx_dbar;
-        if (PASS == 2) sGh[(b ^ 1) * 64 + row] = nx_gh;
+        sLse[((h + 2) & 3) * 64 + row] = nx_lse;
+        sDbar[((h + 2) & 3) * 64 + row] = nx_dbar;
+        if (PASS == 2) sGh[((h + 2) & 3) * 64 + row] = nx_gh;
       }
       incl = incl_next;
       incl_next = incl_next2;
@@ -417,14 +428,14 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
       fence_async_smem();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(tiles);
+      if (lane == 0) mbar_arrive(tiles + (NS == 2 ? 8 * b : 0));
       if (PASS == 0) {
         const float sum = sum_over_lanes(vd, lane);
         if (iq0 + lane < g.tq) atomicAdd(ghat + row_base + iq0 + lane, sum);
       }
     }
   }
-  mbar_wait(sdone, nhalf & 1, ctl, &g_status, kErrWaitMma);
+  mbar_wait(sdone + 8 * (NS - 1), (nhalf / NS) & 1, ctl, &g_status, kErrWaitMma);   // the last commit: every product
   tc_fence_after();
   if (warp < 8) {
     // lane = key: each warpgroup stores half of the columns of dk_main and dv, 32 at a time
@@ -579,8 +590,8 @@ inline int wide_backward(const void* q, const void* k, const void* v, const Geom
 
 // ---------------------------------------------------------------- f(a) / rowsum(f) bids of bf16 heads of 64
 // relu, relu2, softplus.  The row mass and the column sums only need scores and run on the narrow kernels.
-// softplus / inclusive at B4 H8 T8192, forward + backward on one B200: 39.2 ms on the tile kernels -> 7.2 ms (row mass
-// 0.54, column sums 0.67, main pass 1.26, ghat 1.6, reverse pass 3.1); outputs 1.3e-4 -> 1.5e-6 off 64 bits (2-norm),
+// softplus / inclusive at B4 H8 T8192, forward + backward on one B200: 39.2 ms on the tile kernels -> 7.1 ms (row mass
+// 0.54, column sums 0.67, main pass 1.25, ghat 1.6, reverse pass 3.0); outputs 1.3e-4 -> 1.5e-6 off 64 bits (2-norm),
 // gradients 1.7e-3 before and after.  Bound by the special-function unit (four operations per score in the reverse
 // passes, three in the main pass) and, with one CTA per SM in the two product passes, by the hand-over between scores,
 // arithmetic and products.
