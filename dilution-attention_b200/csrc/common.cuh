@@ -134,7 +134,7 @@ struct Geom {
   float eps;
   int carry_rows; // query rows per demand checkpoint (16, 32 or 64)
   int bid;        // FORM of the bid: kBidSoftmax 2^(z - l), kBidSigmoid 1/(1 + 2^(l - z)), or one of the
-                  // four f(a) / rowsum(f) bids (fp32 tile kernels only)
+                  // four f(a) / rowsum(f) bids
   int share;      // share step (kernels_bid.py:123-127): 1 inclusive, 2 exclusive history, 0 none
   int normalised; // the bid divides by its row sum (softmax, relu, relu2, softplus, minshift): there are
                   // row statistics and the backward has the Jacobian correction ghat; otherwise

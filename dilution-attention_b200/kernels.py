@@ -440,7 +440,7 @@ def dilution_decode_append_step(
     """One cached token with the append fused in: what the model does as
     `_append_kv(cache, k1, v1)` (model.py:85-93) followed by
     `dilution_decode_step(q1, cache["k"], cache["v"], cache["committed"], t)`
-    (model.py:236-239), as three kernel launches and no separate copy.
+    (model.py:236-239), as three kernel launches, one where the step is small, and no separate copy.
 
     q1, k1, v1: (B, H, 1, D) of the new token.  cache: the model's dict
     {"k", "v", "len", "committed"} (model.py:76-83, 224-228); its k / v rows at

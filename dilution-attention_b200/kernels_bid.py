@@ -19,8 +19,8 @@ Same entry points and keyword arguments as the reference module (`bid`, `share_c
 (the model passes its context length, model.py:152-156).  The operator itself (softmax, True) is handed to
 `kernels.py`; every other combination goes through the C ABI's dilution_variant_* calls: the
 tcgen05 kernels instantiated for the bid and share step for bf16 tensors of head_dim 64 under
-"bf16" (softmax and the three element-wise bids), the fp32 tile kernels otherwise (fp32 FMAs for
-"ieee", tf32 tensor-core products else; the four f(a) / rowsum(f) bids always).
+"bf16" (softmax, the three element-wise bids, and relu, relu2 and softplus from 641 tokens on), the fp32 tile
+kernels otherwise (fp32 FMAs for "ieee", tf32 tensor-core products else).
 """
 
 from __future__ import annotations

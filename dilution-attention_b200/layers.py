@@ -130,8 +130,8 @@ def split_heads_at(layer, x1, cache):
 
 def softmax_decode_append_step(q1, k1, v1, cache: dict, scratch=None, out=None):
     """One cached token of a softmax layer: `_append_kv(cache, k1, v1)` followed by attention of
-    q1 over the first len+1 cache rows (model.py:112-117), as three launches that stream K and V
-    once.  q1, k1, v1: (B, H, 1, D); cache: the model's dict {"k", "v", "len"}.  Returns
+    q1 over the first len+1 cache rows (model.py:112-117), as launches that stream K and V
+    once (three, or one where the step is small).  q1, k1, v1: (B, H, 1, D); cache: the model's dict {"k", "v", "len"}.  Returns
     (B, H, 1, D) in q1.dtype; cache["len"] grows by one.  With cache["pos_dev"] the length is
     read from the device (see GraphedDecode)."""
     lib = _lib.load()

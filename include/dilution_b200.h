@@ -216,7 +216,8 @@ int dilution_wide_backward(const void* q, const void* k, const void* v, int dtyp
                            const float* ssum, const float* pk, void* scratch, void* dq, void* dk, void* dv,
                            void* stream);
 
-/* Bytes of scratch dilution_decode needs for n rows at this `length`. */
+/* Bytes of scratch dilution_decode needs for n rows at this `length` (a step that runs as one launch leaves
+ * it untouched). */
 size_t dilution_decode_scratch_bytes(int64_t n, int64_t length, int d);
 
 /* Pass 5 — one cached decode step for every (batch, head) row.
@@ -231,7 +232,7 @@ int dilution_decode(const void* q1, const void* k_cache, const void* v_cache, in
 
 /* The same step with the token append fused in: replaces the model's _append_kv
  * (model.py:85-93) followed by dilution_decode_step (kernels.py:994-1038), so a token
- * costs three launches and no separate copy.  k1, v1: (n, d) rows of the new token in
+ * costs three launches, one where the step is small, and no separate copy.  k1, v1: (n, d) rows of the new token in
  * `dtype`; the kernels write them to position length-1 of k_cache / v_cache (which they
  * therefore take as writable) and use them from registers; the demand at length-1 is
  * taken as zero whatever the buffer holds (a new key has none) and set to this step's p.
@@ -345,7 +346,7 @@ int dilution_split_heads_rope_at(void* qkv, void* q, void* k, void* v, const voi
  *          NONE       share = p                           (no share step: out = p v / rowsum p).
  * bf16 tensors of head_dim 64 under DILUTION_PREC_BF16 run on the tcgen05 kernels, instantiated
  * for the bid and share step (softmax and the three element-wise bids); every other dtype,
- * precision and head_dim, and the four f(a) / rowsum(f) bids always, on the fp32 tile kernels
+ * precision and head_dim, and minshift or fewer than 641 tokens of relu, relu2, softplus, on the fp32 tile kernels
  * (IEEE: fp32 FMAs; otherwise tf32 tensor-core products).  Checkpoints every
  * DILUTION_CARRY_ROWS query rows.
  *
