@@ -205,11 +205,14 @@ __device__ __forceinline__ float mass_term(float s, float zscale) {
   if (BID != kBidSoftplus) return fmaxf(s, 0.f);
   const float z = s * zscale;
   const float e = POLY ? poly_exp2<4>(-fabsf(z)) : fast_exp2(-fabsf(z));
-  return fmaxf(z, 0.f) + fast_log2(1.f + e);
+  float top;                                           // max(z, 0) that keeps a NaN, which the polynomial does not
+  asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(top) : "f"(z));
+  return top + fast_log2(1.f + e);
 }
 template <int BID> __device__ __forceinline__ float mass_power(float f) { return BID == kBidRelu2 ? f * f : f; }
 __device__ __forceinline__ float mass_factor(float mass, int i, float mass_scale) {
-  return mass > 0.f ? mass_scale / mass : -1.f / (float)(i + 1);
+  // (a NaN mass stays one: mass_bid hands it on)
+  return mass > 0.f ? mass_scale / mass : mass <= 0.f ? -1.f / (float)(i + 1) : mass;
 }
 __device__ __forceinline__ float mass_bid(float fp, float l) { return l >= 0.f ? fp * l : -l; }
 

@@ -80,3 +80,16 @@ def test_rows_without_mass_bid_uniformly(bid):
     check_grads(True, grads, rgrads, 2e-2)
     if bid != "softplus":
         assert not grads[0][:, :, :40].any()
+
+
+@pytest.mark.parametrize("bid", ["relu", "softplus"])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_values_that_are_not_finite_reach_the_same_outputs(bid, value):
+    """One key and, in another row, one query that are not finite: the outputs that are not finite are the tile kernels'."""
+    pkg = load_package()
+    q, k, v, _ = make_inputs(1, 2, 800, 64, 6, scales=(0.7, 0.7, 1.0, 1.0))
+    k[0, 0, 302, 3] = value
+    q[0, 1, 403, 5] = value
+    x = [t.bfloat16().to(DEV) for t in (q, k, v)]
+    out, tile = (pkg.kernels_bid.dilution_attention_forward(*x, dot_precision=p, bid=bid) for p in ("bf16", "tf32"))
+    assert torch.equal(torch.isfinite(out).all(-1), torch.isfinite(tile).all(-1))
