@@ -365,18 +365,15 @@ __global__ void __launch_bounds__(NT) rowstats_kernel(const T* __restrict__ q,
     }
     tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 1));
     tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 2));
-    const float nm = fmaxf(m, tmax);
+    // no branch on the scores (a row of NaN has no maximum): mma.sync wants whole warps
+    const float nm = fmaxf(m, tmax), ref = nm > -INFINITY ? nm : 0.f;
     float ps = 0.f;
-    if (nm > -INFINITY) {
 #pragma unroll
-      for (int c = 0; c < 16; ++c) ps += pow2<MMA>(z[c] - nm);
-    }
+    for (int c = 0; c < 16; ++c) ps += pow2<MMA>(z[c] - ref);
     ps += __shfl_xor_sync(0xffffffffu, ps, 1);
     ps += __shfl_xor_sync(0xffffffffu, ps, 2);
-    if (nm > -INFINITY) {
-      s = s * pow2<MMA>(m - nm) + ps;
-      m = nm;
-    }
+    s = s * pow2<MMA>(m - ref) + ps;
+    m = nm;
   }
   const int i = ib * TS + r;
   if (mass) {

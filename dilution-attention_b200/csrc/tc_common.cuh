@@ -180,6 +180,7 @@ __device__ __forceinline__ void tmem_alloc(uint32_t slot_smem, uint32_t cols) { 
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_free(uint32_t taddr, uint32_t cols) {         // whole warp
+  __syncwarp();
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols)
                : "memory");
 }

@@ -339,19 +339,21 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) rowstats_kernel(con
           }
           cmax = fmaxf(cmax, v[e]);
         }
-        const float nm = fmaxf(m, cmax * g.zscale);
-        if (nm > -INFINITY) {
-          float ps = 0.f;
+        // No branch on the scores: a row without a finite one so far (a NaN query, all scores -inf) takes the path of
+        // every other row with the reference 0, and what it adds up is scaled by 0 once a reference exists.  A lane
+        // that went another way would still be apart from its warp at the warp-wide tcgen05.ld of the next
+        // chunk and at the tcgen05.dealloc behind the last one.
+        const float nm = fmaxf(m, cmax * g.zscale), ref = nm > -INFINITY ? nm : 0.f;
+        float ps = 0.f;
 #pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            // the pass is bound by the special-function unit: every fourth exponential
-            // is a polynomial on the FMA pipe instead
-            const float z = fmaf(v[e], g.zscale, -nm);
-            ps += (e & 3) == 3 ? poly_exp2<4>(z) : fast_exp2(z);
-          }
-          s = s * fast_exp2(m - nm) + ps;
-          m = nm;
+        for (int e = 0; e < 32; ++e) {
+          // the pass is bound by the special-function unit: every fourth exponential
+          // is a polynomial on the FMA pipe instead
+          const float z = fmaf(v[e], g.zscale, -ref);
+          ps += (e & 3) == 3 ? poly_exp2<4>(z) : fast_exp2(z);
         }
+        s = s * fast_exp2(m - ref) + ps;
+        m = nm;
       }
     };
     if (edge) tile(std::true_type{}); else tile(std::false_type{});
@@ -737,10 +739,10 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
     float rs;
     tmem_ld1(tR + lane_base, &rs);
     tmem_ld_wait();
-    const float inv = 1.f / (rs + g.eps);
     float o[32];
     tmem_ld32(tO + lane_base + kHalf * wg, o);
     tmem_ld_wait(o);
+    const float inv = 1.f / (rs + g.eps);
     if (i < g.tq) {
       float4* dst = reinterpret_cast<float4*>(out + ((int64_t)n * g.tq + i) * kHeadDim + kHalf * wg);
 #pragma unroll
@@ -980,6 +982,7 @@ __global__ void __launch_bounds__(kMainThreads, W == kNarrow ? 2 : 1) forward_ma
     tmem_ld1(tR + lane_base, &rs);
     tmem_ld_wait();
     const float inv = 1.f / (rs + g.eps);
+    __syncwarp();                                     // (a division has paths of its own for NaN and the like)
     const int d = W == kSplit ? g.d : Rows<W>::kHead;
 #pragma unroll
     for (int c0 = 0; c0 < kHalf; c0 += 32) {

@@ -188,7 +188,8 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) rowpass_product_ker
       const float m_new = fmaxf(m_ref, cmax * g.zscale);
       if (__any_sync(0xffffffffu, m_new != m_ref)) {
         const bool fresh = __all_sync(0xffffffffu, m_ref == -INFINITY);   // nothing accumulated yet
-        const float f = m_new == -INFINITY ? 1.f : fast_exp2(m_ref - m_new);
+        // (no branch: the TMEM loads below are warp-wide; a row without a reference has nothing but zeros or NaN yet)
+        const float f = fast_exp2(m_ref - (m_new == -INFINITY ? 0.f : m_new));
         if (!fresh) {
 #pragma unroll
           for (int c = 0; c < kAcc / 16; ++c) {
@@ -271,10 +272,11 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) rowpass_product_ker
     __syncthreads();
     const float4 other = sStat[(1 - WG) * 128 + row];
     const float m = fmaxf(m_ref, other.x);                  // finite: warpgroup 0 always sees key 0
-    const float f_own = m_ref == -INFINITY ? 0.f : fast_exp2(m_ref - m);
-    const float f_oth = other.x == -INFINITY ? 0.f : fast_exp2(other.x - m);
+    const float ref = m == -INFINITY ? 0.f : m;
+    const float f_own = fast_exp2(m_ref - ref), f_oth = fast_exp2(other.x - ref);
     const float den = s * f_own + other.y * f_oth;
     const float inv = (MODE == 1 ? g.scale : 1.f) / den;
+    __syncwarp();                                           // (a division has paths of its own for NaN and the like)
     const float a_own = f_own * inv, a_oth = f_oth * inv;
     const float* take = sX + (WG * 128 + row) * kHalf;
     const int i = ib * kTileRows + row;

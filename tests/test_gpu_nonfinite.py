@@ -1,0 +1,53 @@
+"""Tensors with NaN on the tcgen05 kernels: the same outputs are NaN as on the exact fp32 path, every other output keeps its
+value, and nothing that a value is may steer a warp: its lanes meet in warp-wide TMEM loads and in the release of
+TMEM."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from conftest import load_package, make_inputs
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+SEQ = 300
+PATHS = [(torch.bfloat16, 64, "bf16"), (torch.bfloat16, 128, "bf16"), (torch.float32, 64, "tf32"), (torch.float32, 32, "tf32")]
+
+
+def run(x, dtype, prec, training):
+    """(out, gradients) of one call; no gradients from a forward-only one."""
+    pkg = load_package()
+    leaves = [t.to(DEV, dtype) for t in x]
+    if not training:
+        return pkg.dilution_attention_forward(*leaves, dot_precision=prec), ()
+    leaves = [t.requires_grad_(True) for t in leaves]
+    out = pkg.dilution_attention(*leaves, dot_precision=prec)
+    return out.detach(), torch.autograd.grad(out, leaves, torch.full_like(out, 1e-2))
+
+
+def same_as_exact(x, dtype, prec, training):
+    """Outputs are NaN, infinite and finite where the exact path's are (same operands, fp32 products)."""
+    out, grads = run(x, dtype, prec, training)
+    ref, _ = run([t.to(dtype).float() for t in x], torch.float32, "ieee", False)
+    assert torch.equal(out.isnan(), ref.isnan())
+    assert torch.equal(out.isinf(), ref.isinf()) and torch.equal(out[out.isinf()], ref[ref.isinf()])
+    ok = ref.isfinite()
+    assert (out[ok] - ref[ok]).abs().max().item() < 2e-2
+    return out, ref, grads
+
+
+@pytest.mark.parametrize("training", [False, True])
+@pytest.mark.parametrize("what", ["q", "k"])
+@pytest.mark.parametrize("pos", [0, 34, 130, 258, SEQ - 2])
+@pytest.mark.parametrize("dtype,d,prec", PATHS)
+def test_a_nan_row_leaves_its_warp_whole(dtype, d, prec, pos, what, training):
+    """A NaN query has no score to take a maximum of, at lanes of several warps and in the last, ragged tile."""
+    x = list(make_inputs(1, 2, SEQ, d, 11))[:3]
+    x["qk".index(what)][0, 1, pos, 3] = float("nan")
+    out, _, grads = same_as_exact(x, dtype, prec, training)
+    assert out[0, 1, pos].isnan().all() and out[0, 0].isfinite().all()
+    for g in grads:
+        assert g[0, 0].isfinite().all()
+    # the next call on the same device
+    run([t[:, :1] for t in x], dtype, prec, training)[0].isfinite().all().item()
