@@ -43,10 +43,13 @@ __device__ __forceinline__ float fast_log2(float x) {
 // degree 3) and n is added to the exponent field.  The special-function unit does 16
 // exponentials per clock and SM; kernels bound by it hand a fixed share of their
 // exponentials to this routine, whose ten instructions go to otherwise idle issue slots.
-template <int DEG>
+// A NaN comes out as a finite number; KEEP_NAN hands it on, for one instruction more (2^n multiplied in instead
+// of n added to the exponent: the same value).
+template <int DEG, bool KEEP_NAN = false>
 __device__ __forceinline__ float poly_exp2(float x) {
   static_assert(DEG == 3 || DEG == 4, "degree 3 or 4");
-  x = fmaxf(x, -125.f);
+  if (KEEP_NAN) asm("max.NaN.f32 %0, %0, %1;" : "+f"(x) : "f"(-125.f));
+  else x = fmaxf(x, -125.f);
   const float r = x + 12582912.f;                 // 1.5 * 2^23: round(x) lands in the low mantissa bits
   const float f = x - (r - 12582912.f);
   float p;
@@ -60,6 +63,7 @@ __device__ __forceinline__ float poly_exp2(float x) {
     p = fmaf(p, f, 0.6932609677314758f);
     p = fmaf(p, f, 0.9999280571937561f);
   }
+  if (KEEP_NAN) return p * __int_as_float((__float_as_int(r) << 23) + 0x3f800000);
   return __int_as_float(__float_as_int(p) + (__float_as_int(r) << 23));
 }
 

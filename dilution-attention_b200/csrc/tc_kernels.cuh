@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) rowstats_kernel(con
           // the pass is bound by the special-function unit: every fourth exponential
           // is a polynomial on the FMA pipe instead
           const float z = fmaf(v[e], g.zscale, -ref);
-          ps += (e & 3) == 3 ? poly_exp2<4>(z) : fast_exp2(z);
+          ps += (e & 3) == 3 ? poly_exp2<4, W != kNarrow>(z) : fast_exp2(z);
         }
         s = s * fast_exp2(m - ref) + ps;
         m = nm;
@@ -925,7 +925,7 @@ __global__ void __launch_bounds__(kMainThreads, W == kNarrow ? 2 : 1) forward_ma
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               p[2 * i] = fast_exp2(z[i].x);
-              p[2 * i + 1] = (i & 1) ? poly_exp2<4>(z[i].y) : fast_exp2(z[i].y);
+              p[2 * i + 1] = (i & 1) ? poly_exp2<4, W != kNarrow>(z[i].y) : fast_exp2(z[i].y);
             }
           } else {
 #pragma unroll

@@ -51,3 +51,25 @@ def test_a_nan_row_leaves_its_warp_whole(dtype, d, prec, pos, what, training):
         assert g[0, 0].isfinite().all()
     # the next call on the same device
     run([t[:, :1] for t in x], dtype, prec, training)[0].isfinite().all().item()
+
+
+@pytest.mark.parametrize("training", [False, True])
+@pytest.mark.parametrize("what", ["q", "k", "v"])
+@pytest.mark.parametrize("pos", [3, 128, 129, 130, 131, 259, SEQ - 1])
+@pytest.mark.parametrize("dtype,d,prec", PATHS[1:])
+def test_a_nan_comes_through_every_exponential(dtype, d, prec, pos, what, training):
+    """Every fourth exponential of a row is a polynomial, at each position modulo four and in the last row.  (A masked
+    share of 0 makes NaN of a NaN value: the rows in front of it in its tile, 64 rows of the exact path and 128 here, are
+    left out.)"""
+    x = list(make_inputs(1, 2, SEQ, d, 12))[:3]
+    x["qkv".index(what)][0, 0, pos, 5] = float("nan")
+    if what != "v":
+        same_as_exact(x, dtype, prec, training)
+        return
+    out, _ = run(x, dtype, prec, training)
+    x[2][0, 0, pos, 5] = 0.0
+    clean, _ = run(x, dtype, prec, training)
+    assert out[0, 0, pos:, 5].isnan().all()
+    keep = torch.ones_like(out, dtype=torch.bool)
+    keep[0, 0, pos // 128 * 128:, 5] = False
+    assert torch.equal(out[keep], clean[keep])
