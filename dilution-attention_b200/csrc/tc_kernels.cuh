@@ -216,6 +216,11 @@ __device__ __forceinline__ float mass_factor(float mass, int i, float mass_scale
 }
 __device__ __forceinline__ float mass_bid(float fp, float l) { return l >= 0.f ? fp * l : -l; }
 
+// Whether the masks of a kernel end at the last query too.  A query behind it is a row of zeros with a log-sum-exp of +inf, so
+// that it bids 0 for every finite key, but zero times an infinite key is NaN.  The element-wise bids and softmax of
+// bf16 heads of 64 leave that out: in a long row's passes it is 1% (24.4 -> 24.6 ms at n = 64, T = 16384).
+template <int W, int BID> constexpr bool kMaskEnd = W != kNarrow || row_sum_bid(BID);
+
 // log2-domain log-sum-exp of query i (+inf past the end, so that its p is 0).  The sigmoid bid
 // and the shifted bids have no row statistics: their "lse" is log2 of the shift (0 for the plain
 // sigmoid) for a query that exists and +inf past the end.
@@ -486,7 +491,9 @@ __global__ void __launch_bounds__(256, W != kNarrow ? 2 : row_sum_bid(BID) ? 3 :
     }
     __syncwarp();
     const int i0 = g.q_off + ib * kTileRows + 64 * wg;   // absolute position of this half's first query
-    const bool edge = i0 < k0 + kTileRows - 1;            // part of the diagonal tile
+    const int qend = g.q_off + g.tq;
+    const bool edge = i0 < k0 + kTileRows - 1 ||                      // part of the diagonal tile, or a ragged last one
+                      (kMaskEnd<W, BID> && i0 + 64 > qend);
     const float4* L4 = reinterpret_cast<const float4*>(sL + 128 * b + 64 * wg);
     float colsum0 = 0.f, colsum1 = 0.f;      // queries 0-31 and 32-63 of this warpgroup's half
     auto tile = [&](auto edge_tag) {
@@ -504,7 +511,8 @@ __global__ void __launch_bounds__(256, W != kNarrow ? 2 : row_sum_bid(BID) ? 3 :
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             float p = bid_p<BID>(v[e4 * 4 + u], g.zscale, ls[u]);
-            if (EDGE && ja > i0 + c * 32 + e4 * 4 + u) p = 0.f;
+            const int i = i0 + c * 32 + e4 * 4 + u;
+            if (EDGE && (ja > i || (kMaskEnd<W, BID> && i >= qend))) p = 0.f;
             part[u] += p;
           }
         }
@@ -1060,7 +1068,7 @@ __device__ __forceinline__ float mass_jac(float f, float l, const Geom& g) {
 
 // One thread's 32 queries of the main reverse pass: vs holds their raw scores against the thread's key, vd
 // dO' . v; incle is the key's demand (+ eps) in front of them, R the suffix of dk_share behind them, and query
-// e sees the key when e >= first_q.  Afterwards shp holds the shares as bf16 pairs (SPLIT: their lo plane
+// e sees the key when e >= first_q and, under END, e < end_q (MASK; all of them do otherwise).  Afterwards shp holds the shares as bf16 pairs (SPLIT: their lo plane
 // behind them), vs the Jacobian factor, vd that factor times dp, and R the suffix in front of the queries.
 // Two sweeps.  Forwards: p and 1/(committed+p+eps), the demand
 // accumulated from the checkpoint in front exactly as the forward pass did.  Backwards: the
@@ -1072,10 +1080,10 @@ __device__ __forceinline__ float mass_jac(float f, float l, const Geom& g) {
 // unbounded, takes two passes: 1 leaves p and p * dp in vs and vd, the terms of ghat; 2 subtracts ghat (Gh4) from dp
 // before the factor multiplies.  These bids keep mass_term of a query between the sweeps (-1 where the query does not
 // see the key), which gives p and the factor both.
-template <int BID, int SHARE, bool MASK, bool SPLIT, int PASS = 0>
+template <int BID, int SHARE, bool MASK, bool SPLIT, bool END, int PASS = 0>
 __device__ __forceinline__ void reverse_sweeps(float (&vs)[32], float (&vd)[32], uint32_t* shp, float& R, float incle,
-                                               const float4* Lse4, const float4* Dbar4, const Geom& g, bool dead,
-                                               int first_q, const float4* Gh4 = nullptr) {
+                                               const float4* Lse4, const float4* Dbar4, const Geom& g,
+                                               bool dead, int first_q, int end_q, const float4* Gh4 = nullptr) {
   constexpr bool MASS = row_sum_bid(BID);
   float inv[32];
 #pragma unroll
@@ -1096,13 +1104,13 @@ __device__ __forceinline__ void reverse_sweeps(float (&vs)[32], float (&vd)[32],
       if (MASS) {
         keep = u == 3 ? mass_term<BID, true>(vs[e], g.zscale) : mass_term<BID>(vs[e], g.zscale);
         p = mass_bid(mass_power<BID>(keep), lse[u]);
-        if (MASK && (dead || first_q > e)) keep = -1.f;
+        if (MASK && (dead || first_q > e || (END && e >= end_q))) keep = -1.f;
       } else {
         p = fast_exp2(z[u]);
       }
       if (BID == kBidSigmoid) p = fast_rcp(1.f + p);
       if (MASK) {
-        if (dead || first_q > e) p = 0.f;
+        if (dead || first_q > e || (END && e >= end_q)) p = 0.f;
       }
       if (SHARE == kShareInclusive) {
         incle += p;
@@ -1529,7 +1537,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
       tmem_ld_wait(vd);
       const int qc = (odd ? 0 : 64) + cw;             // first query column of this thread in the step's tile
       const int iq0 = ib * kTileRows + qc;            // its position (q_off == 0 here)
-      const bool masked_tile = dead || (ib * kTileRows + (odd ? 0 : 64) < k0 + kTileRows - 1);
+      const bool masked_tile = dead || (ib * kTileRows + (odd ? 0 : 64) < k0 + kTileRows - 1) ||
+                               (kMaskEnd<kNarrow, BID> && iq0 + 32 > g.tq);
       const float4* Lse4 = reinterpret_cast<const float4*>(sLse + b * 128 + qc);
       const float4* Dbar4 = reinterpret_cast<const float4*>(sDbar + b * 128 + qc);
       uint32_t shp[16];                                // 32 shares as bf16 pairs
@@ -1537,8 +1546,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
       // starts from zero and adds p * (the suffix warpgroup 0 ends with) afterwards: dp is linear in it
       float R = wg == 0 ? sigma : 0.f;
       auto chunk = [&](auto mask_tag) {
-        reverse_sweeps<BID, SHARE, decltype(mask_tag)::value, false, PASS>(
-            vs, vd, shp, R, incl + g.eps, Lse4, Dbar4, g, dead, ja - iq0);
+        reverse_sweeps<BID, SHARE, decltype(mask_tag)::value, false, kMaskEnd<kNarrow, BID>, PASS>(
+            vs, vd, shp, R, incl + g.eps, Lse4, Dbar4, g, dead, ja - iq0, g.tq - iq0);
       };
       if (masked_tile) chunk(std::true_type{}); else chunk(std::false_type{});
       // warpgroup 0: the suffix behind query 32; warpgroup 1: minus its own sum of -dk_share

@@ -422,7 +422,8 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) backward_key_correc
     }
     __syncwarp();
     const int i0 = ib * kTileRows + 64 * odd + 32 * wg;           // first query of this thread's 32
-    const bool masked = dead || t == 0;
+    constexpr bool END = kMaskEnd<W, kBidSoftmax>;
+    const bool masked = dead || t == 0 || (END && i0 + 32 > g.tq);
     const float4* St4 = reinterpret_cast<const float4*>(sStat + b * 128 + 64 * odd + 32 * wg);
     float vs[32];
     uint32_t wt[16], wr[Rows<W>::kPlanes == 2 ? 16 : 1];
@@ -436,8 +437,9 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) backward_key_correc
         float p0 = fast_exp2(fmaf(vs[2 * e2], g.zscale, -st.x));
         float p1 = fast_exp2(fmaf(vs[2 * e2 + 1], g.zscale, -st.z));
         if (MASK) {
-          if (dead || ja > i0 + 2 * e2) p0 = 0.f;
-          if (dead || ja > i0 + 2 * e2 + 1) p1 = 0.f;
+          const int i = i0 + 2 * e2;
+          if (dead || ja > i || (END && i >= g.tq)) p0 = 0.f;
+          if (dead || ja > i + 1 || (END && i + 1 >= g.tq)) p1 = 0.f;
         }
         wt[e2] = pack_bf16(p0 * st.y, p1 * st.w);
         if (Rows<W>::kPlanes == 2) wr[e2] = pack_bf16_rest(p0 * st.y, p1 * st.w, wt[e2]);

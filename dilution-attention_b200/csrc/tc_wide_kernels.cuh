@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
       tmem_ld_wait(vs);
       tmem_ld_wait(vd);
       const int iq0 = hb * 64 + cw;                   // position of this thread's first query
-      const bool masked = dead || hb * 64 < k0 + kTileRows - 1;
+      const bool masked = dead || hb * 64 < k0 + kTileRows - 1 || iq0 + 32 > g.tq;
       const float4* Lse4 = reinterpret_cast<const float4*>(sLse + (h & 3) * 64 + cw);
       const float4* Dbar4 = reinterpret_cast<const float4*>(sDbar + (h & 3) * 64 + cw);
       uint32_t shp[16 * P];
@@ -379,8 +379,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
       // from zero and adds p * (the suffix warpgroup 0 ends with) afterwards: dp is linear in it
       float R = wg == 0 ? sigma : 0.f;
       auto chunk = [&](auto mask_tag) {
-        reverse_sweeps<BID, SHARE, decltype(mask_tag)::value, true, PASS>(
-            vs, vd, shp, R, incl + g.eps, Lse4, Dbar4, g, dead, ja - iq0,
+        reverse_sweeps<BID, SHARE, decltype(mask_tag)::value, true, true, PASS>(
+            vs, vd, shp, R, incl + g.eps, Lse4, Dbar4, g, dead, ja - iq0, g.tq - iq0,
             reinterpret_cast<const float4*>(sGh + (h & 3) * 64 + cw));
       };
       if (masked) chunk(std::true_type{}); else chunk(std::false_type{});

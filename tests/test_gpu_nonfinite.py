@@ -1,5 +1,5 @@
-"""Tensors with NaN on the tcgen05 kernels: the same outputs are NaN as on the exact fp32 path, every other output keeps its
-value, and nothing that a value is may steer a warp: its lanes meet in warp-wide TMEM loads and in the release of
+"""Tensors with NaN and infinities on the tcgen05 kernels: the same outputs are NaN and infinite as on the exact fp32 path,
+every other output keeps its value, and nothing that a value is may steer a warp: its lanes meet in warp-wide TMEM loads and in the release of
 TMEM."""
 
 from __future__ import annotations
@@ -73,3 +73,45 @@ def test_a_nan_comes_through_every_exponential(dtype, d, prec, pos, what, traini
     keep = torch.ones_like(out, dtype=torch.bool)
     keep[0, 0, pos // 128 * 128:, 5] = False
     assert torch.equal(out[keep], clean[keep])
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf")])
+@pytest.mark.parametrize("pos", [4, 129, 130, 131, SEQ - 1])
+@pytest.mark.parametrize("dtype,d,prec", PATHS[1:2])
+def test_a_score_of_minus_infinity_is_a_bid_of_zero(dtype, d, prec, pos, value):
+    """A key's infinite feature against queries of the other sign: its scores are -inf, nobody bids for it and every output
+    is finite."""
+    q, k, v, _ = make_inputs(1, 2, SEQ, d, 13)
+    q[0, 0, :, 5] = -torch.copysign(q[0, 0, :, 5].abs() + 0.1, torch.tensor(value))
+    k[0, 0, pos, 5] = value
+    x = [q, k, v]
+    for training in (False, True):
+        out, ref, grads = same_as_exact(x, dtype, prec, training)
+        assert ref.isfinite().all()
+    _, exact = run([t.to(dtype).float() for t in x], torch.float32, "ieee", True)
+    for name, g, r in zip(("dq", "dk", "dv"), grads, exact):
+        ok = r.isfinite()
+        if name == "dq":             # 0 * inf in the key's feature, for the rows of its 128-row tile too
+            ok[0, 0, pos // 128 * 128:, 5] = False
+        assert ((g.float() - r)[ok].norm() / r[ok].norm()).item() < 1e-2, name
+    _, aux = load_package().dilution_attention_forward(*(t.to(DEV, dtype) for t in x), dot_precision=prec, return_aux=True)
+    assert aux["committed_total"].isfinite().all()
+
+
+@pytest.mark.parametrize("seq", [700, 768])
+def test_a_key_that_nobody_bids_for_under_the_softplus_bid(seq):
+    q, k, v, dout = make_inputs(1, 2, seq, 64, 15)
+    q[0, 0, :, 5] = -(q[0, 0, :, 5].abs() + 0.1)
+    k[0, 0, 131, 5] = float("inf")
+    kb = load_package().kernels_bid
+    got = []
+    for prec in ("bf16", "tf32"):      # tf32 on the same tensors: the tile kernels
+        leaves = [t.to(DEV, torch.bfloat16).requires_grad_(True) for t in (q, k, v)]
+        out = kb.dilution_attention(*leaves, dot_precision=prec, bid="softplus")
+        got.append((out.detach(), *(g.float() for g in torch.autograd.grad(out, leaves, dout.to(DEV)))))
+    for name, a, b in zip(("out", "dq", "dk", "dv"), *got):
+        ok = b.isfinite()
+        if name == "dq":
+            ok[0, 0, 128:, 5] = False
+        assert ok.float().mean().item() > 0.98, name
+        assert ((a - b)[ok].norm() / b[ok].norm()).item() < 1e-2, name
