@@ -33,7 +33,7 @@ constexpr long long kWaitCycles = 4000000000LL;             // ~2 s: a live wait
 //   kNarrow : heads of 64 in bf16, one sub-tile; formed values rounded to bf16;
 //   kWide128: heads of 128 in bf16, two sub-tiles of 64 features;
 //   kPairs64: heads of 64 in bf16, one sub-tile;
-//   kSplit  : heads of up to 64 in fp32, each value as hi + lo with hi = bf16(x), lo = bf16(x - hi):
+//   kSplit  : heads of up to 64 in fp32, each value as hi + lo with hi = bf16(x), lo = bf16(x - hi) (split_pair):
 //             sub-tile 0 holds the hi parts, sub-tile 1 the lo parts (zeros behind the head size).  A product of
 //             two such operands keeps 16 bits of each (2^-17 relative), where tf32 keeps 11.
 // All but kNarrow form hi + lo pairs too (kPlanes), and take do' as hi + lo: [hi | lo] sub-tiles.

@@ -175,6 +175,28 @@ __device__ __forceinline__ uint32_t pack_bf16_rest(float a, float b, uint32_t hi
   return pack_bf16(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xffff0000u));
 }
 
+// Both parts of two fp32 values that come from outside, hi + lo.  An infinity is +-1 + +-inf: the products with another value
+// that are taken (hi hi, hi lo, lo hi) then add up to what the infinity itself gives, of the right sign, NaN with 0
+// — as inf + 0 the hi lo product would be inf * 0, as inf + (inf - inf) all of them are NaN.  A finite value past the largest
+// bf16 is cut, not rounded to inf.  Everything else is rounded.
+__device__ __forceinline__ void split_one(float x, float& hi, float& lo) {
+  const uint32_t u = __float_as_uint(x);
+  hi = isinf(x) ? copysignf(1.f, x) : __uint_as_float(u & 0xffff0000u);
+  lo = isinf(x) ? x : x - hi;
+}
+__device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& lo) {
+  hi = pack_bf16(a, b);
+  lo = pack_bf16_rest(a, b, hi);
+  constexpr float kRoundsToInf = 3.3961775292304601e38f;   // 2^128 - 2^119: half a unit past the largest bf16
+  if (fmaxf(fabsf(a), fabsf(b)) >= kRoundsToInf) {
+    float ha, la, hb, lb;
+    split_one(a, ha, la);
+    split_one(b, hb, lb);
+    hi = pack_bf16(ha, hb);
+    lo = pack_bf16(la, lb);
+  }
+}
+
 // 32 columns of one output row; kSplit rows end after `left` columns (a multiple of 16).
 template <int W>
 __device__ __forceinline__ void store_row32(float* dst, const float* m, int left) {

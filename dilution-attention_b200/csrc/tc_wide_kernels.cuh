@@ -36,10 +36,12 @@ __global__ void split_operands_kernel(SplitArgs a, int64_t rows, int d) {
   const int c = (int)(idx & 15) * 4;
   float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
   if (c < d) x = *reinterpret_cast<const float4*>(a.src[blockIdx.y] + r * d + c);
-  const uint32_t h0 = pack_bf16(x.x, x.y), h1 = pack_bf16(x.z, x.w);
+  uint2 hi, lo;
+  split_pair(x.x, x.y, hi.x, lo.x);
+  split_pair(x.z, x.w, hi.y, lo.y);
   uint2* dst = reinterpret_cast<uint2*>(a.dst[blockIdx.y] + r * 128 + c);
-  dst[0] = make_uint2(h0, h1);
-  dst[16] = make_uint2(pack_bf16_rest(x.x, x.y, h0), pack_bf16_rest(x.z, x.w, h1));
+  dst[0] = hi;
+  dst[16] = lo;
 }
 
 __device__ __forceinline__ void load_vec(const float* p, float (&x)[2]) {
@@ -86,15 +88,17 @@ __global__ void wide_backward_prep_kernel(const TD* __restrict__ dout, const flo
   }
   dot = warp_sum(dot);
   if (W == kWide128) {
-    const uint2 hi = make_uint2(pack_bf16(a[0], a[1]), pack_bf16(a[E - 2], a[E - 1]));
+    uint2 hi, lo;
+    split_pair(a[0], a[1], hi.x, lo.x);
+    split_pair(a[E - 2], a[E - 1], hi.y, lo.y);
     reinterpret_cast<uint2*>(dop + row * 256)[lane] = hi;
-    reinterpret_cast<uint2*>(dop + row * 256 + 128)[lane] =
-        make_uint2(pack_bf16_rest(a[0], a[1], hi.x), pack_bf16_rest(a[E - 2], a[E - 1], hi.y));
+    reinterpret_cast<uint2*>(dop + row * 256 + 128)[lane] = lo;
     reinterpret_cast<float4*>(dq_main + row * 128)[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
   } else {
-    const uint32_t hi = pack_bf16(a[0], a[1]);
+    uint32_t hi, lo;
+    split_pair(a[0], a[1], hi, lo);
     reinterpret_cast<uint32_t*>(dop + row * 128)[lane] = hi;
-    reinterpret_cast<uint32_t*>(dop + row * 128 + 64)[lane] = pack_bf16_rest(a[0], a[1], hi);
+    reinterpret_cast<uint32_t*>(dop + row * 128 + 64)[lane] = lo;
     reinterpret_cast<float2*>(dq_main + row * 64)[lane] = make_float2(0.f, 0.f);
   }
   if (lane == 0) {

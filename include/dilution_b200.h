@@ -200,7 +200,7 @@ int dilution_backward(const void* q, const void* k, const void* v, int dtype, in
  * (kernels.py:328-455, 829-903) for those cases.
  *
  * dilution_split_operands: fp32 (rows, d) -> bf16 (rows, 128), [hi 64 | lo 64] with hi = bf16(x),
- * lo = bf16(x - hi), zeros behind d.  A product of two such operands keeps 16 bits of each, tf32 keeps 11.  For both
+ * lo = bf16(x - hi), zeros behind d; an infinity is hi = +-1, lo = +-inf, and a finite x past the largest bf16 is cut.  A product of two such operands keeps 16 bits of each, tf32 keeps 11.  For both
  * dtypes the shares and the gradient terms formed inside are multiplied as such pairs.
  * out, pk: (n, t, d) fp32; pk may be NULL when no backward follows.  dq, dk, dv: (n, t, d) of `dtype`.
  * scratch: dilution_wide_scratch_bytes. */

@@ -75,12 +75,12 @@ def test_a_nan_comes_through_every_exponential(dtype, d, prec, pos, what, traini
     assert torch.equal(out[keep], clean[keep])
 
 
-@pytest.mark.parametrize("value", [float("inf"), float("-inf")])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), 3.4e38, -3.4e38])
 @pytest.mark.parametrize("pos", [4, 129, 130, 131, SEQ - 1])
-@pytest.mark.parametrize("dtype,d,prec", PATHS[1:2])
+@pytest.mark.parametrize("dtype,d,prec", PATHS[1:])
 def test_a_score_of_minus_infinity_is_a_bid_of_zero(dtype, d, prec, pos, value):
     """A key's infinite feature against queries of the other sign: its scores are -inf, nobody bids for it and every output
-    is finite."""
+    is finite.  3.4e38 is past the largest bf16 and rounds to an infinity there."""
     q, k, v, _ = make_inputs(1, 2, SEQ, d, 13)
     q[0, 0, :, 5] = -torch.copysign(q[0, 0, :, 5].abs() + 0.1, torch.tensor(value))
     k[0, 0, pos, 5] = value
@@ -115,3 +115,11 @@ def test_a_key_that_nobody_bids_for_under_the_softplus_bid(seq):
             ok[0, 0, 128:, 5] = False
         assert ok.float().mean().item() > 0.98, name
         assert ((a - b)[ok].norm() / b[ok].norm()).item() < 1e-2, name
+
+
+@pytest.mark.parametrize("what", ["q", "k"])
+@pytest.mark.parametrize("dtype,d,prec", PATHS[1:])
+def test_an_infinite_score_makes_its_rows_nan(dtype, d, prec, what):
+    x = list(make_inputs(1, 2, SEQ, d, 14))[:3]
+    x["qk".index(what)][0, 0, 131, 5] = float("inf")
+    same_as_exact(x, dtype, prec, True)
