@@ -179,22 +179,21 @@ __device__ __forceinline__ uint32_t pack_bf16_rest(float a, float b, uint32_t hi
 // that are taken (hi hi, hi lo, lo hi) then add up to what the infinity itself gives, of the right sign, NaN with 0
 // — as inf + 0 the hi lo product would be inf * 0, as inf + (inf - inf) all of them are NaN.  A finite value past the largest
 // bf16 is cut, not rounded to inf.  Everything else is rounded.
-__device__ __forceinline__ void split_one(float x, float& hi, float& lo) {
-  const uint32_t u = __float_as_uint(x);
-  hi = isinf(x) ? copysignf(1.f, x) : __uint_as_float(u & 0xffff0000u);
-  lo = isinf(x) ? x : x - hi;
-}
 __device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& lo) {
-  hi = pack_bf16(a, b);
-  lo = pack_bf16_rest(a, b, hi);
   constexpr float kRoundsToInf = 3.3961775292304601e38f;   // 2^128 - 2^119: half a unit past the largest bf16
-  if (fmaxf(fabsf(a), fabsf(b)) >= kRoundsToInf) {
-    float ha, la, hb, lb;
-    split_one(a, ha, la);
-    split_one(b, hb, lb);
-    hi = pack_bf16(ha, hb);
-    lo = pack_bf16(la, lb);
+  float x[2] = {a, b}, rest[2];
+  bool inf[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    inf[i] = isinf(x[i]);
+    rest[i] = x[i];
+    if (inf[i]) x[i] = copysignf(1.f, x[i]);
+    else if (fabsf(x[i]) >= kRoundsToInf) x[i] = __uint_as_float(__float_as_uint(x[i]) & 0xffff0000u);
   }
+  hi = pack_bf16(x[0], x[1]);
+  if (!inf[0]) rest[0] -= __uint_as_float(hi << 16);
+  if (!inf[1]) rest[1] -= __uint_as_float(hi & 0xffff0000u);
+  lo = pack_bf16(rest[0], rest[1]);
 }
 
 // 32 columns of one output row; kSplit rows end after `left` columns (a multiple of 16).

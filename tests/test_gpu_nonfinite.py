@@ -123,3 +123,29 @@ def test_an_infinite_score_makes_its_rows_nan(dtype, d, prec, what):
     x = list(make_inputs(1, 2, SEQ, d, 14))[:3]
     x["qk".index(what)][0, 0, 131, 5] = float("inf")
     same_as_exact(x, dtype, prec, True)
+
+
+def test_hi_and_lo_planes_of_values_that_are_not_finite():
+    """hi + lo of every kind of value, and of its neighbours as if it were not there."""
+    lib = load_package()._lib.load()
+    clean = make_inputs(1, 1, 8, 32, 17)[0][0, 0]
+    x = clean.clone()
+    odd = [float("inf"), float("-inf"), float("nan"), 3.4e38, -3.4e38]
+    for n, value in enumerate(odd):
+        x[n, 6 + n] = value
+    got = []
+    for t in (x.to(DEV), clean.to(DEV)):
+        planes = [torch.empty(8, 128, device=DEV, dtype=torch.bfloat16) for _ in range(3)]
+        assert lib.dilution_split_operands(t.data_ptr(), t.data_ptr(), t.data_ptr(), 8, 32, *(p.data_ptr() for p in planes),
+                                           torch.cuda.current_stream().cuda_stream) == 0
+        got.append(planes[0].float().cpu())
+    hi, lo = got[0][:, :64], got[0][:, 64:]
+    assert (hi[0, 6], lo[0, 6]) == (1.0, float("inf")) and (hi[1, 7], lo[1, 7]) == (-1.0, float("-inf"))
+    assert hi[2, 8].isnan() and lo[2, 8].isnan()
+    for n, sign in ((3, 1), (4, -1)):
+        assert hi[n, 6 + n] == sign * torch.finfo(torch.bfloat16).max
+        assert abs((hi[n, 6 + n].double() + lo[n, 6 + n].double()).item() / x[n, 6 + n].item() - 1) < 2.0 ** -15
+    for n in range(5):
+        for p in got:
+            p[n, [6 + n, 70 + n]] = 0.0
+    assert torch.equal(got[0], got[1])
