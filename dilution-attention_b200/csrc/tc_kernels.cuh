@@ -795,12 +795,37 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
 // of 64 stays on forward_main_kernel: its long rows run at the card's power limit, where this form is 1 to 3% slower
 // (145.2 -> 148 ms for the passes of a 128K prompt, 16 heads).
 constexpr int kMainThreads = 288;
+
+// Shares as hi + lo make NaN of an infinite value (lo may be negative or 0).  Where an output is NaN and its row sum is not, the
+// value is to blame: the output becomes the sum of the infinities that the row sees, NaN if they are of both signs or a
+// value is NaN.  out: this lane's row, columns [col0, col1), if `row` says that there is one; i: its position, -1 where the row
+// sum is NaN; vinf: where a row of v, `stride` apart, holds what is infinite (its lo plane under kSplit); keys: up to the
+// warp's last row.  The warp walks in step, whatever the values: its release of TMEM follows.
+__device__ __noinline__ void restore_infinities(float* out, const __nv_bfloat16* vinf, int stride, int keys, int i, bool row,
+                                                int col0, int col1) {
+  for (int c = col0; c < col1; ++c) {
+    const float x = row ? out[c] : 0.f;
+    const bool want = x != x && i >= 0;
+    if (!__any_sync(0xffffffffu, want)) continue;
+    float sum = 0.f;
+    for (int j = 0; j < keys; ++j) {
+      const float v = __bfloat162float(vinf[(int64_t)j * stride + c]);
+      sum += j <= i && !(fabsf(v) < INFINITY) ? v : 0.f;
+      if ((j & 63) == 63 && __all_sync(0xffffffffu, sum != sum || !want)) break;
+    }
+    const float y = want && sum != 0.f ? sum : x;
+    if (row) out[c] = y;
+  }
+  __syncwarp();
+}
+
 template <int BID = kBidSoftmax, int SHARE = kShareInclusive, int W = kNarrow>
 __global__ void __launch_bounds__(kMainThreads, W == kNarrow ? 2 : 1) forward_main_async_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, Geom g, const float* __restrict__ rmax,
     const float* __restrict__ rden, const float* __restrict__ carry,
-    const float* __restrict__ carry_base, float* __restrict__ out, float* __restrict__ ssum) {
+    const float* __restrict__ carry_base, const __nv_bfloat16* __restrict__ v_rows, float* __restrict__ out,
+    float* __restrict__ ssum) {
   constexpr uint32_t TB = Rows<W>::kBytes;
   constexpr int P = Rows<W>::kPlanes;
   constexpr int kOCols = Rows<W>::kCols + 16;        // O and the row sums: one tile
@@ -1013,6 +1038,7 @@ __global__ void __launch_bounds__(kMainThreads, W == kNarrow ? 2 : 1) forward_ma
     const float inv = 1.f / (rs + g.eps);
     __syncwarp();                                     // (a division has paths of its own for NaN and the like)
     const int d = W == kSplit ? g.d : Rows<W>::kHead;
+    bool nan = false;
 #pragma unroll
     for (int c0 = 0; c0 < kHalf; c0 += 32) {
       const int col = kHalf * wg + c0;
@@ -1033,8 +1059,18 @@ __global__ void __launch_bounds__(kMainThreads, W == kNarrow ? 2 : 1) forward_ma
           if (W != kSplit || col + 4 * c < d)
             dst[c] = make_float4(o[4 * c] * inv, o[4 * c + 1] * inv, o[4 * c + 2] * inv, o[4 * c + 3] * inv);
       }
+      if (P == 2) {
+#pragma unroll
+        for (int e = 0; e < 32; ++e) nan |= o[e] != o[e];
+      }
     }
     if (i < g.tq && wg == 0) ssum[(int64_t)n * g.tq + i] = rs;
+    if (P == 2) {
+      if (__any_sync(0xffffffffu, nan && rs == rs && i < g.tq))
+        restore_infinities(out + ((int64_t)n * g.tq + i) * d, v_rows + (int64_t)n * g.tk * (64 * Rows<W>::kSub) + (W == kSplit ? 64 : 0),
+                           64 * Rows<W>::kSub, min(g.tk, (i | 31) + 1), rs == rs ? i : -1, i < g.tq, kHalf * wg,
+                           min(d, kHalf * (wg + 1)));
+    }
   }
   }
   drain_if_aborted(ctl);
@@ -2006,14 +2042,16 @@ inline int forward_main(const void* q, const void* k, const void* v, const Geom&
   static_assert(2 * (smem + 1024) <= 233472 && 3 * (smem + 1024) > 233472, "exactly two CTAs of the main pass fit one SM");
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
   const unsigned grid = (unsigned)(g.n * nqb);
-  auto launch = [&](auto kern, int threads) -> int {
-    if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
-    kern<<<grid, threads, smem, st>>>(mq, mk, mv, g, rmax, rden, carry, carry_base, out, ssum);
-    return 0;
-  };
   DIL_TC_SHARE(g, {
-    if (int rc = g.bid == kBidSigmoid ? launch(forward_main_async_kernel<kBidSigmoid, SHARE>, kMainThreads)
-                                      : launch(forward_main_kernel<kBidSoftmax, SHARE>, 256)) return rc;
+    if (g.bid == kBidSigmoid) {
+      auto kern = forward_main_async_kernel<kBidSigmoid, SHARE>;
+      if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
+      kern<<<grid, kMainThreads, smem, st>>>(mq, mk, mv, g, rmax, rden, carry, carry_base, nullptr, out, ssum);
+    } else {
+      auto kern = forward_main_kernel<kBidSoftmax, SHARE>;
+      if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
+      kern<<<grid, 256, smem, st>>>(mq, mk, mv, g, rmax, rden, carry, carry_base, out, ssum);
+    }
   })
   return launch_status("tc forward_main", err, errlen);
 }

@@ -149,3 +149,38 @@ def test_hi_and_lo_planes_of_values_that_are_not_finite():
         for p in got:
             p[n, [6 + n, 70 + n]] = 0.0
     assert torch.equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("signs", [(1.0,), (-1.0,), (1.0, 1.0), (1.0, -1.0)])
+@pytest.mark.parametrize("pos", [0, 63, 129, 131, SEQ - 1])
+@pytest.mark.parametrize("path", PATHS[1:] + ["softplus"])
+def test_infinite_values_make_infinite_outputs(path, pos, signs):
+    """The rows that see an infinite value are infinite in its column, and NaN where they see both signs; shares multiplied as
+    hi + lo would make NaN of all of them.  (Rows in front of it in its 128-row tile: 0 * inf, as above.)"""
+    pkg = load_package()
+    dtype, d, prec = (torch.bfloat16, 64, None) if path == "softplus" else path
+    seq = 700 if path == "softplus" else SEQ
+
+    def call(x, exact):
+        if path == "softplus":       # tf32 on the same tensors: the tile kernels
+            return pkg.kernels_bid.dilution_attention_forward(*(t.to(DEV, dtype) for t in x), bid="softplus",
+                                                              dot_precision="tf32" if exact else "bf16")
+        return run([t.to(dtype).float() for t in x], torch.float32, "ieee", False)[0] if exact else run(x, dtype, prec, True)[0]
+
+    x = list(make_inputs(1, 2, seq, d, 16))[:3]
+    clean = call(x, False)
+    at = [pos, pos + 70][:len(signs)] if pos + 70 < seq else [pos - 70 * n for n in range(len(signs))][::-1]
+    pos = at[0]
+    for p, s in zip(at, signs):
+        x[2][0, 1, p, 7] = s * float("inf")
+    out, ref = call(x, False)[0, 1, :, 7].cpu(), call(x, True)[0, 1, :, 7].cpu()
+    want = torch.zeros(seq)
+    for p, s in zip(at, signs):
+        want[p:] += s * float("inf")
+    sees = [i for i in range(pos, seq) if all(i >= p or i < p // 128 * 128 for p in at)]      # no masked infinity in the tile
+    for got in (out, ref):
+        assert torch.equal(got[sees].nan_to_num(5.0, 1.0, -1.0), want[sees].nan_to_num(5.0, 1.0, -1.0))
+    full = call(x, False)
+    keep = torch.ones_like(full, dtype=torch.bool)
+    keep[0, 1, pos // 128 * 128:, 7] = False
+    assert torch.equal(full[keep], clean[keep])
