@@ -201,11 +201,8 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
       : "r"(taddr)
       : "memory");
 }
-__device__ __forceinline__ void tmem_ld_wait() {
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-// The same wait, tied to the 32 registers a load filled: the compiler cannot move
-// a use of them above the wait.
+// Loads fill their registers asynchronously.  Every wait names those it is for, so that the compiler cannot move a use
+// of them above it.
 __device__ __forceinline__ void tmem_ld_wait(float* v) {
   uint32_t* r = reinterpret_cast<uint32_t*>(v);
   asm volatile("tcgen05.wait::ld.sync.aligned;"
@@ -220,9 +217,13 @@ __device__ __forceinline__ void tmem_ld_wait(float* v) {
 
 // One fp32 column of this thread's lane.
 __device__ __forceinline__ void tmem_ld1(uint32_t taddr, float* v) {
-  uint32_t r;
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(taddr) : "memory");
-  *v = __uint_as_float(r);
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];"
+               : "=r"(*reinterpret_cast<uint32_t*>(v))
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_ld_wait1(float* v) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(*reinterpret_cast<uint32_t*>(v)) : : "memory");
 }
 
 // 16 consecutive fp32 columns of this thread's lane.

@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) forward_fused_kernel(
       }
       float rs;
       tmem_ld1(tOb + 64, &rs);
-      tmem_ld_wait();
+      tmem_ld_wait1(&rs);
       fence_async_smem();
       tc_fence_before();
       asm volatile("bar.sync 2, 128;" ::: "memory");         // every warp has read the tile: its buffer is free

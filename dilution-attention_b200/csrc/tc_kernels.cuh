@@ -767,7 +767,7 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
     const int i = ib * kTileRows + row;
     float rs;
     tmem_ld1(tR + lane_base, &rs);
-    tmem_ld_wait();
+    tmem_ld_wait1(&rs);
     float o[32];
     tmem_ld32(tO + lane_base + kHalf * wg, o);
     tmem_ld_wait(o);
@@ -1034,7 +1034,7 @@ __global__ void __launch_bounds__(kMainThreads, W == kNarrow ? 2 : 1) forward_ma
     const int i = ib * kTileRows + row;
     float rs;
     tmem_ld1(tR + lane_base, &rs);
-    tmem_ld_wait();
+    tmem_ld_wait1(&rs);
     const float inv = 1.f / (rs + g.eps);
     __syncwarp();                                     // (a division has paths of its own for NaN and the like)
     const int d = W == kSplit ? g.d : Rows<W>::kHead;
@@ -1519,7 +1519,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
         }
         float gh;
         tmem_ld1(tG + lane_base, &gh);
-        tmem_ld_wait();
+        tmem_ld_wait1(&gh);
         fence_async_smem();
         tc_fence_before();
         asm volatile("bar.sync 2, 128;" ::: "memory");

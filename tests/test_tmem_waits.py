@@ -1,0 +1,30 @@
+"""tcgen05.ld fills its registers asynchronously.  A wait that does not name them lets the compiler use them too early, which
+no run need show: every load in the sources is followed by a wait for the same registers."""
+
+from __future__ import annotations
+
+import glob
+import os
+import re
+
+import pytest
+
+from conftest import ROOT
+
+SOURCES = sorted(glob.glob(os.path.join(ROOT, "dilution-attention_b200", "csrc", "tc_*.cuh")))
+WAIT = {"1": "tmem_ld_wait1", "16": "tmem_ld_wait16", "32": "tmem_ld_wait"}
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=os.path.basename)
+def test_every_load_has_a_wait_that_names_its_registers(path):
+    lines = open(path).read().split("\n")
+    for at, line in enumerate(lines):
+        assert "tmem_ld_wait()" not in line, (at + 1, line)
+        load = re.search(r"^\s*tmem_ld(1|16|32)\((.*), ([&\w]+(?: \+ \d+)?)\);", line)
+        if load:
+            wait = f"{WAIT[load[1]]}({load[3]});"
+            assert any(wait in after for after in lines[at + 1:at + 70]), (at + 1, line, wait)
+
+
+def test_the_sources_are_found():
+    assert sum("tmem_ld32(" in open(p).read() for p in SOURCES) >= 4
