@@ -90,9 +90,22 @@ def _prepare(q, k, v, dot_precision):
         x = x.reshape(n, x.shape[2], head_dim)
         if x.dtype != want:
             x = x.to(want)
-        ops.append(x.contiguous())
+        x = x.contiguous()
+        if x.data_ptr() % 16:
+            raise RuntimeError("dilution attention needs q, k and v on a 16-byte boundary")
+        ops.append(x)
     code = _lib.BF16 if want == torch.bfloat16 else _lib.F32
     return ops, code, _lib.PREC[dot_precision], n
+
+
+def _upstream(dout, n, seq, head_dim, keep_bf16):
+    """The upstream gradient as the backward's kernels read it: contiguous (n, t, d) rows that start on a 16-byte boundary
+    (a slice need not), fp32, or bf16 if it is and keep_bf16."""
+    dout = dout.reshape(n, seq, head_dim)
+    if not (keep_bf16 and dout.dtype == torch.bfloat16):
+        dout = dout.float()
+    dout = dout.contiguous()
+    return dout if dout.data_ptr() % 16 == 0 else dout.clone()
 
 
 def _short_rows(n, seq):
@@ -265,10 +278,7 @@ class _DilutionAttentionFn(torch.autograd.Function):
         # scaled bf16 copy anyway); everything else is widened to fp32 as the reference does
         wide = _lib.wide_path(code, prec, head_dim)
         on_tc = wide or _lib.tensor_core_path(code, prec, head_dim)
-        dof = dout.reshape(n, seq, head_dim)
-        if not (on_tc and dof.dtype == torch.bfloat16):
-            dof = dof.float()
-        dof = dof.contiguous()
+        dof = _upstream(dout, n, seq, head_dim, on_tc)
         do_code = _lib.BF16 if dof.dtype == torch.bfloat16 else _lib.F32
         gdt = torch.bfloat16 if code == _lib.BF16 else torch.float32
         dq, dk, dv = (torch.empty(batch, heads, seq, head_dim, device=dev, dtype=gdt) for _ in range(3))

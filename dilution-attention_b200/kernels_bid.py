@@ -166,7 +166,7 @@ class _VariantFn(torch.autograd.Function):
         lib = _lib.load()
         batch, heads, seq, head_dim = q.shape
         (qf, kf, vf), code, prec, n = K._prepare(q, k, v, dot_precision)
-        dof = dout.reshape(n, seq, head_dim).float().contiguous()
+        dof = K._upstream(dout, n, seq, head_dim, False)
         dq = torch.empty(n, seq, head_dim, device=q.device, dtype=qf.dtype)
         dk, dv = torch.empty_like(dq), torch.empty_like(dq)
         scratch = torch.empty(lib.dilution_backward_scratch_bytes(n, seq, head_dim), device=q.device,

@@ -76,3 +76,21 @@ def test_first_call_in_a_fresh_process(kernels):
     )
     res = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
     assert res.returncode == 0 and "fresh-process ok" in res.stdout, res.stderr[-2000:]
+
+
+@pytest.mark.parametrize("dtype,d,prec", [(torch.float32, 64, "ieee"), (torch.float32, 64, "tf32"), (torch.bfloat16, 64, "bf16"),
+                                          (torch.bfloat16, 128, "bf16"), (torch.bfloat16, 32, "bf16")])
+def test_operands_off_a_16_byte_boundary_are_refused_and_upstream_gradients_copied(kernels, dtype, d, prec):
+    """Every kernel reads its operands 16 bytes at a time."""
+    def off(n):
+        return torch.randn(2 * 70 * d + n, device=DEV).to(dtype)[n:].view(1, 2, 70, d)
+    q, k, v = off(0), off(0), off(0)
+    with pytest.raises(RuntimeError, match="16-byte"):
+        kernels.dilution_attention_forward(q, off(1), v, dot_precision=prec)
+    leaves = [t.requires_grad_(True) for t in (q, k, v)]
+    out = kernels.dilution_attention(*leaves, dot_precision=prec)
+    dout = off(1)
+    got = torch.autograd.grad(out, leaves, dout.to(out.dtype) if dtype == torch.float32 else dout, retain_graph=True)
+    ref = torch.autograd.grad(out, leaves, dout.clone())
+    for a, b in zip(got, ref):
+        assert torch.allclose(a.float(), b.float(), rtol=1e-2, atol=1e-3 * b.abs().max().item())

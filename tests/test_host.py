@@ -132,3 +132,17 @@ def test_variant_install_routes_every_bid_here_and_uninstall_puts_the_module_bac
     assert calls == []
     KB.uninstall(fake)
     assert fake.dilution_attention is original and fake.HAS_TRITON is False
+
+
+@pytest.mark.parametrize("dtype,keep_bf16", [(torch.bfloat16, True), (torch.bfloat16, False), (torch.float32, False)])
+@pytest.mark.parametrize("offset", [0, 1, 3, 8])
+def test_upstream_gradient_is_aligned(dtype, keep_bf16, offset):
+    """The kernels read it 4 to 16 bytes at a time; a contiguous slice may start anywhere."""
+    K = load_package().kernels
+    base = torch.randn(2 * 3 * 16 + 8, dtype=torch.float32).to(dtype)
+    dout = base[offset:offset + 96].view(1, 2, 3, 16)
+    got = K._upstream(dout, 2, 3, 16, keep_bf16)
+    assert got.data_ptr() % 16 == 0 and got.is_contiguous() and torch.equal(got.float(), dout.view(2, 3, 16).float())
+    assert got.dtype == (torch.bfloat16 if keep_bf16 else torch.float32)
+    if offset % 8 == 0 and got.dtype == dtype:
+        assert got.data_ptr() == dout.data_ptr()          # nothing is copied without need
