@@ -22,6 +22,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "once_per_device.cuh"
 #include "tc_common.cuh"
 
 namespace dil {
@@ -1931,30 +1932,16 @@ __global__ void cast_dq_kernel(const float* __restrict__ src, __nv_bfloat16* __r
 // The opt-in to more than 48 KB of dynamic shared memory is per kernel and per device: it is
 // made on the first launch of that kernel on that device and remembered.
 inline int set_smem_attr(const void* fn, int bytes, char* err, size_t errlen) {
-  constexpr int kKernels = 64, kDevices = 64;
-  static std::mutex mu;
-  static const void* fns[kKernels];
-  static bool done[kKernels][kDevices];
+  static OncePerDevice opted_in;
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) dev = -1;
-  int slot = -1;
-  if (dev >= 0) {
-    std::lock_guard<std::mutex> lk(mu);
-    for (int i = 0; i < kKernels && slot < 0; ++i) {
-      if (fns[i] == fn) slot = i;
-      else if (fns[i] == nullptr) { fns[i] = fn; slot = i; }
-    }
-    if (slot >= 0 && done[slot][dev]) return 0;
-  }
+  if (cudaGetDevice(&dev) != cudaSuccess) dev = -1;
+  if (opted_in.done(fn, dev)) return 0;
   const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e != cudaSuccess) {
     snprintf(err, errlen, "cudaFuncSetAttribute(%d): %s", bytes, cudaGetErrorString(e));
     return 3;
   }
-  if (slot >= 0) {
-    std::lock_guard<std::mutex> lk(mu);
-    done[slot][dev] = true;
-  }
+  opted_in.set(fn, dev);
   return 0;
 }
 
