@@ -378,7 +378,7 @@ int launch_decode(const void* q1, const void* kc, const void* vc, int64_t n, int
       attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
       cfg.attrs = attr;
       cfg.numAttrs = 1;
-      Prof prof("decode_scores", st, timing);      // the name that a step has always begun with
+      Prof prof("decode_step", st, timing);
       const cudaError_t e = cudaLaunchKernelEx(
           &cfg, cluster_step_kernel<T, D, MODE>, (const T*)q1, (const T*)kc, (const T*)vc, cap, (int)len, keys,
           scale * dil::kLog2e, eps, committed, (const T*)knew, (const T*)vnew, (T*)const_cast<void*>(kc),

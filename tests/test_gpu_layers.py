@@ -128,7 +128,8 @@ def test_patched_alternating_model_matches_eager(pkg):
     finally:
         pkg.layers.uninstall_layers()
         pkg.uninstall()
-    assert {"split_heads_rope", "merge_heads_rope_grad", "tc_softmax_forward", "decode_scores"} <= names, names
+    assert {"split_heads_rope", "merge_heads_rope_grad", "tc_softmax_forward"} <= names, names
+    assert names & {"decode_step", "decode_scores"}, names      # a step of few keys is one launch
     assert pkg._lib.launch_count() > before
     assert torch.isfinite(got).all()
     assert (got - eager).abs().max().item() < 6e-2
