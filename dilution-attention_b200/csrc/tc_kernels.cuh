@@ -578,9 +578,9 @@ __global__ void __launch_bounds__(256, W != kNarrow ? 2 : row_sum_bid(BID) ? 3 :
 template <int W> constexpr int kMainSmem =
     4 * (int)Rows<W>::kBytes + (1 + 2 * Rows<W>::kPlanes) * (int)kTileBytes + 512 + 128;
 
-// BID / SHARE select the ablations of kernels_bid.py (sigmoid bid; exclusive or absent share step,
-// :254-262); the default instantiation is the operator.
-template <int BID = kBidSoftmax, int SHARE = kShareInclusive>
+// The bids of softmax form: softmax, and expshift, whose log-sum-exp is a constant.  SHARE selects the ablations of
+// kernels_bid.py (exclusive or absent share step, :254-262); the default instantiation is the operator.
+template <int SHARE = kShareInclusive>
 __global__ void __launch_bounds__(256, 2) forward_main_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, Geom g, const float* __restrict__ rmax,
@@ -621,7 +621,7 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
   }
   __syncwarp();
   if (warp == 0) tmem_alloc(smem_u32(&ctl->tmem), kTmem);
-  if (wg == 0) sL[row] = load_lse<BID>(rmax, rden, (int64_t)n * g.tq, ib * kTileRows + row, g.tq, g.lshift);
+  if (wg == 0) sL[row] = load_lse<kBidSoftmax>(rmax, rden, (int64_t)n * g.tq, ib * kTileRows + row, g.tq, g.lshift);
   else {
 #pragma unroll
     for (int c = 0; c < 8; ++c)
@@ -715,7 +715,7 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
             const int e = e8 * 8 + h * 4 + u;
             // two special-function ops per score bind this pass: every fourth exponential of the
             // softmax bid is a polynomial on the FMA pipe (79.7 -> 75.3 ms at the 128K prefill shape)
-            float p = u == 3 ? bid_p<BID, true>(v[e], g.zscale, ls[u]) : bid_p<BID>(v[e], g.zscale, ls[u]);
+            float p = u == 3 ? bid_p<kBidSoftmax, true>(v[e], g.zscale, ls[u]) : bid_p<kBidSoftmax>(v[e], g.zscale, ls[u]);
             if (MASK && (dead || ja > qh + c * 32 + e)) p = 0.f;
             if (SHARE == kShareInclusive) {
               den += p;
@@ -787,7 +787,7 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
 }
 
 // The main pass with its own issuing warp, for rows that leave room for one CTA per SM (W != kNarrow) and the
-// element-wise bids.  The arithmetic is forward_main_kernel's.  A ninth warp issues every copy and product, so that
+// bids of sigmoid form (sigmoid, sigshift).  The arithmetic is forward_main_kernel's.  A ninth warp issues every copy and product, so that
 // no compute warp waits for another one's turn at the tensor pipe: the scores of tile jb + 1 are issued as soon as
 // all warps have read those of tile jb (half of the arithmetic still ahead of them), and share V of tile jb runs under
 // the arithmetic of tile jb + 1, whose first 32 shares per thread wait in registers until it has read the share tile.
@@ -2010,10 +2010,8 @@ inline int colsum_scan(const void* q, const void* k, const Geom& g, const float*
       colsum_scan_kernel<32, BID><<<grid, 256, smem, st>>>(mq, mk, g, rmax, rden, carry_base, carry, total);
     })
   } else {                              // forward-only calls of the operator
-    DIL_TC_PLAIN_BID(g, {
-      if (int rc = set_smem_attr((const void*)colsum_scan_kernel<64, BID>, smem, err, errlen)) return rc;
-      colsum_scan_kernel<64, BID><<<grid, 256, smem, st>>>(mq, mk, g, rmax, rden, carry_base, carry, total);
-    })
+    if (int rc = set_smem_attr((const void*)colsum_scan_kernel<64>, smem, err, errlen)) return rc;
+    colsum_scan_kernel<64><<<grid, 256, smem, st>>>(mq, mk, g, rmax, rden, carry_base, carry, total);
   }
   return launch_status("tc colsum_scan", err, errlen);
 }
@@ -2035,7 +2033,7 @@ inline int forward_main(const void* q, const void* k, const void* v, const Geom&
       if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
       kern<<<grid, kMainThreads, smem, st>>>(mq, mk, mv, g, rmax, rden, carry, carry_base, nullptr, out, ssum);
     } else {
-      auto kern = forward_main_kernel<kBidSoftmax, SHARE>;
+      auto kern = forward_main_kernel<SHARE>;
       if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
       kern<<<grid, 256, smem, st>>>(mq, mk, mv, g, rmax, rden, carry, carry_base, out, ssum);
     }
