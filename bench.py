@@ -23,8 +23,8 @@ Also on the line:
                  heads, 256 steps, heads sharded over ranks) against the measured HBM
                  copy bandwidth;
   other_shapes   (1 GPU) forward + backward at the smaller shapes the reference publishes, and at
-                 an fp32 ("tf32") and a head_dim-128 shape, which run on the fp32 tile kernels with tf32
-                 tensor-core products;
+                 an fp32 ("tf32") and a head_dim-128 shape (`wide_rows`: the tcgen05 kernels' rows of
+                 256 bytes);
   config1_fp32   (1 GPU) BASELINE config 1 on the tile kernels with fp32 FMA products, with the reference's
                  CPU operator at the same shape;
   lm             (1 GPU, when a copy of the reference package is installed under
@@ -300,7 +300,7 @@ def run_triton(args):
         dms = a.elapsed_time(b) / steps
         other = time_other_shapes(rk.dilution_attention, dev)
         try:
-            other_ffma = time_shapes(rk.dilution_attention, dev, TILE_SHAPES, iters=5)
+            other_ffma = time_shapes(rk.dilution_attention, dev, WIDE_SHAPES, iters=5)
         except Exception as e:  # noqa: BLE001
             other_ffma = {"error": f"{type(e).__name__}: {str(e)[:200]}"}
         try:
@@ -327,10 +327,10 @@ def run_triton(args):
 OTHER_SHAPES = ((32, 12, 1024), (8, 8, 4096), (2, 12, 16384))
 
 
-# Shapes that run on the fp32 tile kernels here, with tf32 tensor-core products (fp32 tensors under
-# "tf32", as the model's non-autocast path passes them, and head_dim 128):
+# Shapes that run on the tcgen05 kernels' rows of 256 bytes (fp32 tensors under "tf32", as the model's
+# non-autocast path passes them, as hi + lo planes; bf16 heads of 128):
 # (batch, heads, seq, head_dim, dtype, precision).
-TILE_SHAPES = ((8, 8, 4096, 64, torch.float32, "tf32"), (4, 8, 4096, 128, torch.bfloat16, "bf16"))
+WIDE_SHAPES = ((8, 8, 4096, 64, torch.float32, "tf32"), (4, 8, 4096, 128, torch.bfloat16, "bf16"))
 
 
 def time_shapes(op, dev, shapes, iters=10):
@@ -501,7 +501,7 @@ def run_ours(args):
     K, L = c.K, c.L
     if args.only:
         blocks = {"decode": run_decode, "prefill": run_prefill, "lm": run_lm,
-                  "tile": lambda c_, a_: time_shapes(c_.K.dilution_attention, c_.dev, TILE_SHAPES, iters=3),
+                  "tile": lambda c_, a_: time_shapes(c_.K.dilution_attention, c_.dev, WIDE_SHAPES, iters=3),
                   "variants": lambda c_, a_: time_variants(c_.pkg.kernels_bid.dilution_attention, c_.dev, iters=3)}
         res = blocks[args.only](c, args)
         if c.rank == 0:
@@ -536,7 +536,7 @@ def run_ours(args):
     other = fp32_c1 = None
     if c.world == 1 and not args.no_other:
         other = time_other_shapes(K.dilution_attention, c.dev)
-        other["tile_kernels"] = time_shapes(K.dilution_attention, c.dev, TILE_SHAPES, iters=5)
+        other["wide_rows"] = time_shapes(K.dilution_attention, c.dev, WIDE_SHAPES, iters=5)
         other["variants"] = time_variants(c.pkg.kernels_bid.dilution_attention, c.dev)
         fp32_c1 = run_config1(c)
     sharded = None if args.no_sharded else run_train_sharded(c, args, devt)

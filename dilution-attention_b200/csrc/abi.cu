@@ -894,8 +894,8 @@ int dilution_softmax_decode_append(const void* q1, const void* k1, const void* v
 // bf16 heads of 64 under "bf16" take the tcgen05 kernels; of the f(a) / rowsum(f) bids the three whose f needs no row
 // minimum, from kMassMinSeq tokens on: 780 -> 213 us forward + backward at n = 32, t = 1024 (softplus), 39.2 -> 7.1 ms
 // at t = 8192.  Shorter rows would gain too (tile kernels 350 us at n = 4, t = 512; the host's launches are 200 us of
-// either), but up to 520 tokens the tests hold them to the tile kernels' route; the line is the next tile boundary that
-// leaves that contract alone.
+// either): the line is not where the times meet, it only leaves the route of short rows, which the tests hold up to 520
+// tokens, as it has been.
 constexpr int64_t kMassMinSeq = 5 * 128 + 1;
 static bool tc_variant(int dtype, int precision, int64_t t, int d, int bid, float scale) {
   if (!dil::tc::supported(dtype, precision, d, 0)) return false;

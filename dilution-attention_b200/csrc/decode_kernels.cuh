@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(NT) sweep_kernel(const T* __restrict__ vc, int
 
 // ---- the whole step in one launch, one cluster per (batch, head) row -----------------------------------------
 // For short caches the three launches and the scratch round trips between them are the step: 16 rows of 3001 keys are
-// 2 us of memory traffic and took 9.3 us in a CUDA graph and 30 us called from Python; now 7.2 and 24 us.  A cluster of up to 8 CTAs splits the row's
+// 2 us of memory traffic and took 9.3 us in a CUDA graph; now 7.2 us.  A cluster of up to 8 CTAs splits the row's
 // keys; scores stay in shared memory, chunk statistics and partial outputs cross CTAs through distributed
 // shared memory, and two cluster barriers take the place of the launch boundaries.  Values are those of the three
 // kernels; only partial sums are taken over other chunks.  No scratch.

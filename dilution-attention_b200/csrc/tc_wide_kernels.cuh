@@ -10,10 +10,12 @@
 // kernels in tc_kernels.cuh and tc_rowpass_kernels.cuh; the reverse main pass has a kernel of its own, since the
 // narrow one's accumulators would need 656 of the 512 TMEM columns.
 //
-// Forward + backward at B4 H8 T4096 on one B200, before (tile kernels with tf32 products) and after:
+// Forward + backward at B4 H8 T4096 on one B200, before (tile kernels with tf32 products) and after, the same tensors call
+// after call (other tensors every call: 2.02 and 1.97 ms):
 //   bf16 d = 128  14.8 ms -> 1.93 ms  (reverse pass 7.24 -> 0.94, main pass 3.82 -> 0.31)
 //   fp32 d = 64    7.1 ms -> 1.84 ms  (reverse pass 3.51 -> 0.81, main pass 1.61 -> 0.31)
-// (with single bf16 values bf16 d = 128 takes 1.64 ms, its outputs 1.0e-3 off).  Against 64 bits, 2-norm: bf16 outputs
+// (with single bf16 values bf16 d = 128 takes 1.64 ms, its outputs 1.0e-3 off; with exponentials that lose a NaN and
+// masks that end at the last key only both are 0.9% faster).  Against 64 bits, 2-norm: bf16 outputs
 // 1.3e-4 -> 1.6e-6, gradients 1.7e-3 before and after (their own rounding to bf16); fp32 outputs 2.8e-4 -> about 1e-5.
 #pragma once
 

@@ -106,7 +106,7 @@ def test_bf16_tensors(KB, key, bid, share):
     check_grads(share, (qs.grad, ks.grad, vs.grad), (rdq, rdk, rdv), 2e-2)
 
 
-ROW_SUM = ("relu", "relu2", "softplus", "minshift")     # f(a) / rowsum(f): the tile kernels, always
+ROW_SUM = ("relu", "relu2", "softplus", "minshift")     # f(a) / rowsum(f): the tile kernels up to 640 tokens
 
 
 @pytest.mark.parametrize("seq", [300, 1100, 2049])
@@ -142,7 +142,7 @@ def test_bf16_head_dim_64_runs_on_the_tensor_core_kernels(KB, key, bid, share, s
 
 @pytest.mark.parametrize("key,bid,share", [x for x in VARIANTS if x[1] in ROW_SUM])
 def test_row_sum_bids_on_bf16_heads_of_64_take_the_tile_kernels(KB, key, bid, share):
-    """The four f(a) / rowsum(f) bids have no tcgen05 instantiation: bf16 tensors with heads of 64
+    """The four f(a) / rowsum(f) bids of up to 640 tokens (minshift of any number): bf16 tensors with heads of 64
     run on the tile kernels (tf32 products, exact on bf16 values), with the row statistics, the
     saved jac K product and the key correction of a row-normalised bid."""
     pkg = load_package()
