@@ -102,10 +102,11 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   return r;
 }
 
-// Barrier of every thread of the cluster; what was written before it is visible behind it.
+// Barrier of every thread of the cluster; what was written before it is visible behind it.  Not the .aligned form, which
+// takes whole warps for granted: it stands behind work of thread 0 alone and behind loops of unequal length.
 __device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
 // A float of CTA `rank`'s shared memory, by its address in this CTA's.
 __device__ __forceinline__ float ld_cluster(const float* p, int rank) {

@@ -1,5 +1,6 @@
-"""tcgen05.ld fills its registers asynchronously.  A wait that does not name them lets the compiler use them too early, which
-no run need show: every load in the sources is followed by a wait for the same registers."""
+"""What the sources promise the hardware and no run need show.  tcgen05.ld fills its registers asynchronously, and a wait that
+does not name them lets the compiler use them too early: every load is followed by a wait for the same registers.  The
+.aligned cluster barrier wants whole warps, where the code in front of it has work for thread 0 alone."""
 
 from __future__ import annotations
 
@@ -28,3 +29,9 @@ def test_every_load_has_a_wait_that_names_its_registers(path):
 
 def test_the_sources_are_found():
     assert sum("tmem_ld32(" in open(p).read() for p in SOURCES) >= 4
+
+
+def test_cluster_barriers_do_not_take_whole_warps_for_granted():
+    for path in glob.glob(os.path.join(ROOT, "dilution-attention_b200", "csrc", "*.cuh")):
+        for line in open(path):
+            assert not re.search(r'asm.*barrier\.cluster\..*\.aligned', line), (path, line)
