@@ -151,36 +151,6 @@ dil::Geom make_geom(int64_t n, int64_t tq, int64_t tk, int64_t q_offset, float s
   if ((precision) == DILUTION_PREC_IEEE) { constexpr bool MMA = false; __VA_ARGS__; } \
   else { constexpr bool MMA = true; __VA_ARGS__; }
 
-template <typename T, int D, bool MMA>
-int launch_rowstats(const void* q, const void* k, const dil::Geom& g, float* rmax, float* rden,
-                    cudaStream_t st) {
-  using namespace dil::simt;
-  auto kern = rowstats_kernel<T, D, MMA>;
-  if (int rc = set_smem(kern, smem_rowstats<D>())) return rc;
-  const int nqb = (g.tq + TS - 1) / TS;
-  {
-    Prof prof("simt_rowstats", st);
-    kern<<<(unsigned)(g.n * nqb), NT, smem_rowstats<D>(), st>>>((const T*)q, (const T*)k, g, rmax, rden);
-  }
-  return check_launch("rowstats");
-}
-
-template <typename T, int D, bool MMA>
-int launch_colsum(const void* q, const void* k, const dil::Geom& g, const float* rmax,
-                  const float* rden, const float* base, float* carry, float* total,
-                  cudaStream_t st) {
-  using namespace dil::simt;
-  auto kern = colsum_scan_kernel<T, D, MMA>;
-  if (int rc = set_smem(kern, smem_colsum<D>())) return rc;
-  const int nkb = (g.tk + TS - 1) / TS;
-  {
-    Prof prof("simt_colsum_scan", st);
-    kern<<<(unsigned)(g.n * nkb), NT, smem_colsum<D>(), st>>>((const T*)q, (const T*)k, g, rmax, rden,
-                                                               base, carry, total);
-  }
-  return check_launch("colsum_scan");
-}
-
 // CTAs per block of the FFMA passes (Part in simt_kernels.cuh): the largest power of two up to 8 that keeps the
 // grid within two CTAs per SM and leaves every rank a tile of the longest block.
 int split_of(unsigned grid, int tiles) {
@@ -205,6 +175,39 @@ int launch_split(K kern, unsigned grid, int split, size_t smem, cudaStream_t st,
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
   if (e != cudaSuccess) return fail(DILUTION_ERR_CUDA, "cluster launch: %s", cudaGetErrorString(e));
   return check_launch("cluster launch");
+}
+
+template <typename T, int D, bool MMA>
+int launch_rowstats(const void* q, const void* k, const dil::Geom& g, float* rmax, float* rden,
+                    cudaStream_t st) {
+  using namespace dil::simt;
+  const int nqb = (g.tq + TS - 1) / TS;
+  const unsigned grid = (unsigned)(g.n * nqb);
+  Prof prof("simt_rowstats", st);
+  if (const int split = MMA ? 1 : split_of(grid, nqb); split > 1)
+    return launch_split(rowstats_kernel<T, D, false, true>, grid, split, smem_rowstats<D>(), st, (const T*)q, (const T*)k, g,
+                        rmax, rden, split);
+  auto kern = rowstats_kernel<T, D, MMA>;
+  if (int rc = set_smem(kern, smem_rowstats<D>())) return rc;
+  kern<<<grid, NT, smem_rowstats<D>(), st>>>((const T*)q, (const T*)k, g, rmax, rden, 1);
+  return check_launch("rowstats");
+}
+
+template <typename T, int D, bool MMA>
+int launch_colsum(const void* q, const void* k, const dil::Geom& g, const float* rmax,
+                  const float* rden, const float* base, float* carry, float* total,
+                  cudaStream_t st) {
+  using namespace dil::simt;
+  const int nkb = (g.tk + TS - 1) / TS;
+  const unsigned grid = (unsigned)(g.n * nkb);
+  Prof prof("simt_colsum_scan", st);
+  if (const int split = MMA ? 1 : split_of(grid, (g.tq + TS - 1) / TS); split > 1)
+    return launch_split(colsum_scan_kernel<T, D, false, true>, grid, split, smem_colsum<D>(), st, (const T*)q, (const T*)k,
+                        g, rmax, rden, base, carry, total, split);
+  auto kern = colsum_scan_kernel<T, D, MMA>;
+  if (int rc = set_smem(kern, smem_colsum<D>())) return rc;
+  kern<<<grid, NT, smem_colsum<D>(), st>>>((const T*)q, (const T*)k, g, rmax, rden, base, carry, total, 1);
+  return check_launch("colsum_scan");
 }
 
 template <typename T, int D, bool MMA>

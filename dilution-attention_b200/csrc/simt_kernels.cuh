@@ -26,8 +26,7 @@ constexpr int SL = 68;    // leading dimension of score tiles (4 mod 32: conflic
 
 template <int D> __host__ __device__ constexpr int ld() { return D + 4; }
 
-// SPLIT (FFMA products, few blocks): a cluster of `split` CTAs shares one block of the main, reverse and key-correction
-// passes.  Rank r of the cluster takes a part of the tiles the block would walk through one after the other (about
+// SPLIT (FFMA products, few blocks): a cluster of `split` CTAs shares one block of a pass.  Rank r of the cluster takes a part of the tiles the block would walk through one after the other (about
 // 20 us each in the reverse pass, on a chip that is mostly idle), and the cluster adds up the accumulators through
 // distributed shared memory, each rank a slice of the rows, always in rank order.  The reverse pass is a
 // chain over query tiles by way of the suffix of dk_share: every rank first forms its tiles' sums, the ranks
@@ -315,19 +314,20 @@ __device__ __forceinline__ int first_query_block(int jb, int q_off) {
 
 // ---------------------------------------------------------------- pass 1
 // grid = n * ceil(tq/64), longest rows first.
-template <typename T, int D, bool MMA>
+template <typename T, int D, bool MMA, bool SPLIT = false>
 __global__ void __launch_bounds__(NT) rowstats_kernel(const T* __restrict__ q,
                                                       const T* __restrict__ k, Geom g,
                                                       float* __restrict__ rmax,
-                                                      float* __restrict__ rden) {
+                                                      float* __restrict__ rden, int split) {
+  const Part pt = part_of<SPLIT>(split);
   extern __shared__ __align__(16) float smem[];
   constexpr int LD = ld<D>();
   float* sQ = smem;
   float* sK = sQ + TS * LD;
   float* sS = sK + TS * LD;
   const int nqb = (g.tq + TS - 1) / TS;
-  const int64_t n = blockIdx.x % g.n;
-  const int ib = nqb - 1 - (int)(blockIdx.x / g.n);
+  const int64_t n = pt.block % g.n;
+  const int ib = nqb - 1 - (int)(pt.block / g.n);
   load_tile<T, D, MMA>(sQ, q + n * g.tq * D, ib * TS, g.tq);
 
   const int r = threadIdx.x >> 2, part = threadIdx.x & 3;
@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(NT) rowstats_kernel(const T* __restrict__ q,
   float m = mass ? INFINITY : -INFINITY, s = 0.f;
   const int last_key = min(g.tk - 1, g.q_off + ib * TS + TS - 1);
   const int njb = last_key / TS + 1;
-  for (int jb = 0; jb < njb; ++jb) {
+  for (int jb = pt.rank; jb < njb; jb += pt.size) {
     __syncthreads();
     load_tile<T, D, MMA>(sK, k + n * g.tk * D, jb * TS, g.tk);
     __syncthreads();
@@ -381,6 +381,31 @@ __global__ void __launch_bounds__(NT) rowstats_kernel(const T* __restrict__ q,
     s += __shfl_xor_sync(0xffffffffu, s, 2);
     m = fminf(m, __shfl_xor_sync(0xffffffffu, m, 1));
     m = fminf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+  }
+  if (SPLIT) {
+    __syncthreads();                           // the score tile has been read
+    float *sM = sS, *sSum = sS + TS;
+    if (part == 0) {
+      sM[r] = m;
+      sSum[r] = s;
+    }
+    cluster_sync();
+    if (part == 0) {                           // (every rank forms every row, and stores a slice)
+      for (int o = 0; o < pt.size; ++o) {
+        const float om = ld_cluster(&sM[r], o);
+        m = mass ? fminf(m, om) : fmaxf(m, om);
+      }
+      const float ref = mass || !(m > -INFINITY) ? 0.f : m;
+      s = 0.f;
+      for (int o = 0; o < pt.size; ++o) {
+        const float os = ld_cluster(&sSum[r], o);
+        s += mass ? os : os * pow2<MMA>(ld_cluster(&sM[r], o) - ref);
+      }
+    }
+    cluster_sync();                            // a CTA's shared memory stays until its peers have read it
+    if (r / (TS / pt.size) != pt.rank) return;
+  }
+  if (mass) {
     if (g.bid == kBidMinshift) {
       // sum(a - rmin) over the window (kernels_bid.py:338-340); the rmax buffer holds rmin
       s = fmaxf(s - (float)(min(ia, g.tk - 1) + 1) * m, 0.f);
@@ -398,11 +423,14 @@ __global__ void __launch_bounds__(NT) rowstats_kernel(const T* __restrict__ q,
 // Key-stationary: one CTA per (row n, 64-key block), query blocks in causal
 // order; the running per-key demand is the exclusive scan, written as a
 // checkpoint before each query block.  grid = n * ceil(tk/64).
-template <typename T, int D, bool MMA>
+// SPLIT: rank r takes the r-th run of query tiles, stores its checkpoints without what earlier ranks commit and adds that
+// once the ranks have exchanged their sums.
+template <typename T, int D, bool MMA, bool SPLIT = false>
 __global__ void __launch_bounds__(NT) colsum_scan_kernel(
     const T* __restrict__ q, const T* __restrict__ k, Geom g, const float* __restrict__ rmax,
     const float* __restrict__ rden, const float* __restrict__ carry_base,
-    float* __restrict__ carry, float* __restrict__ total) {
+    float* __restrict__ carry, float* __restrict__ total, int split) {
+  const Part pt = part_of<SPLIT>(split);
   extern __shared__ __align__(16) float smem[];
   constexpr int LD = ld<D>();
   float* sK = smem;
@@ -414,15 +442,17 @@ __global__ void __launch_bounds__(NT) colsum_scan_kernel(
   float* sPart = sU + TS;  // [4][64]
   const int nqb = (g.tq + TS - 1) / TS;
   const int ncb = (g.tq + kCarryRows - 1) / kCarryRows;
-  const int64_t n = blockIdx.x % g.n;
-  const int jb = (int)(blockIdx.x / g.n);
+  const int64_t n = pt.block % g.n;
+  const int jb = (int)(pt.block / g.n);
   load_tile<T, D, MMA>(sK, k + n * g.tk * D, jb * TS, g.tk);
 
   const int col = threadIdx.x & 63, seg = threadIdx.x >> 6;
   const int ja = jb * TS + col;
   const float base = (seg == 0 && carry_base != nullptr && ja < g.tk) ? carry_base[n * g.tk + ja] : 0.f;
   float local = 0.f;
-  for (int ib = first_query_block(jb, g.q_off); ib < nqb; ++ib) {
+  const int first = first_query_block(jb, g.q_off), per = (max(0, nqb - first) + pt.size - 1) / pt.size;
+  const int ib_lo = first + pt.rank * per, ib_hi = min(nqb, ib_lo + per);
+  for (int ib = ib_lo; ib < ib_hi; ++ib) {
     __syncthreads();
     load_tile<T, D, MMA>(sQ, q + n * g.tq * D, ib * TS, g.tq);
     load_stats(sM, sRinv, sU, rmax, rden, n, ib, g);
@@ -447,6 +477,23 @@ __global__ void __launch_bounds__(NT) colsum_scan_kernel(
       }
       local += half0 + (sPart[2 * TS + col] + sPart[3 * TS + col]);
     }
+  }
+  if (SPLIT) {
+    __syncthreads();
+    if (seg == 0) sPart[col] = local;
+    cluster_sync();
+    float before = 0.f;
+    if (seg == 0)
+      for (int r = 0; r < pt.rank; ++r) before += ld_cluster(&sPart[col], r);
+    cluster_sync();            // a CTA's shared memory stays until its peers have read it
+    if (seg == 0 && ja < g.tk && pt.rank > 0) {
+      float* c = carry + (n * ncb + 2 * ib_lo) * (int64_t)g.tk + ja;
+      const int rows = min(ncb, 2 * ib_hi) - 2 * ib_lo;
+#pragma unroll 4
+      for (int r = 0; r < rows; ++r) c[r * (int64_t)g.tk] += before;
+    }
+    if (pt.rank + 1 < pt.size) return;
+    local += before;
   }
   if (seg == 0 && ja < g.tk) total[n * g.tk + ja] = local;
 }
