@@ -284,17 +284,33 @@ __host__ __device__ constexpr uint32_t instr_desc(int m, int n, int a_mn, int b_
          ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
+// Whole warps issue MMAs: every lane runs the issuing code, in step, and the instruction itself is predicated on one elected
+// lane.  An MMA takes its addresses and descriptors from uniform registers; where a single lane runs the code (if (lane == 0))
+// the compiler holds them in ordinary ones and moves each of them over in front of each instruction, 80 cycles per MMA in
+// the row pass (8 of them and the commit: 650 cycles, as uniform code 120; n = 64, T = 8192).  Everything the operands
+// are made of must be uniform in the compiler's eyes too: uniform() for what comes out of memory, uniform_warp() for the
+// branch.  lead: elect_one(), asked once per thread, where the warp is in step.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t uniform(uint32_t x) { return __shfl_sync(0xffffffffu, x, 0); }
+__device__ __forceinline__ int uniform_warp() { return (int)uniform(threadIdx.x >> 5); }
+
 // Arrive on an mbarrier once every MMA issued so far by this thread has completed.
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-               : "memory");
+__device__ __forceinline__ void mma_commit(uint32_t lead, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+      ::"r"(bar), "r"(lead)
+      : "memory");
 }
 
 // A descriptor is kept as two 32-bit halves.  The start address sits in the low half, so
 // stepping through a tile is one 32-bit add of a constant to a value built once outside
-// the loop: the issuing thread's own arithmetic, not the tensor pipe, limits the issue
-// rate of small MMAs (about 45 cycles per instruction back to back, about 100 when each
-// descriptor is rebuilt from an address).
+// the loop.
 struct Desc {
   uint32_t lo, hi;
 };
@@ -304,58 +320,60 @@ __device__ __forceinline__ Desc make_desc(uint32_t saddr, uint32_t lbo_bytes, ui
 }
 // D[tmem] (+)= A[smem] * B[smem]; one instruction covers 16 contraction elements.
 // Offsets are added in descriptor units of 16 bytes.
-__device__ __forceinline__ void mma_ss(uint32_t d_tmem, Desc a, uint32_t a_off16, Desc b, uint32_t b_off16,
+__device__ __forceinline__ void mma_ss(uint32_t lead, uint32_t d_tmem, Desc a, uint32_t a_off16, Desc b, uint32_t b_off16,
                                        uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
       "mov.b64 da, {%1, %2};\n\t"
       "mov.b64 db, {%3, %4};\n\t"
       "setp.ne.b32 p, %6, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}"
+      "setp.ne.b32 q, %7, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}"
       :
       : "r"(d_tmem), "r"(a.lo + a_off16), "r"(a.hi), "r"(b.lo + b_off16), "r"(b.hi), "r"(idesc),
-        "r"(accumulate)
+        "r"(accumulate), "r"(lead)
       : "memory");
 }
 // D[tmem] (+)= A[tmem] * B[smem]: A is an M x 16 bf16 operand held in TMEM, row m on
 // lane m, two consecutive contraction elements per 32-bit column (8 columns).
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, Desc b, uint32_t b_off16,
+__device__ __forceinline__ void mma_ts(uint32_t lead, uint32_t d_tmem, uint32_t a_tmem, Desc b, uint32_t b_off16,
                                        uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 db;\n\t"
       "mov.b64 db, {%2, %3};\n\t"
       "setp.ne.b32 p, %5, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
+      "setp.ne.b32 q, %6, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
       :
-      : "r"(d_tmem), "r"(a_tmem), "r"(b.lo + b_off16), "r"(b.hi), "r"(idesc), "r"(accumulate)
+      : "r"(d_tmem), "r"(a_tmem), "r"(b.lo + b_off16), "r"(b.hi), "r"(idesc), "r"(accumulate), "r"(lead)
       : "memory");
 }
 
 // S[128 x n_cols] = A[128 rows] * B[n_cols rows]^T over the features of a row, both K-major: four instructions per
 // pair of sub-tiles, which lie a_sub and b_sub bytes apart.
 template <int W>
-__device__ __forceinline__ void mma_scores_wide(uint32_t d_tmem, Desc a, uint32_t a_sub, Desc b, uint32_t b_sub,
+__device__ __forceinline__ void mma_scores_wide(uint32_t lead, uint32_t d_tmem, Desc a, uint32_t a_sub, Desc b, uint32_t b_sub,
                                                 uint32_t idesc) {
 #pragma unroll
   for (int i = 0; i < Rows<W>::kPairs; ++i)
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk)
-      mma_ss(d_tmem, a, (a_sub >> 4) * Rows<W>::pair_a(i) + 2 * kk, b, (b_sub >> 4) * Rows<W>::pair_b(i) + 2 * kk, idesc,
+      mma_ss(lead, d_tmem, a, (a_sub >> 4) * Rows<W>::pair_a(i) + 2 * kk, b, (b_sub >> 4) * Rows<W>::pair_b(i) + 2 * kk, idesc,
              i > 0 || kk > 0);
 }
 // The same of V do'^T.
 template <int W>
-__device__ __forceinline__ void mma_dov_wide(uint32_t d_tmem, Desc a, uint32_t a_sub, Desc b, uint32_t b_sub, uint32_t idesc) {
+__device__ __forceinline__ void mma_dov_wide(uint32_t lead, uint32_t d_tmem, Desc a, uint32_t a_sub, Desc b, uint32_t b_sub, uint32_t idesc) {
 #pragma unroll
   for (int i = 0; i < Rows<W>::kDoPairs; ++i)
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk)
-      mma_ss(d_tmem, a, (a_sub >> 4) * Rows<W>::do_a(i) + 2 * kk, b, (b_sub >> 4) * Rows<W>::do_b(i) + 2 * kk, idesc,
+      mma_ss(lead, d_tmem, a, (a_sub >> 4) * Rows<W>::do_a(i) + 2 * kk, b, (b_sub >> 4) * Rows<W>::do_b(i) + 2 * kk, idesc,
              i > 0 || kk > 0);
 }
 template <int W>
-__device__ __forceinline__ void mma_scores_w(uint32_t d_tmem, uint32_t a_smem, uint32_t b_smem, int n_cols) {
-  mma_scores_wide<W>(d_tmem, make_desc(a_smem, 16, 1024), kTileBytes, make_desc(b_smem, 16, 1024), kTileBytes,
+__device__ __forceinline__ void mma_scores_w(uint32_t lead, uint32_t d_tmem, uint32_t a_smem, uint32_t b_smem, int n_cols) {
+  mma_scores_wide<W>(lead, d_tmem, make_desc(a_smem, 16, 1024), kTileBytes, make_desc(b_smem, 16, 1024), kTileBytes,
                      instr_desc(128, n_cols, 0, 0));
 }
 

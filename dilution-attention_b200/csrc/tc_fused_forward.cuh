@@ -52,6 +52,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) forward_fused_kernel(
   const uint32_t shready = smem_u32(bars + 7), odone = smem_u32(bars + 8); // odone[2]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wg = tid >> 7, row = tid & 127;
+  const int warp_u = uniform_warp();
+  const uint32_t lead = elect_one();
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
   const int ncb = (g.tq + 31) / 32;
   const int n = (int)(blockIdx.x % g.n);
@@ -96,7 +98,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) forward_fused_kernel(
     }
   }
   __syncwarp();
-  const uint32_t tmem = ctl->tmem;
+  const uint32_t tmem = uniform(ctl->tmem);
   const uint32_t tS = tmem, tO = tmem + 256;              // O | rs tile b at tO + 128 b
   const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
 
@@ -113,9 +115,9 @@ __global__ void __launch_bounds__(kFusedThreads, 1) forward_fused_kernel(
     auto issue_scores = [&](int a, int st) {
       const uint32_t off = st * 1024 + a * 512;              // 16-byte units: a tile is 1024, 64 rows 512
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk) mma_ss(tS + 64 * a, dK0, 2 * kk, dQ, off + 2 * kk, id_s, kk > 0);
+      for (int kk = 0; kk < 4; ++kk) mma_ss(lead, tS + 64 * a, dK0, 2 * kk, dQ, off + 2 * kk, id_s, kk > 0);
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk) mma_ss(tS + 128 + 64 * a, dK1, 2 * kk, dQ, off + 2 * kk, id_s, kk > 0);
+      for (int kk = 0; kk < 4; ++kk) mma_ss(lead, tS + 128 + 64 * a, dK1, 2 * kk, dQ, off + 2 * kk, id_s, kk > 0);
     };
     // O | rs of step s-1 from TMEM to global memory: lane = query
     auto read_out = [&](int s1) {
@@ -153,19 +155,19 @@ __global__ void __launch_bounds__(kFusedThreads, 1) forward_fused_kernel(
       const int i = ibq * kTileRows + row;
       if (i < g.tq) atomicAdd(ssum + row_base + i, rs);
     };
-    if (tid == 256) {
+    if (warp_u == 8) {
       mbar_wait(kfull, 0, ctl, &g_status, kErrWaitTma);
       mbar_wait(qfull, 0, ctl, &g_status, kErrWaitTma);
       tc_fence_after();
       issue_scores(0, 0);
-      mma_commit(sdone);
+      mma_commit(lead, sdone);
       issue_scores(1, 0);
-      mma_commit(sdone + 8);
+      mma_commit(lead, sdone + 8);
     }
     __syncwarp();
     for (int s = 0; s < nsteps; ++s) {
       if (s >= 1) read_out(s - 1);
-      if (tid == 256) {
+      if (warp_u == 8) {
         const int b = s & 1;
         if (s + 1 < nsteps) {
           // scores of step s+1, each query half as soon as the compute warps have taken that
@@ -174,21 +176,21 @@ __global__ void __launch_bounds__(kFusedThreads, 1) forward_fused_kernel(
           mbar_wait(sfree, s & 1, ctl, &g_status, kErrWaitTile);
           tc_fence_after();
           issue_scores(0, b ^ 1);
-          mma_commit(sdone);
+          mma_commit(lead, sdone);
           mbar_wait(sfree + 8, s & 1, ctl, &g_status, kErrWaitTile);
           tc_fence_after();
           issue_scores(1, b ^ 1);
-          mma_commit(sdone + 8);
+          mma_commit(lead, sdone + 8);
         }
         mbar_wait(shready, s & 1, ctl, &g_status, kErrWaitTile);
         tc_fence_after();
         const uint32_t tOb = tO + 128 * b;
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) mma_ss(tOb, dSh0, 128 * kk, dV0, 128 * kk, id_o, kk > 0);
+        for (int kk = 0; kk < 8; ++kk) mma_ss(lead, tOb, dSh0, 128 * kk, dV0, 128 * kk, id_o, kk > 0);
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) mma_ss(tOb, dSh1, 128 * kk, dV1, 128 * kk, id_o, 1);
-        mma_commit(odone + 8 * b);
-        if (s + 2 < nsteps) {
+        for (int kk = 0; kk < 8; ++kk) mma_ss(lead, tOb, dSh1, 128 * kk, dV1, 128 * kk, id_o, 1);
+        mma_commit(lead, odone + 8 * b);
+        if (lead && s + 2 < nsteps) {
           // the scores of step s are complete (its shares exist), so its Q stage takes step s+2
           mbar_expect_tx(qfull + 8 * b, kTileBytes);
           tma_load_tile(sQ + kTileBytes * b, &map_q, (ib0 + s + 2) * kTileRows, n, qfull + 8 * b);

@@ -290,6 +290,8 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) rowstats_kernel(con
   const uint32_t kfull = smem_u32(bars), sdone = smem_u32(bars + 2);
 
   const int tid = threadIdx.x, warp = tid >> 5, wg = tid >> 7, row = tid & 127;
+  const int warp_u = uniform_warp();
+  const uint32_t lead = elect_one();
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
   const int n = (int)(blockIdx.x % g.n);
   const int ib = nqb - 1 - (int)(blockIdx.x / g.n);
@@ -306,7 +308,7 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) rowstats_kernel(con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = ctl->tmem;
+  const uint32_t tmem = uniform(ctl->tmem);
 
   if (tid == 0) {
     mbar_expect_tx(kfull, 2 * TB);
@@ -322,11 +324,11 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) rowstats_kernel(con
   const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 64 * wg;
   for (int jb = 0; jb < njb; ++jb) {
     const int b = jb & 1;
-    if (tid == 0) {
+    if (warp_u == 0) {
       mbar_wait(kfull + 8 * b, (jb >> 1) & 1, ctl, &g_status, kErrWaitTma);
       tc_fence_after();
-      mma_scores_w<W>(tmem, sQ, sK0 + TB * b, 128);
-      mma_commit(sdone);
+      mma_scores_w<W>(lead, tmem, sQ, sK0 + TB * b, 128);
+      mma_commit(lead, sdone);
     }
     __syncwarp();
     mbar_wait(sdone, jb & 1, ctl, &g_status, kErrWaitMma);
@@ -437,6 +439,8 @@ __global__ void __launch_bounds__(256, W != kNarrow ? 2 : row_sum_bid(BID) ? 3 :
   const uint32_t qfull = smem_u32(bars), sdone = smem_u32(bars + 2);
 
   const int tid = threadIdx.x, warp = tid >> 5, wg = tid >> 7, row = tid & 127;
+  const int warp_u = uniform_warp();
+  const uint32_t lead = elect_one();
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
   const int ncb = (g.tq + CR - 1) / CR;
   const int n = (int)(blockIdx.x % g.n);
@@ -457,7 +461,7 @@ __global__ void __launch_bounds__(256, W != kNarrow ? 2 : row_sum_bid(BID) ? 3 :
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = ctl->tmem;
+  const uint32_t tmem = uniform(ctl->tmem);
 
   if (tid == 0 && nib > 0) {
     mbar_expect_tx(qfull, 2 * TB);
@@ -494,11 +498,11 @@ __global__ void __launch_bounds__(256, W != kNarrow ? 2 : row_sum_bid(BID) ? 3 :
   const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 64 * wg;
   for (int it = 0; it < nib; ++it) {
     const int ib = ib0 + it, b = it & 1;
-    if (tid == 0) {
+    if (warp_u == 0) {
       mbar_wait(qfull + 8 * b, (it >> 1) & 1, ctl, &g_status, kErrWaitTma);
       tc_fence_after();
-      mma_scores_w<W>(tmem, sK, sQ0 + TB * b, 128);
-      mma_commit(sdone);
+      mma_scores_w<W>(lead, tmem, sK, sQ0 + TB * b, 128);
+      mma_commit(lead, sdone);
     }
     __syncwarp();
     // while the MMA runs: next tile's statistics, and the checkpoints of the previous tile
@@ -607,6 +611,8 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
   const uint32_t kfull = smem_u32(bars), vfull = smem_u32(bars + 2), sdone = smem_u32(bars + 3);
 
   const int tid = threadIdx.x, warp = tid >> 5, wg = tid >> 7, row = tid & 127;
+  const int warp_u = uniform_warp();
+  const uint32_t lead = elect_one();
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
   const int ncb = (g.tq + g.carry_rows - 1) / g.carry_rows;
   const int n = (int)(blockIdx.x % g.n);
@@ -631,7 +637,7 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = ctl->tmem;
+  const uint32_t tmem = uniform(ctl->tmem);
   const uint32_t tS = tmem, tO = tmem + 128, tR = tO + Rows<W>::kCols;
 
   if (tid == 0) {
@@ -644,10 +650,13 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
       mbar_expect_tx(kfull + 8, TB);
       tma_load_rows<W>(sK0 + TB, &map_k, kTileRows, n, kfull + 8);
     }
+  }
+  if (warp_u == 0) {
+    __syncwarp();
     mbar_wait(kfull, 0, ctl, &g_status, kErrWaitTma);
     tc_fence_after();
-    mma_scores_w<W>(tS, sK0, sQ, 128);
-    mma_commit(sdone);
+    mma_scores_w<W>(lead, tS, sK0, sQ, 128);
+    mma_commit(lead, sdone);
   }
   __syncwarp();
 
@@ -741,7 +750,7 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
-    if (tid == 0) {
+    if (warp_u == 0) {
       tc_fence_after();
       mbar_wait(vfull, jb & 1, ctl, &g_status, kErrWaitTma);
       tc_fence_after();
@@ -749,13 +758,13 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
       // descriptors are built once per tile; a k-step is a constant 2048 B (128 units) further
       const Desc dSh = make_desc(sSh, kTileBytes, 1024), dVm = make_desc(sV, kTileBytes, 1024);
 #pragma unroll
-      for (int kk = 0; kk < 8; ++kk) mma_ss(tO, dSh, 128 * kk, dVm, 128 * kk, id_o, (jb > 0 || kk > 0));
+      for (int kk = 0; kk < 8; ++kk) mma_ss(lead, tO, dSh, 128 * kk, dVm, 128 * kk, id_o, (jb > 0 || kk > 0));
       if (jb + 1 < njb) {
         mbar_wait(kfull + 8 * (b ^ 1), ((jb + 1) >> 1) & 1, ctl, &g_status, kErrWaitTma);
         tc_fence_after();
-        mma_scores_w<W>(tS, sK0 + TB * (b ^ 1), sQ, 128);
+        mma_scores_w<W>(lead, tS, sK0 + TB * (b ^ 1), sQ, 128);
       }
-      mma_commit(sdone);
+      mma_commit(lead, sdone);
     }
     __syncwarp();
   }
@@ -849,6 +858,8 @@ __global__ void __launch_bounds__(kMainThreads, W == kNarrow ? 2 : 1) forward_ma
   const uint32_t odone = smem_u32(bars + 4), sfree = smem_u32(bars + 5), shready = smem_u32(bars + 6);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wg = tid >> 7, row = tid & 127;
+  const int warp_u = uniform_warp();
+  const uint32_t lead = elect_one();
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
   const int ncb = (g.tq + g.carry_rows - 1) / g.carry_rows;
   const int n = (int)(blockIdx.x % g.n);
@@ -875,11 +886,11 @@ __global__ void __launch_bounds__(kMainThreads, W == kNarrow ? 2 : 1) forward_ma
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = ctl->tmem;
+  const uint32_t tmem = uniform(ctl->tmem);
   const uint32_t tS = tmem, tO = tmem + 128, tR = tO + Rows<W>::kCols;
 
-  if (warp == 8) {
-    if (lane == 0) {
+  if (warp_u == 8) {
+    if (lead) {
       mbar_expect_tx(kfull, 2 * TB);
       tma_load_rows<W>(sQ, &map_q, ib * kTileRows, n, kfull);
       tma_load_rows<W>(sK0, &map_k, 0, n, kfull);
@@ -889,31 +900,35 @@ __global__ void __launch_bounds__(kMainThreads, W == kNarrow ? 2 : 1) forward_ma
         mbar_expect_tx(kfull + 8, TB);
         tma_load_rows<W>(sK0 + TB, &map_k, kTileRows, n, kfull + 8);
       }
+    }
+    {
       constexpr uint32_t id_s = instr_desc(128, 128, 0, 0), id_o = instr_desc(128, kOCols, 1, 1);
       // descriptors are built once; a k-step of O is a constant 2048 B (128 units) further
       const Desc dK0 = make_desc(sK0, 16, 1024), dK1 = make_desc(sK0 + TB, 16, 1024), dQ = make_desc(sQ, 16, 1024);
       const Desc dSh = make_desc(sSh, kTileBytes, 1024), dVm = make_desc(sV, kTileBytes, 1024);
       mbar_wait(kfull, 0, ctl, &g_status, kErrWaitTma);
       tc_fence_after();
-      mma_scores_wide<W>(tS, dK0, kTileBytes, dQ, kTileBytes, id_s);
-      mma_commit(sdone);
+      mma_scores_wide<W>(lead, tS, dK0, kTileBytes, dQ, kTileBytes, id_s);
+      mma_commit(lead, sdone);
       for (int jb = 0; jb < njb; ++jb) {
         const int b = jb & 1;
         if (jb + 1 < njb) {
           mbar_wait(kfull + 8 * (b ^ 1), ((jb + 1) >> 1) & 1, ctl, &g_status, kErrWaitTma);
           mbar_wait(sfree, jb & 1, ctl, &g_status, kErrWaitTile);
           tc_fence_after();
-          mma_scores_wide<W>(tS, b ? dK0 : dK1, kTileBytes, dQ, kTileBytes, id_s);
-          mma_commit(sdone);
-          if (jb + 2 < njb) {             // the scores of jb have been read, so its K stage is free
+          mma_scores_wide<W>(lead, tS, b ? dK0 : dK1, kTileBytes, dQ, kTileBytes, id_s);
+          mma_commit(lead, sdone);
+          if (lead && jb + 2 < njb) {     // the scores of jb have been read, so its K stage is free
             mbar_expect_tx(kfull + 8 * b, TB);
             tma_load_rows<W>(sK0 + TB * b, &map_k, (jb + 2) * kTileRows, n, kfull + 8 * b);
           }
         }
         if (jb >= 1) {                    // V is free once the previous share V has completed
           mbar_wait(odone, (jb - 1) & 1, ctl, &g_status, kErrWaitMma);
-          mbar_expect_tx(vfull, TB);
-          tma_load_rows<W>(sV, &map_v, jb * kTileRows, n, vfull);
+          if (lead) {
+            mbar_expect_tx(vfull, TB);
+            tma_load_rows<W>(sV, &map_v, jb * kTileRows, n, vfull);
+          }
         }
         mbar_wait(shready, jb & 1, ctl, &g_status, kErrWaitTile);
         mbar_wait(vfull, jb & 1, ctl, &g_status, kErrWaitTma);
@@ -922,8 +937,8 @@ __global__ void __launch_bounds__(kMainThreads, W == kNarrow ? 2 : 1) forward_ma
         for (int pl = 0; pl < P; ++pl)
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)
-            mma_ss(tO, dSh, 2048 * pl + 128 * kk, dVm, 128 * kk, id_o, (jb > 0 || pl > 0 || kk > 0));
-        mma_commit(odone);
+            mma_ss(lead, tO, dSh, 2048 * pl + 128 * kk, dVm, 128 * kk, id_o, (jb > 0 || pl > 0 || kk > 0));
+        mma_commit(lead, odone);
       }
     }
     __syncwarp();
@@ -1332,6 +1347,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
   const uint32_t dqdone = smem_u32(bars + 8);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wg = tid >> 7, row = tid & 127;
+  const int warp_u = uniform_warp();
+  const uint32_t lead = elect_one();
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
   const int ncb = (g.tq + kCarryRows - 1) / kCarryRows;
   const int n = (int)(blockIdx.x % g.n);
@@ -1374,7 +1391,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = ctl->tmem;
+  const uint32_t tmem = uniform(ctl->tmem);
   const uint32_t tS0 = tmem, tDOV0 = tmem + 128, tDV = tmem + 256, tDK = tmem + 320, tDQ = tmem + 384,
                  tG = tmem + 448, tV = tmem + 464;
   const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
@@ -1438,28 +1455,28 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
       constexpr int ODD = decltype(odd_c)::value, ST = decltype(st_c)::value;
       constexpr uint32_t off = ST * 1024 + (ODD ? 0 : 512);
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk) mma_ss(tS0 + 64 * ODD, dKk, 2 * kk, dQk, off + 2 * kk, id_s, kk > 0);
+      for (int kk = 0; kk < 4; ++kk) mma_ss(lead, tS0 + 64 * ODD, dKk, 2 * kk, dQk, off + 2 * kk, id_s, kk > 0);
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk) mma_ts(tDOV0 + 64 * ODD, tV + 8 * kk, dDk, off + 2 * kk, id_s, kk > 0);
+      for (int kk = 0; kk < 4; ++kk) mma_ts(lead, tDOV0 + 64 * ODD, tV + 8 * kk, dDk, off + 2 * kk, id_s, kk > 0);
 #pragma unroll
       for (int kk = 0; PASS == 1 && kk < 4; ++kk)            // + V (lo part of do')^T
-        mma_ts(tDOV0 + 64 * ODD, tV + 8 * kk, make_desc(sPd, 16, 1024), off + 2 * kk, id_s, 1);
+        mma_ts(lead, tDOV0 + 64 * ODD, tV + 8 * kk, make_desc(sPd, 16, 1024), off + 2 * kk, id_s, 1);
     };
-    if (tid == 256) {
+    if (warp_u == 8) {
       mbar_wait(kfull, 0, ctl, &g_status, kErrWaitTma);
       mbar_wait(qfull, 0, ctl, &g_status, kErrWaitTma);
       tc_fence_after();
       issue_scores(std::integral_constant<int, 0>{}, std::integral_constant<int, 0>{});
-      mma_commit(sdone);
+      mma_commit(lead, sdone);
       issue_scores(std::integral_constant<int, 1>{}, std::integral_constant<int, 0>{});
-      mma_commit(sdone + 8);
+      mma_commit(lead, sdone + 8);
     }
     __syncwarp();
     // half-step h = 2s + ODD of step s, whose Q and dO' tiles sit in stage ST = s % 3
     auto half = [&](auto odd_c, auto st_c, int s) {
       constexpr int ODD = decltype(odd_c)::value, ST = decltype(st_c)::value;
       constexpr int ST1 = (ST + 1) % 3, ST2 = (ST + 2) % 3;
-      if (tid == 256) {
+      if (warp_u == 8) {
         mbar_wait(tiles + 8 * ODD, s & 1, ctl, &g_status, kErrWaitTile);
         tc_fence_after();
 #pragma unroll
@@ -1468,14 +1485,14 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
           // warpgroup's 32-column range (warpgroup 1 owns queries 0..31)
           constexpr uint32_t base = ST * 1024 + (ODD ? 0 : 4) * 128;
           const uint32_t col = 64 * ODD + 32 * (kq >> 1) + 8 * (kq & 1);
-          mma_ts(tDV, tS0 + col, dDm, base + 128 * kq, id_kd, 1);
-          mma_ts(tDK, tDOV0 + col, dQm, base + 128 * kq, id_kd, 1);
+          mma_ts(lead, tDV, tS0 + col, dDm, base + 128 * kq, id_kd, 1);
+          mma_ts(lead, tDK, tDOV0 + col, dQm, base + 128 * kq, id_kd, 1);
         }
         if (ODD && PASS != 1) {
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)                    // contraction over the 128 keys
-            mma_ss(tDQ, dPm, 128 * kk, dKm, 128 * kk, id_qd, kk > 0);
-          mma_commit(dqdone);
+            mma_ss(lead, tDQ, dPm, 128 * kk, dKm, 128 * kk, id_qd, kk > 0);
+          mma_commit(lead, dqdone);
         }
         if (s + 1 < nsteps) {                               // half-step h + 2 belongs to step s + 1
           if (!ODD) {
@@ -1484,15 +1501,17 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
           }
           issue_scores(odd_c, std::integral_constant<int, ST1>{});
         }
-        mma_commit(sdone + 8 * ODD);
+        mma_commit(lead, sdone + 8 * ODD);
         if (!ODD && s >= 1 && s + 2 < nsteps) {
           // every MMA of step s-1 has completed once the commit of its second half-step has:
           // its Q and dO' stage takes step s+2
           mbar_wait(sdone + 8, s & 1, ctl, &g_status, kErrWaitMma);
+          if (lead) {
           mbar_expect_tx(qfull + 8 * ST2, kStageTx);
           tma_load_tile(sQ0 + kTileBytes * ST2, &map_q, (nqb - 3 - s) * kTileRows, n, qfull + 8 * ST2);
           tma_load_tile(sD0 + kTileBytes * ST2, &map_do, (nqb - 3 - s) * kTileRows, n, qfull + 8 * ST2);
           if (PASS == 1) tma_load_tile(sPd + kTileBytes * ST2, &map_do, (nqb - 3 - s) * kTileRows, n, qfull + 8 * ST2, 64);
+          }
         }
       }
       __syncwarp();
@@ -1716,6 +1735,8 @@ __global__ void __launch_bounds__(256, 2) backward_correction_kernel(
   const uint32_t qfull = smem_u32(bars), sdone = smem_u32(bars + 2), dqdone = smem_u32(bars + 3);
 
   const int tid = threadIdx.x, warp = tid >> 5, wg = tid >> 7, row = tid & 127;
+  const int warp_u = uniform_warp();
+  const uint32_t lead = elect_one();
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
   const int n = (int)(blockIdx.x % g.n);
   const int jb = (int)(blockIdx.x / g.n);
@@ -1741,7 +1762,7 @@ __global__ void __launch_bounds__(256, 2) backward_correction_kernel(
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = ctl->tmem;
+  const uint32_t tmem = uniform(ctl->tmem);
   const uint32_t tS = tmem, tDK = tmem + 128, tDQ = tmem + 192;
 
   if (tid == 0) {
@@ -1752,10 +1773,13 @@ __global__ void __launch_bounds__(256, 2) backward_correction_kernel(
       mbar_expect_tx(qfull + 8, kTileBytes);
       tma_load_tile(sQ0 + kTileBytes, &map_q, (jb + 1) * kTileRows, n, qfull + 8);
     }
+  }
+  if (warp_u == 0) {
+    __syncwarp();
     mbar_wait(qfull, 0, ctl, &g_status, kErrWaitTma);
     tc_fence_after();
-    mma_scores_w<kNarrow>(tS, sK, sQ0, 128);
-    mma_commit(sdone);
+    mma_scores_w<kNarrow>(lead, tS, sK, sQ0, 128);
+    mma_commit(lead, sdone);
   }
   __syncwarp();
 
@@ -1837,7 +1861,7 @@ __global__ void __launch_bounds__(256, 2) backward_correction_kernel(
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
-    if (tid == 0) {
+    if (warp_u == 0) {
       tc_fence_after();
       constexpr uint32_t id_kd = instr_desc(128, 64, 0, 1), id_qd = instr_desc(128, 64, 1, 1);
       // descriptors are built once per tile; a k-step is a constant 2048 B (128 units) further
@@ -1847,18 +1871,18 @@ __global__ void __launch_bounds__(256, 2) backward_correction_kernel(
       // memory W tile (the staging area of that read-out); dKc takes W from TMEM and runs,
       // with the next scores, under the read-out
 #pragma unroll
-      for (int kk = 0; kk < 8; ++kk) mma_ss(tDQ, dWm, 128 * kk, dKm, 128 * kk, id_qd, kk > 0);
-      mma_commit(dqdone);
+      for (int kk = 0; kk < 8; ++kk) mma_ss(lead, tDQ, dWm, 128 * kk, dKm, 128 * kk, id_qd, kk > 0);
+      mma_commit(lead, dqdone);
 #pragma unroll
       for (int kq = 0; kq < 8; ++kq)
-        mma_ts(tDK, tS + 64 * (kq >> 2) + 32 * ((kq & 3) >> 1) + 8 * (kq & 1), dQm, 128 * kq, id_kd,
+        mma_ts(lead, tDK, tS + 64 * (kq >> 2) + 32 * ((kq & 3) >> 1) + 8 * (kq & 1), dQm, 128 * kq, id_kd,
                (t > 0 || kq > 0));
       if (t + 1 < nsteps) {
         mbar_wait(qfull + 8 * (b ^ 1), ((t + 1) >> 1) & 1, ctl, &g_status, kErrWaitTma);
         tc_fence_after();
-        mma_scores_w<kNarrow>(tS, sK, sQ0 + kTileBytes * (b ^ 1), 128);
+        mma_scores_w<kNarrow>(lead, tS, sK, sQ0 + kTileBytes * (b ^ 1), 128);
       }
-      mma_commit(sdone);
+      mma_commit(lead, sdone);
     }
     __syncwarp();
     mbar_wait(dqdone, t & 1, ctl, &g_status, kErrWaitMma);

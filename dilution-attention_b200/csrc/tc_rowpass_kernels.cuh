@@ -61,6 +61,8 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) rowpass_product_ker
   float* sX = reinterpret_cast<float*>(smem + TB);    // merge area over the K stages: [2][128][half a row]
 
   const int tid = threadIdx.x, warp = tid >> 5, wg = tid >> 7, row = tid & 127;
+  const int warp_u = uniform_warp();
+  const uint32_t lead = elect_one();
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
   const int n = (int)(blockIdx.x % g.n);
   const int ib = nqb - 1 - (int)(blockIdx.x / g.n);
@@ -79,7 +81,7 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) rowpass_product_ker
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = ctl->tmem;
+  const uint32_t tmem = uniform(ctl->tmem);
   const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
   const uint32_t tS = tmem, tO = tmem + 128 + kAcc * wg;      // this warpgroup's accumulator
   {
@@ -106,11 +108,11 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) rowpass_product_ker
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (tid == 0) {
+  if (warp_u == 0) {
     mbar_wait(kfull, 0, ctl, &g_status, kErrWaitTma);
     tc_fence_after();
-    mma_scores_w<W>(tS, sQ, sK0, 128);
-    mma_commit(sdone);
+    mma_scores_w<W>(lead, tS, sQ, sK0, 128);
+    mma_commit(lead, sdone);
   }
   __syncwarp();
 
@@ -219,7 +221,7 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) rowpass_product_ker
     tmem_st_wait();
     tc_fence_before();
     __syncthreads();
-    if (tid == 0) {
+    if (warp_u == 0) {
       tc_fence_after();
       constexpr uint32_t id_pv = instr_desc(128, kAcc, 0, 1);   // A from TMEM (M = queries), B MN-major
       const Desc dB = make_desc(sB0 + TB * st, kTileBytes, 1024);
@@ -229,14 +231,14 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) rowpass_product_ker
         for (int pl = 0; pl < Rows<W>::kPlanes; ++pl)
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)      // 16 keys per instruction: 16 rows of 128 B = 128 units
-            mma_ts(tmem + 128 + kAcc * w, tS + 64 * w + 32 * pl + 8 * kk, dB, 128 * (4 * w + kk), id_pv, 1);
+            mma_ts(lead, tmem + 128 + kAcc * w, tS + 64 * w + 32 * pl + 8 * kk, dB, 128 * (4 * w + kk), id_pv, 1);
       if (jb + 1 < njb) {
         const int sn = (jb + 1) % kRowpassStages;
         mbar_wait(kfull + 8 * sn, ((jb + 1) / kRowpassStages) & 1, ctl, &g_status, kErrWaitTma);
         tc_fence_after();
-        mma_scores_w<W>(tS, sQ, sK0 + TB * sn, 128);
+        mma_scores_w<W>(lead, tS, sQ, sK0 + TB * sn, 128);
       }
-      mma_commit(sdone);
+      mma_commit(lead, sdone);
     }
     __syncwarp();
   }
@@ -351,6 +353,8 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) backward_key_correc
   const uint32_t qfull = smem_u32(bars), sdone = smem_u32(bars + 2);
 
   const int tid = threadIdx.x, warp = tid >> 5, wg = tid >> 7, row = tid & 127;
+  const int warp_u = uniform_warp();
+  const uint32_t lead = elect_one();
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
   const int n = (int)(blockIdx.x % g.n);
   const int jb = (int)(blockIdx.x / g.n);
@@ -374,13 +378,13 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) backward_key_correc
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = ctl->tmem;
+  const uint32_t tmem = uniform(ctl->tmem);
   const uint32_t tS = tmem, tDK = tmem + 64;
   constexpr uint32_t id_s = instr_desc(128, 64, 0, 0), id_kd = instr_desc(128, kAcc, 0, 1);
   // scores of half-step (stage, odd): queries 64*odd.. of the Q tile in that stage (K-major: a
   // row is 128 B)
   auto issue_scores = [&](int stage, int odd) {
-    mma_scores_wide<W>(tS, make_desc(sK, 16, 1024), kTileBytes,
+    mma_scores_wide<W>(lead, tS, make_desc(sK, 16, 1024), kTileBytes,
                        make_desc(sQ0 + TB * stage + 8192 * odd, 16, 1024), kTileBytes, id_s);
   };
 
@@ -392,10 +396,13 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) backward_key_correc
       mbar_expect_tx(qfull + 8, TB);
       tma_load_rows<W>(sQ0 + TB, &map_q, (jb + 1) * kTileRows, n, qfull + 8);
     }
+  }
+  if (warp_u == 0) {
+    __syncwarp();
     mbar_wait(qfull, 0, ctl, &g_status, kErrWaitTma);
     tc_fence_after();
     issue_scores(0, 0);
-    mma_commit(sdone);
+    mma_commit(lead, sdone);
   }
   __syncwarp();
 
@@ -452,14 +459,14 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) backward_key_correc
     tmem_st_wait();
     tc_fence_before();
     __syncthreads();
-    if (tid == 0) {
+    if (warp_u == 0) {
       tc_fence_after();
       const Desc dQm = make_desc(sQ0 + TB * b, kTileBytes, 1024);
 #pragma unroll
       for (int pl = 0; pl < Rows<W>::kPlanes; ++pl)
 #pragma unroll
         for (int kq = 0; kq < 4; ++kq)        // 16 queries per instruction: 16 rows of 128 B = 128 units
-          mma_ts(tDK, tS + 32 * (kq >> 1) + 16 * pl + 8 * (kq & 1), dQm, 128 * (4 * odd + kq), id_kd,
+          mma_ts(lead, tDK, tS + 32 * (kq >> 1) + 16 * pl + 8 * (kq & 1), dQm, 128 * (4 * odd + kq), id_kd,
                  (h > 0 || pl > 0 || kq > 0));
       if (h + 1 < nhalf) {
         if (odd) {                          // the next half-step opens step t+1
@@ -470,7 +477,7 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) backward_key_correc
           issue_scores(b, 1);
         }
       }
-      mma_commit(sdone);
+      mma_commit(lead, sdone);
     }
     __syncwarp();
   }

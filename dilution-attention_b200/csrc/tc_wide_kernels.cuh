@@ -184,6 +184,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
   const uint32_t sdone = smem_u32(bars + 5), tiles = smem_u32(bars + 7), dqdone = smem_u32(bars + 9);   // [2], [2]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wg = tid >> 7, row = tid & 127;
+  const int warp_u = uniform_warp();
+  const uint32_t lead = elect_one();
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
   const int ncb = (g.tq + kCarryRows - 1) / kCarryRows;
   const int n = (int)(blockIdx.x % g.n);
@@ -221,7 +223,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = ctl->tmem;
+  const uint32_t tmem = uniform(ctl->tmem);
   // score stage s at tS + 128 s and tDOV + 128 s
   const uint32_t tS = tmem, tDOV = tmem + 64, tDV = tmem + 128 * NS, tDK = tDV + Rows<W>::kCols, tDQ = tDK + Rows<W>::kCols;
   const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
@@ -264,20 +266,20 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
       const uint32_t col = NS == 2 ? 128 * (h & 1) : 0;
       mbar_wait(qfull + 8 * st, (h / NR) & 1, ctl, &g_status, kErrWaitTma);
       tc_fence_after();
-      mma_scores_wide<W>(tS + col, dKk, kTileBytes, make_desc(sQ0 + HB * st, 16, 1024), HSub, id_s);
-      mma_dov_wide<W>(tDOV + col, dVk, kTileBytes, make_desc(sD0 + HBd * st, 16, 1024), HSub, id_s);
+      mma_scores_wide<W>(lead, tS + col, dKk, kTileBytes, make_desc(sQ0 + HB * st, 16, 1024), HSub, id_s);
+      mma_dov_wide<W>(lead, tDOV + col, dVk, kTileBytes, make_desc(sD0 + HBd * st, 16, 1024), HSub, id_s);
     };
-    if (tid == 256) {
+    if (warp_u == 8) {
       mbar_wait(kfull, 0, ctl, &g_status, kErrWaitTma);
       for (int h = 0; h < NS; ++h) {
         issue_scores(h);
-        mma_commit(sdone + 8 * h);
+        mma_commit(lead, sdone + 8 * h);
       }
     }
     __syncwarp();
     for (int h = 0; h < nhalf; ++h) {
       const int st = h % NR, sc = NS == 2 ? h & 1 : 0;      // stage of q and do', stage of the scores
-      if (tid == 256) {
+      if (warp_u == 8) {
         mbar_wait(tiles + 8 * sc, (h / NS) & 1, ctl, &g_status, kErrWaitTile);
         tc_fence_after();
         const Desc dQm = make_desc(sQ0 + HB * st, HSub, 1024), dDm = make_desc(sD0 + HBd * st, HSub, 1024);
@@ -286,29 +288,29 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
 #pragma unroll
           for (int kq = 0; kq < 4; ++kq) {                    // contraction over the 64 queries, 16 each
             const uint32_t col = 128 * sc + 32 * (kq >> 1) + 16 * pl + 8 * (kq & 1);
-            mma_ts(tDV, tS + col, dDm, 128 * kq, id_kd, 1);
+            mma_ts(lead, tDV, tS + col, dDm, 128 * kq, id_kd, 1);
             if (Rows<W>::kDoParts == 2 && pl == 0)            // share_hi do'_lo; share_lo do'_lo is left out (2^-18)
-              mma_ts(tDV, tS + col, dDm, (HSub >> 4) * Rows<W>::kSub + 128 * kq, id_kd, 1);
-            mma_ts(tDK, tDOV + col, dQm, 128 * kq, id_kd, 1);
+              mma_ts(lead, tDV, tS + col, dDm, (HSub >> 4) * Rows<W>::kSub + 128 * kq, id_kd, 1);
+            mma_ts(lead, tDK, tDOV + col, dQm, 128 * kq, id_kd, 1);
           }
         if (h + NS < nhalf) issue_scores(h + NS);
-        mma_commit(sdone + 8 * sc);
+        mma_commit(lead, sdone + 8 * sc);
 #pragma unroll
         for (int pl = 0; pl < P; ++pl)
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)                      // contraction over the 128 keys
-            mma_ss(tDQ, dKm, 128 * kk, dPm, 1024 * pl + 128 * kk, id_qd, (pl > 0 || kk > 0));
-        mma_commit(dqdone);
+            mma_ss(lead, tDQ, dKm, 128 * kk, dPm, 1024 * pl + 128 * kk, id_qd, (pl > 0 || kk > 0));
+        mma_commit(lead, dqdone);
         if (NS == 1) {
           if (h + 2 < nhalf) {
             // the products that read this stage come before the scores of h + 1, whose commit covers them
             mbar_wait(sdone, (h + 1) & 1, ctl, &g_status, kErrWaitMma);
-            load_stage(h + 2);
+            if (lead) load_stage(h + 2);
           }
         } else if (h >= 1 && h + 3 < nhalf) {
           // the products of h - 1 have completed once the commit behind them has: their stage takes h + 3
           mbar_wait(sdone + 8 * ((h - 1) & 1), ((h - 1) / 2 + 1) & 1, ctl, &g_status, kErrWaitMma);
-          load_stage(h + 3);
+          if (lead) load_stage(h + 3);
         }
       }
       __syncwarp();
