@@ -30,6 +30,7 @@ constexpr int kFusedKeys = 2 * kTileRows;
 // K[2] V[2] ones Q[2] shares[4] staging[2] + lse + barriers
 constexpr int kFusedSmem = 13 * kTileBytes + 2048 + 256 + 1024;
 
+template <bool PAIR>
 __global__ void __launch_bounds__(kFusedThreads, 1) forward_fused_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_out, Geom g,
@@ -235,7 +236,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) forward_fused_kernel(
           for (int e4 = 0; e4 < 8; ++e4) {
             const float4 l = L4[e4];
             const float ls[4] = {l.x, l.y, l.z, l.w};
-            float sh[4];
+            float sh[4], dn[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
               // two special-function ops per score on two warps per scheduler: every fourth
@@ -244,7 +245,14 @@ __global__ void __launch_bounds__(kFusedThreads, 1) forward_fused_kernel(
               float p = u == 3 ? poly_exp2<4>(z) : fast_exp2(z);
               if (MASK && (dead || ja > q0 + e4 * 4 + u)) p = 0.f;
               den += p;
-              sh[u] = p * fast_rcp(den);
+              sh[u] = p;
+              dn[u] = den;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u += 2) {
+              const float2 s2 = mul2(make_float2(sh[u], sh[u + 1]), rcp_two<PAIR>(dn[u], dn[u + 1]));
+              sh[u] = s2.x;
+              sh[u + 1] = s2.y;
             }
             packed[e4 * 2] = pack_bf16(sh[0], sh[1]);
             packed[e4 * 2 + 1] = pack_bf16(sh[2], sh[3]);
@@ -329,13 +337,13 @@ inline int forward_fused(const void* q, const void* k, const void* v, const Geom
   if (int rc = make_map_f32(&mo, out, g.n, g.tq, err, errlen)) return rc;
   constexpr int smem = kFusedSmem;
   static_assert(smem <= 232448, "the fused forward pass fits one SM's shared memory");
-  if (int rc = set_smem_attr((const void*)forward_fused_kernel, smem, err, errlen)) return rc;
+  auto kern = pair_demands(g) ? forward_fused_kernel<true> : forward_fused_kernel<false>;
+  if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
   const int64_t rows = g.n * g.tq;
   cudaMemsetAsync(out, 0, sizeof(float) * (size_t)rows * kHeadDim, st);
   cudaMemsetAsync(ssum, 0, sizeof(float) * (size_t)rows, st);
   const int nsb = (g.tk + kFusedKeys - 1) / kFusedKeys;
-  forward_fused_kernel<<<(unsigned)(g.n * nsb), kFusedThreads, smem, st>>>(mq, mk, mv, mo, g, rmax, rden, carry,
-                                                                         total, ssum);
+  kern<<<(unsigned)(g.n * nsb), kFusedThreads, smem, st>>>(mq, mk, mv, mo, g, rmax, rden, carry, total, ssum);
   return launch_status("tc forward_fused", err, errlen);
 }
 

@@ -212,6 +212,23 @@ __device__ __forceinline__ void store_row32(__nv_bfloat16* dst, const float* m, 
                                                     pack_bf16(m[e + 4], m[e + 5]), pack_bf16(m[e + 6], m[e + 7]));
 }
 
+// 1/a and 1/b, two consecutive demands of a key.  PAIR: from one special-function operation, of which the passes that form
+// shares are short, and the product of the two, instead of two; a NaN b leaves 1/a alone.  For demands between 1e-18 and
+// 1e18 (pair_demands); two more roundings, 1e-7.  Main pass of the sigmoid bid 0.883 -> 0.777 ms (n = 32, T = 8192), of
+// 384 rows of 1024 tokens 206 -> 197 us.  In the reverse passes, whose two warps per scheduler wait for each other
+// rather than for that unit, it loses: 10.5 -> 10.9 ms (n = 64, T = 16384).
+template <bool PAIR>
+__device__ __forceinline__ float2 rcp_two(float a, float b) {
+  if (!PAIR) return make_float2(fast_rcp(a), fast_rcp(b));
+  const float m = fminf(b, 1e18f);
+  const float r = fast_rcp(a * m);
+  return mul2(make_float2(r, r), make_float2(m, a));
+}
+// Whether every demand of a call stays in that range: eps in front, bids of at most 1 (expshift has no row sum: any size).
+inline bool pair_demands(const Geom& g) {
+  return g.eps >= 1e-18f && (g.normalised || g.bid == kBidSigmoid);
+}
+
 // Byte offset of the 16-byte chunk holding queries [q, q+8) of `key` in an
 // MN-major [128 keys][128 queries] bf16 tile (q a multiple of 8): two 64-query
 // sub-tiles of 16 KB, rows of 128 B, 16-byte chunks XOR-swizzled by the row.
@@ -584,7 +601,7 @@ template <int W> constexpr int kMainSmem =
 
 // The bids of softmax form: softmax, and expshift, whose log-sum-exp is a constant.  SHARE selects the ablations of
 // kernels_bid.py (exclusive or absent share step, :254-262); the default instantiation is the operator.
-template <int SHARE = kShareInclusive>
+template <int SHARE = kShareInclusive, bool PAIR = true>
 __global__ void __launch_bounds__(256, 2) forward_main_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, Geom g, const float* __restrict__ rmax,
@@ -718,7 +735,7 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const float ls[4] = {lcur[h].x, lcur[h].y, lcur[h].z, lcur[h].w};
-          float sh[4];
+          float sh[4], dn[4];
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             const int e = e8 * 8 + h * 4 + u;
@@ -728,12 +745,21 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
             if (MASK && (dead || ja > qh + c * 32 + e)) p = 0.f;
             if (SHARE == kShareInclusive) {
               den += p;
-              sh[u] = p * fast_rcp(den);
+              sh[u] = p;
+              dn[u] = den;
             } else if (SHARE == kShareExclusive) {     // earlier queries' demand only
               sh[u] = p * fast_rcp(den);
               den += p;
             } else {                                   // no share step
               sh[u] = p;
+            }
+          }
+          if (SHARE == kShareInclusive) {
+#pragma unroll
+            for (int u = 0; u < 4; u += 2) {
+              const float2 s2 = mul2(make_float2(sh[u], sh[u + 1]), rcp_two<PAIR>(dn[u], dn[u + 1]));
+              sh[u] = s2.x;
+              sh[u + 1] = s2.y;
             }
           }
           packed[h * 2 + 0] = pack_bf16(sh[0], sh[1]);
@@ -829,7 +855,7 @@ __device__ __noinline__ void restore_infinities(float* out, const __nv_bfloat16*
   __syncwarp();
 }
 
-template <int BID = kBidSoftmax, int SHARE = kShareInclusive, int W = kNarrow>
+template <int BID = kBidSoftmax, int SHARE = kShareInclusive, int W = kNarrow, bool PAIR = true>
 __global__ void __launch_bounds__(kMainThreads, W == kNarrow ? 2 : 1) forward_main_async_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, Geom g, const float* __restrict__ rmax,
@@ -1010,7 +1036,15 @@ __global__ void __launch_bounds__(kMainThreads, W == kNarrow ? 2 : 1) forward_ma
               den += p[u];
             } else if (SHARE == kShareInclusive) {
               den += p[u];
-              r[u] = fast_rcp(den);
+              r[u] = den;
+            }
+          }
+          if (SHARE == kShareInclusive) {
+#pragma unroll
+            for (int u = 0; u < 8; u += 2) {
+              const float2 i2 = rcp_two<PAIR>(r[u], r[u + 1]);
+              r[u] = i2.x;
+              r[u + 1] = i2.y;
             }
           }
 #pragma unroll
@@ -1989,6 +2023,10 @@ static_assert(5 * (kRowstatsSmem<kNarrow> + 1024) > 233472 && 5 * (kColsumSmem<k
   if ((g).share == kShareInclusive) { constexpr int SHARE = kShareInclusive; __VA_ARGS__; }        \
   else if ((g).share == kShareExclusive) { constexpr int SHARE = kShareExclusive; __VA_ARGS__; }   \
   else { constexpr int SHARE = kShareNone; __VA_ARGS__; }
+// (only the inclusive share step takes reciprocals of consecutive demands together)
+#define DIL_TC_PAIR(g, SHARE, ...)                                                                       \
+  if (SHARE != kShareInclusive || pair_demands(g)) { constexpr bool PAIR = true; __VA_ARGS__; }          \
+  else { constexpr bool PAIR = SHARE != kShareInclusive; __VA_ARGS__; }
 #define DIL_TC_PLAIN_BID(g, ...)                                               \
   if ((g).bid == kBidSigmoid) { constexpr int BID = kBidSigmoid; __VA_ARGS__; } \
   else { constexpr int BID = kBidSoftmax; __VA_ARGS__; }
@@ -2051,17 +2089,17 @@ inline int forward_main(const void* q, const void* k, const void* v, const Geom&
   static_assert(2 * (smem + 1024) <= 233472 && 3 * (smem + 1024) > 233472, "exactly two CTAs of the main pass fit one SM");
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
   const unsigned grid = (unsigned)(g.n * nqb);
-  DIL_TC_SHARE(g, {
+  DIL_TC_SHARE(g, DIL_TC_PAIR(g, SHARE, {
     if (g.bid == kBidSigmoid) {
-      auto kern = forward_main_async_kernel<kBidSigmoid, SHARE>;
+      auto kern = forward_main_async_kernel<kBidSigmoid, SHARE, kNarrow, PAIR>;
       if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
       kern<<<grid, kMainThreads, smem, st>>>(mq, mk, mv, g, rmax, rden, carry, carry_base, nullptr, out, ssum);
     } else {
-      auto kern = forward_main_kernel<SHARE>;
+      auto kern = forward_main_kernel<SHARE, PAIR>;
       if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
       kern<<<grid, 256, smem, st>>>(mq, mk, mv, g, rmax, rden, carry, carry_base, out, ssum);
     }
-  })
+  }))
   return launch_status("tc forward_main", err, errlen);
 }
 

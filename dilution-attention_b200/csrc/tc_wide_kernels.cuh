@@ -529,7 +529,8 @@ inline int wide_forward(const void* q, const void* k, const void* v, const Geom&
   {
     constexpr int smem = kMainSmem<W>;
     static_assert(smem <= 232448 && 2 * smem > 233472, "one CTA (512 TMEM columns) per SM");
-    auto kern = forward_main_async_kernel<kBidSoftmax, kShareInclusive, W>;
+    auto kern = pair_demands(g) ? forward_main_async_kernel<kBidSoftmax, kShareInclusive, W, true>
+                                : forward_main_async_kernel<kBidSoftmax, kShareInclusive, W, false>;
     if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
     mark("tc_wide_forward_main", st, 0);
     kern<<<grid, kMainThreads, smem, st>>>(m.q, m.k, m.v, g, rmax, rden, carry, nullptr, (const __nv_bfloat16*)v, out,
@@ -614,11 +615,11 @@ inline int mass_forward_main(const void* q, const void* k, const void* v, const 
   constexpr int smem = kMainSmem<kPairs64>;
   static_assert(smem <= 232448 && 2 * smem > 233472, "one CTA (512 TMEM columns) per SM");
   const unsigned grid = (unsigned)(g.n * ((g.tq + kTileRows - 1) / kTileRows));
-  DIL_TC_MASS_BID(g, DIL_TC_SHARE(g, {
-    auto kern = forward_main_async_kernel<BID, SHARE, kPairs64>;
+  DIL_TC_MASS_BID(g, DIL_TC_SHARE(g, DIL_TC_PAIR(g, SHARE, {
+    auto kern = forward_main_async_kernel<BID, SHARE, kPairs64, PAIR>;
     if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
     kern<<<grid, kMainThreads, smem, st>>>(mq, mk, mv, g, rmax, rden, carry, nullptr, (const __nv_bfloat16*)v, out, ssum);
-  }))
+  })))
   return launch_status("tc forward_main", err, errlen);
 }
 
