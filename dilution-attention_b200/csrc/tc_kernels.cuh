@@ -830,7 +830,12 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
 // softplus bid 1.55 -> 1.26 ms (n = 32, T = 8192); with two CTAs: sigmoid bid 0.98 -> 0.89 ms.  The softmax bid of heads
 // of 64 stays on forward_main_kernel: its long rows run at the card's power limit, where this form is 1 to 3% slower
 // (145.2 -> 148 ms for the passes of a 128K prompt, 16 heads).
-constexpr int kMainThreads = 288;
+// Compute warpgroups: with one CTA per SM two are two warps per scheduler, which leave it idle while they wait for each
+// other's hand-over; four take 32 queries of a tile per thread instead of 64 (bf16 heads of 128 0.303 -> 0.277 ms, fp32 heads of
+// 64 0.306 -> 0.277, softplus bid 1.205 -> 1.164 ms at the sizes above, both with reciprocals by pairs).  Where two CTAs share
+// an SM there are four per scheduler already.
+template <int W> constexpr int kMainGroups = W == kNarrow ? 2 : 4;
+template <int W> constexpr int kMainThreads = 128 * kMainGroups<W> + 32;
 
 // Shares as hi + lo make NaN of an infinite value (lo may be negative or 0).  Where an output is NaN and its row sum is not, the
 // value is to blame: the output becomes the sum of the infinities that the row sees, NaN if they are of both signs or a
@@ -856,7 +861,7 @@ __device__ __noinline__ void restore_infinities(float* out, const __nv_bfloat16*
 }
 
 template <int BID = kBidSoftmax, int SHARE = kShareInclusive, int W = kNarrow, bool PAIR = true>
-__global__ void __launch_bounds__(kMainThreads, W == kNarrow ? 2 : 1) forward_main_async_kernel(
+__global__ void __launch_bounds__(kMainThreads<W>, W == kNarrow ? 2 : 1) forward_main_async_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, Geom g, const float* __restrict__ rmax,
     const float* __restrict__ rden, const float* __restrict__ carry,
@@ -864,6 +869,7 @@ __global__ void __launch_bounds__(kMainThreads, W == kNarrow ? 2 : 1) forward_ma
     float* __restrict__ ssum) {
   constexpr uint32_t TB = Rows<W>::kBytes;
   constexpr int P = Rows<W>::kPlanes;
+  constexpr int NW = kMainGroups<W>, CW = kTileRows / NW;      // queries of a tile per thread
   constexpr int kOCols = Rows<W>::kCols + 16;        // O and the row sums: one tile
   constexpr int kTmem = W == kNarrow ? 256 : 512;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -896,8 +902,8 @@ __global__ void __launch_bounds__(kMainThreads, W == kNarrow ? 2 : 1) forward_ma
   if (tid == 0) {
     ctl->abort = 0;
     for (int i = 0; i < 5; ++i) mbar_init(kfull + 8 * i, 1);      // kfull[2], vfull, sdone, odone
-    mbar_init(sfree, 8);
-    mbar_init(shready, 8);
+    mbar_init(sfree, 4 * NW);
+    mbar_init(shready, 4 * NW);
     fence_barrier_init();
   }
   __syncwarp();
@@ -915,7 +921,7 @@ __global__ void __launch_bounds__(kMainThreads, W == kNarrow ? 2 : 1) forward_ma
   const uint32_t tmem = uniform(ctl->tmem);
   const uint32_t tS = tmem, tO = tmem + 128, tR = tO + Rows<W>::kCols;
 
-  if (warp_u == 8) {
+  if (warp_u == 4 * NW) {
     if (lead) {
       mbar_expect_tx(kfull, 2 * TB);
       tma_load_rows<W>(sQ, &map_q, ib * kTileRows, n, kfull);
@@ -969,13 +975,13 @@ __global__ void __launch_bounds__(kMainThreads, W == kNarrow ? 2 : 1) forward_ma
     }
     __syncwarp();
   } else {
-  // the checkpoint row this warpgroup starts from: the one in front of query 0 / query 64 of the block
-  const int rb = (ib * kTileRows + 64 * wg) / g.carry_rows;
-  const bool have_rows = rb < ncb;                 // false only for a ragged last half block
+  // the checkpoint row this warpgroup starts from: the one in front of its first query of the block
+  const int rb = (ib * kTileRows + CW * wg) / g.carry_rows;
+  const bool have_rows = rb < ncb;                 // false only in a ragged last block
   const int64_t carry_row = ((int64_t)n * ncb + (have_rows ? rb : 0)) * g.tk;
-  const float4* L4 = reinterpret_cast<const float4*>(sL + 64 * wg);
-  const uint32_t taddr = tS + ((uint32_t)((warp & 3) * 32) << 16) + 64 * wg;
-  const int qh = q0 + 64 * wg;                     // absolute position of this half's first query
+  const float4* L4 = reinterpret_cast<const float4*>(sL + CW * wg);
+  const uint32_t taddr = tS + ((uint32_t)((warp & 3) * 32) << 16) + CW * wg;
+  const int qh = q0 + CW * wg;                     // absolute position of this warpgroup's first query
   auto load_den = [&](int jbx) {
     const int jx = jbx * kTileRows + row;
     float d = g.eps;
@@ -995,12 +1001,12 @@ __global__ void __launch_bounds__(kMainThreads, W == kNarrow ? 2 : 1) forward_ma
     mbar_wait(sdone, jb & 1, ctl, &g_status, kErrWaitMma);
     tc_fence_after();
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
+    for (int c = 0; c < CW / 32; ++c) {
       float v[32];
       uint32_t packed[16], rest[P == 2 ? 16 : 1];
       tmem_ld32(taddr + 32 * c, v);
       tmem_ld_wait(v);
-      if (c == 1) {
+      if (c == CW / 32 - 1) {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(sfree);
@@ -1061,7 +1067,7 @@ __global__ void __launch_bounds__(kMainThreads, W == kNarrow ? 2 : 1) forward_ma
       if (c == 0 && jb >= 1) mbar_wait(odone, (jb - 1) & 1, ctl, &g_status, kErrWaitMma);
 #pragma unroll
       for (int e8 = 0; e8 < 4; ++e8) {
-        const uint32_t dst = sSh + share_chunk_offset(row, wg * 64 + c * 32 + e8 * 8);
+        const uint32_t dst = sSh + share_chunk_offset(row, wg * CW + c * 32 + e8 * 8);
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(packed[4 * e8]),
                      "r"(packed[4 * e8 + 1]), "r"(packed[4 * e8 + 2]), "r"(packed[4 * e8 + 3])
                      : "memory");
@@ -1077,8 +1083,8 @@ __global__ void __launch_bounds__(kMainThreads, W == kNarrow ? 2 : 1) forward_ma
   }
   mbar_wait(odone, (njb - 1) & 1, ctl, &g_status, kErrWaitMma);
   tc_fence_after();
-  {
-    // lane = query now: each warpgroup stores half of the output columns of row `row`, 32 at a time
+  if (wg < 2) {
+    // lane = query now: each of two warpgroups stores half of the output columns of row `row`, 32 at a time
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     constexpr int kHalf = Rows<W>::kHead / 2;
     const int i = ib * kTileRows + row;
@@ -2093,7 +2099,7 @@ inline int forward_main(const void* q, const void* k, const void* v, const Geom&
     if (g.bid == kBidSigmoid) {
       auto kern = forward_main_async_kernel<kBidSigmoid, SHARE, kNarrow, PAIR>;
       if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
-      kern<<<grid, kMainThreads, smem, st>>>(mq, mk, mv, g, rmax, rden, carry, carry_base, nullptr, out, ssum);
+      kern<<<grid, kMainThreads<kNarrow>, smem, st>>>(mq, mk, mv, g, rmax, rden, carry, carry_base, nullptr, out, ssum);
     } else {
       auto kern = forward_main_kernel<SHARE, PAIR>;
       if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;

@@ -533,7 +533,7 @@ inline int wide_forward(const void* q, const void* k, const void* v, const Geom&
                                 : forward_main_async_kernel<kBidSoftmax, kShareInclusive, W, false>;
     if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
     mark("tc_wide_forward_main", st, 0);
-    kern<<<grid, kMainThreads, smem, st>>>(m.q, m.k, m.v, g, rmax, rden, carry, nullptr, (const __nv_bfloat16*)v, out,
+    kern<<<grid, kMainThreads<W>, smem, st>>>(m.q, m.k, m.v, g, rmax, rden, carry, nullptr, (const __nv_bfloat16*)v, out,
                                            ssum);
     mark("tc_wide_forward_main", st, 1);
   }
@@ -618,7 +618,7 @@ inline int mass_forward_main(const void* q, const void* k, const void* v, const 
   DIL_TC_MASS_BID(g, DIL_TC_SHARE(g, DIL_TC_PAIR(g, SHARE, {
     auto kern = forward_main_async_kernel<BID, SHARE, kPairs64, PAIR>;
     if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
-    kern<<<grid, kMainThreads, smem, st>>>(mq, mk, mv, g, rmax, rden, carry, nullptr, (const __nv_bfloat16*)v, out, ssum);
+    kern<<<grid, kMainThreads<kPairs64>, smem, st>>>(mq, mk, mv, g, rmax, rden, carry, nullptr, (const __nv_bfloat16*)v, out, ssum);
   })))
   return launch_status("tc forward_main", err, errlen);
 }
