@@ -645,12 +645,20 @@ int dilution_forward_main(const void* q, const void* k, const void* v, int dtype
 int dilution_forward_fused(const void* q, const void* k, const void* v, int dtype, int precision, int64_t n,
                            int64_t t, int d, float scale, float eps, const float* rmax, const float* rden,
                            float* carry, float* total, float* out, float* ssum, void* stream) {
+  return dilution_forward_fused_rows(q, k, v, dtype, precision, n, t, d, scale, eps, rmax, rden, 32, carry, total, out, ssum,
+                                     stream);
+}
+
+int dilution_forward_fused_rows(const void* q, const void* k, const void* v, int dtype, int precision, int64_t n,
+                                int64_t t, int d, float scale, float eps, const float* rmax, const float* rden,
+                                int carry_rows, float* carry, float* total, float* out, float* ssum, void* stream) {
   if (int rc = check_common("dilution_forward_fused", dtype, precision, n, t, t, 0, d)) return rc;
   if (!q || !k || !v || !rmax || !rden || !carry || !total || !out || !ssum)
     return fail(DILUTION_ERR_ARG, "dilution_forward_fused: null pointer");
 #if defined(DILUTION_TENSOR_PATH) && DILUTION_TC_HAS_MAIN
   if (dil::tc::supported(dtype, precision, d, 0)) {
-    const dil::Geom g = make_geom(n, t, t, 0, scale, eps, 32);
+    if (int rc = check_carry_rows("dilution_forward_fused", dtype, precision, d, 0, carry_rows)) return rc;
+    const dil::Geom g = make_geom(n, t, t, 0, scale, eps, carry_rows);
     cudaStream_t st = (cudaStream_t)stream;
     {
       Prof prof("tc_forward_fused", st);

@@ -2,21 +2,23 @@
 // (the reference's training forward, _dilution_key_forward + _dilution_normalize,
 // kernels.py:200-248, does the same on its side of the fence).
 //
-// A CTA owns 256 keys (two 128-key halves, one per compute warpgroup; lane = key) and walks
-// the query blocks that can see them in causal order.  The demand of a key is ONE register
-// for the whole sweep, so no checkpoint is read; the checkpoints the backward needs
-// (every 32 query rows) and the demand totals are stored on the way.  Per 128-query step:
-//   S^T  = K Q^T            two 64-query halves per key half (so that the next step's scores run
-//                           under this step's arithmetic): 16 MMAs of N = 64
-//   p, den += p, share      exactly the arithmetic of forward_main_kernel
-//   O | rs = share [V|1]    M = 128 queries, K = 256 keys, N = 80: 16 MMAs, a FRESH tile per step
-// and the O | rs tile is added to `out` / `ssum` in global memory: a third warpgroup
-// (lane = query) moves it from TMEM to a swizzled fp32 staging tile and issues two TMA
-// tensor reductions, the row sums go by atomics.  `out` and `ssum` therefore start at zero and
-// a small kernel divides at the end.  One exponential and one QK^T sweep per score less than
+// A CTA owns 512 keys, 128 per compute warpgroup (lane = key), and walks the queries that can see them in causal
+// order, 64 at a time.  The demand of a key is ONE register for the whole sweep, so no checkpoint is read; the checkpoints that
+// the backward needs (every 32 query rows, or 64) and the demand totals are stored on the way.  Per half tile of 64 queries and
+// warpgroup:
+//   S^T  = K Q^T            A = the keys' rows in TMEM, written there once: 4 MMAs of N = 64
+//   p, den += p, share      exactly the arithmetic of forward_main_kernel, 64 queries per thread
+//   O^T | rs                = [V | 1]^T share, M = 64 features and 64 copies of the row sums, K = 128 keys, N = 64: 8 MMAs into a
+//                           FRESH tile per half tile that all four warpgroups add to
+// and the tile is added to `out` / `ssum` in global memory: two warps of a fifth warpgroup (lane = feature) move it from TMEM
+// to a staging tile and issue a TMA tensor reduction each, the row sums go by atomics from the other two.  `out` and `ssum`
+// therefore start at zero and a small kernel divides at the end.  One exponential and one QK^T sweep per score less than
 // column-sum pass + query-stationary main pass.
 //
-// 384 threads, one CTA per SM (TMEM: S^T 256 columns, two O | rs tiles of 80).  Thread 256
+// Four warpgroups are four warps per scheduler.  They fit because the keys are a TMEM operand and O comes out transposed
+// (64 columns): S^T 4 x 64, K 4 x 32, O^T 2 x 64 = 512 columns, V + ones + shares + q + staging = 192 KB.  Two warpgroups of 128
+// keys with S^T double-buffered took 6.5 ms at n = 64, T = 16384 (now 6.1) and left the special-function unit idle
+// whenever both waited; output tiles are added half as often.  640 threads, one CTA per SM; a fifth-warpgroup warp
 // issues every TMA copy and MMA.  Every wait is bounded.
 #pragma once
 
@@ -25,58 +27,53 @@
 namespace dil {
 namespace tc {
 
-constexpr int kFusedThreads = 384;
-constexpr int kFusedKeys = 2 * kTileRows;
-// K[2] V[2] ones Q[2] shares[4] staging[2] + lse + barriers
-constexpr int kFusedSmem = 13 * kTileBytes + 2048 + 256 + 1024;
+constexpr int kFusedRing = 4;                              // half tiles of q
+// V[G] ones shares[G] | Q[4] (8 KB each) | staging (16 KB) | lse [4][64] | barriers
+template <int G> constexpr int kFusedSmem = (2 * G + 1) * kTileBytes + kFusedRing * kTileBytes / 2 + kTileBytes + 1024 + 256 + 1024;
 
-template <bool PAIR>
-__global__ void __launch_bounds__(kFusedThreads, 1) forward_fused_kernel(
-    const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-    const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_out, Geom g,
+// G: compute warpgroups of 128 keys.  CR: query rows per checkpoint.
+template <int G, int CR, bool PAIR>
+__global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_kernel(
+    const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_v,
+    const __grid_constant__ CUtensorMap map_out, Geom g, const __nv_bfloat16* __restrict__ k,
     const float* __restrict__ rmax, const float* __restrict__ rden, float* __restrict__ carry,
     float* __restrict__ total, float* __restrict__ ssum) {
+  constexpr int R = kFusedRing, kTmem = G == 1 ? 256 : 512;
+  constexpr uint32_t HB = kTileBytes / 2;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
-  const uint32_t sK = smem_u32(smem);                       // [2] K-major
-  const uint32_t sV = sK + 2 * kTileBytes;                  // [2], then the ones tile: [V | 1] MN-major
-  const uint32_t sOnes = sK + 4 * kTileBytes;
-  uint8_t* ones_ptr = smem + 4 * kTileBytes;
-  const uint32_t sQ = sK + 5 * kTileBytes;                  // [2] stages
-  const uint32_t sSh = sK + 7 * kTileBytes;                 // [2 key halves][2 query halves] MN-major shares
-  const uint32_t sStage = sK + 11 * kTileBytes;             // 32 KB fp32 O tile for the reductions
-  float* sL = reinterpret_cast<float*>(smem + 13 * kTileBytes);            // [2 warpgroups][2][128] lse of a step's queries
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 13 * kTileBytes + 2048);
-  Ctl* ctl = reinterpret_cast<Ctl*>(bars + 16);
-  const uint32_t kfull = smem_u32(bars), qfull = smem_u32(bars + 1);       // qfull[2]
-  const uint32_t sdone = smem_u32(bars + 3), sfree = smem_u32(bars + 5);   // [2] each: query halves
-  const uint32_t shready = smem_u32(bars + 7), odone = smem_u32(bars + 8); // odone[2]
+  const uint32_t sV = smem_u32(smem), sOnes = sV + G * kTileBytes;           // A of O^T: [V | ones], MN-major
+  uint8_t* ones_ptr = smem + G * kTileBytes;
+  const uint32_t sSh = sOnes + kTileBytes;                                   // [G][128 keys][64 queries]
+  const uint32_t sQ = sSh + G * kTileBytes, sStage = sQ + R * HB;            // staging: [2 warps][64 queries][32 features] fp32
+  float* sL = reinterpret_cast<float*>(smem + (sStage - sV) + kTileBytes);   // [4][64] lse of a half tile's queries
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sL + 256);
+  const uint32_t vfull = smem_u32(bars), qfull = vfull + 8, ofull = qfull + 8 * R;            // 1, [R], [2]
+  const uint32_t sdone = ofull + 16, odone = sdone + 8 * G, sfree = odone + 8 * G, shready = sfree + 8 * G;   // [G] each
+  Ctl* ctl = reinterpret_cast<Ctl*>(bars + 3 + R + 4 * G);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wg = tid >> 7, row = tid & 127;
   const int warp_u = uniform_warp();
   const uint32_t lead = elect_one();
-  const int nqb = (g.tq + kTileRows - 1) / kTileRows;
-  const int ncb = (g.tq + 31) / 32;
+  const int ncb = (g.tq + CR - 1) / CR;
   const int n = (int)(blockIdx.x % g.n);
-  const int kb = (int)(blockIdx.x / g.n);
-  const int k0 = kb * kFusedKeys;
-  const int ib0 = 2 * kb;                       // first query block that sees these keys
-  const int nsteps = nqb - ib0;                 // >= 1
+  const int k0 = (int)(blockIdx.x / g.n) * (G * kTileRows);
+  const int h0 = k0 / 64, nh = (g.tq + 63) / 64;          // half tiles of queries; warpgroup w sees those from h0 + 2 w on
+  const int groups = min(G, (g.tk - k0 + kTileRows - 1) / kTileRows);
   const int64_t row_base = (int64_t)n * g.tq;
 
   if (tid == 0) {
     ctl->abort = 0;
-    for (int i = 0; i < 5; ++i) mbar_init(kfull + 8 * i, 1);        // kfull, qfull[2], sdone[2]
-    mbar_init(sfree, 8);
-    mbar_init(sfree + 8, 8);
-    mbar_init(shready, 8);
-    mbar_init(odone, 1);
-    mbar_init(odone + 8, 1);
+    for (int i = 0; i < 3 + R + 2 * G; ++i) mbar_init(vfull + 8 * i, 1);
+    for (int i = 0; i < 2 * G; ++i) mbar_init(sfree + 8 * i, 4);
     fence_barrier_init();
   }
   __syncwarp();
-  if (warp == 0) tmem_alloc(smem_u32(&ctl->tmem), 512);
-  if (wg == 1) {
+  if (warp == 0) tmem_alloc(smem_u32(&ctl->tmem), kTmem);
+  if (wg == G) {
+    sL[row] = load_lse(rmax, rden, row_base, h0 * 64 + row, g.tq);         // of the first three half tiles
+  } else if (wg == 0) {
+    if (row < 64) sL[128 + row] = load_lse(rmax, rden, row_base, h0 * 64 + 128 + row, g.tq);
 #pragma unroll
     for (int c = 0; c < 8; ++c)
       reinterpret_cast<uint4*>(ones_ptr)[row * 8 + c] = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
@@ -85,151 +82,168 @@ __global__ void __launch_bounds__(kFusedThreads, 1) forward_fused_kernel(
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  // only now: the barriers these copies complete on were initialised by thread 0, and nothing but
-  // the CTA-wide barrier above orders that against another warp's use of them
-  if (tid == 256) {
-    mbar_expect_tx(kfull, 4 * kTileBytes);
-    tma_load_tile(sK, &map_k, k0, n, kfull);
-    tma_load_tile(sK + kTileBytes, &map_k, k0 + kTileRows, n, kfull);
-    tma_load_tile(sV, &map_v, k0, n, kfull);
-    tma_load_tile(sV + kTileBytes, &map_v, k0 + kTileRows, n, kfull);
-    for (int s = 0; s < 2 && s < nsteps; ++s) {
-      mbar_expect_tx(qfull + 8 * s, kTileBytes);
-      tma_load_tile(sQ + kTileBytes * s, &map_q, (ib0 + s) * kTileRows, n, qfull + 8 * s);
-    }
-  }
-  __syncwarp();
   const uint32_t tmem = uniform(ctl->tmem);
-  const uint32_t tS = tmem, tO = tmem + 256;              // O | rs tile b at tO + 128 b
+  const uint32_t tS = tmem, tK = tmem + 64 * G, tO = tmem + 96 * G;        // O^T tile b at tO + 64 b
   const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-
-  if (wg == 2) {
-    // ------------------------------------------------------------ issue, and the O read-out
-    constexpr uint32_t id_s = instr_desc(128, 64, 0, 0);     // scores: both operands K-major
-    constexpr uint32_t id_o = instr_desc(128, 80, 1, 1);     // O | rs: A and B MN-major
-    const Desc dK0 = make_desc(sK, 16, 1024), dK1 = make_desc(sK + kTileBytes, 16, 1024);
-    const Desc dQ = make_desc(sQ, 16, 1024);
-    const Desc dSh0 = make_desc(sSh, kTileBytes, 1024), dSh1 = make_desc(sSh + 2 * kTileBytes, kTileBytes, 1024);
-    const Desc dV0 = make_desc(sV, sOnes - sV, 1024);
-    const Desc dV1 = make_desc(sV + kTileBytes, sOnes - (sV + kTileBytes), 1024);
-    // scores of query half `a` of the step whose Q tile sits in stage `st`, both key halves
-    auto issue_scores = [&](int a, int st) {
-      const uint32_t off = st * 1024 + a * 512;              // 16-byte units: a tile is 1024, 64 rows 512
+  const int ja = k0 + wg * kTileRows + row;
+  const bool dead = ja >= g.tk;
+  if (wg < G) {
+    // this key's row as an A operand: two head-dim elements per 32-bit column
+    uint32_t w[32];
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk) mma_ss(lead, tS + 64 * a, dK0, 2 * kk, dQ, off + 2 * kk, id_s, kk > 0);
-#pragma unroll
-      for (int kk = 0; kk < 4; ++kk) mma_ss(lead, tS + 128 + 64 * a, dK1, 2 * kk, dQ, off + 2 * kk, id_s, kk > 0);
-    };
-    // O | rs of step s-1 from TMEM to global memory: lane = query
-    auto read_out = [&](int s1) {
-      const int b = s1 & 1;
-      if (lane == 0) mbar_wait(odone + 8 * b, (s1 >> 1) & 1, ctl, &g_status, kErrWaitMma);
-      __syncwarp();
-      tc_fence_after();
-      if (tid == 256) tma_wait_read_all();                   // the previous reductions have read the staging tile
-      asm volatile("bar.sync 2, 128;" ::: "memory");
-      const uint32_t stage = sStage + row * 128;
-      const uint32_t tOb = tO + 128 * b + lane_base;
-#pragma unroll 1
-      for (int j = 0; j < 4; ++j) {                          // 16 columns at a time
-        float o[16];
-        tmem_ld16(tOb + 16 * j, o);
-        tmem_ld_wait16(o);
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-          asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(stage + kTileBytes * (j >> 1) + (((4 * (j & 1) + c) ^ (row & 7)) << 4)),
-                       "f"(o[4 * c]), "f"(o[4 * c + 1]), "f"(o[4 * c + 2]), "f"(o[4 * c + 3])
-                       : "memory");
-      }
-      float rs;
-      tmem_ld1(tOb + 64, &rs);
-      tmem_ld_wait1(&rs);
-      fence_async_smem();
-      tc_fence_before();
-      asm volatile("bar.sync 2, 128;" ::: "memory");         // every warp has read the tile: its buffer is free
-      const int ibq = ib0 + s1;
-      if (tid == 256) {
-        tc_fence_after();
-        tma_reduce_add_tile(&map_out, sStage, 0, ibq * kTileRows, n);
-        tma_reduce_add_tile(&map_out, sStage + kTileBytes, 32, ibq * kTileRows, n);
-      }
-      const int i = ibq * kTileRows + row;
-      if (i < g.tq) atomicAdd(ssum + row_base + i, rs);
-    };
-    if (warp_u == 8) {
-      mbar_wait(kfull, 0, ctl, &g_status, kErrWaitTma);
-      mbar_wait(qfull, 0, ctl, &g_status, kErrWaitTma);
-      tc_fence_after();
-      issue_scores(0, 0);
-      mma_commit(lead, sdone);
-      issue_scores(1, 0);
-      mma_commit(lead, sdone + 8);
+    for (int c = 0; c < 8; ++c) {
+      uint4 x = make_uint4(0u, 0u, 0u, 0u);
+      if (!dead) x = reinterpret_cast<const uint4*>(k + ((int64_t)n * g.tk + ja) * kHeadDim)[c];
+      w[4 * c] = x.x; w[4 * c + 1] = x.y; w[4 * c + 2] = x.z; w[4 * c + 3] = x.w;
     }
     __syncwarp();
-    for (int s = 0; s < nsteps; ++s) {
-      if (s >= 1) read_out(s - 1);
-      if (warp_u == 8) {
-        const int b = s & 1;
-        if (s + 1 < nsteps) {
-          // scores of step s+1, each query half as soon as the compute warps have taken that
-          // half of step s out of TMEM
-          mbar_wait(qfull + 8 * (b ^ 1), ((s + 1) >> 1) & 1, ctl, &g_status, kErrWaitTma);
-          mbar_wait(sfree, s & 1, ctl, &g_status, kErrWaitTile);
-          tc_fence_after();
-          issue_scores(0, b ^ 1);
-          mma_commit(lead, sdone);
-          mbar_wait(sfree + 8, s & 1, ctl, &g_status, kErrWaitTile);
-          tc_fence_after();
-          issue_scores(1, b ^ 1);
-          mma_commit(lead, sdone + 8);
-        }
-        mbar_wait(shready, s & 1, ctl, &g_status, kErrWaitTile);
-        tc_fence_after();
-        const uint32_t tOb = tO + 128 * b;
+    tmem_st16(tK + 32 * wg + lane_base, w);
+    tmem_st16(tK + 32 * wg + lane_base + 16, w + 16);
+    tmem_st_wait();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+
+  if (wg == G) {
+    // ------------------------------------------------------------ issue, and the O read-out
+    // (registers of G = 4: 5 x 96 at launch, then 4 x 104 + 64)
+    if (G == 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    constexpr uint32_t id_s = instr_desc(128, 64, 0, 0);     // scores: A from TMEM, B K-major
+    constexpr uint32_t id_o = instr_desc(128, 64, 1, 1);     // O^T: A and B MN-major
+    const Desc dQ = make_desc(sQ, 16, 1024), dSh = make_desc(sSh, kTileBytes, 1024);
+    const bool issuer = warp_u == 4 * G;
+    auto load_q = [&](int h) {
+      const int st = (h - h0) % R;
+      if (!lead) return;
+      mbar_expect_tx(qfull + 8 * st, HB);
+      tma_load_tile(sQ + HB * st, &map_q, h * 64, n, qfull + 8 * st);
+    };
+    auto issue_scores = [&](int w, int h) {
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) mma_ss(lead, tOb, dSh0, 128 * kk, dV0, 128 * kk, id_o, kk > 0);
+      for (int kk = 0; kk < 4; ++kk)
+        mma_ts(lead, tS + 64 * w, tK + 32 * w + 8 * kk, dQ, (HB >> 4) * ((h - h0) % R) + 2 * kk, id_s, kk > 0);
+      mma_commit(lead, sdone + 8 * w);
+    };
+    // O^T of half tile h, lane = feature (and the row sums on the lanes behind them), to global memory.  On the way, the
+    // lse of h + 3: the barrier of the four warps and the scores of h + 3 lie between the store and the use, the
+    // hand-over of h, which ofull waits for, behind the last use of the slot (h - 1).
+    auto read_out = [&](int h) {
+      float nx_max = INFINITY, nx_den = 1.f;
+      const int i3 = (h + 3) * 64 + row;
+      const bool fetch = row < 64 && h + 3 < nh;
+      if (fetch && i3 < g.tq) {
+        nx_max = rmax[row_base + i3];
+        nx_den = rden[row_base + i3];
+      }
+      const int u = h - h0, w4 = warp & 3;
+      if (lane == 0) mbar_wait(ofull + 8 * (u & 1), (u >> 1) & 1, ctl, &g_status, kErrWaitMma);
+      __syncwarp();
+      tc_fence_after();
+      if (fetch) sL[64 * ((u + 3) & 3) + row] = nx_max + log2f(nx_den);
+      __syncwarp();
+      const uint32_t tOb = tO + 64 * (u & 1) + lane_base;
+      if (w4 < 2) {
+        const uint32_t stage = sStage + HB * w4;
+        if (lane == 0) tma_wait_read_all();                  // the previous reduction has read this warp's staging
+        __syncwarp();
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) mma_ss(lead, tOb, dSh1, 128 * kk, dV1, 128 * kk, id_o, 1);
-        mma_commit(lead, odone + 8 * b);
-        if (lead && s + 2 < nsteps) {
-          // the scores of step s are complete (its shares exist), so its Q stage takes step s+2
-          mbar_expect_tx(qfull + 8 * b, kTileBytes);
-          tma_load_tile(sQ + kTileBytes * b, &map_q, (ib0 + s + 2) * kTileRows, n, qfull + 8 * b);
+        for (int c = 0; c < 4; ++c) {
+          float o[16];
+          tmem_ld16(tOb + 16 * c, o);
+          tmem_ld_wait16(o);
+#pragma unroll
+          for (int e = 0; e < 16; ++e)
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(stage + lane * 4 + (16 * c + e) * 128), "f"(o[e]) : "memory");
         }
+        fence_async_smem();
+        __syncwarp();
+        if (lane == 0) tma_reduce_add_tile(&map_out, stage, 32 * w4, h * 64, n);
+      } else {
+        // any of these lanes holds the row sums of all queries: lane l takes query 32 (w4 - 2) + l
+        float rs = 0.f;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          float o[16];
+          tmem_ld16(tOb + 32 * (w4 - 2) + 16 * c, o);
+          tmem_ld_wait16(o);
+#pragma unroll
+          for (int e = 0; e < 16; ++e) rs = lane == 16 * c + e ? o[e] : rs;
+        }
+        const int i = h * 64 + 32 * (w4 - 2) + lane;
+        if (i < g.tq) atomicAdd(ssum + row_base + i, rs);
+        __syncwarp();
+      }
+      tc_fence_before();
+      __syncwarp();
+      asm volatile("bar.sync 2, 128;" ::: "memory");         // every warp has read the tile: its buffer is free
+      tc_fence_after();
+    };
+    if (issuer) {
+      if (lead) {
+        mbar_expect_tx(vfull, groups * kTileBytes);
+        for (int w = 0; w < groups; ++w) tma_load_tile(sV + kTileBytes * w, &map_v, k0 + w * kTileRows, n, vfull);
+      }
+      for (int h = h0; h < h0 + R && h < nh; ++h) load_q(h);
+      mbar_wait(qfull, 0, ctl, &g_status, kErrWaitTma);
+      tc_fence_after();
+      issue_scores(0, h0);
+      mbar_wait(vfull, 0, ctl, &g_status, kErrWaitTma);
+    }
+    __syncwarp();
+    for (int h = h0; h < nh; ++h) {
+      const int u = h - h0;
+      if (h > h0) read_out(h - 1);
+      if (issuer) {
+        if (h + 1 < nh) {
+          // scores of h + 1, as soon as a warpgroup has taken those of h out of TMEM
+          mbar_wait(qfull + 8 * ((u + 1) % R), ((u + 1) / R) & 1, ctl, &g_status, kErrWaitTma);
+          for (int w = 0; w < groups; ++w) {
+            const int t = u - 2 * w;                         // the warpgroup's own count of half tiles
+            if (t + 1 < 0) break;
+            if (t >= 0) mbar_wait(sfree + 8 * w, t & 1, ctl, &g_status, kErrWaitTile);
+            tc_fence_after();
+            issue_scores(w, h + 1);
+          }
+        }
+        for (int w = 0; w < groups; ++w) {
+          const int t = u - 2 * w;
+          if (t < 0) break;
+          mbar_wait(shready + 8 * w, t & 1, ctl, &g_status, kErrWaitTile);
+          tc_fence_after();
+          const Desc dVw = make_desc(sV + kTileBytes * w, sOnes - sV - kTileBytes * w, 1024);
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)
+            mma_ss(lead, tO + 64 * (u & 1), dVw, 128 * kk, dSh, 1024 * w + 128 * kk, id_o, w > 0 || kk > 0);
+          mma_commit(lead, odone + 8 * w);
+        }
+        mma_commit(lead, ofull + 8 * (u & 1));
+        if (h + R < nh) load_q(h + R);                       // every share of h exists, so its scores are complete
       }
       __syncwarp();
     }
-    read_out(nsteps - 1);
-    if (tid == 256) tma_wait_read_all();
+    read_out(nh - 1);
+    if (lane == 0) tma_wait_read_all();
+    __syncwarp();
   } else {
+    if (G == 4) asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
     // ------------------------------------------------------------ the compute warps: lane = key
-    // Each warpgroup keeps its own copy of a step's lse values, so the two only meet through the
-    // issuing thread's barriers.
-    const int ja = k0 + wg * kTileRows + row;
-    const bool dead = ja >= g.tk;
-    const uint32_t tSw = tS + 128 * wg + lane_base;
-    const uint32_t sShw = sSh + 2 * kTileBytes * wg;
-    float* sLw = sL + 256 * wg;                              // [2][128]
+    const uint32_t tSw = tS + 64 * wg + lane_base;
+    const uint32_t sShw = sSh + kTileBytes * wg;
+    const int kw = k0 + wg * kTileRows;
     float den = g.eps;                                       // committed + eps, for the whole sweep
-    sLw[row] = load_lse(rmax, rden, row_base, ib0 * kTileRows + row, g.tq);
-    if (wg == 0) asm volatile("bar.sync 3, 128;" ::: "memory"); else asm volatile("bar.sync 4, 128;" ::: "memory");
-    for (int s = 0; s < nsteps; ++s) {
-      const int ib = ib0 + s, b = s & 1;
-      float lse_next = INFINITY;
-      if (s + 1 < nsteps) lse_next = load_lse(rmax, rden, row_base, (ib + 1) * kTileRows + row, g.tq);
-      // The step's four 32-query chunks (query half a = IDX / 2).  The TMEM load of the next chunk
-      // is issued before this chunk's arithmetic; the shares of the first two chunks wait in
-      // registers until the O MMAs of the previous step have read the share tile.
+    for (int h = h0 + 2 * wg; h < nh && wg < groups; ++h) {
+      const int t = h - h0 - 2 * wg;
       float v0[32], v1[32];
-      uint32_t pk0[16], pk1[16];
-      mbar_wait(sdone, s & 1, ctl, &g_status, kErrWaitMma);
-      tc_fence_after();
-      tmem_ld32(tSw, v0);
-      auto arith = [&](const float* v, uint32_t* packed, int q0) {
-        const int rb = q0 >> 5;                              // checkpoint in front of the chunk's first query
-        if (!dead && rb < ncb) carry[((int64_t)n * ncb + rb) * g.tk + ja] = den - g.eps;
-        const float4* L4 = reinterpret_cast<const float4*>(sLw + 128 * b + (q0 - ib * kTileRows));
-        const bool masked = dead || (k0 + wg * kTileRows + kTileRows - 1 > q0);
+      uint32_t pk[16];
+      auto arith = [&](const float* v, int c) {
+        const int q0 = h * 64 + 32 * c;
+        if (CR == 32 || c == 0) {                            // checkpoint in front of the chunk's first query
+          const int rb = q0 / CR;
+          if (!dead && rb < ncb) carry[((int64_t)n * ncb + rb) * g.tk + ja] = den - g.eps;
+        }
+        const float4* L4 = reinterpret_cast<const float4*>(sL + 64 * ((h - h0) & 3) + 32 * c);
+        const bool masked = dead || kw + kTileRows - 1 > q0;
         auto chunk = [&](auto mask_tag) {
           constexpr bool MASK = decltype(mask_tag)::value;
 #pragma unroll
@@ -239,8 +253,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) forward_fused_kernel(
             float sh[4], dn[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-              // two special-function ops per score on two warps per scheduler: every fourth
-              // exponential is a degree-4 polynomial on the FMA pipe instead (7.30 -> 7.08 ms)
+              // the special-function unit binds: every fourth exponential is a degree-4 polynomial on the FMA pipe
               const float z = fmaf(v[e4 * 4 + u], g.zscale, -ls[u]);
               float p = u == 3 ? poly_exp2<4>(z) : fast_exp2(z);
               if (MASK && (dead || ja > q0 + e4 * 4 + u)) p = 0.f;
@@ -254,64 +267,45 @@ __global__ void __launch_bounds__(kFusedThreads, 1) forward_fused_kernel(
               sh[u] = s2.x;
               sh[u + 1] = s2.y;
             }
-            packed[e4 * 2] = pack_bf16(sh[0], sh[1]);
-            packed[e4 * 2 + 1] = pack_bf16(sh[2], sh[3]);
+            pk[e4 * 2] = pack_bf16(sh[0], sh[1]);
+            pk[e4 * 2 + 1] = pack_bf16(sh[2], sh[3]);
           }
         };
         if (masked) chunk(std::true_type{}); else chunk(std::false_type{});
-      };
-      auto store = [&](const uint32_t* packed, int ql) {      // ql: first query of the chunk within the step
-#pragma unroll
-        for (int e8 = 0; e8 < 4; ++e8) {
-          const uint32_t dst = sShw + share_chunk_offset(row, ql + e8 * 8);
-          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(packed[4 * e8]),
-                       "r"(packed[4 * e8 + 1]), "r"(packed[4 * e8 + 2]), "r"(packed[4 * e8 + 3])
-                       : "memory");
-        }
-      };
-      auto release = [&](int a) {                            // this half of the scores is out of TMEM
-        tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(sfree + 8 * a);
       };
-      const int qs = ib * kTileRows;
-      // chunk 0
+      auto store = [&](int c) {
+#pragma unroll
+        for (int e8 = 0; e8 < 4; ++e8)
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sShw + share_chunk_offset(row, 32 * c + 8 * e8)),
+                       "r"(pk[4 * e8]), "r"(pk[4 * e8 + 1]), "r"(pk[4 * e8 + 2]), "r"(pk[4 * e8 + 3])
+                       : "memory");
+      };
+      mbar_wait(sdone + 8 * wg, t & 1, ctl, &g_status, kErrWaitMma);
+      tc_fence_after();
+      tmem_ld32(tSw, v0);
       tmem_ld_wait(v0);
       tmem_ld32(tSw + 32, v1);
-      arith(v0, pk0, qs);
-      // chunk 1
+      arith(v0, 0);
       tmem_ld_wait(v1);
-      release(0);
-      mbar_wait(sdone + 8, s & 1, ctl, &g_status, kErrWaitMma);
-      tc_fence_after();
-      tmem_ld32(tSw + 64, v0);
-      arith(v1, pk1, qs + 32);
-      if (s >= 1) mbar_wait(odone + 8 * (b ^ 1), ((s - 1) >> 1) & 1, ctl, &g_status, kErrWaitMma);
-      store(pk0, 0);
-      store(pk1, 32);
-      // chunk 2
-      tmem_ld_wait(v0);
-      tmem_ld32(tSw + 96, v1);
-      arith(v0, pk0, qs + 64);
-      store(pk0, 64);
-      // chunk 3
-      tmem_ld_wait(v1);
-      release(1);
-      arith(v1, pk1, qs + 96);
-      store(pk1, 96);
-      if (s + 1 < nsteps) sLw[128 * (b ^ 1) + row] = lse_next;
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(sfree + 8 * wg);            // these scores are out of TMEM
+      // the products of the previous half tile have read this warpgroup's share tile
+      if (t >= 1) mbar_wait(odone + 8 * wg, (t - 1) & 1, ctl, &g_status, kErrWaitMma);
+      store(0);
+      arith(v1, 1);
+      store(1);
       fence_async_smem();
       __syncwarp();
-      if (lane == 0) mbar_arrive(shready);
-      // the next step's lse is visible to the warpgroup
-      if (wg == 0) asm volatile("bar.sync 3, 128;" ::: "memory"); else asm volatile("bar.sync 4, 128;" ::: "memory");
+      if (lane == 0) mbar_arrive(shready + 8 * wg);
     }
     if (!dead) total[(int64_t)n * g.tk + ja] = den - g.eps;
   }
   drain_if_aborted(ctl);
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_free(tmem, 512);
+  if (warp == 0) tmem_free(tmem, kTmem);
 }
 
 // out = O / (rs + eps) in place, four columns per thread (grid over n*t*16 float4).
@@ -325,25 +319,46 @@ __global__ void normalize_out_kernel(float* __restrict__ out, const float* __res
   reinterpret_cast<float4*>(out)[i] = x;
 }
 
-// Passes 2 and 3 of a training forward (q_off = 0, tq = tk, checkpoints every 32 rows) in one
-// key-stationary sweep.  carry: (n, ceil(t/32), t); total: (n, t); out: (n, t, 64) fp32; ssum: (n, t).
+// Compute warpgroups per CTA.  Four need blocks of 512 keys for the SMs; with fewer than 256 of them a CTA of 128 keys, two to
+// an SM, is faster, and as fast as the sweep of 256 keys that it replaces.  Passes 2 and 3, one / four warpgroups / two
+// passes, in us: n = 64, T = 3000 324 / 277 / 291; n = 4, T = 32768 1963 / 1573 / 1676; n = 16, T = 65536 29.4 / 21.8 / 26.3 ms;
+// n = 16, T = 3000 (96 blocks) 115 / 166 / 100; n = 16, T = 1024 (32) 51 / 68 / 42.
+inline int fused_groups(int64_t n, int64_t t) { return n * ((t + 511) / 512) >= 256 ? 4 : 1; }
+
+// Passes 2 and 3 of a call over whole rows (q_off = 0, tq = tk) in one
+// key-stationary sweep.  carry: (n, ceil(t/32 or t/64), t); total: (n, t); out: (n, t, 64) fp32; ssum: (n, t).
 inline int forward_fused(const void* q, const void* k, const void* v, const Geom& g, const float* rmax,
                          const float* rden, float* carry, float* total, float* out, float* ssum,
                          cudaStream_t st, char* err, size_t errlen) {
-  CUtensorMap mq, mk, mv, mo;
-  if (int rc = make_map(&mq, q, g.n, g.tq, err, errlen)) return rc;
-  if (int rc = make_map(&mk, k, g.n, g.tk, err, errlen)) return rc;
+  CUtensorMap mq, mv, mo;
+  if (int rc = make_map(&mq, q, g.n, g.tq, err, errlen, kHeadDim, 64)) return rc;
   if (int rc = make_map(&mv, v, g.n, g.tk, err, errlen)) return rc;
-  if (int rc = make_map_f32(&mo, out, g.n, g.tq, err, errlen)) return rc;
-  constexpr int smem = kFusedSmem;
-  static_assert(smem <= 232448, "the fused forward pass fits one SM's shared memory");
-  auto kern = pair_demands(g) ? forward_fused_kernel<true> : forward_fused_kernel<false>;
-  if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
+  if (int rc = make_map_f32(&mo, out, g.n, g.tq, err, errlen, kHeadDim, 64, false)) return rc;
+  if ((uintptr_t)k & 15) {
+    snprintf(err, errlen, "bf16 tensor-core path needs 16-byte aligned q/k/v");
+    return 1;
+  }
   const int64_t rows = g.n * g.tq;
   cudaMemsetAsync(out, 0, sizeof(float) * (size_t)rows * kHeadDim, st);
   cudaMemsetAsync(ssum, 0, sizeof(float) * (size_t)rows, st);
-  const int nsb = (g.tk + kFusedKeys - 1) / kFusedKeys;
-  kern<<<(unsigned)(g.n * nsb), kFusedThreads, smem, st>>>(mq, mk, mv, mo, g, rmax, rden, carry, total, ssum);
+  auto launch = [&](auto groups_c, auto cr_c, auto pair_c) -> int {
+    constexpr int G = decltype(groups_c)::value, smem = kFusedSmem<G>;
+    static_assert(smem <= 232448 && (G > 1 || 2 * (smem + 1024) <= 233472), "one or two CTAs fit one SM's shared memory");
+    auto kern = forward_fused_kernel<G, decltype(cr_c)::value, decltype(pair_c)::value>;
+    if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
+    const int nsb = (g.tk + G * kTileRows - 1) / (G * kTileRows);
+    kern<<<(unsigned)(g.n * nsb), 128 * (G + 1), smem, st>>>(mq, mv, mo, g, (const __nv_bfloat16*)k, rmax, rden, carry, total,
+                                                            ssum);
+    return 0;
+  };
+  using std::integral_constant;
+  auto by_pair = [&](auto groups_c, auto cr_c) {
+    return pair_demands(g) ? launch(groups_c, cr_c, std::true_type{}) : launch(groups_c, cr_c, std::false_type{});
+  };
+  auto by_rows = [&](auto groups_c) {
+    return g.carry_rows == 64 ? by_pair(groups_c, integral_constant<int, 64>{}) : by_pair(groups_c, integral_constant<int, 32>{});
+  };
+  if (int rc = fused_groups(g.n, g.tk) == 4 ? by_rows(integral_constant<int, 4>{}) : by_rows(integral_constant<int, 1>{})) return rc;
   return launch_status("tc forward_fused", err, errlen);
 }
 

@@ -48,9 +48,9 @@ HAS_CUDA_LIB = _lib.available()
 # key half left.  False (or DILUTION_SAVE_PK=0 in the environment): nothing is saved and the
 # correction pass recomputes the query half.
 TC_SAVE_PK = os.environ.get("DILUTION_SAVE_PK", "1") != "0"
-# Training forward on the tensor-core path: one key-stationary sweep for passes 2 and 3
-# (dilution_forward_fused) instead of the column-sum pass plus the query-stationary main pass, which short rows keep
-# (_short_rows).
+# Forward of whole rows on the tensor-core path: one key-stationary sweep for passes 2 and 3
+# (dilution_forward_fused_rows) instead of the column-sum pass plus the query-stationary main pass, which short rows and calls of
+# few rows keep (_two_passes).
 TC_FUSED_FORWARD = os.environ.get("DILUTION_FUSED_FORWARD", "1") != "0"
 
 
@@ -108,14 +108,19 @@ def _upstream(dout, n, seq, head_dim, keep_bf16):
     return dout if dout.data_ptr() % 16 == 0 else dout.clone()
 
 
-def _short_rows(n, seq):
-    """Training forwards that take the column-sum and main passes instead of the fused sweep.  The sweep owns
-    256 keys per block: a short row is mostly diagonal blocks, and the output that it adds up in memory is zeroed,
-    reduced into and divided once per row of few tiles.  Passes 2 and 3 of a call, fused sweep with its division against
-    two passes: n = 384, T = 1024 327 / 295 us, n = 16, T = 1777 79 / 69, n = 256, T = 2048 639 / 607; n = 64, T = 4096
-    521 / 528; n = 64, T = 16384 7.66 / 8.06 ms.  With fewer than 74 super-blocks (half of the SMs) the host's launches
-    outlast either."""
-    return seq <= 2048 and n * -(-seq // 256) >= 74
+def _two_passes(n, seq, carry_rows):
+    """Calls that take the column-sum and main passes instead of the fused sweep.  With 256 blocks of 512 keys or more
+    the sweep fills the chip and is the faster one beyond 2048 tokens, before a backward or not; a short row is mostly diagonal blocks, and
+    the output that the sweep adds up in memory is zeroed, reduced into and divided once per row of few tiles.  With fewer
+    blocks the two passes are faster.  Passes 2 and 3 of a call, sweep / two passes: n = 64, T = 3000
+    277 / 291 us, n = 64, T = 16384 6.1 / 6.8 ms, n = 16, T = 131072 90 / 104 ms; n = 384, T = 1024 283 / 274 us, n = 16,
+    T = 4096 158 / 141 us.  Training calls of at most 2559 tokens and few blocks stay with the sweep, whose shape for
+    few blocks is as fast as it ever was: below 74 blocks of 256 keys (half of the SMs) the host's launches outlast either."""
+    if seq > 2048 and n * -(-seq // 512) >= 256:
+        return False
+    if carry_rows != 32:
+        return True
+    return n * -(-seq // 256) >= 74 if seq <= 2048 else seq >= 2560
 
 
 def _forward_rows(lib, qf, kf, vf, code, prec, scale, out, ssum, rmax, rden, carry, total, pk,
@@ -133,12 +138,12 @@ def _forward_rows(lib, qf, kf, vf, code, prec, scale, out, ssum, rmax, rden, car
     else:
         _lib.check(lib.dilution_rowstats(qf.data_ptr(), kf.data_ptr(), code, prec, n, tq, tk, q_offset,
                                          d, scale, rmax.data_ptr(), rden.data_ptr(), st), "dilution_rowstats")
-    if (TC_FUSED_FORWARD and carry_rows == 32 and carry_base is None and q_offset == 0 and tq == tk
-            and _lib.tensor_core_path(code, prec, d) and not _short_rows(n, tq)):
-        _lib.check(lib.dilution_forward_fused(qf.data_ptr(), kf.data_ptr(), vf.data_ptr(), code, prec, n, tq, d,
-                                              scale, EPS, rmax.data_ptr(), rden.data_ptr(), carry.data_ptr(),
-                                              total.data_ptr(), out.data_ptr(), ssum.data_ptr(), st),
-                   "dilution_forward_fused")
+    if (TC_FUSED_FORWARD and carry_base is None and q_offset == 0 and tq == tk
+            and _lib.tensor_core_path(code, prec, d) and not _two_passes(n, tq, carry_rows)):
+        _lib.check(lib.dilution_forward_fused_rows(qf.data_ptr(), kf.data_ptr(), vf.data_ptr(), code, prec, n, tq, d,
+                                                   scale, EPS, rmax.data_ptr(), rden.data_ptr(), carry_rows,
+                                                   carry.data_ptr(), total.data_ptr(), out.data_ptr(), ssum.data_ptr(), st),
+                   "dilution_forward_fused_rows")
         return
     _lib.check(lib.dilution_colsum_scan(qf.data_ptr(), kf.data_ptr(), code, prec, n, tq, tk, q_offset,
                                         d, scale, rmax.data_ptr(), rden.data_ptr(), None, carry_rows,

@@ -172,6 +172,11 @@ int dilution_forward_main(const void* q, const void* k, const void* v, int dtype
 int dilution_forward_fused(const void* q, const void* k, const void* v, int dtype, int precision, int64_t n,
                            int64_t t, int d, float scale, float eps, const float* rmax, const float* rden,
                            float* carry, float* total, float* out, float* ssum, void* stream);
+/* The same with a checkpoint every 32 or 64 query rows (carry: (n, ceil(t/carry_rows), t)): 64 for calls that no backward
+ * follows. */
+int dilution_forward_fused_rows(const void* q, const void* k, const void* v, int dtype, int precision, int64_t n,
+                                int64_t t, int d, float scale, float eps, const float* rmax, const float* rden,
+                                int carry_rows, float* carry, float* total, float* out, float* ssum, void* stream);
 
 size_t dilution_backward_scratch_bytes(int64_t n, int64_t t, int d);
 

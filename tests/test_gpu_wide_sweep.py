@@ -1,0 +1,58 @@
+"""The key-stationary sweep in blocks of 512 keys (256 of them or more) at the edges of its blocks, warpgroups and half tiles,
+with checkpoints every 32 rows (a training forward) and every 64 (a prompt), against the two passes and, in the first and last
+row, the oracle; and the choice between the two at its edges."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from conftest import load_package, make_inputs, rel_err
+from oracle import dilution_oracle as O
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _forward(K, x, training, fused):
+    saved, K.TC_FUSED_FORWARD = K.TC_FUSED_FORWARD, fused
+    try:
+        out, aux = K.dilution_attention_forward(*x, dot_precision="bf16", return_aux=True, _training=training)
+    finally:
+        K.TC_FUSED_FORWARD = saved
+    return out, aux
+
+
+@pytest.mark.parametrize("training", [True, False])
+@pytest.mark.parametrize("rows,seq", [(52, 2049), (52, 2111), (52, 2175), (52, 2176), (52, 2177), (52, 2305), (43, 2561),
+                                      (43, 3072), (37, 3137)])
+def test_sweep_of_512_keys(rows, seq, training):
+    pkg = load_package()
+    K = pkg.kernels
+    x = [t.bfloat16().to(DEV) for t in make_inputs(1, rows, seq, 64, 60 + seq, scales=(1.0, 1.0, 1.0, 1.0))[:3]]
+    pkg._lib.profile(True)
+    pkg._lib.profile_collect()
+    out, aux = _forward(K, x, training, True)
+    names = set(pkg._lib.profile_collect())
+    pkg._lib.profile(False)
+    assert "tc_forward_fused" in names and "tc_forward_main" not in names, names
+    ref_out, ref = _forward(K, x, training, False)
+    assert aux["bwd_block_m"] == ref["bwd_block_m"] == (32 if training else 64)
+    assert (out - ref_out).abs().max().item() < 1e-2                     # both round their shares to bf16
+    assert rel_err(aux["committed_total"], ref["committed_total"]) < 1e-4
+    assert rel_err(aux["ssum"], ref["ssum"]) < 1e-2
+    step = aux["bwd_block_m"]
+    scale = max(1.0, ref["carry"][:, -1].abs().max().item())
+    for rb in range(aux["carry"].shape[1]):
+        end = min((rb + 1) * step, seq)
+        assert (aux["carry"][:, rb, :end] - ref["carry"][:, rb, :end]).abs().max().item() < 1e-4 * scale, rb
+    for r in (0, rows - 1):
+        want = O.dilution_chunked(*(t[:, r:r + 1].float().cpu() for t in x), chunk=512)
+        assert (out[:, r:r + 1].cpu() - want).abs().max().item() < 2e-2
+
+
+@pytest.mark.parametrize("rows,seq,training,sweep", [(52, 2048, False, False), (52, 2049, False, True), (51, 2049, False, False),
+                                                     (10, 2559, True, True), (10, 2560, True, False), (32, 4096, True, True),
+                                                     (31, 4096, True, False)])
+def test_route(rows, seq, training, sweep):
+    assert load_package().kernels._two_passes(rows, seq, 32 if training else 64) is not sweep
