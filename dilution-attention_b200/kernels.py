@@ -123,36 +123,24 @@ def _two_passes(n, seq, carry_rows):
     return n * -(-seq // 256) >= 74 if seq <= 2048 else seq >= 2560
 
 
-def _forward_rows(lib, qf, kf, vf, code, prec, scale, out, ssum, rmax, rden, carry, total, pk,
-                  carry_rows, q_offset=0, carry_base=None):
-    """Passes 1-3 on a slab of (batch*head) rows.  On the tensor-core path a requested pk comes
-    out of pass 1; otherwise out of pass 3 (the fp32 kernel)."""
-    n, tq, d = qf.shape
-    tk = kf.shape[1]
-    st = _stream(qf.device)
-    if pk is not None and _lib.tensor_core_path(code, prec, d) and q_offset == 0 and tq == tk:
-        _lib.check(lib.dilution_rowstats_pk(qf.data_ptr(), kf.data_ptr(), code, prec, n, tq, d, scale,
-                                            rmax.data_ptr(), rden.data_ptr(), pk.data_ptr(), st),
-                   "dilution_rowstats_pk")
+def _forward_rows(lib, q, k, v, sizes, code, prec, scale, out, ssum, rmax, rden, carry, total, pk, carry_rows, st):
+    """Passes 1-3 on a slab of (batch*head) rows, all tensors as addresses.  sizes: (rows, queries, keys, head size).  On the
+    tensor-core path a requested pk comes out of pass 1; otherwise out of pass 3 (the fp32 kernel)."""
+    n, tq, tk, d = sizes
+    tc = _lib.tensor_core_path(code, prec, d) and tq == tk
+    if pk is not None and tc:
+        _lib.check(lib.dilution_rowstats_pk(q, k, code, prec, n, tq, d, scale, rmax, rden, pk, st), "dilution_rowstats_pk")
         pk = None
     else:
-        _lib.check(lib.dilution_rowstats(qf.data_ptr(), kf.data_ptr(), code, prec, n, tq, tk, q_offset,
-                                         d, scale, rmax.data_ptr(), rden.data_ptr(), st), "dilution_rowstats")
-    if (TC_FUSED_FORWARD and carry_base is None and q_offset == 0 and tq == tk
-            and _lib.tensor_core_path(code, prec, d) and not _two_passes(n, tq, carry_rows)):
-        _lib.check(lib.dilution_forward_fused_rows(qf.data_ptr(), kf.data_ptr(), vf.data_ptr(), code, prec, n, tq, d,
-                                                   scale, EPS, rmax.data_ptr(), rden.data_ptr(), carry_rows,
-                                                   carry.data_ptr(), total.data_ptr(), out.data_ptr(), ssum.data_ptr(), st),
-                   "dilution_forward_fused_rows")
+        _lib.check(lib.dilution_rowstats(q, k, code, prec, n, tq, tk, 0, d, scale, rmax, rden, st), "dilution_rowstats")
+    if TC_FUSED_FORWARD and tc and not _two_passes(n, tq, carry_rows):
+        _lib.check(lib.dilution_forward_fused_rows(q, k, v, code, prec, n, tq, d, scale, EPS, rmax, rden, carry_rows, carry,
+                                                   total, out, ssum, st), "dilution_forward_fused_rows")
         return
-    _lib.check(lib.dilution_colsum_scan(qf.data_ptr(), kf.data_ptr(), code, prec, n, tq, tk, q_offset,
-                                        d, scale, rmax.data_ptr(), rden.data_ptr(), None, carry_rows,
-                                        carry.data_ptr(), total.data_ptr(), st), "dilution_colsum_scan")
-    _lib.check(lib.dilution_forward_main(qf.data_ptr(), kf.data_ptr(), vf.data_ptr(), code, prec,
-                                         n, tq, tk, q_offset, d, scale, EPS,
-                                         rmax.data_ptr(), rden.data_ptr(), carry.data_ptr(), carry_rows,
-                                         _ptr(carry_base), out.data_ptr(), ssum.data_ptr(), _ptr(pk), st),
-               "dilution_forward_main")
+    _lib.check(lib.dilution_colsum_scan(q, k, code, prec, n, tq, tk, 0, d, scale, rmax, rden, None, carry_rows, carry, total,
+                                        st), "dilution_colsum_scan")
+    _lib.check(lib.dilution_forward_main(q, k, v, code, prec, n, tq, tk, 0, d, scale, EPS, rmax, rden, carry, carry_rows,
+                                         None, out, ssum, pk, st), "dilution_forward_main")
 
 
 def _wide_operands(lib, qf, kf, vf, code):
@@ -197,7 +185,7 @@ def dilution_attention_forward(
     quadratic carry scratch stays under scratch_budget_gib; rows are independent,
     so this changes nothing numerically.
     """
-    result, aux, _ = _attention_forward(q, k, v, dot_precision, return_aux, _save_pk, scratch_budget_gib, _training)
+    result, aux = _attention_forward(q, k, v, dot_precision, return_aux, _save_pk, scratch_budget_gib, _training)
     if return_aux:
         aux.update(block_m=block_m, block_n=block_n, dot_precision=dot_precision, num_warps=num_warps)
         return result, aux
@@ -205,7 +193,7 @@ def dilution_attention_forward(
 
 
 def _attention_forward(q, k, v, dot_precision, return_aux, _save_pk, scratch_budget_gib=16.0, _training=None):
-    """(out, aux, operands): aux without the caller's tuning arguments, operands as the kernels took q, k and v."""
+    """(out, aux): aux without the caller's tuning arguments."""
     lib = _lib.load()
     (qf, kf, vf), code, prec, n = _prepare(q, k, v, dot_precision)
     batch, heads, seq, head_dim = q.shape
@@ -233,52 +221,106 @@ def _attention_forward(q, k, v, dot_precision, return_aux, _save_pk, scratch_bud
     carry = torch.empty(rows, ncb, seq, **f32)
     for a in range(0, n, rows):
         b = min(a + rows, n)
+        # (a slice costs 2 us, and most calls are one slab)
+        qs, ks, vs, o, ss, mx, dn, tot, pks = (
+            x if rows == n or x is None else x[a:b] for x in (qf, kf, vf, out, ssum, rmax, rden, total, pk))
         if wide:
             _lib.check(lib.dilution_wide_forward(
-                qf[a:b].data_ptr(), kf[a:b].data_ptr(), vf[a:b].data_ptr(), code, b - a, seq, head_dim, scale, EPS,
-                rmax[a:b].data_ptr(), rden[a:b].data_ptr(), carry.data_ptr(), total[a:b].data_ptr(),
-                out[a:b].data_ptr(), ssum[a:b].data_ptr(), None if pk is None else pk[a:b].data_ptr(), _stream(dev)),
+                qs.data_ptr(), ks.data_ptr(), vs.data_ptr(), code, b - a, seq, head_dim, scale, EPS, mx.data_ptr(),
+                dn.data_ptr(), carry.data_ptr(), tot.data_ptr(), o.data_ptr(), ss.data_ptr(), _ptr(pks), _stream(dev)),
                 "dilution_wide_forward")
             continue
-        _forward_rows(lib, qf[a:b], kf[a:b], vf[a:b], code, prec, scale, out[a:b], ssum[a:b],
-                      rmax[a:b], rden[a:b], carry[: b - a], total[a:b],
-                      None if pk is None else pk[a:b], carry_rows)
+        _forward_rows(lib, qs.data_ptr(), ks.data_ptr(), vs.data_ptr(), (b - a, seq, kf.shape[1], head_dim), code, prec, scale,
+                      o.data_ptr(), ss.data_ptr(), mx.data_ptr(), dn.data_ptr(), carry.data_ptr(), tot.data_ptr(), _ptr(pks),
+                      carry_rows, _stream(dev))
 
     aux = dict(pk=pk, rmax=rmax, rden=rden, carry=carry, ssum=ssum, bwd_block_m=carry_rows,
                committed_total=total.reshape(batch, heads, seq))
-    return out.reshape(batch, heads, seq, head_dim), aux, (qf, kf, vf)
+    return out.reshape(batch, heads, seq, head_dim), aux
+
+
+def _operands(q, k, v, dot_precision):
+    """What _prepare gives for three tensors of one shape: contiguous operands (not folded to three dimensions: the
+    kernels take addresses), the dtype code and the precision code."""
+    if not (q.is_cuda and q.dim() == 4 and q.shape == k.shape == v.shape):
+        batch, heads, seq, head_dim = q.shape
+        ops, code, prec, _ = _prepare(q, k, v, dot_precision)
+        return [x.reshape(batch, heads, seq, head_dim) for x in ops], code, prec
+    want = torch.bfloat16 if (dot_precision == "bf16" or q.dtype == torch.bfloat16) else torch.float32
+    ops = []
+    for x in (q, k, v):
+        if x.dtype != want:
+            x = x.to(want)
+        x = x.contiguous()
+        if x.data_ptr() % 16:
+            raise RuntimeError("dilution attention needs q, k and v on a 16-byte boundary")
+        ops.append(x)
+    return ops, _lib.BF16 if want == torch.bfloat16 else _lib.F32, _lib.PREC[dot_precision]
+
+
+def _workspace(device, **parts):
+    """One fp32 allocation for what a training forward leaves for its backward besides the output, and the byte offset of each
+    part (sizes in fp32 elements, parts on 256-byte boundaries).  A call of few rows takes as long as the host needs for it, and
+    every allocation from Python is 1.8 us of that."""
+    at, offsets = 0, {}
+    for name, count in parts.items():
+        offsets[name] = 4 * at
+        at += (count + 63) // 64 * 64
+    return torch.empty(at, device=device, dtype=torch.float32), offsets
 
 
 class _DilutionAttentionFn(torch.autograd.Function):
-    """Autograd op (kernels.py:829-903): fp32 output; dq, dk, dv in the input dtypes."""
+    """Autograd op (kernels.py:829-903): fp32 output; dq, dk, dv in the input dtypes.
+
+    Saved for the backward: the operands as the kernels took them (casts, copies of strided views and hi | lo planes are made
+    once), the output and one workspace with the row statistics, the checkpoints, the demand totals and pk.  Tensors of
+    the workspace are handed to the kernels by their addresses, without views.  Host time of forward + backward of one short
+    row, of which a Function that does nothing takes 50 us: 190 -> 150 us."""
 
     @staticmethod
     def forward(ctx, q, k, v, dot_precision):
+        _resolve_precision(dot_precision)
+        if not any(ctx.needs_input_grad[:3]):
+            return _attention_forward(q, k, v, dot_precision, True, False, _training=False)[0]
+        lib = _lib.load()
+        ops, code, prec = _operands(q, k, v, dot_precision)
+        batch, heads, seq, head_dim = q.shape
+        n, dev = batch * heads, q.device
+        wide = _lib.wide_path(code, prec, head_dim)
         # the tensor-core backward can apply the dq correction itself, without a saved pk
-        lowp, _ = _resolve_precision(dot_precision)
-        on_tc = _lib.tensor_core_path(_lib.BF16 if (lowp or q.dtype == torch.bfloat16) else _lib.F32,
-                                      _lib.PREC[dot_precision], q.shape[-1])
-        out, aux, operands = _attention_forward(
-            q, k, v, dot_precision, True, any(ctx.needs_input_grad[:3]) and (TC_SAVE_PK or not on_tc),
-            _training=any(ctx.needs_input_grad[:3]))
-        ctx.carry_rows = aux["bwd_block_m"]
-        # what the backward's kernels read: the operands as the forward took them (casts, copies of strided views
-        # and hi | lo planes are made once)
-        ctx.save_for_backward(*operands, out, aux["rmax"], aux["rden"], aux["carry"], aux["ssum"], aux["pk"],
-                              aux["committed_total"])
-        ctx.dot_precision = dot_precision
+        save_pk = TC_SAVE_PK or not _lib.tensor_core_path(code, prec, head_dim)
+        rows = n * seq
+        ws, at = _workspace(dev, rmax=rows, rden=rows, ssum=rows, total=rows, pk=rows * head_dim if save_pk else 0,
+                            carry=rows * ((seq + CARRY_ROWS - 1) // CARRY_ROWS),
+                            planes=3 * 64 * rows if wide and code == _lib.F32 else 0)
+        out = torch.empty(q.shape, device=dev, dtype=torch.float32)
+        scale, st, base = 1.0 / math.sqrt(head_dim), _stream(dev), ws.data_ptr()
+        rmax, rden, ssum, total, carry = (base + at[x] for x in ("rmax", "rden", "ssum", "total", "carry"))
+        pk = base + at["pk"] if save_pk else None
+        addr = [x.data_ptr() for x in ops]
+        if wide:
+            if code == _lib.F32:
+                planes = [base + at["planes"] + 256 * rows * i for i in range(3)]
+                _lib.check(lib.dilution_split_operands(*addr, rows, head_dim, *planes, st), "dilution_split_operands")
+                addr, ops = planes, ()
+            _lib.check(lib.dilution_wide_forward(*addr, code, n, seq, head_dim, scale, EPS, rmax, rden, carry, total,
+                                                 out.data_ptr(), ssum, pk, st), "dilution_wide_forward")
+        else:
+            _forward_rows(lib, *addr, (n, seq, seq, head_dim), code, prec, scale, out.data_ptr(), ssum, rmax, rden, carry,
+                          total, pk, CARRY_ROWS, st)
+        ctx.save_for_backward(*ops, out, ws)
+        ctx.call = (code, prec, at, save_pk)
         ctx.dtypes = (q.dtype, k.dtype, v.dtype)
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        qf, kf, vf, out, rmax, rden, carry, ssum, pk, total = ctx.saved_tensors
+        *ops, out, ws = ctx.saved_tensors
+        code, prec, at, save_pk = ctx.call
         lib = _lib.load()
         batch, heads, seq, head_dim = out.shape
-        lowp, _ = _resolve_precision(ctx.dot_precision)
-        code = _lib.BF16 if (lowp or ctx.dtypes[0] == torch.bfloat16) else _lib.F32
-        prec = _lib.PREC[ctx.dot_precision]
         n, dev = batch * heads, out.device
+        rows = n * seq
         # the tensor-core paths read a bf16 upstream gradient as it is (their first kernel makes a
         # scaled bf16 copy anyway); everything else is widened to fp32 as the reference does
         wide = _lib.wide_path(code, prec, head_dim)
@@ -286,25 +328,24 @@ class _DilutionAttentionFn(torch.autograd.Function):
         dof = _upstream(dout, n, seq, head_dim, on_tc)
         do_code = _lib.BF16 if dof.dtype == torch.bfloat16 else _lib.F32
         gdt = torch.bfloat16 if code == _lib.BF16 else torch.float32
-        dq, dk, dv = (torch.empty(batch, heads, seq, head_dim, device=dev, dtype=gdt) for _ in range(3))
+        dq, dk, dv = (torch.empty(out.shape, device=dev, dtype=gdt) for _ in range(3))
         nbytes = (lib.dilution_wide_scratch_bytes(code, n, seq, head_dim) if wide
                   else lib.dilution_backward_scratch_bytes(n, seq, head_dim))
         scratch = torch.empty(nbytes, device=dev, dtype=torch.uint8)
-        scale = 1.0 / math.sqrt(head_dim)
+        scale, st, base = 1.0 / math.sqrt(head_dim), _stream(dev), ws.data_ptr()
+        rmax, rden, ssum, total, carry = (base + at[x] for x in ("rmax", "rden", "ssum", "total", "carry"))
+        pk = base + at["pk"] if save_pk else None
+        addr = [x.data_ptr() for x in ops] or [base + at["planes"] + 256 * rows * i for i in range(3)]
         if wide:
             _lib.check(lib.dilution_wide_backward(
-                qf.data_ptr(), kf.data_ptr(), vf.data_ptr(), code, n, seq, head_dim, scale, EPS, dof.data_ptr(), do_code,
-                out.data_ptr(), rmax.data_ptr(), rden.data_ptr(), carry.data_ptr(), total.data_ptr(), ssum.data_ptr(),
-                pk.data_ptr(), scratch.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), _stream(dev)),
-                "dilution_wide_backward")
+                *addr, code, n, seq, head_dim, scale, EPS, dof.data_ptr(), do_code, out.data_ptr(), rmax, rden, carry, total,
+                ssum, pk, scratch.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), st), "dilution_wide_backward")
         else:
             _lib.check(lib.dilution_backward(
-                qf.data_ptr(), kf.data_ptr(), vf.data_ptr(), code, prec, n, seq, head_dim,
-                scale, EPS, dof.data_ptr(), do_code, out.data_ptr(),
-                rmax.data_ptr(), rden.data_ptr(), carry.data_ptr(), ctx.carry_rows, total.data_ptr(), ssum.data_ptr(),
-                _ptr(pk), scratch.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), _stream(dev)),
+                *addr, code, prec, n, seq, head_dim, scale, EPS, dof.data_ptr(), do_code, out.data_ptr(), rmax, rden, carry,
+                CARRY_ROWS, total, ssum, pk, scratch.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), st),
                 "dilution_backward")
-        return (*(x.to(dt) for x, dt in zip((dq, dk, dv), ctx.dtypes)), None)
+        return (*(x if x.dtype == dt else x.to(dt) for x, dt in zip((dq, dk, dv), ctx.dtypes)), None)
 
 
 def dilution_attention(
@@ -356,21 +397,25 @@ def softmax_attention_forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
     batch, heads, seq, head_dim = q.shape
     if q.dtype != torch.bfloat16 or head_dim != 64:
         raise ValueError("softmax_attention_forward takes bfloat16 tensors with head_dim 64")
-    (qf, kf, vf), code, prec, n = _prepare(q, k, v, "bf16")
-    out = torch.empty(n, seq, head_dim, device=q.device, dtype=torch.bfloat16)
+    n = batch * heads
+    if q.shape == k.shape == v.shape:
+        (qf, kf, vf), code, prec = _operands(q, k, v, "bf16")
+        keys = seq
+    else:
+        (qf, kf, vf), code, prec, n = _prepare(q, k, v, "bf16")
+        keys = kf.shape[1]
+    out = torch.empty(batch, heads, seq, head_dim, device=q.device, dtype=torch.bfloat16)
     rmax = rden = None
     if return_lse:
-        rmax = torch.empty(n, seq, device=q.device, dtype=torch.float32)
+        rmax = torch.empty(batch, heads, seq, device=q.device, dtype=torch.float32)
         rden = torch.empty_like(rmax)
     _lib.check(lib.dilution_softmax_forward(qf.data_ptr(), kf.data_ptr(), vf.data_ptr(), code, prec, n, seq,
-                                            kf.shape[1], 0, head_dim, 1.0 / math.sqrt(head_dim), _ptr(rmax),
+                                            keys, 0, head_dim, 1.0 / math.sqrt(head_dim), _ptr(rmax),
                                             _ptr(rden), out.data_ptr(), _stream(q.device)),
                "dilution_softmax_forward")
-    result = out.reshape(batch, heads, seq, head_dim)
     if return_lse:
-        lse = (rmax + torch.log2(rden)) * math.log(2.0)
-        return result, lse.reshape(batch, heads, seq)
-    return result
+        return out, (rmax + torch.log2(rden)) * math.log(2.0)
+    return out
 
 
 def decode_scratch(n: int, capacity: int, head_dim: int, device) -> torch.Tensor:
@@ -400,8 +445,17 @@ def _decode_args(q1, k_cache, v_cache, committed, length):
 
 
 def _rows(x, n, head_dim):
+    """One contiguous row per (batch, head), which the kernels read by its address (folding a tensor that is laid out so
+    already would cost 2 us)."""
+    if x.is_contiguous() and x.numel() == n * head_dim:
+        return x
     x = x.reshape(n, head_dim)
     return x if x.is_contiguous() else x.contiguous()
+
+
+def _cache_rows(x, *shape):
+    """A cache buffer as the kernels read it by its address.  It must be contiguous: .view refuses others."""
+    return x if x.is_contiguous() and x.numel() == math.prod(shape) else x.view(*shape)
 
 
 def dilution_decode_step(
@@ -428,11 +482,10 @@ def dilution_decode_step(
     batch, heads, head_dim, capacity = _decode_args(q1, k_cache, v_cache, committed, length)
     n = batch * heads
     qf = _rows(q1, n, head_dim)
-    kf = k_cache.view(n, capacity, head_dim)      # .view: the caches must be contiguous
-    vf = v_cache.view(n, capacity, head_dim)
-    cf = committed.view(n, capacity)
+    kf, vf = _cache_rows(k_cache, n, capacity, head_dim), _cache_rows(v_cache, n, capacity, head_dim)
+    cf = _cache_rows(committed, n, capacity)
     if out is None:
-        out = torch.empty(n, head_dim, device=q1.device, dtype=q1.dtype)
+        out = torch.empty(batch, heads, 1, head_dim, device=q1.device, dtype=q1.dtype)
     need = lib.dilution_decode_scratch_bytes(n, length, head_dim)
     if scratch is None or scratch.numel() * scratch.element_size() < need:
         scratch = torch.empty(need, device=q1.device, dtype=torch.uint8)
@@ -441,7 +494,7 @@ def dilution_decode_step(
                                    length, head_dim, 1.0 / math.sqrt(head_dim), EPS,
                                    cf.data_ptr(), out.data_ptr(), scratch.data_ptr(),
                                    _stream(q1.device)), "dilution_decode")
-    return out.view(batch, heads, 1, head_dim)
+    return out if out.dim() == 4 else out.view(batch, heads, 1, head_dim)
 
 
 def dilution_decode_append_step(
@@ -477,12 +530,11 @@ def dilution_decode_append_step(
         raise ValueError("k1 and v1 must have q1's dtype")
     n = batch * heads
     qf, kn, vn = (_rows(x, n, head_dim) for x in (q1, k1, v1))
-    kf = k_cache.view(n, capacity, head_dim)
-    vf = v_cache.view(n, capacity, head_dim)
-    cf = committed.view(n, capacity)
+    kf, vf = _cache_rows(k_cache, n, capacity, head_dim), _cache_rows(v_cache, n, capacity, head_dim)
+    cf = _cache_rows(committed, n, capacity)
     pos_dev = cache.get("pos_dev")
     if out is None:
-        out = torch.empty(n, head_dim, device=q1.device, dtype=q1.dtype)
+        out = torch.empty(batch, heads, 1, head_dim, device=q1.device, dtype=q1.dtype)
     need = lib.dilution_decode_scratch_bytes(n, capacity if pos_dev is not None else t + 1, head_dim)
     if scratch is None or scratch.numel() * scratch.element_size() < need:
         scratch = torch.empty(need, device=q1.device, dtype=torch.uint8)
@@ -498,7 +550,7 @@ def dilution_decode_append_step(
                                               1.0 / math.sqrt(head_dim), EPS, cf.data_ptr(), out.data_ptr(),
                                               scratch.data_ptr(), _stream(q1.device)), "dilution_decode_append")
     cache["len"] = t + 1
-    return out.view(batch, heads, 1, head_dim)
+    return out if out.dim() == 4 else out.view(batch, heads, 1, head_dim)
 
 
 _COPY_STREAMS: dict = {}

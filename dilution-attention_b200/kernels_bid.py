@@ -62,10 +62,9 @@ def _is_operator(bid: str, share_cumsum) -> bool:
     return bid == "softmax" and _share_code(share_cumsum) == 1
 
 
-def _variant_forward(q, k, v, dot_precision, bid, share, shift, save_pk, scratch_budget_gib=16.0,
-                     keep_carry=False, need_total=True):
-    """All forward passes of one call, (batch*head) rows in slabs under the scratch budget unless
-    the checkpoints are kept for a backward.  Without a share step nothing reads the checkpoints:
+def _variant_forward(q, k, v, dot_precision, bid, share, shift, scratch_budget_gib=16.0, keep_carry=False, need_total=True):
+    """All forward passes of one call that no backward follows, (batch*head) rows in slabs under the scratch budget unless
+    the checkpoints are kept.  Without a share step nothing reads the checkpoints:
     unless the demand totals are asked for, the column-sum pass is skipped altogether."""
     lib = _lib.load()
     (qf, kf, vf), code, prec, n = K._prepare(q, k, v, dot_precision)
@@ -78,7 +77,6 @@ def _variant_forward(q, k, v, dot_precision, bid, share, shift, save_pk, scratch
     total = torch.empty(n, seq, **f32) if scan else None
     rmax = torch.empty(n, seq, **f32) if stats else None
     rden = torch.empty(n, seq, **f32) if stats else None
-    pk = torch.empty(n, seq, head_dim, **f32) if (save_pk and bid == _lib.BID["softmax"]) else None
     ncb = (seq + _lib.CARRY_ROWS - 1) // _lib.CARRY_ROWS
     rows = n
     if not keep_carry:
@@ -86,14 +84,14 @@ def _variant_forward(q, k, v, dot_precision, bid, share, shift, save_pk, scratch
     carry = torch.empty(rows, ncb, seq, **f32) if scan else None
     scale = 1.0 / math.sqrt(head_dim)
     st = K._stream(q.device)
-    part = lambda x, a, b: None if x is None else x[a:b].data_ptr()
     for a in range(0, n, rows):
         b = min(a + rows, n)
-        _lib.check(lib.dilution_variant_forward(
-            qf[a:b].data_ptr(), kf[a:b].data_ptr(), vf[a:b].data_ptr(), code, prec, b - a, seq, head_dim,
-            scale, EPS, bid, share, float(shift), part(rmax, a, b), part(rden, a, b), K._ptr(carry), part(total, a, b),
-            out[a:b].data_ptr(), ssum[a:b].data_ptr(), part(pk, a, b), st), "dilution_variant_forward")
-    return out, dict(rmax=rmax, rden=rden, carry=carry, ssum=ssum, pk=pk, total=total)
+        qs, ks, vs, o, ss, mx, dn, tot = (K._ptr(x if rows == n or x is None else x[a:b])
+                                          for x in (qf, kf, vf, out, ssum, rmax, rden, total))
+        _lib.check(lib.dilution_variant_forward(qs, ks, vs, code, prec, b - a, seq, head_dim, scale, EPS, bid, share,
+                                                float(shift), mx, dn, K._ptr(carry), tot, o, ss, None, st),
+                   "dilution_variant_forward")
+    return out, dict(rmax=rmax, rden=rden, carry=carry, ssum=ssum, total=total)
 
 
 def dilution_attention_forward(
@@ -123,8 +121,8 @@ def dilution_attention_forward(
             res[1].update(bid=bid, share_cumsum=share_cumsum, shift=shift)
         return res
     batch, heads, seq, head_dim = q.shape
-    out, aux = _variant_forward(q, k, v, dot_precision, code_b, code_s, shift, save_pk=False,
-                                keep_carry=return_aux, need_total=return_aux)
+    out, aux = _variant_forward(q, k, v, dot_precision, code_b, code_s, shift, keep_carry=return_aux,
+                                need_total=return_aux)
     result = out.reshape(batch, heads, seq, head_dim)
     if return_aux:
         return result, dict(rmax=aux["rmax"], rden=aux["rden"], carry=aux["carry"], ssum=aux["ssum"],
@@ -140,45 +138,52 @@ class _VariantFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, v, dot_precision, bid, share, shift):
-        training = any(ctx.needs_input_grad[:3])
-        # without a share step the softmax bid's Jacobian correction is identically zero: no pk
-        out, aux = _variant_forward(q, k, v, dot_precision, bid, share, shift, save_pk=training and share != 0,
-                                    keep_carry=True, need_total=False)
-        ctx.args = (dot_precision, bid, share, shift)
-        stats = [x for x in (aux["rmax"], aux["rden"]) if x is not None]
-        ctx.n_stats = len(stats)
-        ctx.has_pk = aux["pk"] is not None
-        if ctx.has_pk:
-            stats.append(aux["pk"])
-        scan = [x for x in (aux["carry"], aux["total"]) if x is not None]
-        ctx.n_scan = len(scan)
-        ctx.save_for_backward(q, k, v, out, aux["ssum"], *scan, *stats)
-        return out.reshape(q.shape)
+        lib = _lib.load()
+        ops, code, prec = K._operands(q, k, v, dot_precision)
+        batch, heads, seq, head_dim = q.shape
+        n = batch * heads
+        rows = n * seq
+        parts = dict(ssum=rows)
+        if bid in _lib.ROW_SUM_BIDS:           # bids that divide by a row sum have row statistics
+            parts.update(rmax=rows, rden=rows)
+        if share != 0:                         # without a share step nothing reads the checkpoints
+            parts.update(total=rows, carry=rows * ((seq + _lib.CARRY_ROWS - 1) // _lib.CARRY_ROWS))
+            if any(ctx.needs_input_grad[:3]) and bid == _lib.BID["softmax"]:
+                parts.update(pk=rows * head_dim)      # (and the softmax bid's Jacobian correction is identically zero)
+        ws, at = K._workspace(q.device, **parts)
+        out = torch.empty(q.shape, device=q.device, dtype=torch.float32)
+        rmax, rden, carry, total, ssum, pk = _parts(ws, at)
+        _lib.check(lib.dilution_variant_forward(
+            *(x.data_ptr() for x in ops), code, prec, n, seq, head_dim, 1.0 / math.sqrt(head_dim), EPS, bid, share,
+            float(shift), rmax, rden, carry, total, out.data_ptr(), ssum, pk, K._stream(q.device)), "dilution_variant_forward")
+        ctx.save_for_backward(q, k, v, out, ws)
+        ctx.call = (dot_precision, bid, share, shift, at)
+        return out
 
     @staticmethod
     def backward(ctx, dout):
-        q, k, v, out, ssum, *rest = ctx.saved_tensors
-        carry, total = rest[:2] if ctx.n_scan == 2 else (None, None)
-        stats = rest[ctx.n_scan:]
-        rmax, rden = stats[:2] if ctx.n_stats == 2 else (None, None)
-        pk = stats[-1] if ctx.has_pk else None
-        dot_precision, bid, share, shift = ctx.args
+        q, k, v, out, ws = ctx.saved_tensors
+        dot_precision, bid, share, shift, at = ctx.call
         lib = _lib.load()
         batch, heads, seq, head_dim = q.shape
-        (qf, kf, vf), code, prec, n = K._prepare(q, k, v, dot_precision)
+        ops, code, prec = K._operands(q, k, v, dot_precision)
+        n = batch * heads
         dof = K._upstream(dout, n, seq, head_dim, False)
-        dq = torch.empty(n, seq, head_dim, device=q.device, dtype=qf.dtype)
-        dk, dv = torch.empty_like(dq), torch.empty_like(dq)
-        scratch = torch.empty(lib.dilution_backward_scratch_bytes(n, seq, head_dim), device=q.device,
-                              dtype=torch.uint8)
+        dq, dk, dv = (torch.empty(q.shape, device=q.device, dtype=ops[0].dtype) for _ in range(3))
+        scratch = torch.empty(lib.dilution_backward_scratch_bytes(n, seq, head_dim), device=q.device, dtype=torch.uint8)
+        rmax, rden, carry, total, ssum, pk = _parts(ws, at)
         _lib.check(lib.dilution_variant_backward(
-            qf.data_ptr(), kf.data_ptr(), vf.data_ptr(), code, prec, n, seq, head_dim, 1.0 / math.sqrt(head_dim),
-            EPS, bid, share, float(shift), dof.data_ptr(), out.data_ptr(), K._ptr(rmax), K._ptr(rden), K._ptr(carry),
-            K._ptr(total), ssum.data_ptr(), K._ptr(pk), scratch.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+            *(x.data_ptr() for x in ops), code, prec, n, seq, head_dim, 1.0 / math.sqrt(head_dim),
+            EPS, bid, share, float(shift), dof.data_ptr(), out.data_ptr(), rmax, rden, carry,
+            total, ssum, pk, scratch.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
             K._stream(q.device)), "dilution_variant_backward")
-        shape4 = (batch, heads, seq, head_dim)
-        return (dq.reshape(shape4).to(q.dtype), dk.reshape(shape4).to(k.dtype), dv.reshape(shape4).to(v.dtype),
-                None, None, None, None)
+        return (*(x if x.dtype == t.dtype else x.to(t.dtype) for x, t in zip((dq, dk, dv), (q, k, v))), None, None, None, None)
+
+
+def _parts(ws, at):
+    """Addresses of a workspace's parts, None for those that this bid and share step do without."""
+    base = ws.data_ptr()
+    return [base + at[x] if x in at else None for x in ("rmax", "rden", "carry", "total", "ssum", "pk")]
 
 
 def dilution_attention(
@@ -241,18 +246,18 @@ def dilution_decode_step(
     n = batch * heads
     qf = K._rows(q1, n, head_dim)
     if out is None:
-        out = torch.empty(n, head_dim, device=q1.device, dtype=q1.dtype)
+        out = torch.empty(batch, heads, 1, head_dim, device=q1.device, dtype=q1.dtype)
     need = lib.dilution_decode_scratch_bytes(n, length, head_dim)
     if scratch is None or scratch.numel() * scratch.element_size() < need:
         scratch = torch.empty(need, device=q1.device, dtype=torch.uint8)
     code = _lib.BF16 if q1.dtype == torch.bfloat16 else _lib.F32
     _lib.check(lib.dilution_variant_decode(
-        qf.data_ptr(), None, None, k_cache.view(n, capacity, head_dim).data_ptr(),
-        v_cache.view(n, capacity, head_dim).data_ptr(), code, n, capacity, length, head_dim,
-        1.0 / math.sqrt(head_dim), EPS, code_b, code_s, float(shift), committed.view(n, capacity).data_ptr(),
+        qf.data_ptr(), None, None, K._cache_rows(k_cache, n, capacity, head_dim).data_ptr(),
+        K._cache_rows(v_cache, n, capacity, head_dim).data_ptr(), code, n, capacity, length, head_dim,
+        1.0 / math.sqrt(head_dim), EPS, code_b, code_s, float(shift), K._cache_rows(committed, n, capacity).data_ptr(),
         out.data_ptr(),
         scratch.data_ptr(), K._stream(q1.device)), "dilution_variant_decode")
-    return out.view(batch, heads, 1, head_dim)
+    return out if out.dim() == 4 else out.view(batch, heads, 1, head_dim)
 
 
 _PATCHED = ("dilution_attention_forward", "dilution_attention", "dilution_decode_step")

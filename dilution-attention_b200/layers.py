@@ -147,7 +147,7 @@ def softmax_decode_append_step(q1, k1, v1, cache: dict, scratch=None, out=None):
     n, capacity = batch * heads, k_cache.shape[2]
     qf, kn, vn = (K._rows(x, n, d) for x in (q1, k1, v1))
     if out is None:
-        out = torch.empty(n, d, device=q1.device, dtype=q1.dtype)
+        out = torch.empty(batch, heads, 1, d, device=q1.device, dtype=q1.dtype)
     pos_dev = cache.get("pos_dev")
     need = lib.dilution_decode_scratch_bytes(n, capacity if pos_dev is not None else t + 1, d)
     if scratch is None or scratch.numel() * scratch.element_size() < need:
@@ -155,16 +155,16 @@ def softmax_decode_append_step(q1, k1, v1, cache: dict, scratch=None, out=None):
     code = _lib.BF16 if q1.dtype == torch.bfloat16 else _lib.F32
     if pos_dev is not None:
         _lib.check(lib.dilution_softmax_decode_append_at(
-            qf.data_ptr(), kn.data_ptr(), vn.data_ptr(), k_cache.view(n, capacity, d).data_ptr(),
-            v_cache.view(n, capacity, d).data_ptr(), code, n, capacity, pos_dev.data_ptr(), d, 1.0 / math.sqrt(d),
+            qf.data_ptr(), kn.data_ptr(), vn.data_ptr(), K._cache_rows(k_cache, n, capacity, d).data_ptr(),
+            K._cache_rows(v_cache, n, capacity, d).data_ptr(), code, n, capacity, pos_dev.data_ptr(), d, 1.0 / math.sqrt(d),
             out.data_ptr(), scratch.data_ptr(), K._stream(q1.device)), "dilution_softmax_decode_append_at")
     else:
         _lib.check(lib.dilution_softmax_decode_append(
-            qf.data_ptr(), kn.data_ptr(), vn.data_ptr(), k_cache.view(n, capacity, d).data_ptr(),
-            v_cache.view(n, capacity, d).data_ptr(), code, n, capacity, t + 1, d, 1.0 / math.sqrt(d),
+            qf.data_ptr(), kn.data_ptr(), vn.data_ptr(), K._cache_rows(k_cache, n, capacity, d).data_ptr(),
+            K._cache_rows(v_cache, n, capacity, d).data_ptr(), code, n, capacity, t + 1, d, 1.0 / math.sqrt(d),
             out.data_ptr(), scratch.data_ptr(), K._stream(q1.device)), "dilution_softmax_decode_append")
     cache["len"] = t + 1
-    return out.view(batch, heads, 1, d)
+    return out if out.dim() == 4 else out.view(batch, heads, 1, d)
 
 
 class GraphedDecode:
