@@ -102,6 +102,22 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   return r;
 }
 
+// poly_exp2 of two values, NaN kept: 13 instructions for the pair, where two single ones that keep a NaN take 20 and two that
+// do not 18.
+__device__ __forceinline__ float2 poly_exp2_two(float2 x) {
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x.x) : "f"(-125.f));
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x.y) : "f"(-125.f));
+  const float2 big = make_float2(12582912.f, 12582912.f);
+  const float2 r = add2(x, big), f = sub2(x, sub2(r, big));
+  float2 p = fma2(f, make_float2(0.009570085443556309f, 0.009570085443556309f),
+                  make_float2(0.05591784790158272f, 0.05591784790158272f));
+  p = fma2(p, f, make_float2(0.240247443318367f, 0.240247443318367f));
+  p = fma2(p, f, make_float2(0.6931217908859253f, 0.6931217908859253f));
+  p = fma2(p, f, make_float2(0.9999992847442627f, 0.9999992847442627f));
+  return mul2(p, make_float2(__int_as_float((__float_as_int(r.x) << 23) + 0x3f800000),
+                             __int_as_float((__float_as_int(r.y) << 23) + 0x3f800000)));
+}
+
 // Barrier of every thread of the cluster; what was written before it is visible behind it.  Not the .aligned form, which
 // takes whole warps for granted: it stands behind work of thread 0 alone and behind loops of unequal length.
 __device__ __forceinline__ void cluster_sync() {

@@ -247,28 +247,27 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
         auto chunk = [&](auto mask_tag) {
           constexpr bool MASK = decltype(mask_tag)::value;
 #pragma unroll
-          for (int e4 = 0; e4 < 8; ++e4) {
-            const float4 l = L4[e4];
-            const float ls[4] = {l.x, l.y, l.z, l.w};
-            float sh[4], dn[4];
+          for (int e8 = 0; e8 < 4; ++e8) {
+            const float4 la = L4[2 * e8], lb = L4[2 * e8 + 1];
+            const float ls[8] = {la.x, la.y, la.z, la.w, lb.x, lb.y, lb.z, lb.w};
+            float z[8], sh[8], dn[8];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              // the special-function unit binds: every fourth exponential is a degree-4 polynomial on the FMA pipe
-              const float z = fmaf(v[e4 * 4 + u], g.zscale, -ls[u]);
-              float p = u == 3 ? poly_exp2<4>(z) : fast_exp2(z);
-              if (MASK && (dead || ja > q0 + e4 * 4 + u)) p = 0.f;
+            for (int u = 0; u < 8; ++u) z[u] = fmaf(v[e8 * 8 + u], g.zscale, -ls[u]);
+            // every fourth exponential is a degree-4 polynomial on the FMA pipe
+            const float2 fourth = poly_exp2_two(make_float2(z[3], z[7]));
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+              float p = (u & 3) != 3 ? fast_exp2(z[u]) : u == 3 ? fourth.x : fourth.y;
+              if (MASK && (dead || ja > q0 + e8 * 8 + u)) p = 0.f;
               den += p;
               sh[u] = p;
               dn[u] = den;
             }
 #pragma unroll
-            for (int u = 0; u < 4; u += 2) {
+            for (int u = 0; u < 8; u += 2) {
               const float2 s2 = mul2(make_float2(sh[u], sh[u + 1]), rcp_two<PAIR>(dn[u], dn[u + 1]));
-              sh[u] = s2.x;
-              sh[u + 1] = s2.y;
+              pk[e8 * 4 + u / 2] = pack_bf16(s2.x, s2.y);
             }
-            pk[e4 * 2] = pack_bf16(sh[0], sh[1]);
-            pk[e4 * 2 + 1] = pack_bf16(sh[2], sh[3]);
           }
         };
         if (masked) chunk(std::true_type{}); else chunk(std::false_type{});

@@ -276,13 +276,13 @@ __device__ __forceinline__ float load_lse(const float* __restrict__ rmax, const 
 }
 
 // The bid of one raw score s (kernels_bid.py:191-204) given the row's lse l:
-// softmax 2^(s*zscale - l); sigmoid 1 / (1 + 2^(l - s*zscale)), which is 0 for l = +inf.
+// softmax 2^(s*zscale - l); sigmoid 1 / (1 + 2^(l - s*zscale)), which is 0 for l = +inf.  POLY: softplus's exponential on
+// the FMA pipe.
 template <int BID, bool POLY = false>
 __device__ __forceinline__ float bid_p(float s, float zscale, float l) {
   if (row_sum_bid(BID)) return mass_bid(mass_power<BID>(mass_term<BID, POLY>(s, zscale)), l);
   if (BID == kBidSigmoid) return fast_rcp(1.f + fast_exp2(fmaf(s, -zscale, l)));
-  // POLY: the exponential on the FMA pipe (a share of them, where the special-function unit binds)
-  return POLY ? poly_exp2<4>(fmaf(s, zscale, -l)) : fast_exp2(fmaf(s, zscale, -l));
+  return fast_exp2(fmaf(s, zscale, -l));
 }
 
 // ---------------------------------------------------------------- pass 1: row statistics
@@ -732,6 +732,10 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
           lnext[0] = L4[c * 8 + e8 * 2 + 2];
           lnext[1] = L4[c * 8 + e8 * 2 + 3];
         }
+        // two special-function ops per score bind this pass: every fourth exponential of the
+        // softmax bid is a polynomial on the FMA pipe (79.7 -> 75.3 ms at the 128K prefill shape)
+        const float2 fourth = poly_exp2_two(make_float2(fmaf(v[e8 * 8 + 3], g.zscale, -lcur[0].w),
+                                                        fmaf(v[e8 * 8 + 7], g.zscale, -lcur[1].w)));
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const float ls[4] = {lcur[h].x, lcur[h].y, lcur[h].z, lcur[h].w};
@@ -739,9 +743,7 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             const int e = e8 * 8 + h * 4 + u;
-            // two special-function ops per score bind this pass: every fourth exponential of the
-            // softmax bid is a polynomial on the FMA pipe (79.7 -> 75.3 ms at the 128K prefill shape)
-            float p = u == 3 ? bid_p<kBidSoftmax, true>(v[e], g.zscale, ls[u]) : bid_p<kBidSoftmax>(v[e], g.zscale, ls[u]);
+            float p = u < 3 ? bid_p<kBidSoftmax>(v[e], g.zscale, ls[u]) : h == 0 ? fourth.x : fourth.y;
             if (MASK && (dead || ja > qh + c * 32 + e)) p = 0.f;
             if (SHARE == kShareInclusive) {
               den += p;

@@ -184,3 +184,35 @@ def test_infinite_values_make_infinite_outputs(path, pos, signs):
     keep = torch.ones_like(full, dtype=torch.bool)
     keep[0, 1, pos // 128 * 128:, 7] = False
     assert torch.equal(full[keep], clean[keep])
+
+
+@pytest.mark.parametrize("training", [False, True])
+@pytest.mark.parametrize("what", ["q", "k"])
+@pytest.mark.parametrize("pos", [3, 128, 129, 130, 131, 259, SEQ - 1])
+def test_a_nan_comes_through_every_exponential_of_bf16_heads_of_64(pos, what, training):
+    x = list(make_inputs(1, 2, SEQ, 64, 12))[:3]
+    x["qk".index(what)][0, 0, pos, 5] = float("nan")
+    same_as_exact(x, torch.bfloat16, "bf16", training)
+
+
+@pytest.mark.parametrize("training", [False, True])
+@pytest.mark.parametrize("what", ["q", "k"])
+@pytest.mark.parametrize("pos", [1000, 1001, 1002, 1003])
+def test_a_nan_in_a_sweep_of_512_keys(pos, what, training):
+    """A NaN query makes every demand NaN that it bids for, a NaN key its own, and both every output from there on, in a call
+    of 256 blocks of 512 keys or more."""
+    rows, seq = 52, 2049
+    x = [t.bfloat16().to(DEV) for t in make_inputs(1, rows, seq, 64, 18)[:3]]
+    x["qk".index(what)][0, 1, pos, 5] = float("nan")
+    pkg = load_package()
+    pkg._lib.profile(True)
+    pkg._lib.profile_collect()
+    out, aux = pkg.kernels.dilution_attention_forward(*x, dot_precision="bf16", return_aux=True, _training=training)
+    names = set(pkg._lib.profile_collect())
+    pkg._lib.profile(False)
+    assert "tc_forward_fused" in names
+    total = aux["committed_total"]
+    assert out[0, 1, pos:].isnan().all() and out[0, 1, :pos].isfinite().all()
+    assert total[0, 1, pos].isnan() and (what == "k" or total[0, 1, :pos].isnan().all())
+    for other in (0, 2, rows - 1):
+        assert out[0, other].isfinite().all() and total[0, other].isfinite().all()
