@@ -102,18 +102,28 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   return r;
 }
 
-// poly_exp2 of two values, NaN kept: 13 instructions for the pair, where two single ones that keep a NaN take 20 and two that
-// do not 18.
+// poly_exp2 of two values, NaN kept: 13 instructions for the pair at degree 4, where two single ones that keep a NaN take 20
+// and two that do not 18.  Degree 5 is as exact as the special-function unit (2.1e-7).
+template <int DEG>
 __device__ __forceinline__ float2 poly_exp2_two(float2 x) {
+  static_assert(DEG == 4 || DEG == 5, "degree 4 or 5");
+  auto both = [](float c) { return make_float2(c, c); };
   asm("max.NaN.f32 %0, %0, %1;" : "+f"(x.x) : "f"(-125.f));
   asm("max.NaN.f32 %0, %0, %1;" : "+f"(x.y) : "f"(-125.f));
-  const float2 big = make_float2(12582912.f, 12582912.f);
-  const float2 r = add2(x, big), f = sub2(x, sub2(r, big));
-  float2 p = fma2(f, make_float2(0.009570085443556309f, 0.009570085443556309f),
-                  make_float2(0.05591784790158272f, 0.05591784790158272f));
-  p = fma2(p, f, make_float2(0.240247443318367f, 0.240247443318367f));
-  p = fma2(p, f, make_float2(0.6931217908859253f, 0.6931217908859253f));
-  p = fma2(p, f, make_float2(0.9999992847442627f, 0.9999992847442627f));
+  const float2 r = add2(x, both(12582912.f)), f = sub2(x, sub2(r, both(12582912.f)));
+  float2 p;
+  if (DEG == 5) {
+    p = fma2(f, both(0.0013276472454890609f), both(0.009675540961325169f));
+    p = fma2(p, f, both(0.05550713092088699f));
+    p = fma2(p, f, both(0.24022120237350464f));
+    p = fma2(p, f, both(0.6931469440460205f));
+    p = fma2(p, f, both(1.f));
+  } else {
+    p = fma2(f, both(0.009570085443556309f), both(0.05591784790158272f));
+    p = fma2(p, f, both(0.240247443318367f));
+    p = fma2(p, f, both(0.6931217908859253f));
+    p = fma2(p, f, both(0.9999992847442627f));
+  }
   return mul2(p, make_float2(__int_as_float((__float_as_int(r.x) << 23) + 0x3f800000),
                              __int_as_float((__float_as_int(r.y) << 23) + 0x3f800000)));
 }

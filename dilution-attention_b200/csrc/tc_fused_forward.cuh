@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
   uint8_t* ones_ptr = smem + G * kTileBytes;
   const uint32_t sSh = sOnes + kTileBytes;                                   // [G][128 keys][64 queries]
   const uint32_t sQ = sSh + G * kTileBytes, sStage = sQ + R * HB;            // staging: [2 warps][64 queries][32 features] fp32
-  float* sL = reinterpret_cast<float*>(smem + (sStage - sV) + kTileBytes);   // [4][64] lse of a half tile's queries
+  float* sL = reinterpret_cast<float*>(smem + (sStage - sV) + kTileBytes);   // [4][64] -lse of a half tile's queries
   uint64_t* bars = reinterpret_cast<uint64_t*>(sL + 256);
   const uint32_t vfull = smem_u32(bars), qfull = vfull + 8, ofull = qfull + 8 * R;            // 1, [R], [2]
   const uint32_t sdone = ofull + 16, odone = sdone + 8 * G, sfree = odone + 8 * G, shready = sfree + 8 * G;   // [G] each
@@ -71,9 +71,9 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
   __syncwarp();
   if (warp == 0) tmem_alloc(smem_u32(&ctl->tmem), kTmem);
   if (wg == G) {
-    sL[row] = load_lse(rmax, rden, row_base, h0 * 64 + row, g.tq);         // of the first three half tiles
+    sL[row] = -load_lse(rmax, rden, row_base, h0 * 64 + row, g.tq);         // of the first three half tiles
   } else if (wg == 0) {
-    if (row < 64) sL[128 + row] = load_lse(rmax, rden, row_base, h0 * 64 + 128 + row, g.tq);
+    if (row < 64) sL[128 + row] = -load_lse(rmax, rden, row_base, h0 * 64 + 128 + row, g.tq);
 #pragma unroll
     for (int c = 0; c < 8; ++c)
       reinterpret_cast<uint4*>(ones_ptr)[row * 8 + c] = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
       if (lane == 0) mbar_wait(ofull + 8 * (u & 1), (u >> 1) & 1, ctl, &g_status, kErrWaitMma);
       __syncwarp();
       tc_fence_after();
-      if (fetch) sL[64 * ((u + 3) & 3) + row] = nx_max + log2f(nx_den);
+      if (fetch) sL[64 * ((u + 3) & 3) + row] = -(nx_max + log2f(nx_den));
       __syncwarp();
       const uint32_t tOb = tO + 64 * (u & 1) + lane_base;
       if (w4 < 2) {
@@ -231,7 +231,9 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
     const uint32_t tSw = tS + 64 * wg + lane_base;
     const uint32_t sShw = sSh + kTileBytes * wg;
     const int kw = k0 + wg * kTileRows;
-    float den = g.eps;                                       // committed + eps, for the whole sweep
+    // committed + eps in front of a chunk of 32 queries, and what its sum has rounded off: the bids of a chunk are added up from
+    // zero and folded in once, so that neither thousands of roundings nor bids under half an ulp of a large demand add up
+    float base = g.eps, low = 0.f;
     for (int h = h0 + 2 * wg; h < nh && wg < groups; ++h) {
       const int t = h - h0 - 2 * wg;
       float v0[32], v1[32];
@@ -240,8 +242,9 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
         const int q0 = h * 64 + 32 * c;
         if (CR == 32 || c == 0) {                            // checkpoint in front of the chunk's first query
           const int rb = q0 / CR;
-          if (!dead && rb < ncb) carry[((int64_t)n * ncb + rb) * g.tk + ja] = den - g.eps;
+          if (!dead && rb < ncb) carry[((int64_t)n * ncb + rb) * g.tk + ja] = base - g.eps;
         }
+        float chunk_sum = 0.f;
         const float4* L4 = reinterpret_cast<const float4*>(sL + 64 * ((h - h0) & 3) + 32 * c);
         const bool masked = dead || kw + kTileRows - 1 > q0;
         auto chunk = [&](auto mask_tag) {
@@ -252,25 +255,34 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
             const float ls[8] = {la.x, la.y, la.z, la.w, lb.x, lb.y, lb.z, lb.w};
             float z[8], sh[8], dn[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) z[u] = fmaf(v[e8 * 8 + u], g.zscale, -ls[u]);
-            // every fourth exponential is a degree-4 polynomial on the FMA pipe
-            const float2 fourth = poly_exp2_two(make_float2(z[3], z[7]));
+            for (int u = 0; u < 8; u += 2) {
+              const float2 z2 = fma2(make_float2(v[e8 * 8 + u], v[e8 * 8 + u + 1]), make_float2(g.zscale, g.zscale),
+                                     make_float2(ls[u], ls[u + 1]));
+              z[u] = z2.x;
+              z[u + 1] = z2.y;
+            }
+            // every fourth exponential is a polynomial on the FMA pipe, of degree 5: the demand is an output in fp32
+            const float2 fourth = poly_exp2_two<5>(make_float2(z[3], z[7]));
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
               float p = (u & 3) != 3 ? fast_exp2(z[u]) : u == 3 ? fourth.x : fourth.y;
               if (MASK && (dead || ja > q0 + e8 * 8 + u)) p = 0.f;
-              den += p;
+              chunk_sum += p;
               sh[u] = p;
-              dn[u] = den;
+              dn[u] = chunk_sum;
             }
 #pragma unroll
             for (int u = 0; u < 8; u += 2) {
-              const float2 s2 = mul2(make_float2(sh[u], sh[u + 1]), rcp_two<PAIR>(dn[u], dn[u + 1]));
+              const float2 den = add2(make_float2(base, base), make_float2(dn[u], dn[u + 1]));
+              const float2 s2 = mul2(make_float2(sh[u], sh[u + 1]), rcp_two<PAIR>(den.x, den.y));
               pk[e8 * 4 + u / 2] = pack_bf16(s2.x, s2.y);
             }
           }
         };
         if (masked) chunk(std::true_type{}); else chunk(std::false_type{});
+        const float add = chunk_sum - low, sum = base + add;
+        low = (sum - base) - add;
+        base = sum;
         __syncwarp();
       };
       auto store = [&](int c) {
@@ -299,7 +311,7 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
       __syncwarp();
       if (lane == 0) mbar_arrive(shready + 8 * wg);
     }
-    if (!dead) total[(int64_t)n * g.tk + ja] = den - g.eps;
+    if (!dead) total[(int64_t)n * g.tk + ja] = base - g.eps;
   }
   drain_if_aborted(ctl);
   tc_fence_before();

@@ -734,7 +734,7 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
         }
         // two special-function ops per score bind this pass: every fourth exponential of the
         // softmax bid is a polynomial on the FMA pipe (79.7 -> 75.3 ms at the 128K prefill shape)
-        const float2 fourth = poly_exp2_two(make_float2(fmaf(v[e8 * 8 + 3], g.zscale, -lcur[0].w),
+        const float2 fourth = poly_exp2_two<4>(make_float2(fmaf(v[e8 * 8 + 3], g.zscale, -lcur[0].w),
                                                         fmaf(v[e8 * 8 + 7], g.zscale, -lcur[1].w)));
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
