@@ -112,6 +112,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, Ctl* ct
   return true;
 }
 
+// The wait of a whole warp that issues: its lanes meet behind it.  Every lane polls for itself, but only the elected one's
+// MMAs, commits and copies make the barriers go on; a lane that was still polling when the phase after the next began
+// would wait for a parity that comes back no more.  No such lane can exist if nothing is issued before all have seen the phase.
+__device__ __forceinline__ void mbar_wait_warp(uint32_t bar, uint32_t parity, Ctl* ctl, int* status, int code) {
+  mbar_wait(bar, parity, ctl, status, code);
+  __syncwarp();
+}
+
 // After a wait has given up, the CTA runs to its end without waiting for anything, so copies and
 // MMAs it issued may still be in flight when it gets there.  Every kernel calls this in front of its
 // last CTA-wide barrier: a CTA that gave up idles for a fixed grace period (about 0.2 ms, three

@@ -185,10 +185,10 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
         for (int w = 0; w < groups; ++w) tma_load_tile(sV + kTileBytes * w, &map_v, k0 + w * kTileRows, n, vfull);
       }
       for (int h = h0; h < h0 + R && h < nh; ++h) load_q(h);
-      mbar_wait(qfull, 0, ctl, &g_status, kErrWaitTma);
+      mbar_wait_warp(qfull, 0, ctl, &g_status, kErrWaitTma);
       tc_fence_after();
       issue_scores(0, h0);
-      mbar_wait(vfull, 0, ctl, &g_status, kErrWaitTma);
+      mbar_wait_warp(vfull, 0, ctl, &g_status, kErrWaitTma);
     }
     __syncwarp();
     for (int h = h0; h < nh; ++h) {
@@ -197,11 +197,11 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
       if (issuer) {
         if (h + 1 < nh) {
           // scores of h + 1, as soon as a warpgroup has taken those of h out of TMEM
-          mbar_wait(qfull + 8 * ((u + 1) % R), ((u + 1) / R) & 1, ctl, &g_status, kErrWaitTma);
+          mbar_wait_warp(qfull + 8 * ((u + 1) % R), ((u + 1) / R) & 1, ctl, &g_status, kErrWaitTma);
           for (int w = 0; w < groups; ++w) {
             const int t = u - 2 * w;                         // the warpgroup's own count of half tiles
             if (t + 1 < 0) break;
-            if (t >= 0) mbar_wait(sfree + 8 * w, t & 1, ctl, &g_status, kErrWaitTile);
+            if (t >= 0) mbar_wait_warp(sfree + 8 * w, t & 1, ctl, &g_status, kErrWaitTile);
             tc_fence_after();
             issue_scores(w, h + 1);
           }
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
         for (int w = 0; w < groups; ++w) {
           const int t = u - 2 * w;
           if (t < 0) break;
-          mbar_wait(shready + 8 * w, t & 1, ctl, &g_status, kErrWaitTile);
+          mbar_wait_warp(shready + 8 * w, t & 1, ctl, &g_status, kErrWaitTile);
           tc_fence_after();
           const Desc dVw = make_desc(sV + kTileBytes * w, sOnes - sV - kTileBytes * w, 1024);
 #pragma unroll

@@ -940,15 +940,15 @@ __global__ void __launch_bounds__(kMainThreads<W>, W == kNarrow ? 2 : 1) forward
       // descriptors are built once; a k-step of O is a constant 2048 B (128 units) further
       const Desc dK0 = make_desc(sK0, 16, 1024), dK1 = make_desc(sK0 + TB, 16, 1024), dQ = make_desc(sQ, 16, 1024);
       const Desc dSh = make_desc(sSh, kTileBytes, 1024), dVm = make_desc(sV, kTileBytes, 1024);
-      mbar_wait(kfull, 0, ctl, &g_status, kErrWaitTma);
+      mbar_wait_warp(kfull, 0, ctl, &g_status, kErrWaitTma);
       tc_fence_after();
       mma_scores_wide<W>(lead, tS, dK0, kTileBytes, dQ, kTileBytes, id_s);
       mma_commit(lead, sdone);
       for (int jb = 0; jb < njb; ++jb) {
         const int b = jb & 1;
         if (jb + 1 < njb) {
-          mbar_wait(kfull + 8 * (b ^ 1), ((jb + 1) >> 1) & 1, ctl, &g_status, kErrWaitTma);
-          mbar_wait(sfree, jb & 1, ctl, &g_status, kErrWaitTile);
+          mbar_wait_warp(kfull + 8 * (b ^ 1), ((jb + 1) >> 1) & 1, ctl, &g_status, kErrWaitTma);
+          mbar_wait_warp(sfree, jb & 1, ctl, &g_status, kErrWaitTile);
           tc_fence_after();
           mma_scores_wide<W>(lead, tS, b ? dK0 : dK1, kTileBytes, dQ, kTileBytes, id_s);
           mma_commit(lead, sdone);
@@ -958,14 +958,14 @@ __global__ void __launch_bounds__(kMainThreads<W>, W == kNarrow ? 2 : 1) forward
           }
         }
         if (jb >= 1) {                    // V is free once the previous share V has completed
-          mbar_wait(odone, (jb - 1) & 1, ctl, &g_status, kErrWaitMma);
+          mbar_wait_warp(odone, (jb - 1) & 1, ctl, &g_status, kErrWaitMma);
           if (lead) {
             mbar_expect_tx(vfull, TB);
             tma_load_rows<W>(sV, &map_v, jb * kTileRows, n, vfull);
           }
         }
-        mbar_wait(shready, jb & 1, ctl, &g_status, kErrWaitTile);
-        mbar_wait(vfull, jb & 1, ctl, &g_status, kErrWaitTma);
+        mbar_wait_warp(shready, jb & 1, ctl, &g_status, kErrWaitTile);
+        mbar_wait_warp(vfull, jb & 1, ctl, &g_status, kErrWaitTma);
         tc_fence_after();
 #pragma unroll
         for (int pl = 0; pl < P; ++pl)
@@ -1505,8 +1505,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
         mma_ts(lead, tDOV0 + 64 * ODD, tV + 8 * kk, make_desc(sPd, 16, 1024), off + 2 * kk, id_s, 1);
     };
     if (warp_u == 8) {
-      mbar_wait(kfull, 0, ctl, &g_status, kErrWaitTma);
-      mbar_wait(qfull, 0, ctl, &g_status, kErrWaitTma);
+      mbar_wait_warp(kfull, 0, ctl, &g_status, kErrWaitTma);
+      mbar_wait_warp(qfull, 0, ctl, &g_status, kErrWaitTma);
       tc_fence_after();
       issue_scores(std::integral_constant<int, 0>{}, std::integral_constant<int, 0>{});
       mma_commit(lead, sdone);
@@ -1519,7 +1519,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
       constexpr int ODD = decltype(odd_c)::value, ST = decltype(st_c)::value;
       constexpr int ST1 = (ST + 1) % 3, ST2 = (ST + 2) % 3;
       if (warp_u == 8) {
-        mbar_wait(tiles + 8 * ODD, s & 1, ctl, &g_status, kErrWaitTile);
+        mbar_wait_warp(tiles + 8 * ODD, s & 1, ctl, &g_status, kErrWaitTile);
         tc_fence_after();
 #pragma unroll
         for (int kq = 0; PASS != 1 && kq < 4; ++kq) {       // contraction over the 64 queries
@@ -1538,7 +1538,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
         }
         if (s + 1 < nsteps) {                               // half-step h + 2 belongs to step s + 1
           if (!ODD) {
-            mbar_wait(qfull + 8 * ST1, ((s + 1) / 3) & 1, ctl, &g_status, kErrWaitTma);
+            mbar_wait_warp(qfull + 8 * ST1, ((s + 1) / 3) & 1, ctl, &g_status, kErrWaitTma);
             tc_fence_after();
           }
           issue_scores(odd_c, std::integral_constant<int, ST1>{});
@@ -1547,12 +1547,12 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
         if (!ODD && s >= 1 && s + 2 < nsteps) {
           // every MMA of step s-1 has completed once the commit of its second half-step has:
           // its Q and dO' stage takes step s+2
-          mbar_wait(sdone + 8, s & 1, ctl, &g_status, kErrWaitMma);
+          mbar_wait_warp(sdone + 8, s & 1, ctl, &g_status, kErrWaitMma);
           if (lead) {
-          mbar_expect_tx(qfull + 8 * ST2, kStageTx);
-          tma_load_tile(sQ0 + kTileBytes * ST2, &map_q, (nqb - 3 - s) * kTileRows, n, qfull + 8 * ST2);
-          tma_load_tile(sD0 + kTileBytes * ST2, &map_do, (nqb - 3 - s) * kTileRows, n, qfull + 8 * ST2);
-          if (PASS == 1) tma_load_tile(sPd + kTileBytes * ST2, &map_do, (nqb - 3 - s) * kTileRows, n, qfull + 8 * ST2, 64);
+            mbar_expect_tx(qfull + 8 * ST2, kStageTx);
+            tma_load_tile(sQ0 + kTileBytes * ST2, &map_q, (nqb - 3 - s) * kTileRows, n, qfull + 8 * ST2);
+            tma_load_tile(sD0 + kTileBytes * ST2, &map_do, (nqb - 3 - s) * kTileRows, n, qfull + 8 * ST2);
+            if (PASS == 1) tma_load_tile(sPd + kTileBytes * ST2, &map_do, (nqb - 3 - s) * kTileRows, n, qfull + 8 * ST2, 64);
           }
         }
       }

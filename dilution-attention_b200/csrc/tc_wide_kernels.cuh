@@ -264,13 +264,13 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
     auto issue_scores = [&](int h) {
       const int st = h % NR;
       const uint32_t col = NS == 2 ? 128 * (h & 1) : 0;
-      mbar_wait(qfull + 8 * st, (h / NR) & 1, ctl, &g_status, kErrWaitTma);
+      mbar_wait_warp(qfull + 8 * st, (h / NR) & 1, ctl, &g_status, kErrWaitTma);
       tc_fence_after();
       mma_scores_wide<W>(lead, tS + col, dKk, kTileBytes, make_desc(sQ0 + HB * st, 16, 1024), HSub, id_s);
       mma_dov_wide<W>(lead, tDOV + col, dVk, kTileBytes, make_desc(sD0 + HBd * st, 16, 1024), HSub, id_s);
     };
     if (warp_u == 8) {
-      mbar_wait(kfull, 0, ctl, &g_status, kErrWaitTma);
+      mbar_wait_warp(kfull, 0, ctl, &g_status, kErrWaitTma);
       for (int h = 0; h < NS; ++h) {
         issue_scores(h);
         mma_commit(lead, sdone + 8 * h);
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
     for (int h = 0; h < nhalf; ++h) {
       const int st = h % NR, sc = NS == 2 ? h & 1 : 0;      // stage of q and do', stage of the scores
       if (warp_u == 8) {
-        mbar_wait(tiles + 8 * sc, (h / NS) & 1, ctl, &g_status, kErrWaitTile);
+        mbar_wait_warp(tiles + 8 * sc, (h / NS) & 1, ctl, &g_status, kErrWaitTile);
         tc_fence_after();
         const Desc dQm = make_desc(sQ0 + HB * st, HSub, 1024), dDm = make_desc(sD0 + HBd * st, HSub, 1024);
 #pragma unroll
@@ -304,12 +304,12 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
         if (NS == 1) {
           if (h + 2 < nhalf) {
             // the products that read this stage come before the scores of h + 1, whose commit covers them
-            mbar_wait(sdone, (h + 1) & 1, ctl, &g_status, kErrWaitMma);
+            mbar_wait_warp(sdone, (h + 1) & 1, ctl, &g_status, kErrWaitMma);
             if (lead) load_stage(h + 2);
           }
         } else if (h >= 1 && h + 3 < nhalf) {
           // the products of h - 1 have completed once the commit behind them has: their stage takes h + 3
-          mbar_wait(sdone + 8 * ((h - 1) & 1), ((h - 1) / 2 + 1) & 1, ctl, &g_status, kErrWaitMma);
+          mbar_wait_warp(sdone + 8 * ((h - 1) & 1), ((h - 1) / 2 + 1) & 1, ctl, &g_status, kErrWaitMma);
           if (lead) load_stage(h + 3);
         }
       }
