@@ -28,6 +28,8 @@ namespace dil {
 namespace tc {
 
 constexpr int kFusedRing = 4;                              // half tiles of q
+constexpr int kFusedRegs = 96;                             // per thread at launch of four compute warpgroups, by the launch bounds
+static_assert(4 * 104 + 64 <= 5 * kFusedRegs, "setmaxnreg hands out what the block was launched with");
 // V[G] ones shares[G] | Q[4] (8 KB each) | staging (16 KB) | lse [4][64] | barriers
 template <int G> constexpr int kFusedSmem = (2 * G + 1) * kTileBytes + kFusedRing * kTileBytes / 2 + kTileBytes + 1024 + 256 + 1024;
 
@@ -107,7 +109,6 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
 
   if (wg == G) {
     // ------------------------------------------------------------ issue, and the O read-out
-    // (registers of G = 4: 5 x 96 at launch, then 4 x 104 + 64)
     if (G == 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
     constexpr uint32_t id_s = instr_desc(128, 64, 0, 0);     // scores: A from TMEM, B K-major
     constexpr uint32_t id_o = instr_desc(128, 64, 1, 1);     // O^T: A and B MN-major
@@ -356,7 +357,7 @@ inline int forward_fused(const void* q, const void* k, const void* v, const Geom
     constexpr int G = decltype(groups_c)::value, smem = kFusedSmem<G>;
     static_assert(smem <= 232448 && (G > 1 || 2 * (smem + 1024) <= 233472), "one or two CTAs fit one SM's shared memory");
     auto kern = forward_fused_kernel<G, decltype(cr_c)::value, decltype(pair_c)::value>;
-    if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
+    if (int rc = set_smem_attr((const void*)kern, smem, err, errlen, G == 4 ? kFusedRegs : 0)) return rc;
     const int nsb = (g.tk + G * kTileRows - 1) / (G * kTileRows);
     kern<<<(unsigned)(g.n * nsb), 128 * (G + 1), smem, st>>>(mq, mv, mo, g, (const __nv_bfloat16*)k, rmax, rden, carry, total,
                                                             ssum);

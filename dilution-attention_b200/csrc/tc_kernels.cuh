@@ -1353,6 +1353,8 @@ __device__ __forceinline__ float sum_over_lanes(float (&x)[32], int lane) {
 // the arithmetic of h + 1.  Q and dO' tiles are triple-buffered.  After setup the third
 // warpgroup gives registers up (setmaxnreg) and the compute warpgroups take them.
 constexpr int kBwdThreads = 384;
+constexpr int kBwdRegs = 168;      // per thread at launch, by the launch bounds; the reverse passes' splits stay within them
+static_assert(128 + 2 * 184 <= 3 * kBwdRegs && 104 + 2 * 200 <= 3 * kBwdRegs, "setmaxnreg hands out what the block was launched with");
 constexpr int kBwdSmem = 12 * kTileBytes + 2048 + 2048 + 256 + 1024;
 
 // PASS 1 (reverse_sweeps; pass 2 is wide_backward_main_kernel) forms only the scores and adds up ghat, p * dp over the
@@ -1997,11 +1999,22 @@ __global__ void cast_dq_kernel(const float* __restrict__ src, __nv_bfloat16* __r
 
 // The opt-in to more than 48 KB of dynamic shared memory is per kernel and per device: it is
 // made on the first launch of that kernel on that device and remembered.
-inline int set_smem_attr(const void* fn, int bytes, char* err, size_t errlen) {
+// regs: registers per thread that the kernel's setmaxnreg split needs at launch.  An increase beyond what the block was launched
+// with waits for ever, so a build in which the compiler took fewer is refused here.
+inline int set_smem_attr(const void* fn, int bytes, char* err, size_t errlen, int regs = 0) {
   static OncePerDevice opted_in;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) dev = -1;
   if (opted_in.done(fn, dev)) return 0;
+  if (regs > 0) {
+    cudaFuncAttributes at;
+    const cudaError_t e = cudaFuncGetAttributes(&at, fn);
+    if (e != cudaSuccess || at.numRegs < regs) {
+      if (e != cudaSuccess) snprintf(err, errlen, "cudaFuncGetAttributes: %s", cudaGetErrorString(e));
+      else snprintf(err, errlen, "kernel built with %d registers, its split needs %d", at.numRegs, regs);
+      return 3;
+    }
+  }
   const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e != cudaSuccess) {
     snprintf(err, errlen, "cudaFuncSetAttribute(%d): %s", bytes, cudaGetErrorString(e));
@@ -2148,7 +2161,7 @@ inline int backward(const void* q, const void* k, const void* v, const Geom& g, 
     mark("tc_backward_main", st, 0);
     const unsigned grid = (unsigned)(g.n * nkb);
     DIL_TC_PLAIN_BID(g, DIL_TC_SHARE(g, {
-      if (int rc = set_smem_attr((const void*)backward_main_kernel<BID, SHARE>, smem_bwd, err, errlen)) return rc;
+      if (int rc = set_smem_attr((const void*)backward_main_kernel<BID, SHARE>, smem_bwd, err, errlen, kBwdRegs)) return rc;
       backward_main_kernel<BID, SHARE><<<grid, kBwdThreads, smem_bwd, st>>>(
           mq, mk, md, mdq, g, (const __nv_bfloat16*)v, rmax, rden, dbarp, carry, total, dq_main, dk_main,
           (__nv_bfloat16*)dv, ghat);

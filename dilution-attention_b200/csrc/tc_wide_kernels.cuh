@@ -570,7 +570,7 @@ inline int wide_backward(const void* q, const void* k, const void* v, const Geom
     constexpr int smem = kBwdWideSmem<W>;
     static_assert(smem <= 232448 && 2 * smem > 233472, "the wide reverse pass runs one CTA per SM");
     auto kern = wide_backward_main_kernel<W, TOut>;
-    if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
+    if (int rc = set_smem_attr((const void*)kern, smem, err, errlen, kBwdRegs)) return rc;
     mark("tc_wide_backward_main", st, 0);
     kern<<<grid, kBwdThreads, smem, st>>>(mq64, m.k, m.v, md64, mdq, g, rmax, rden, dbarp, carry, total, dk_main,
                                           (TOut*)dv, ghat);
@@ -648,7 +648,7 @@ inline int mass_backward(const void* q, const void* k, const void* v, const Geom
   // factor of 1 / (row mass) would multiply what that leaves of it
   DIL_TC_MASS_BID(g, DIL_TC_SHARE(g, {
     auto kern = backward_main_kernel<BID, SHARE, 1>;
-    if (int rc = set_smem_attr((const void*)kern, kBwdSmem, err, errlen)) return rc;
+    if (int rc = set_smem_attr((const void*)kern, kBwdSmem, err, errlen, kBwdRegs)) return rc;
     mark("tc_backward_ghat", st, 0);
     kern<<<grid, kBwdThreads, kBwdSmem, st>>>(mq, mk, md, mdq, g, (const bf*)v, rmax, rden, dbarp, carry, total, nullptr,
                                               nullptr, nullptr, ghat);
@@ -657,7 +657,7 @@ inline int mass_backward(const void* q, const void* k, const void* v, const Geom
     auto main = wide_backward_main_kernel<kPairs64, bf, BID, SHARE, 2>;
     constexpr int smem = kBwdWideSmem<kPairs64>;
     static_assert(smem <= 232448 && 2 * smem > 233472, "the wide reverse pass runs one CTA per SM");
-    if (int rc = set_smem_attr((const void*)main, smem, err, errlen)) return rc;
+    if (int rc = set_smem_attr((const void*)main, smem, err, errlen, kBwdRegs)) return rc;
     mark("tc_backward_main", st, 0);
     main<<<grid, kBwdThreads, smem, st>>>(mq64, mk, mv, md64, mdq, g, rmax, rden, dbarp, carry, total, (bf*)dk, (bf*)dv,
                                           ghat);
