@@ -225,8 +225,13 @@ __device__ __forceinline__ float2 rcp_two(float a, float b) {
   return mul2(make_float2(r, r), make_float2(m, a));
 }
 // Whether every demand of a call stays in that range: eps in front, bids of at most 1 (expshift has no row sum: any size).
+// Demands that a caller hands in (carry_base) are held at the upper end, where a share is nothing: capped_demand.
 inline bool pair_demands(const Geom& g) {
-  return g.eps >= 1e-18f && (g.normalised || g.bid == kBidSigmoid);
+  return g.eps >= 1e-18f && g.eps <= 1e18f && (g.normalised || g.bid == kBidSigmoid);
+}
+template <bool PAIR, int SHARE>
+__device__ __forceinline__ float capped_demand(float d) {
+  return PAIR && SHARE == kShareInclusive && d > 1e18f ? 1e18f : d;      // (a NaN stays one)
 }
 
 // Byte offset of the 16-byte chunk holding queries [q, q+8) of `key` in an
@@ -691,7 +696,7 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
       d += carry[carry_row + jx];
       if (carry_base != nullptr) d += carry_base[(int64_t)n * g.tk + jx];
     }
-    return d;
+    return capped_demand<PAIR, SHARE>(d);
   };
   float den_next = load_den(0);
   for (int jb = 0; jb < njb; ++jb) {
@@ -991,7 +996,7 @@ __global__ void __launch_bounds__(kMainThreads<W>, W == kNarrow ? 2 : 1) forward
       d += carry[carry_row + jx];
       if (carry_base != nullptr) d += carry_base[(int64_t)n * g.tk + jx];
     }
-    return d;
+    return capped_demand<PAIR, SHARE>(d);
   };
   float den_next = load_den(0);
   for (int jb = 0; jb < njb; ++jb) {
