@@ -453,6 +453,12 @@ def _rows(x, n, head_dim):
     return x if x.is_contiguous() else x.contiguous()
 
 
+def _step_output(out, batch, heads, head_dim):
+    """A step's output, or the caller's buffer for it in any shape, as (batch, heads, 1, head_dim) (a view of what has that
+    shape already would cost 1 us)."""
+    return out if out.shape == (batch, heads, 1, head_dim) else out.view(batch, heads, 1, head_dim)
+
+
 def _cache_rows(x, *shape):
     """A cache buffer as the kernels read it by its address.  It must be contiguous: .view refuses others."""
     return x if x.is_contiguous() and x.numel() == math.prod(shape) else x.view(*shape)
@@ -494,7 +500,7 @@ def dilution_decode_step(
                                    length, head_dim, 1.0 / math.sqrt(head_dim), EPS,
                                    cf.data_ptr(), out.data_ptr(), scratch.data_ptr(),
                                    _stream(q1.device)), "dilution_decode")
-    return out if out.dim() == 4 else out.view(batch, heads, 1, head_dim)
+    return _step_output(out, batch, heads, head_dim)
 
 
 def dilution_decode_append_step(
@@ -550,7 +556,7 @@ def dilution_decode_append_step(
                                               1.0 / math.sqrt(head_dim), EPS, cf.data_ptr(), out.data_ptr(),
                                               scratch.data_ptr(), _stream(q1.device)), "dilution_decode_append")
     cache["len"] = t + 1
-    return out if out.dim() == 4 else out.view(batch, heads, 1, head_dim)
+    return _step_output(out, batch, heads, head_dim)
 
 
 _COPY_STREAMS: dict = {}

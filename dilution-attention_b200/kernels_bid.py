@@ -257,7 +257,7 @@ def dilution_decode_step(
         1.0 / math.sqrt(head_dim), EPS, code_b, code_s, float(shift), K._cache_rows(committed, n, capacity).data_ptr(),
         out.data_ptr(),
         scratch.data_ptr(), K._stream(q1.device)), "dilution_variant_decode")
-    return out if out.dim() == 4 else out.view(batch, heads, 1, head_dim)
+    return K._step_output(out, batch, heads, head_dim)
 
 
 _PATCHED = ("dilution_attention_forward", "dilution_attention", "dilution_decode_step")

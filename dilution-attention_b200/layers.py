@@ -164,7 +164,7 @@ def softmax_decode_append_step(q1, k1, v1, cache: dict, scratch=None, out=None):
             K._cache_rows(v_cache, n, capacity, d).data_ptr(), code, n, capacity, t + 1, d, 1.0 / math.sqrt(d),
             out.data_ptr(), scratch.data_ptr(), K._stream(q1.device)), "dilution_softmax_decode_append")
     cache["len"] = t + 1
-    return out if out.dim() == 4 else out.view(batch, heads, 1, d)
+    return K._step_output(out, batch, heads, d)
 
 
 class GraphedDecode:

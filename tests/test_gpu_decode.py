@@ -5,7 +5,7 @@ from __future__ import annotations
 import pytest
 import torch
 
-from conftest import golden, make_inputs, rel_err
+from conftest import golden, load_package, make_inputs, rel_err
 from oracle import dilution_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -198,3 +198,30 @@ def test_position_past_the_capacity_stays_inside_the_cache(kernels, pkg):
         row = cap - 1 if position >= cap else 0
         got_k = kc.view(n, cap, d)[:, row]
         assert torch.equal(got_k, k1)
+
+
+@pytest.mark.parametrize("step", ["plain", "append", "sigmoid", "softmax"])
+@pytest.mark.parametrize("shape", [(6, 64), (2, 3, 1, 64), (1, 2, 3, 64), (3, 2, 1, 64), (384,)])
+def test_a_buffer_for_the_output_comes_back_as_one_row_per_head(kernels, step, shape):
+    pkg = load_package()
+    b, h, t, d = 2, 3, 40, 64
+    q, k, v, _ = make_inputs(b, h, t, d, 91)
+    k, v = k.cuda(), v.cuda()
+    q1 = q[:, :, -1:].contiguous().cuda()
+    committed = torch.rand(b, h, t, generator=torch.Generator().manual_seed(3)).cuda()
+
+    def call(out):
+        cache = dict(k=k.clone(), v=v.clone(), committed=committed.clone(), len=t - 1)
+        if step == "plain":
+            return kernels.dilution_decode_step(q1, cache["k"], cache["v"], cache["committed"], t, out=out)
+        if step == "sigmoid":
+            return pkg.kernels_bid.dilution_decode_step(q1, cache["k"], cache["v"], cache["committed"], t, bid="sigmoid",
+                                                        share_cumsum=True, out=out)
+        append = kernels.dilution_decode_append_step if step == "append" else pkg.layers.softmax_decode_append_step
+        return append(q1, k[:, :, -1:].contiguous(), v[:, :, -1:].contiguous(), cache, out=out)
+
+    want = call(None)
+    buffer = torch.empty(shape, device="cuda")
+    got = call(buffer)
+    assert got.shape == want.shape == (b, h, 1, d) and got.data_ptr() == buffer.data_ptr()
+    assert torch.equal(got, want)
