@@ -123,9 +123,16 @@ def _two_passes(n, seq, carry_rows):
     return n * -(-seq // 256) >= 74 if seq <= 2048 else seq >= 2560
 
 
-def _forward_rows(lib, q, k, v, sizes, code, prec, scale, out, ssum, rmax, rden, carry, total, pk, carry_rows, st):
+def _takes_sweep(code, prec, n, tq, tk, head_dim, carry_rows):
+    """Whether passes 2 and 3 of a call are the fused sweep; asked once per call, so that slabs do not differ in their kernels."""
+    return (TC_FUSED_FORWARD and tq == tk and _lib.tensor_core_path(code, prec, head_dim)
+            and not _two_passes(n, tq, carry_rows))
+
+
+def _forward_rows(lib, q, k, v, sizes, code, prec, scale, out, ssum, rmax, rden, carry, total, pk, carry_rows, sweep, st):
     """Passes 1-3 on a slab of (batch*head) rows, all tensors as addresses.  sizes: (rows, queries, keys, head size).  On the
-    tensor-core path a requested pk comes out of pass 1; otherwise out of pass 3 (the fp32 kernel)."""
+    tensor-core path a requested pk comes out of pass 1; otherwise out of pass 3 (the fp32 kernel).  sweep: what _takes_sweep
+    says of the whole call."""
     n, tq, tk, d = sizes
     tc = _lib.tensor_core_path(code, prec, d) and tq == tk
     if pk is not None and tc:
@@ -133,7 +140,7 @@ def _forward_rows(lib, q, k, v, sizes, code, prec, scale, out, ssum, rmax, rden,
         pk = None
     else:
         _lib.check(lib.dilution_rowstats(q, k, code, prec, n, tq, tk, 0, d, scale, rmax, rden, st), "dilution_rowstats")
-    if TC_FUSED_FORWARD and tc and not _two_passes(n, tq, carry_rows):
+    if sweep:
         _lib.check(lib.dilution_forward_fused_rows(q, k, v, code, prec, n, tq, d, scale, EPS, rmax, rden, carry_rows, carry,
                                                    total, out, ssum, st), "dilution_forward_fused_rows")
         return
@@ -182,8 +189,10 @@ def dilution_attention_forward(
     reference stores every 32 or 64 in the same way, kernels.py:374-377).
 
     Without return_aux the (batch*head) rows are processed in slabs so that the
-    quadratic carry scratch stays under scratch_budget_gib; rows are independent,
-    so this changes nothing numerically.
+    quadratic carry scratch stays under scratch_budget_gib; rows are independent, and
+    all slabs take the kernels that the whole call takes, so this changes nothing but the
+    order in which an output's partial sums are added (kernels pick their blocks by a
+    slab's rows).
     """
     result, aux = _attention_forward(q, k, v, dot_precision, return_aux, _save_pk, scratch_budget_gib, _training)
     if return_aux:
@@ -219,6 +228,7 @@ def _attention_forward(q, k, v, dot_precision, return_aux, _save_pk, scratch_bud
         per_row = ncb * seq * 4
         rows = max(1, min(n, int(scratch_budget_gib * 2**30) // max(per_row, 1)))
     carry = torch.empty(rows, ncb, seq, **f32)
+    sweep = _takes_sweep(code, prec, n, seq, kf.shape[1], head_dim, carry_rows)
     for a in range(0, n, rows):
         b = min(a + rows, n)
         # (a slice costs 2 us, and most calls are one slab)
@@ -232,7 +242,7 @@ def _attention_forward(q, k, v, dot_precision, return_aux, _save_pk, scratch_bud
             continue
         _forward_rows(lib, qs.data_ptr(), ks.data_ptr(), vs.data_ptr(), (b - a, seq, kf.shape[1], head_dim), code, prec, scale,
                       o.data_ptr(), ss.data_ptr(), mx.data_ptr(), dn.data_ptr(), carry.data_ptr(), tot.data_ptr(), _ptr(pks),
-                      carry_rows, _stream(dev))
+                      carry_rows, sweep, _stream(dev))
 
     aux = dict(pk=pk, rmax=rmax, rden=rden, carry=carry, ssum=ssum, bwd_block_m=carry_rows,
                committed_total=total.reshape(batch, heads, seq))
@@ -307,7 +317,7 @@ class _DilutionAttentionFn(torch.autograd.Function):
                                                  out.data_ptr(), ssum, pk, st), "dilution_wide_forward")
         else:
             _forward_rows(lib, *addr, (n, seq, seq, head_dim), code, prec, scale, out.data_ptr(), ssum, rmax, rden, carry,
-                          total, pk, CARRY_ROWS, st)
+                          total, pk, CARRY_ROWS, _takes_sweep(code, prec, n, seq, seq, head_dim, CARRY_ROWS), st)
         ctx.save_for_backward(*ops, out, ws)
         ctx.call = (code, prec, at, save_pk)
         ctx.dtypes = (q.dtype, k.dtype, v.dtype)

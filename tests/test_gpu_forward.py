@@ -8,7 +8,7 @@ import math
 import pytest
 import torch
 
-from conftest import golden, make_inputs, rel_err, seeded
+from conftest import golden, load_package, make_inputs, rel_err, seeded
 from oracle import dilution_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -200,3 +200,21 @@ def test_size_independent_properties_at_16k(kernels):
     ref = O.dilution_chunked(qb.float().cpu()[..., :2048, :], kb.float().cpu()[..., :2048, :],
                              va.float().cpu()[..., :2048, :], chunk=512)
     assert (oa.cpu()[..., :2048, :] - ref).abs().max().item() < 2e-2
+
+
+@pytest.mark.parametrize("rows,seq", [(56, 2049), (60, 2176)])
+def test_slabs_take_the_kernels_of_the_whole_call(kernels, rows, seq):
+    """The last slab alone (4 rows) would be a call of few blocks, with other kernels."""
+    pkg = load_package()
+    x = [t.bfloat16().cuda() for t in make_inputs(1, rows, seq, 64, 23, scales=(1.0, 1.0, 1.0, 1.0))[:3]]
+    per_row = -(-seq // 64) * seq * 4
+    got = []
+    for budget in (16.0, (rows - 4) * per_row / 2 ** 30 + 1e-9):
+        pkg._lib.profile(True)
+        pkg._lib.profile_collect()
+        got.append(kernels.dilution_attention_forward(*x, dot_precision="bf16", scratch_budget_gib=budget))
+        launches = {name: count for name, (count, _) in pkg._lib.profile_collect().items()}
+        pkg._lib.profile(False)
+        assert launches.get("tc_forward_fused") == len(got) and "tc_forward_main" not in launches, launches
+    # sums in another order: 32 accumulations of 16 keys in a block of 512, then at most 17 blocks, over a row sum of as many
+    assert (got[0] - got[1]).abs().max().item() <= 2 * (32 + 17) * 2.0 ** -23 * got[0].abs().max().item()
