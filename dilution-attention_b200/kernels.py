@@ -124,9 +124,14 @@ def _two_passes(n, seq, carry_rows):
 
 
 def _takes_sweep(code, prec, n, tq, tk, head_dim, carry_rows):
-    """Whether passes 2 and 3 of a call are the fused sweep; asked once per call, so that slabs do not differ in their kernels."""
-    return (TC_FUSED_FORWARD and tq == tk and _lib.tensor_core_path(code, prec, head_dim)
-            and not _two_passes(n, tq, carry_rows))
+    """Whether passes 2 and 3 of a call are the fused sweep; asked once per call, so that slabs do not differ in their kernels.
+    The sweep adds up outputs in memory in no fixed order: under torch.use_deterministic_algorithms a call that no backward
+    follows keeps the two passes, which repeat bit for bit (a backward adds up dq the same way)."""
+    if not (TC_FUSED_FORWARD and tq == tk and _lib.tensor_core_path(code, prec, head_dim)):
+        return False
+    if carry_rows != 32 and torch.are_deterministic_algorithms_enabled():
+        return False
+    return not _two_passes(n, tq, carry_rows)
 
 
 def _forward_rows(lib, q, k, v, sizes, code, prec, scale, out, ssum, rmax, rden, carry, total, pk, carry_rows, sweep, st):
@@ -193,6 +198,11 @@ def dilution_attention_forward(
     all slabs take the kernels that the whole call takes, so this changes nothing but the
     order in which an output's partial sums are added (kernels pick their blocks by a
     slab's rows).
+
+    On the tensor-core path a call of 256 blocks of 512 keys or more adds up its output in
+    no fixed order and repeats to fp32 rounding only; under
+    torch.use_deterministic_algorithms(True) it takes kernels that repeat bit for bit
+    (unless a backward will follow), a fifth slower at 128K tokens.
     """
     result, aux = _attention_forward(q, k, v, dot_precision, return_aux, _save_pk, scratch_budget_gib, _training)
     if return_aux:

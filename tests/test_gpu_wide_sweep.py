@@ -56,3 +56,23 @@ def test_sweep_of_512_keys(rows, seq, training):
                                                      (31, 4096, True, False)])
 def test_route(rows, seq, training, sweep):
     assert load_package().kernels._two_passes(rows, seq, 32 if training else 64) is not sweep
+
+
+def test_deterministic_algorithms_keep_the_two_passes():
+    pkg = load_package()
+    x = [t.bfloat16().to(DEV) for t in make_inputs(1, 52, 2111, 64, 71, scales=(1.0, 1.0, 1.0, 1.0))[:3]]
+    sweep = pkg.kernels.dilution_attention_forward(*x, dot_precision="bf16")
+    torch.use_deterministic_algorithms(True)
+    try:
+        pkg._lib.profile(True)
+        pkg._lib.profile_collect()
+        got = [pkg.kernels.dilution_attention_forward(*x, dot_precision="bf16", return_aux=True) for _ in range(3)]
+        names = set(pkg._lib.profile_collect())
+        pkg._lib.profile(False)
+        assert pkg.kernels._takes_sweep(pkg._lib.BF16, pkg._lib.PREC["bf16"], 52, 2111, 2111, 64, 32)      # a training forward
+    finally:
+        torch.use_deterministic_algorithms(False)
+    assert "tc_forward_main" in names and "tc_forward_fused" not in names, names
+    for out, aux in got[1:]:
+        assert torch.equal(out, got[0][0]) and torch.equal(aux["committed_total"], got[0][1]["committed_total"])
+    assert (sweep - got[0][0]).abs().max().item() < 1e-2                  # both round their shares to bf16
