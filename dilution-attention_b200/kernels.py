@@ -289,12 +289,17 @@ def _workspace(device, **parts):
     return torch.empty(at, device=device, dtype=torch.float32), offsets
 
 
+def _plane_addresses(planes, rows):
+    """The hi | lo planes of q, k and v in one tensor: 128 bf16 values per row."""
+    return [planes.data_ptr() + 256 * rows * i for i in range(3)]
+
+
 class _DilutionAttentionFn(torch.autograd.Function):
     """Autograd op (kernels.py:829-903): fp32 output; dq, dk, dv in the input dtypes.
 
     Saved for the backward: the operands as the kernels took them (casts, copies of strided views and hi | lo planes are made
-    once), the output and one workspace with the row statistics, the checkpoints, the demand totals and pk.  Tensors of
-    the workspace are handed to the kernels by their addresses, without views.  Host time of forward + backward of one short
+    once; the planes are one tensor), the output and one workspace with the row statistics, the checkpoints, the demand totals
+    and pk.  Tensors of the workspace are handed to the kernels by their addresses, without views.  Host time of forward + backward of one short
     row, of which a Function that does nothing takes 50 us: 190 -> 150 us."""
 
     @staticmethod
@@ -311,8 +316,7 @@ class _DilutionAttentionFn(torch.autograd.Function):
         save_pk = TC_SAVE_PK or not _lib.tensor_core_path(code, prec, head_dim)
         rows = n * seq
         ws, at = _workspace(dev, rmax=rows, rden=rows, ssum=rows, total=rows, pk=rows * head_dim if save_pk else 0,
-                            carry=rows * ((seq + CARRY_ROWS - 1) // CARRY_ROWS),
-                            planes=3 * 64 * rows if wide and code == _lib.F32 else 0)
+                            carry=rows * ((seq + CARRY_ROWS - 1) // CARRY_ROWS))
         out = torch.empty(q.shape, device=dev, dtype=torch.float32)
         scale, st, base = 1.0 / math.sqrt(head_dim), _stream(dev), ws.data_ptr()
         rmax, rden, ssum, total, carry = (base + at[x] for x in ("rmax", "rden", "ssum", "total", "carry"))
@@ -320,9 +324,11 @@ class _DilutionAttentionFn(torch.autograd.Function):
         addr = [x.data_ptr() for x in ops]
         if wide:
             if code == _lib.F32:
-                planes = [base + at["planes"] + 256 * rows * i for i in range(3)]
+                # (a tensor of their own type: a saved-tensor hook may round what it takes for fp32)
+                ops = [torch.empty(3, rows, 128, device=dev, dtype=torch.bfloat16)]
+                planes = _plane_addresses(ops[0], rows)
                 _lib.check(lib.dilution_split_operands(*addr, rows, head_dim, *planes, st), "dilution_split_operands")
-                addr, ops = planes, ()
+                addr = planes
             _lib.check(lib.dilution_wide_forward(*addr, code, n, seq, head_dim, scale, EPS, rmax, rden, carry, total,
                                                  out.data_ptr(), ssum, pk, st), "dilution_wide_forward")
         else:
@@ -355,7 +361,7 @@ class _DilutionAttentionFn(torch.autograd.Function):
         scale, st, base = 1.0 / math.sqrt(head_dim), _stream(dev), ws.data_ptr()
         rmax, rden, ssum, total, carry = (base + at[x] for x in ("rmax", "rden", "ssum", "total", "carry"))
         pk = base + at["pk"] if save_pk else None
-        addr = [x.data_ptr() for x in ops] or [base + at["planes"] + 256 * rows * i for i in range(3)]
+        addr = [x.data_ptr() for x in ops] if len(ops) == 3 else _plane_addresses(ops[0], rows)
         if wide:
             _lib.check(lib.dilution_wide_backward(
                 *addr, code, n, seq, head_dim, scale, EPS, dof.data_ptr(), do_code, out.data_ptr(), rmax, rden, carry, total,

@@ -6,7 +6,7 @@ from __future__ import annotations
 import pytest
 import torch
 
-from conftest import golden, make_inputs, rel_err
+from conftest import golden, load_package, make_inputs, rel_err
 from oracle import dilution_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -236,3 +236,32 @@ def test_bf16_backward_peaked_attention(kernels, scale):
     for name, gr, t in (("dq", ref[1], qs), ("dk", ref[2], ks), ("dv", ref[3], vs)):
         assert torch.isfinite(t.grad).all(), name
         assert rel_err(t.grad.float().cpu(), gr) < 3e-2, name
+
+
+@pytest.mark.parametrize("dtype,d,prec", [(torch.bfloat16, 64, "bf16"), (torch.bfloat16, 128, "bf16"),
+                                          (torch.float32, 64, "tf32"), (torch.float32, 32, "tf32"),
+                                          (torch.float32, 64, "ieee")])
+@pytest.mark.parametrize("bid", ["softmax", "sigmoid", "softplus"])
+def test_saved_tensor_hooks_that_round(kernels, bid, dtype, d, prec):
+    """A hook that keeps 12 bits of the mantissa of what is saved as fp32 costs about that much in the gradients: nothing but
+    fp32 values may be saved as fp32.  Bound: 2^-12 on the demands, 1/(row sums), log-sum-exps of up to 16 (2^-8 of a bid) and pk
+    of sums that cancel to a tenth."""
+    def rounding(x):
+        return (x.view(torch.int32) & ~0x7FF).view(torch.float32) if x.dtype == torch.float32 else x
+
+    pkg = load_package()
+    q, k, v, dout = (x.to(DEV) for x in make_inputs(1, 2, 200, d, 77))
+    leaves = [x.to(dtype).requires_grad_(True) for x in (q, k, v)]
+
+    def grads():
+        if bid == "softmax":
+            out = kernels.dilution_attention(*leaves, dot_precision=prec)
+        else:
+            out = pkg.kernels_bid.dilution_attention(*leaves, dot_precision=prec, bid=bid)
+        return torch.autograd.grad(out, leaves, dout)
+
+    plain = grads()
+    with torch.autograd.graph.saved_tensors_hooks(rounding, lambda x: x):
+        rounded = grads()
+    for name, a, b in zip(("dq", "dk", "dv"), rounded, plain):
+        assert ((a.float() - b.float()).norm() / b.float().norm()).item() < 4e-2, name
