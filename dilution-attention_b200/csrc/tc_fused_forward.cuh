@@ -332,9 +332,8 @@ __global__ void normalize_out_kernel(float* __restrict__ out, const float* __res
 }
 
 // Compute warpgroups per CTA.  Four need blocks of 512 keys for the SMs; with fewer than 256 of them a CTA of 128 keys, two to
-// an SM, is faster, and as fast as the sweep of 256 keys that it replaces.  Passes 2 and 3, one / four warpgroups / two
-// passes, in us: n = 64, T = 3000 324 / 277 / 291; n = 4, T = 32768 1963 / 1573 / 1676; n = 16, T = 65536 29.4 / 21.8 / 26.3 ms;
-// n = 16, T = 3000 (96 blocks) 115 / 166 / 100; n = 16, T = 1024 (32) 51 / 68 / 42.
+// an SM, is faster.  Passes 2 and 3, one / four warpgroups, in us: n = 64, T = 3000 324 / 277; n = 4, T = 32768 1963 / 1573;
+// n = 16, T = 65536 29.4 / 21.2 ms; n = 16, T = 3000 (96 blocks) 115 / 166; n = 16, T = 1024 (32) 45 / 68.
 inline int fused_groups(int64_t n, int64_t t) { return n * ((t + 511) / 512) >= 256 ? 4 : 1; }
 
 // Passes 2 and 3 of a call over whole rows (q_off = 0, tq = tk) in one

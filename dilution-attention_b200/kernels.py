@@ -109,18 +109,20 @@ def _upstream(dout, n, seq, head_dim, keep_bf16):
 
 
 def _two_passes(n, seq, carry_rows):
-    """Calls that take the column-sum and main passes instead of the fused sweep.  With 256 blocks of 512 keys or more
-    the sweep fills the chip and is the faster one beyond 2048 tokens, before a backward or not; a short row is mostly diagonal blocks, and
-    the output that the sweep adds up in memory is zeroed, reduced into and divided once per row of few tiles.  With fewer
-    blocks the two passes are faster.  Passes 2 and 3 of a call, sweep / two passes: n = 64, T = 3000
-    277 / 291 us, n = 64, T = 16384 6.1 / 6.8 ms, n = 16, T = 131072 90 / 104 ms; n = 384, T = 1024 283 / 274 us, n = 16,
-    T = 4096 158 / 141 us.  Training calls of at most 2559 tokens and few blocks stay with the sweep, whose shape for
-    few blocks is as fast as it ever was: below 74 blocks of 256 keys (half of the SMs) the host's launches outlast either."""
+    """Calls that take the column-sum and main passes instead of the fused sweep.  With 256 blocks of 512 keys or more the sweep
+    fills the chip and is the faster one beyond 2048 tokens, before a backward or not; a short row is mostly diagonal blocks,
+    and the output that the sweep adds up in memory is zeroed, reduced into and divided once per row of few tiles.  Passes 2 and
+    3 of a call, sweep / two passes: n = 64, T = 16384 5.8 / 6.6 ms, n = 2, T = 65536 3.04 / 3.31 ms, n = 32, T = 4096 229 / 247 us,
+    n = 64, T = 3000 276 / 289, n = 52, T = 2560 180 / 175; n = 384, T = 1024 280 / 271.  With fewer blocks (the sweep then has 128
+    keys per block) the two passes are faster: n = 31, T = 4096 276 / 239, n = 1, T = 65536 2044 / 1859, n = 16, T = 2304 87 / 72,
+    n = 8, T = 2048 74 / 62.  Training calls of few short rows stay with the sweep all the same, below 74 blocks of 256 keys (half
+    of the SMs) up to 2048 tokens and up to 100 of them below 2560: the host's launches, 150 us a step, outlast either."""
     if seq > 2048 and n * -(-seq // 512) >= 256:
         return False
     if carry_rows != 32:
         return True
-    return n * -(-seq // 256) >= 74 if seq <= 2048 else seq >= 2560
+    blocks = n * -(-seq // 256)
+    return blocks >= 74 if seq <= 2048 else seq >= 2560 or blocks > 100
 
 
 def _takes_sweep(code, prec, n, tq, tk, head_dim, carry_rows):

@@ -76,3 +76,10 @@ def test_deterministic_algorithms_keep_the_two_passes():
     for out, aux in got[1:]:
         assert torch.equal(out, got[0][0]) and torch.equal(aux["committed_total"], got[0][1]["committed_total"])
     assert (sweep - got[0][0]).abs().max().item() < 1e-2                  # both round their shares to bf16
+
+
+@pytest.mark.parametrize("rows,seq,sweep", [(11, 2304, True), (12, 2304, False), (10, 2559, True), (11, 2559, False),
+                                            (51, 2559, False), (52, 2559, True)])
+def test_route_of_training_calls_a_little_longer_than_short_rows(rows, seq, sweep):
+    """Beyond 100 blocks of 256 keys the sweep of few blocks is slower than the two passes by more than the host hides."""
+    assert load_package().kernels._two_passes(rows, seq, 32) is not sweep
