@@ -39,7 +39,8 @@ template <int MODE, int W = kNarrow> struct RowpassSmem {
   static constexpr int kBytes = kTiles * (int)Rows<W>::kBytes + 4096 + 256 + 1024;
 };
 
-template <int MODE, typename TOut, int W = kNarrow>
+// ONE_POLLS: one lane of the issuing warp waits for the next tiles, the others behind it (kOnePollsAbove).
+template <int MODE, typename TOut, int W = kNarrow, bool ONE_POLLS = false>
 __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) rowpass_product_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, Geom g, float* __restrict__ rmax, float* __restrict__ rden,
@@ -234,7 +235,8 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) rowpass_product_ker
             mma_ts(lead, tmem + 128 + kAcc * w, tS + 64 * w + 32 * pl + 8 * kk, dB, 128 * (4 * w + kk), id_pv, 1);
       if (jb + 1 < njb) {
         const int sn = (jb + 1) % kRowpassStages;
-        mbar_wait(kfull + 8 * sn, ((jb + 1) / kRowpassStages) & 1, ctl, &g_status, kErrWaitTma);
+        if (!ONE_POLLS || (tid & 31) == 0) mbar_wait(kfull + 8 * sn, ((jb + 1) / kRowpassStages) & 1, ctl, &g_status, kErrWaitTma);
+        if (ONE_POLLS) __syncwarp();
         tc_fence_after();
         mma_scores_w<W>(lead, tS, sQ, sK0 + TB * sn, 128);
       }
@@ -548,6 +550,13 @@ inline int rowstats_pk(const void* q, const void* k, const Geom& g, float* rmax,
   return launch_status("tc rowstats_pk", err, errlen);
 }
 
+// Softmax pass, blocks above which one lane of the issuing warp polls for the next tiles instead of 32: where two CTAs share
+// every SM for long, it is the faster form, on a chip that is not full the other, whose scores are issued sooner.  One lane
+// issuing everything (with operands in ordinary registers) / all lanes polling / one: n = 64, T = 8192 840 / 861 / 846 us, n = 16, T = 16384
+// 736 / 744 / 722, n = 64, T = 4096 218 / 210 / 207, n = 128, T = 2048 131 / 123 / 123; n = 16, T = 2048 (256 blocks) 29.9 / 25.8 / 27.2,
+// n = 2, T = 3000 (48) 39.0 / 32.9 / 34.9.
+constexpr unsigned kOnePollsAbove = 2 * 148;
+
 // Causal softmax attention forward: out = softmax(q k^T * scale) v in bf16; rmax / rden
 // (optional) as pass 1 writes them.
 inline int softmax_forward(const void* q, const void* k, const void* v, const Geom& g, float* rmax,
@@ -556,12 +565,14 @@ inline int softmax_forward(const void* q, const void* k, const void* v, const Ge
   if (int rc = make_map(&mq, q, g.n, g.tq, err, errlen)) return rc;
   if (int rc = make_map(&mk, k, g.n, g.tk, err, errlen)) return rc;
   if (int rc = make_map(&mv, v, g.n, g.tk, err, errlen)) return rc;
-  auto kern = rowpass_product_kernel<2, __nv_bfloat16>;
+  const int nqb = (g.tq + kTileRows - 1) / kTileRows;
+  const unsigned grid = (unsigned)(g.n * nqb);
+  auto kern = grid > kOnePollsAbove ? rowpass_product_kernel<2, __nv_bfloat16, kNarrow, true>
+                                    : rowpass_product_kernel<2, __nv_bfloat16>;
   constexpr int smem = RowpassSmem<2>::kBytes;
   static_assert(2 * (smem + 1024) <= 233472 && 3 * (smem + 1024) > 233472, "two CTAs of the softmax pass fit one SM");
   if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
-  const int nqb = (g.tq + kTileRows - 1) / kTileRows;
-  kern<<<(unsigned)(g.n * nqb), 256, smem, st>>>(mq, mk, mv, g, rmax, rden, (__nv_bfloat16*)out);
+  kern<<<grid, 256, smem, st>>>(mq, mk, mv, g, rmax, rden, (__nv_bfloat16*)out);
   return launch_status("tc softmax_forward", err, errlen);
 }
 

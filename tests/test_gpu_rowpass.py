@@ -99,3 +99,12 @@ def test_softmax_attention_on_model_views(kernels):
     q, k, v = (y.view(b, t, h, d).transpose(1, 2) for y in x.split(h * d, dim=2))
     got = kernels.softmax_attention_forward(q.to(DEV), k.to(DEV), v.to(DEV))
     assert (got.float().cpu() - O.softmax_attention(q.float(), k.float(), v.float())).abs().max().item() < 2e-2
+
+
+@pytest.mark.parametrize("rows,seq", [(296, 128), (297, 128), (100, 385), (99, 257), (75, 500)])
+def test_softmax_attention_of_a_full_chip(kernels, rows, seq):
+    """Around and above two blocks of 128 queries per SM, where the issuing warp waits in another way."""
+    q, k, v, _ = (x.bfloat16().to(DEV) for x in make_inputs(1, rows, seq, 64, 61))
+    got = kernels.softmax_attention_forward(q, k, v)
+    ref = F.scaled_dot_product_attention(q.float(), k.float(), v.float(), is_causal=True)
+    assert (got.float() - ref).abs().max().item() < 2e-2
