@@ -26,9 +26,10 @@ constexpr int SL = 68;    // leading dimension of score tiles (4 mod 32: conflic
 
 template <int D> __host__ __device__ constexpr int ld() { return D + 4; }
 
-// SPLIT (FFMA products, few blocks): a cluster of `split` CTAs shares one block of a pass.  Rank r of the cluster takes a part of the tiles the block would walk through one after the other (about
-// 20 us each in the reverse pass, on a chip that is mostly idle), and the cluster adds up the accumulators through
-// distributed shared memory, each rank a slice of the rows, always in rank order.  The reverse pass is a
+// SPLIT (FFMA products, few blocks): a cluster of `split` CTAs shares one block of a pass.  Rank r of the cluster takes a
+// part of the tiles the block would walk through one after the other (about 20 us each in the reverse pass, on a chip that is
+// mostly idle), and the cluster adds up the accumulators through distributed shared memory, each rank a slice of the
+// rows, always in rank order.  The reverse pass is a
 // chain over query tiles by way of the suffix of dk_share: every rank first forms its tiles' sums, the ranks
 // exchange them, and each goes on from the sum behind its tiles.  n = 4, T = 512, d = 64, forward + backward on one B200:
 // 410 -> 196 us (the host's launches; main pass 97 -> 31, reverse pass 170 -> 43, key correction 69 -> 22);
