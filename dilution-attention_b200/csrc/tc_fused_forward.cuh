@@ -1,13 +1,14 @@
-// Key-stationary training forward on the tensor cores: passes 2 and 3 in one sweep
+// Key-stationary forward of whole rows on the tensor cores: passes 2 and 3 in one sweep
 // (the reference's training forward, _dilution_key_forward + _dilution_normalize,
 // kernels.py:200-248, does the same on its side of the fence).
 //
 // A CTA owns 512 keys, 128 per compute warpgroup (lane = key), and walks the queries that can see them in causal
-// order, 64 at a time.  The demand of a key is ONE register for the whole sweep, so no checkpoint is read; the checkpoints that
+// order, 64 at a time.  The demand of a key stays in its thread for the whole sweep, so no checkpoint is read; the checkpoints that
 // the backward needs (every 32 query rows, or 64) and the demand totals are stored on the way.  Per half tile of 64 queries and
 // warpgroup:
 //   S^T  = K Q^T            A = the keys' rows in TMEM, written there once: 4 MMAs of N = 64
-//   p, den += p, share      exactly the arithmetic of forward_main_kernel, 64 queries per thread
+//   p, demand, share        64 queries per thread, the arithmetic of forward_main_kernel but for the demand, which is an output
+//                           here: bids of 32 queries are summed from zero and folded into a compensated total
 //   O^T | rs                = [V | 1]^T share, M = 64 features and 64 copies of the row sums, K = 128 keys, N = 64: 8 MMAs into a
 //                           FRESH tile per half tile that all four warpgroups add to
 // and the tile is added to `out` / `ssum` in global memory: two warps of a fifth warpgroup (lane = feature) move it from TMEM
@@ -17,9 +18,11 @@
 //
 // Four warpgroups are four warps per scheduler.  They fit because the keys are a TMEM operand and O comes out transposed
 // (64 columns): S^T 4 x 64, K 4 x 32, O^T 2 x 64 = 512 columns, V + ones + shares + q + staging = 192 KB.  Two warpgroups of 128
-// keys with S^T double-buffered took 6.5 ms at n = 64, T = 16384 (now 6.1) and left the special-function unit idle
+// keys with S^T double-buffered took 6.5 ms at n = 64, T = 16384 (now 5.8) and left the special-function unit idle
 // whenever both waited; output tiles are added half as often.  640 threads, one CTA per SM; a fifth-warpgroup warp
-// issues every TMA copy and MMA.  Every wait is bounded.
+// issues every TMA copy and MMA.  Every wait is bounded.  No unit binds it: special-function unit 41%, issue slots 52%, tensor
+// pipe 25%, DRAM 0.8 TB/s (n = 64, T = 4096); what is left is the issuing warp, which also moves O out and serves the four
+// warpgroups in a fixed order.
 #pragma once
 
 #include "tc_kernels.cuh"
@@ -262,7 +265,8 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
               z[u] = z2.x;
               z[u + 1] = z2.y;
             }
-            // every fourth exponential is a polynomial on the FMA pipe, of degree 5: the demand is an output in fp32
+            // every fourth exponential is a polynomial on the FMA pipe (7.30 -> 7.08 ms when two warps shared a scheduler), of
+            // degree 5: with degree 4 the demand, an output in fp32, is off by up to 4.6e-6 instead of 2.5e-6
             const float2 fourth = poly_exp2_two<5>(make_float2(z[3], z[7]));
 #pragma unroll
             for (int u = 0; u < 8; ++u) {

@@ -1327,7 +1327,7 @@ __device__ __forceinline__ float sum_over_lanes(float (&x)[32], int lane) {
 
 // Main reverse pass (the reference's BA, kernels.py:677-775).  grid = n * ceil(t/128),
 // key blocks with the most query blocks first; one CTA per SM, three warpgroups: two of
-// compute warps and one whose first thread issues every TMA copy and every MMA and whose
+// compute warps and one whose first warp issues every TMA copy and every MMA and whose
 // four warps move the finished dQ tiles out.
 // TMEM (496 of 512 columns): two stages of S^T (64 columns each) | two stages of dOV^T
 // (64 each) | dV 64 | dK 64 | dQ 64 + ghat 16 as one 80-column tile | the V tile as a
@@ -1352,7 +1352,7 @@ __device__ __forceinline__ float sum_over_lanes(float (&x)[32], int lane) {
 // to shared memory as the MN-major A operand (M = queries) of one N = 80 MMA per 128
 // queries against B = [K | ones], which yields dQ = pdp K in 64 columns and ghat = pdp 1
 // in the next 16.
-// The issuing thread runs two half-steps ahead of the arithmetic: when the tiles of
+// The issuing warp runs two half-steps ahead of the arithmetic: when the tiles of
 // half-step h are complete it issues dV, dK (and dQ | ghat after the second half) of h and
 // the score MMAs of h + 2 into the stage h has just left, so the tensor pipe works under
 // the arithmetic of h + 1.  Q and dO' tiles are triple-buffered.  After setup the third
@@ -1485,7 +1485,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
 
   if (wg == 2) {
     // ------------------------------------------------------------ warpgroup 2: issue and dQ read-out
-    // Thread 256 issues every MMA and TMA copy.  After the second half-step of a step all
+    // Warp 8 issues every MMA and TMA copy.  After the second half-step of a step all
     // four warps (lane = query) move the finished dQ | ghat tile out, so that the compute
     // warps never touch it.  The warpgroup hands most of its registers to the other two.
     asm volatile("setmaxnreg.dec.sync.aligned.u32 128;");

@@ -136,8 +136,8 @@ __global__ void split_dq_from_pk_kernel(const float* __restrict__ dq_main, const
 //  * V stays in shared memory (as a TMEM operand it would take 64 columns);
 //  * ghat, the sum of pdp over keys, is formed by shuffles in fp32 once the half-step's tiles are handed over, while
 //    the compute warps would wait for the next scores (as a product of its own against a tile of ones it was 16 of
-//    the 76 MMAs of a kWide128 half-step, each about 50 cycles of the issuing thread: 1.11 -> 0.94 ms, kSplit 0.92 ->
-//    0.81 ms, n = 32, T = 4096).
+//    the 76 MMAs of a kWide128 half-step: 1.11 -> 0.94 ms, kSplit 0.92 -> 0.81 ms, n = 32, T = 4096, when one thread
+//    issued them at about 50 cycles each).
 //  * share and pdp are multiplied as hi and lo planes (two A operands side by side in TMEM, two pdp tiles); for kSplit
 //    dQ^T rows 64..127 (K_lo) are reduced into the same columns of dq_main as rows 0..63;
 //  * kWide128 stages 32 queries of dQ at a time (16 KB instead of 32): its do' takes 64 KB.
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
     for (int c = 0; c < Rows<W>::kCols / 16; ++c) tmem_st16((wg == 0 ? tDV : tDK) + lane_base + 16 * c, z);
     tmem_st_wait();
   }
-  auto load_stage = [&](int h) {                     // thread 256: q and do' of half-step h
+  auto load_stage = [&](int h) {                     // one lane: q and do' of half-step h
     const int st = h % NR, r0 = (2 * nqb - 1 - h) * 64;
     mbar_expect_tx(qfull + 8 * st, HB + HBd);
     tma_load_rows<W>(sQ0 + HB * st, &map_q, r0, n, qfull + 8 * st, HSub);

@@ -204,7 +204,7 @@ def dilution_attention_forward(
     On the tensor-core path a call of 256 blocks of 512 keys or more adds up its output in
     no fixed order and repeats to fp32 rounding only; under
     torch.use_deterministic_algorithms(True) it takes kernels that repeat bit for bit
-    (unless a backward will follow), a fifth slower at 128K tokens.
+    (unless a backward will follow), a sixth slower at 128K tokens.
     """
     result, aux = _attention_forward(q, k, v, dot_precision, return_aux, _save_pk, scratch_budget_gib, _training)
     if return_aux:
@@ -301,8 +301,8 @@ class _DilutionAttentionFn(torch.autograd.Function):
 
     Saved for the backward: the operands as the kernels took them (casts, copies of strided views and hi | lo planes are made
     once; the planes are one tensor), the output and one workspace with the row statistics, the checkpoints, the demand totals
-    and pk.  Tensors of the workspace are handed to the kernels by their addresses, without views.  Host time of forward + backward of one short
-    row, of which a Function that does nothing takes 50 us: 190 -> 150 us."""
+    and pk.  Tensors of the workspace are handed to the kernels by their addresses, without views.  Host time of forward +
+    backward of one short row, of which a Function that does nothing takes 50 us: 190 -> 150 us."""
 
     @staticmethod
     def forward(ctx, q, k, v, dot_precision):
