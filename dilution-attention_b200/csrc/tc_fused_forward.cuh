@@ -9,20 +9,23 @@
 //   S^T  = K Q^T            A = the keys' rows in TMEM, written there once: 4 MMAs of N = 64
 //   p, demand, share        64 queries per thread, the arithmetic of forward_main_kernel but for the demand, which is an output
 //                           here: bids of 32 queries are summed from zero and folded into a compensated total
-//   O^T | rs                = [V | 1]^T share, M = 64 features and 64 copies of the row sums, K = 128 keys, N = 64: 8 MMAs into a
+//   O^T | rs                = [V | 1 0 .. 0]^T share, M = 64 features, the row sums and 63 rows of zeros (as 64 copies of the sums
+//                           they cost power, which long rows are short of: 5.08 -> 5.00 ms), K = 128 keys, N = 64: 8 MMAs into a
 //                           FRESH tile per half tile that all four warpgroups add to
 // and the tile is added to `out` / `ssum` in global memory: two warps of a fifth warpgroup (lane = feature) move it from TMEM
-// to a staging tile and issue a TMA tensor reduction each, the row sums go by atomics from the other two.  `out` and `ssum`
+// to a staging tile and issue a TMA tensor reduction each, the row sums go by atomics from the third.  `out` and `ssum`
 // therefore start at zero and a small kernel divides at the end.  One exponential and one QK^T sweep per score less than
 // column-sum pass + query-stationary main pass.
 //
 // Four warpgroups are four warps per scheduler.  They fit because the keys are a TMEM operand and O comes out transposed
 // (64 columns): S^T 4 x 64, K 4 x 32, O^T 2 x 64 = 512 columns, V + ones + shares + q + staging = 192 KB.  Two warpgroups of 128
-// keys with S^T double-buffered took 6.5 ms at n = 64, T = 16384 (now 5.8) and left the special-function unit idle
-// whenever both waited; output tiles are added half as often.  640 threads, one CTA per SM; a fifth-warpgroup warp
-// issues every TMA copy and MMA.  Every wait is bounded.  No unit binds it: special-function unit 41%, issue slots 52%, tensor
-// pipe 25%, DRAM 0.8 TB/s (n = 64, T = 4096); what is left is the issuing warp, which also moves O out and serves the four
-// warpgroups in a fixed order.
+// keys with S^T double-buffered took 6.5 ms at n = 64, T = 16384 and left the special-function unit idle
+// whenever both waited; output tiles are added half as often.  640 threads, one CTA per SM.  Every wait is bounded.
+//
+// The fifth warpgroup's last warp does nothing but issue every TMA copy and MMA: as one of the four that move O out (two took the
+// row sums then) it was in the middle of that whenever a warpgroup wanted its next scores.  Moved out of the read-out, at
+// n = 64, T = 16384 5.9 -> 4.7 ms, n = 16, T = 131072 86 -> 75 ms, n = 384, T = 1024 279 -> 251 us, n = 16, T = 1777 (128 keys
+// per CTA) 70 -> 55 us.  What is left: half of the special-function unit's rate; long rows run at the card's power limit.
 #pragma once
 
 #include "tc_kernels.cuh"
@@ -47,15 +50,16 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
   constexpr uint32_t HB = kTileBytes / 2;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
-  const uint32_t sV = smem_u32(smem), sOnes = sV + G * kTileBytes;           // A of O^T: [V | ones], MN-major
+  const uint32_t sV = smem_u32(smem), sOnes = sV + G * kTileBytes;           // A of O^T: [V | 1 0 .. 0], MN-major
   uint8_t* ones_ptr = smem + G * kTileBytes;
   const uint32_t sSh = sOnes + kTileBytes;                                   // [G][128 keys][64 queries]
   const uint32_t sQ = sSh + G * kTileBytes, sStage = sQ + R * HB;            // staging: [2 warps][64 queries][32 features] fp32
   float* sL = reinterpret_cast<float*>(smem + (sStage - sV) + kTileBytes);   // [4][64] -lse of a half tile's queries
   uint64_t* bars = reinterpret_cast<uint64_t*>(sL + 256);
   const uint32_t vfull = smem_u32(bars), qfull = vfull + 8, ofull = qfull + 8 * R;            // 1, [R], [2]
-  const uint32_t sdone = ofull + 16, odone = sdone + 8 * G, sfree = odone + 8 * G, shready = sfree + 8 * G;   // [G] each
-  Ctl* ctl = reinterpret_cast<Ctl*>(bars + 3 + R + 4 * G);
+  const uint32_t sdone = ofull + 16, odone = sdone + 8 * G, sfree = odone + 8 * G, shready = sfree + 8 * G,   // [G] each
+                 ofree = shready + 8 * G;                                                                  // [2]
+  Ctl* ctl = reinterpret_cast<Ctl*>(bars + 5 + R + 4 * G);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wg = tid >> 7, row = tid & 127;
   const int warp_u = uniform_warp();
@@ -71,6 +75,7 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
     ctl->abort = 0;
     for (int i = 0; i < 3 + R + 2 * G; ++i) mbar_init(vfull + 8 * i, 1);
     for (int i = 0; i < 2 * G; ++i) mbar_init(sfree + 8 * i, 4);
+    for (int i = 0; i < 2; ++i) mbar_init(ofree + 8 * i, 3);
     fence_barrier_init();
   }
   __syncwarp();
@@ -81,7 +86,7 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
     if (row < 64) sL[128 + row] = -load_lse(rmax, rden, row_base, h0 * 64 + 128 + row, g.tq);
 #pragma unroll
     for (int c = 0; c < 8; ++c)
-      reinterpret_cast<uint4*>(ones_ptr)[row * 8 + c] = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
+      reinterpret_cast<uint4*>(ones_ptr)[row * 8 + c] = make_uint4(c == (row & 7) ? 0x3f80u : 0u, 0u, 0u, 0u);
   }
   fence_async_smem();
   tc_fence_before();
@@ -111,79 +116,24 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
   tc_fence_after();
 
   if (wg == G) {
-    // ------------------------------------------------------------ issue, and the O read-out
+    // ------------------------------------------------------------ issue (its last warp), and the O read-out
     if (G == 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
-    constexpr uint32_t id_s = instr_desc(128, 64, 0, 0);     // scores: A from TMEM, B K-major
-    constexpr uint32_t id_o = instr_desc(128, 64, 1, 1);     // O^T: A and B MN-major
-    const Desc dQ = make_desc(sQ, 16, 1024), dSh = make_desc(sSh, kTileBytes, 1024);
-    const bool issuer = warp_u == 4 * G;
-    auto load_q = [&](int h) {
-      const int st = (h - h0) % R;
-      if (!lead) return;
-      mbar_expect_tx(qfull + 8 * st, HB);
-      tma_load_tile(sQ + HB * st, &map_q, h * 64, n, qfull + 8 * st);
-    };
-    auto issue_scores = [&](int w, int h) {
+    if (warp_u == 4 * G + 3) {
+      constexpr uint32_t id_s = instr_desc(128, 64, 0, 0);     // scores: A from TMEM, B K-major
+      constexpr uint32_t id_o = instr_desc(128, 64, 1, 1);     // O^T: A and B MN-major
+      const Desc dQ = make_desc(sQ, 16, 1024), dSh = make_desc(sSh, kTileBytes, 1024);
+      auto load_q = [&](int h) {
+        const int st = (h - h0) % R;
+        if (!lead) return;
+        mbar_expect_tx(qfull + 8 * st, HB);
+        tma_load_tile(sQ + HB * st, &map_q, h * 64, n, qfull + 8 * st);
+      };
+      auto issue_scores = [&](int w, int h) {
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk)
-        mma_ts(lead, tS + 64 * w, tK + 32 * w + 8 * kk, dQ, (HB >> 4) * ((h - h0) % R) + 2 * kk, id_s, kk > 0);
-      mma_commit(lead, sdone + 8 * w);
-    };
-    // O^T of half tile h, lane = feature (and the row sums on the lanes behind them), to global memory.  On the way, the
-    // lse of h + 3: the barrier of the four warps and the scores of h + 3 lie between the store and the use, the
-    // hand-over of h, which ofull waits for, behind the last use of the slot (h - 1).
-    auto read_out = [&](int h) {
-      float nx_max = INFINITY, nx_den = 1.f;
-      const int i3 = (h + 3) * 64 + row;
-      const bool fetch = row < 64 && h + 3 < nh;
-      if (fetch && i3 < g.tq) {
-        nx_max = rmax[row_base + i3];
-        nx_den = rden[row_base + i3];
-      }
-      const int u = h - h0, w4 = warp & 3;
-      if (lane == 0) mbar_wait(ofull + 8 * (u & 1), (u >> 1) & 1, ctl, &g_status, kErrWaitMma);
-      __syncwarp();
-      tc_fence_after();
-      if (fetch) sL[64 * ((u + 3) & 3) + row] = -(nx_max + log2f(nx_den));
-      __syncwarp();
-      const uint32_t tOb = tO + 64 * (u & 1) + lane_base;
-      if (w4 < 2) {
-        const uint32_t stage = sStage + HB * w4;
-        if (lane == 0) tma_wait_read_all();                  // the previous reduction has read this warp's staging
-        __syncwarp();
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          float o[16];
-          tmem_ld16(tOb + 16 * c, o);
-          tmem_ld_wait16(o);
-#pragma unroll
-          for (int e = 0; e < 16; ++e)
-            asm volatile("st.shared.f32 [%0], %1;" ::"r"(stage + lane * 4 + (16 * c + e) * 128), "f"(o[e]) : "memory");
-        }
-        fence_async_smem();
-        __syncwarp();
-        if (lane == 0) tma_reduce_add_tile(&map_out, stage, 32 * w4, h * 64, n);
-      } else {
-        // any of these lanes holds the row sums of all queries: lane l takes query 32 (w4 - 2) + l
-        float rs = 0.f;
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          float o[16];
-          tmem_ld16(tOb + 32 * (w4 - 2) + 16 * c, o);
-          tmem_ld_wait16(o);
-#pragma unroll
-          for (int e = 0; e < 16; ++e) rs = lane == 16 * c + e ? o[e] : rs;
-        }
-        const int i = h * 64 + 32 * (w4 - 2) + lane;
-        if (i < g.tq) atomicAdd(ssum + row_base + i, rs);
-        __syncwarp();
-      }
-      tc_fence_before();
-      __syncwarp();
-      asm volatile("bar.sync 2, 128;" ::: "memory");         // every warp has read the tile: its buffer is free
-      tc_fence_after();
-    };
-    if (issuer) {
+        for (int kk = 0; kk < 4; ++kk)
+          mma_ts(lead, tS + 64 * w, tK + 32 * w + 8 * kk, dQ, (HB >> 4) * ((h - h0) % R) + 2 * kk, id_s, kk > 0);
+        mma_commit(lead, sdone + 8 * w);
+      };
       if (lead) {
         mbar_expect_tx(vfull, groups * kTileBytes);
         for (int w = 0; w < groups; ++w) tma_load_tile(sV + kTileBytes * w, &map_v, k0 + w * kTileRows, n, vfull);
@@ -193,17 +143,15 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
       tc_fence_after();
       issue_scores(0, h0);
       mbar_wait_warp(vfull, 0, ctl, &g_status, kErrWaitTma);
-    }
-    __syncwarp();
-    for (int h = h0; h < nh; ++h) {
-      const int u = h - h0;
-      if (h > h0) read_out(h - 1);
-      if (issuer) {
+      for (int h = h0; h < nh; ++h) {
+        const int u = h - h0;
+        // O^T of h - 2 is out of its buffer, and the lse of h + 1 are in place
+        if (u >= 2) mbar_wait_warp(ofree + 8 * (u & 1), ((u >> 1) + 1) & 1, ctl, &g_status, kErrWaitDrain);
         if (h + 1 < nh) {
           // scores of h + 1, as soon as a warpgroup has taken those of h out of TMEM
           mbar_wait_warp(qfull + 8 * ((u + 1) % R), ((u + 1) / R) & 1, ctl, &g_status, kErrWaitTma);
           for (int w = 0; w < groups; ++w) {
-            const int t = u - 2 * w;                         // the warpgroup's own count of half tiles
+            const int t = u - 2 * w;                           // the warpgroup's own count of half tiles
             if (t + 1 < 0) break;
             if (t >= 0) mbar_wait_warp(sfree + 8 * w, t & 1, ctl, &g_status, kErrWaitTile);
             tc_fence_after();
@@ -222,13 +170,72 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
           mma_commit(lead, odone + 8 * w);
         }
         mma_commit(lead, ofull + 8 * (u & 1));
-        if (h + R < nh) load_q(h + R);                       // every share of h exists, so its scores are complete
+        if (h + R < nh) load_q(h + R);                         // every share of h exists, so its scores are complete
       }
       __syncwarp();
+    } else {
+      // O^T of half tile h, lane = feature (and the row sums on the lanes behind them), to global memory.  On the way, the
+      // lse of h + 3: the issuing warp waits for this tile's release before it issues the scores of h + 3, and the hand-over of
+      // h, which ofull waits for, lies behind the last use of the slot (h - 1).
+      for (int h = h0; h < nh; ++h) {
+        float nx_max = INFINITY, nx_den = 1.f;
+        const int i3 = (h + 3) * 64 + row;
+        const bool fetch = row < 64 && h + 3 < nh;
+        if (fetch && i3 < g.tq) {
+          nx_max = rmax[row_base + i3];
+          nx_den = rden[row_base + i3];
+        }
+        const int u = h - h0, w4 = warp & 3;
+        if (lane == 0) mbar_wait(ofull + 8 * (u & 1), (u >> 1) & 1, ctl, &g_status, kErrWaitMma);
+        __syncwarp();
+        tc_fence_after();
+        if (fetch) sL[64 * ((u + 3) & 3) + row] = -(nx_max + log2f(nx_den));
+        __syncwarp();
+        const uint32_t tOb = tO + 64 * (u & 1) + lane_base;
+        const uint32_t stage = sStage + HB * w4;
+        float rs[2] = {0.f, 0.f};
+        if (w4 < 2) {
+          if (lane == 0) tma_wait_read_all();                  // the previous reduction has read this warp's staging
+          __syncwarp();
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            float o[16];
+            tmem_ld16(tOb + 16 * c, o);
+            tmem_ld_wait16(o);
+#pragma unroll
+            for (int e = 0; e < 16; ++e)
+              asm volatile("st.shared.f32 [%0], %1;" ::"r"(stage + lane * 4 + (16 * c + e) * 128), "f"(o[e]) : "memory");
+          }
+          fence_async_smem();
+        } else {
+          // the first of these lanes holds the row sums of all queries: lane l takes those of queries l and 32 + l from it
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            float o[16];
+            tmem_ld16(tOb + 16 * c, o);
+            tmem_ld_wait16(o);
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+              const float x = __shfl_sync(0xffffffffu, o[e], 0);
+              rs[c >> 1] = lane == 16 * (c & 1) + e ? x : rs[c >> 1];
+            }
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(ofree + 8 * (u & 1));       // this warp has read the tile
+        if (w4 < 2) {
+          if (lane == 0) tma_reduce_add_tile(&map_out, stage, 32 * w4, h * 64, n);
+        } else {
+          const int i = h * 64 + lane;
+          if (i < g.tq) atomicAdd(ssum + row_base + i, rs[0]);
+          if (i + 32 < g.tq) atomicAdd(ssum + row_base + i + 32, rs[1]);
+        }
+        __syncwarp();
+      }
+      if (lane == 0) tma_wait_read_all();
+      __syncwarp();
     }
-    read_out(nh - 1);
-    if (lane == 0) tma_wait_read_all();
-    __syncwarp();
   } else {
     if (G == 4) asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
     // ------------------------------------------------------------ the compute warps: lane = key
@@ -324,6 +331,14 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
   if (warp == 0) tmem_free(tmem, kTmem);
 }
 
+// Zeroes what the sweep adds up (one launch where two memsets cost the host twice).
+__global__ void zero_sums_kernel(float* __restrict__ out, float* __restrict__ ssum, int64_t rows) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= rows * (kHeadDim / 4)) return;
+  reinterpret_cast<float4*>(out)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (i < rows) ssum[i] = 0.f;
+}
+
 // out = O / (rs + eps) in place, four columns per thread (grid over n*t*16 float4).
 __global__ void normalize_out_kernel(float* __restrict__ out, const float* __restrict__ ssum, float eps,
                                      int64_t n4) {
@@ -335,10 +350,11 @@ __global__ void normalize_out_kernel(float* __restrict__ out, const float* __res
   reinterpret_cast<float4*>(out)[i] = x;
 }
 
-// Compute warpgroups per CTA.  Four need blocks of 512 keys for the SMs; with fewer than 256 of them a CTA of 128 keys, two to
-// an SM, is faster.  Passes 2 and 3, one / four warpgroups, in us: n = 64, T = 3000 324 / 277; n = 4, T = 32768 1963 / 1573;
-// n = 16, T = 65536 29.4 / 21.2 ms; n = 16, T = 3000 (96 blocks) 115 / 166; n = 16, T = 1024 (32) 45 / 68.
-inline int fused_groups(int64_t n, int64_t t) { return n * ((t + 511) / 512) >= 256 ? 4 : 1; }
+// Compute warpgroups per CTA.  Four need blocks of 512 keys for the SMs; with fewer than 200 of them a CTA of 128 keys, two to
+// an SM, is faster.  Passes 2 and 3, one / four warpgroups, in us: 384 blocks (n = 64, T = 3000) 262 / 231; 248 (n = 31, T = 4096)
+// 220 / 189; 200 (n = 100, T = 768) 60.0 / 56.6; 192 (n = 24, T = 4096) 180 / 180; 144 (n = 48, T = 1536) 74 / 83; 128 (n = 16,
+// T = 4096) 120 / 173.
+inline int fused_groups(int64_t n, int64_t t) { return n * ((t + 511) / 512) >= 200 ? 4 : 1; }
 
 // Passes 2 and 3 of a call over whole rows (q_off = 0, tq = tk) in one
 // key-stationary sweep.  carry: (n, ceil(t/32 or t/64), t); total: (n, t); out: (n, t, 64) fp32; ssum: (n, t).
@@ -354,8 +370,7 @@ inline int forward_fused(const void* q, const void* k, const void* v, const Geom
     return 1;
   }
   const int64_t rows = g.n * g.tq;
-  cudaMemsetAsync(out, 0, sizeof(float) * (size_t)rows * kHeadDim, st);
-  cudaMemsetAsync(ssum, 0, sizeof(float) * (size_t)rows, st);
+  zero_sums_kernel<<<(unsigned)((rows * (kHeadDim / 4) + 255) / 256), 256, 0, st>>>(out, ssum, rows);
   auto launch = [&](auto groups_c, auto cr_c, auto pair_c) -> int {
     constexpr int G = decltype(groups_c)::value, smem = kFusedSmem<G>;
     static_assert(smem <= 232448 && (G > 1 || 2 * (smem + 1024) <= 233472), "one or two CTAs fit one SM's shared memory");

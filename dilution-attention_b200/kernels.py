@@ -49,8 +49,8 @@ HAS_CUDA_LIB = _lib.available()
 # correction pass recomputes the query half.
 TC_SAVE_PK = os.environ.get("DILUTION_SAVE_PK", "1") != "0"
 # Forward of whole rows on the tensor-core path: one key-stationary sweep for passes 2 and 3
-# (dilution_forward_fused_rows) instead of the column-sum pass plus the query-stationary main pass, which short rows and calls of
-# few rows keep (_two_passes).
+# (dilution_forward_fused_rows) instead of the column-sum pass plus the query-stationary main pass, which short rows keep
+# (_sweep_is_faster, _two_passes).
 TC_FUSED_FORWARD = os.environ.get("DILUTION_FUSED_FORWARD", "1") != "0"
 
 
@@ -108,15 +108,29 @@ def _upstream(dout, n, seq, head_dim, keep_bf16):
     return dout if dout.data_ptr() % 16 == 0 else dout.clone()
 
 
+def _sweep_is_faster(n, seq, carry_rows):
+    """Calls that take the fused sweep instead of the column-sum and main passes.  Passes 2 and 3 of a call, sweep / two passes,
+    in us: n = 1, T = 4096 91 / 107; n = 31, T = 4096 189 / 238; n = 12, T = 2304 66 / 70; n = 1, T = 65536 1449 / 1845; n = 64,
+    T = 16384 4.7 / 7.0 ms.  A row of under 1536 tokens is mostly diagonal blocks, and the output that the sweep adds up in memory
+    is zeroed, reduced into and divided once per row of few tiles: n = 48, T = 1536 74 / 74, n = 16, T = 1536 49 / 51, n = 64,
+    T = 1024 57 / 55, n = 384, T = 512 107 / 103, n = 1024, T = 128 61 / 52; with 256 blocks of 512 keys it still wins from 1024
+    tokens on: n = 384, T = 1024 251 / 271, n = 128, T = 1024 93 / 98, but n = 512, T = 768 236 / 233.  Training calls of fewer
+    than 74 blocks of 256 keys (half of the SMs) take it at any length, and those of up to 100 that are no longer than 2048 tokens
+    the two passes: within 5 us of each other, where a step's launches take the host 150.  Calls that no backward follows keep the
+    two passes up to 2048 tokens, where those repeat bit for bit."""
+    if carry_rows != 32:
+        return seq > 2048
+    blocks = n * -(-seq // 256)
+    if blocks < 74 or seq > 2048:
+        return True
+    return blocks > 100 if seq >= 1536 else seq >= 1024 and n * -(-seq // 512) >= 256
+
+
 def _two_passes(n, seq, carry_rows):
-    """Calls that take the column-sum and main passes instead of the fused sweep.  With 256 blocks of 512 keys or more the sweep
-    fills the chip and is the faster one beyond 2048 tokens, before a backward or not; a short row is mostly diagonal blocks,
-    and the output that the sweep adds up in memory is zeroed, reduced into and divided once per row of few tiles.  Passes 2 and
-    3 of a call, sweep / two passes: n = 64, T = 16384 5.8 / 6.6 ms, n = 2, T = 65536 3.04 / 3.31 ms, n = 32, T = 4096 229 / 247 us,
-    n = 64, T = 3000 276 / 289, n = 52, T = 2560 180 / 175; n = 384, T = 1024 280 / 271.  With fewer blocks (the sweep then has 128
-    keys per block) the two passes are faster: n = 31, T = 4096 276 / 239, n = 1, T = 65536 2044 / 1859, n = 16, T = 2304 87 / 72,
-    n = 8, T = 2048 74 / 62.  Training calls of few short rows stay with the sweep all the same, below 74 blocks of 256 keys (half
-    of the SMs) up to 2048 tokens and up to 100 of them below 2560: the host's launches, 150 us a step, outlast either."""
+    """Calls that keep the column-sum and main passes under torch.use_deterministic_algorithms, whose outputs and demands repeat bit
+    for bit; the sweep adds up outputs in memory in no fixed order.  Calls that no backward follows all do (_takes_sweep).  A
+    training call's gradients do not repeat either way, so it gives up the sweep only where the sweep does not fill the chip, or
+    rows are short, and the host's launches outlast neither."""
     if seq > 2048 and n * -(-seq // 512) >= 256:
         return False
     if carry_rows != 32:
@@ -126,14 +140,12 @@ def _two_passes(n, seq, carry_rows):
 
 
 def _takes_sweep(code, prec, n, tq, tk, head_dim, carry_rows):
-    """Whether passes 2 and 3 of a call are the fused sweep; asked once per call, so that slabs do not differ in their kernels.
-    The sweep adds up outputs in memory in no fixed order: under torch.use_deterministic_algorithms a call that no backward
-    follows keeps the two passes, which repeat bit for bit (a backward adds up dq the same way)."""
+    """Whether passes 2 and 3 of a call are the fused sweep; asked once per call, so that slabs do not differ in their kernels."""
     if not (TC_FUSED_FORWARD and tq == tk and _lib.tensor_core_path(code, prec, head_dim)):
         return False
-    if carry_rows != 32 and torch.are_deterministic_algorithms_enabled():
-        return False
-    return not _two_passes(n, tq, carry_rows)
+    if torch.are_deterministic_algorithms_enabled():
+        return carry_rows == 32 and not _two_passes(n, tq, carry_rows)
+    return _sweep_is_faster(n, tq, carry_rows)
 
 
 def _forward_rows(lib, q, k, v, sizes, code, prec, scale, out, ssum, rmax, rden, carry, total, pk, carry_rows, sweep, st):
