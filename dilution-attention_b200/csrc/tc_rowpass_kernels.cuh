@@ -326,6 +326,219 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) rowpass_product_ker
   if (warp == 0) tmem_free(tmem, kTmem);
 }
 
+// The same of bf16 heads of 64 where there are many blocks (kPairsFrom): two query tiles of 128 per CTA, one per compute warpgroup (lane
+// = query, so that a row's sums and output need no merge), and a ninth warp that issues every TMA copy and MMA.  The keys come in
+// half tiles of 64: S = Q K^T (N = 64) and O take 128 TMEM columns of a warpgroup, P~ goes over the scores that were read, and two
+// CTAs give a scheduler four warps in four phases.  The issuing warp serves a warpgroup's P~ B and, behind it in the pipe, its next
+// scores as soon as its P~ is written; while those are on their way the other three warps of the scheduler compute.  A step of 64 keys
+// takes a warp 1240 cycles of arithmetic alone and 2150 in all with three others beside it (the special-function unit's floor: 2048);
+// continuous calls run at the card's power limit (1.72 GHz, 995 W), so that polynomials for some of the exponentials give nothing.
+// grid = n * ceil(tq/256), longest rows first.
+constexpr int kRowRing = 4;                           // half tiles of K (and V)
+constexpr int kRowThreads = 288;
+template <int MODE> constexpr int kRowSmem = 2 * (int)kTileBytes + kRowRing * MODE * (int)kTileBytes / 2 + 256 + 1024;
+
+template <int MODE, typename TOut>
+__global__ void __launch_bounds__(kRowThreads, 2) rowpass_tiles_kernel(
+    const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+    const __grid_constant__ CUtensorMap map_v, Geom g, float* __restrict__ rmax, float* __restrict__ rden,
+    TOut* __restrict__ out) {
+  static_assert(MODE == 1 || MODE == 2, "1: B = K (pk); 2: B = V (softmax attention)");
+  constexpr int R = kRowRing;
+  constexpr uint32_t HB = kTileBytes / 2;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = align1024(smem_raw);
+  const uint32_t sQ = smem_u32(smem), sK = sQ + 2 * kTileBytes, sB = MODE == 2 ? sK + R * HB : sK;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 2 * kTileBytes + MODE * R * HB);
+  const uint32_t qfull = smem_u32(bars), kfull = qfull + 8, kfree = kfull + 8 * R, sdone = kfree + 8 * R, pready = sdone + 16;
+  Ctl* ctl = reinterpret_cast<Ctl*>(bars + 5 + 2 * R);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wg = tid >> 7, row = tid & 127;
+  const int warp_u = uniform_warp();
+  const uint32_t lead = elect_one();
+  const int npair = (g.tq + 2 * kTileRows - 1) / (2 * kTileRows);
+  const int n = (int)(blockIdx.x % g.n);
+  const int t0 = (npair - 1 - (int)(blockIdx.x / g.n)) * 2;       // query tiles t0 and t0 + 1
+  // half tiles of keys that a tile's queries see; none for a tile behind the last query
+  auto half_tiles = [&](int w) {
+    return (t0 + w) * kTileRows < g.tq ? min(g.tk - 1, g.q_off + (t0 + w) * kTileRows + kTileRows - 1) / 64 + 1 : 0;
+  };
+  const int nh0 = half_tiles(0), nh1 = half_tiles(1), nh = max(nh0, nh1);
+
+  if (tid == 0) {
+    ctl->abort = 0;
+    for (int i = 0; i < 3 + 2 * R; ++i) mbar_init(qfull + 8 * i, 1);          // qfull, kfull[R], kfree[R], sdone[2]
+    mbar_init(pready, 4);
+    mbar_init(pready + 8, 4);
+    fence_barrier_init();
+  }
+  __syncwarp();
+  if (warp == 0) tmem_alloc(smem_u32(&ctl->tmem), 256);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = uniform(ctl->tmem);
+
+  if (warp_u == 8) {
+    // ------------------------------------------------------------ the issuing warp
+    constexpr uint32_t id_s = instr_desc(128, 64, 0, 0), id_p = instr_desc(128, 64, 0, 1);
+    const Desc dQ = make_desc(sQ, 16, 1024), dK = make_desc(sK, 16, 1024), dB = make_desc(sB, kTileBytes, 1024);
+    auto load_keys = [&](int h) {
+      const int st = h % R;
+      if (!lead) return;
+      mbar_expect_tx(kfull + 8 * st, MODE * HB);
+      tma_load_tile(sK + HB * st, &map_k, h * 64, n, kfull + 8 * st);
+      if (MODE == 2) tma_load_tile(sB + HB * st, &map_v, h * 64, n, kfull + 8 * st);
+    };
+    if (lead) {
+      mbar_expect_tx(qfull, (nh1 > 0 ? 2 : 1) * kTileBytes);
+      for (int w = 0; w < (nh1 > 0 ? 2 : 1); ++w) tma_load_tile(sQ + kTileBytes * w, &map_q, (t0 + w) * kTileRows, n, qfull);
+    }
+    for (int h = 0; h < R && h < nh; ++h) load_keys(h);
+    mbar_wait_warp(qfull, 0, ctl, &g_status, kErrWaitTma);
+    for (int h = 0; h <= nh; ++h) {
+      if (h < nh) mbar_wait_warp(kfull + 8 * (h % R), (h / R) & 1, ctl, &g_status, kErrWaitTma);
+      for (int w = 0; w < 2; ++w) {
+        const int nw = w ? nh1 : nh0;
+        if (h > nw || nw == 0) continue;
+        const uint32_t tS = tmem + 128 * w;
+        if (h > 0) {
+          mbar_wait_warp(pready + 8 * w, (h - 1) & 1, ctl, &g_status, kErrWaitTile);
+          tc_fence_after();
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)                          // 16 keys per instruction: 16 rows of 128 B = 128 units
+            mma_ts(lead, tS + 64, tS + 8 * kk, dB, (HB >> 4) * ((h - 1) % R) + 128 * kk, id_p, h > 1 || kk > 0);
+        }
+        if (h < nw) {
+          tc_fence_after();
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk) mma_ss(lead, tS, dQ, 1024 * w + 2 * kk, dK, (HB >> 4) * (h % R) + 2 * kk, id_s, kk > 0);
+        }
+        mma_commit(lead, sdone + 8 * w);                          // P~ B of h - 1 and the scores of h
+      }
+      if (h > 0) mma_commit(lead, kfree + 8 * ((h - 1) % R));
+      if (h > 1 && h - 2 + R < nh) {
+        mbar_wait_warp(kfree + 8 * ((h - 2) % R), ((h - 2) / R) & 1, ctl, &g_status, kErrWaitMma);
+        load_keys(h - 2 + R);
+      }
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------ the compute warps: lane = query
+    const uint32_t tS = tmem + 128 * wg + ((uint32_t)((warp & 3) * 32) << 16), tO = tS + 64;
+    const int nw = wg ? nh1 : nh0, i = (t0 + wg) * kTileRows + row, q0 = g.q_off + (t0 + wg) * kTileRows, ia = q0 + row;
+    float m_ref = -INFINITY, s = 0.f;
+    for (int h = 0; h < nw; ++h) {
+      mbar_wait(sdone + 8 * wg, h & 1, ctl, &g_status, kErrWaitMma);
+      tc_fence_after();
+      __syncwarp();
+      float v[64];
+      tmem_ld32(tS, v);
+      tmem_ld32(tS + 32, v + 32);
+      tmem_ld_wait(v);
+      tmem_ld_wait(v + 32);
+      uint32_t pw[32];
+      float ps = 0.f;
+      // P~ = 2^(z - reference) for the thread's 64 scores, two per instruction; their sum in ps
+      auto exponentials = [&]() {
+        const float mr = m_ref == -INFINITY ? 0.f : m_ref;
+        const float2 zs = make_float2(g.zscale, g.zscale), off = make_float2(-mr, -mr);
+        float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int e = 0; e < 64; e += 4) {
+          const float2 z0 = fma2(make_float2(v[e], v[e + 1]), zs, off);
+          const float2 z1 = fma2(make_float2(v[e + 2], v[e + 3]), zs, off);
+          const float2 p0 = make_float2(fast_exp2(z0.x), fast_exp2(z0.y));
+          const float2 p1 = make_float2(fast_exp2(z1.x), fast_exp2(z1.y));
+          acc0 = add2(acc0, p0);
+          acc1 = add2(acc1, p1);
+          pw[e >> 1] = pack_bf16(p0.x, p0.y);
+          pw[(e >> 1) + 1] = pack_bf16(p1.x, p1.y);
+        }
+        const float2 acc = add2(acc0, acc1);
+        ps = acc.x + acc.y;
+      };
+      // (the reference, the common half tile and the slow path are those of rowpass_product_kernel)
+      const bool edge = (h * 64 + 63 > q0) || ((h + 1) * 64 > g.tk);
+      bool slow = edge || __any_sync(0xffffffffu, m_ref == -INFINITY);
+      if (!slow) {
+        exponentials();
+        slow = __any_sync(0xffffffffu, !(ps < kRefLimit));
+        if (slow) {                      // rare: the scores are still in TMEM, fetch them again
+          tmem_ld32(tS, v);
+          tmem_ld32(tS + 32, v + 32);
+          tmem_ld_wait(v);
+          tmem_ld_wait(v + 32);
+        }
+      }
+      if (slow) {
+        float cmax = -INFINITY;
+#pragma unroll
+        for (int e = 0; e < 64; ++e) {
+          const int ja = h * 64 + e;
+          if (edge && (ja > ia || ja >= g.tk)) v[e] = -INFINITY;
+          cmax = fmaxf(cmax, v[e]);
+        }
+        const float m_new = fmaxf(m_ref, cmax * g.zscale);
+        if (__any_sync(0xffffffffu, m_new != m_ref)) {
+          const bool fresh = __all_sync(0xffffffffu, m_ref == -INFINITY);   // nothing accumulated yet
+          const float f = fast_exp2(m_ref - (m_new == -INFINITY ? 0.f : m_new));
+          if (!fresh && h > 0) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              float o[16];
+              tmem_ld16(tO + 16 * c, o);
+              tmem_ld_wait16(o);
+              uint32_t w[16];
+#pragma unroll
+              for (int e = 0; e < 16; ++e) w[e] = __float_as_uint(o[e] * f);
+              tmem_st16(tO + 16 * c, w);
+            }
+          }
+          s *= f;
+          m_ref = m_new;
+        }
+        exponentials();
+      }
+      s += ps;
+      // over the first 32 of the 64 scores: keys 2c, 2c+1 in column c
+      tmem_st16(tS, pw);
+      tmem_st16(tS + 16, pw + 16);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(pready + 8 * wg);
+    }
+    if (nw > 0) {
+      mbar_wait(sdone + 8 * wg, nw & 1, ctl, &g_status, kErrWaitMma);
+      tc_fence_after();
+      __syncwarp();
+      const float inv = (MODE == 1 ? g.scale : 1.f) / s;
+      __syncwarp();                                           // (a division has paths of its own for NaN and the like)
+      TOut* dst = out + ((int64_t)n * g.tq + i) * kHeadDim;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        float o[32];
+        tmem_ld32(tO + 32 * c, o);
+        tmem_ld_wait(o);
+#pragma unroll
+        for (int e = 0; e < 32; ++e) o[e] *= inv;
+        if (i < g.tq) store_row32<kNarrow>(dst + 32 * c, o, 32);
+      }
+      if (i < g.tq && rmax != nullptr) {
+        // the reference, not necessarily the row maximum (it lags behind it by design); every consumer uses the pair only as
+        // the log-sum-exp rmax + log2(rden)
+        rmax[(int64_t)n * g.tq + i] = m_ref;
+        rden[(int64_t)n * g.tq + i] = s;
+      }
+    }
+  }
+  drain_if_aborted(ctl);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_free(tmem, 256);
+}
+
 // Key half of the softmax-Jacobian correction alone (the reference's BC, kernels.py:777-809),
 // for a backward that has pk saved:  dk = dk_main - scale * P^T (ghat * Q).
 // grid = n * ceil(t/128) key blocks; S^T = K Q^T, lane = key; W = p * ghat goes back into TMEM
@@ -536,12 +749,29 @@ __global__ void dq_from_pk_kernel(const float* __restrict__ dq_main, const float
 }
 
 // ---------------------------------------------------------------- host launchers
+// Pairs of query tiles from which a row pass takes rowpass_tiles_kernel.  Two CTAs of two tiles each want 296 of them at a time, and a
+// CTA takes twice the tiles of one of rowpass_product_kernel, whose warpgroups share a row's keys: on a chip that is not full that one
+// is done sooner.  Row pass with pk, one tile / pairs, in us: n = 64, T = 16384 (4096 pairs) 3134 / 2681; n = 128, T = 2048 (1024)
+// 131 / 125; n = 384, T = 1024 (1536) 128.7 / 128.2; n = 32, T = 4096 (512) 111.1 / 111.0; n = 16, T = 1777 (112) 24 / 36.
+// Softmax: n = 64, T = 8192 (2048) 805 / 732; n = 64, T = 4096 (1024) 211 / 197; n = 4, T = 32768 (512) 714 / 691; n = 64, T = 1024
+// (256) 27.5 / 28.8; n = 2, T = 3000 (24) 33 / 51.
+constexpr int64_t kPairsFrom = 512;
+inline int64_t tile_pairs(const Geom& g) { return g.n * ((g.tq + 2 * kTileRows - 1) / (2 * kTileRows)); }
+
 // Pass 1 with the saved query correction: rmax, rden and pk = scale * softmax(q k^T) k.
 inline int rowstats_pk(const void* q, const void* k, const Geom& g, float* rmax, float* rden, float* pk,
                        cudaStream_t st, char* err, size_t errlen) {
   CUtensorMap mq, mk;
+  const int64_t pairs = tile_pairs(g);
   if (int rc = make_map(&mq, q, g.n, g.tq, err, errlen)) return rc;
-  if (int rc = make_map(&mk, k, g.n, g.tk, err, errlen)) return rc;
+  if (int rc = make_map(&mk, k, g.n, g.tk, err, errlen, kHeadDim, pairs >= kPairsFrom ? 64 : kTileRows)) return rc;
+  if (pairs >= kPairsFrom) {
+    auto kern = rowpass_tiles_kernel<1, float>;
+    constexpr int smem = kRowSmem<1> > kTwoPerSm ? kRowSmem<1> : kTwoPerSm;
+    if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
+    kern<<<(unsigned)pairs, kRowThreads, smem, st>>>(mq, mk, mk, g, rmax, rden, pk);
+    return launch_status("tc rowstats_pk", err, errlen);
+  }
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
   auto kern = rowpass_product_kernel<1, float>;
   constexpr int smem = RowpassSmem<1>::kBytes > kTwoPerSm ? RowpassSmem<1>::kBytes : kTwoPerSm;
@@ -551,10 +781,8 @@ inline int rowstats_pk(const void* q, const void* k, const Geom& g, float* rmax,
 }
 
 // Softmax pass, blocks above which one lane of the issuing warp polls for the next tiles instead of 32: where two CTAs share
-// every SM for long, it is the faster form, on a chip that is not full the other, whose scores are issued sooner.  One lane
-// issuing everything (with operands in ordinary registers) / all lanes polling / one: n = 64, T = 8192 840 / 861 / 846 us, n = 16, T = 16384
-// 736 / 744 / 722, n = 64, T = 4096 218 / 210 / 207, n = 128, T = 2048 131 / 123 / 123; n = 16, T = 2048 (256 blocks) 29.9 / 25.8 / 27.2,
-// n = 2, T = 3000 (48) 39.0 / 32.9 / 34.9.
+// every SM for long, it is the faster form, on a chip that is not full the other, whose scores are issued sooner.  All lanes polling /
+// one: n = 4, T = 16384 (512 blocks) 196 / 193, n = 16, T = 2048 (256) 25.8 / 27.2, n = 2, T = 3000 (48) 32.9 / 34.9.
 constexpr unsigned kOnePollsAbove = 2 * 148;
 
 // Causal softmax attention forward: out = softmax(q k^T * scale) v in bf16; rmax / rden
@@ -562,9 +790,19 @@ constexpr unsigned kOnePollsAbove = 2 * 148;
 inline int softmax_forward(const void* q, const void* k, const void* v, const Geom& g, float* rmax,
                            float* rden, void* out, cudaStream_t st, char* err, size_t errlen) {
   CUtensorMap mq, mk, mv;
+  const int64_t pairs = tile_pairs(g);
+  const int key_rows = pairs >= kPairsFrom ? 64 : kTileRows;
   if (int rc = make_map(&mq, q, g.n, g.tq, err, errlen)) return rc;
-  if (int rc = make_map(&mk, k, g.n, g.tk, err, errlen)) return rc;
-  if (int rc = make_map(&mv, v, g.n, g.tk, err, errlen)) return rc;
+  if (int rc = make_map(&mk, k, g.n, g.tk, err, errlen, kHeadDim, key_rows)) return rc;
+  if (int rc = make_map(&mv, v, g.n, g.tk, err, errlen, kHeadDim, key_rows)) return rc;
+  if (pairs >= kPairsFrom) {
+    auto kern = rowpass_tiles_kernel<2, __nv_bfloat16>;
+    constexpr int smem = kRowSmem<2>;
+    static_assert(2 * (smem + 1024) <= 233472 && 3 * (smem + 1024) > 233472, "two CTAs of the softmax pass fit one SM");
+    if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
+    kern<<<(unsigned)pairs, kRowThreads, smem, st>>>(mq, mk, mv, g, rmax, rden, (__nv_bfloat16*)out);
+    return launch_status("tc softmax_forward", err, errlen);
+  }
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
   const unsigned grid = (unsigned)(g.n * nqb);
   auto kern = grid > kOnePollsAbove ? rowpass_product_kernel<2, __nv_bfloat16, kNarrow, true>
