@@ -54,6 +54,7 @@ SIGNATURES = {
     "dilution_split_heads_rope_at": (_I, [_P, _P, _P, _P, _P, _P, _L, _L, _I, _I, _P, _P]),
     "dilution_variant_forward": (_I, [_P, _P, _P, _I, _I, _L, _L, _I, _F, _F, _I, _I, _F,
                                       _P, _P, _P, _P, _P, _P, _P, _P]),
+    "dilution_variant_forward_fused": (_I, [_P, _P, _P, _I, _I, _L, _L, _I, _F, _F, _I, _F, _P, _P, _P, _P, _P]),
     "dilution_variant_backward": (_I, [_P, _P, _P, _I, _I, _L, _L, _I, _F, _F, _I, _I, _F,
                                        _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
     "dilution_variant_decode": (_I, [_P, _P, _P, _P, _P, _I, _L, _L, _L, _I, _F, _F, _I, _I, _F, _P, _P, _P, _P]),

@@ -975,6 +975,29 @@ int dilution_variant_forward(const void* q, const void* k, const void* v, int dt
   return DILUTION_OK;
 }
 
+int dilution_variant_forward_fused(const void* q, const void* k, const void* v, int dtype, int precision, int64_t n, int64_t t,
+                                   int d, float scale, float eps, int bid, float shift, float* carry, float* total, float* out,
+                                   float* ssum, void* stream) {
+  if (int rc = check_common("dilution_variant_forward_fused", dtype, precision, n, t, t, 0, d)) return rc;
+  if (int rc = check_variant("dilution_variant_forward_fused", bid, dil::kShareInclusive, shift)) return rc;
+  if (!q || !k || !v || !carry || !total || !out || !ssum)
+    return fail(DILUTION_ERR_ARG, "dilution_variant_forward_fused: null pointer");
+#if defined(DILUTION_TENSOR_PATH) && DILUTION_TC_HAS_MAIN
+  if (bid != dil::kBidSoftmax && !dil::row_sum_bid(bid) && dil::tc::supported(dtype, precision, d, 0)) {
+    const dil::Geom g = make_geom(n, t, t, 0, scale, eps, dil::kCarryRows, bid, dil::kShareInclusive, shift);
+    cudaStream_t st = (cudaStream_t)stream;
+    {
+      Prof prof("tc_forward_fused", st);
+      if (int rc = dil::tc::forward_fused(q, k, v, g, nullptr, nullptr, carry, total, out, ssum, st, g_err, sizeof(g_err))) return rc;
+    }
+    Prof prof("tc_normalize_out", st);
+    return dil::tc::normalize_out(g, out, ssum, st, g_err, sizeof(g_err));
+  }
+#endif
+  return fail(DILUTION_ERR_UNSUPPORTED, "dilution_variant_forward_fused: element-wise bids (sigmoid, expshift, sigshift) of bf16 inputs, "
+              "BF16 precision and head_dim 64 only (other cases run dilution_variant_forward)");
+}
+
 int dilution_variant_backward(const void* q, const void* k, const void* v, int dtype, int precision, int64_t n,
                               int64_t t, int d, float scale, float eps, int bid, int share, float shift, const float* dout,
                               const float* out, const float* rmax, const float* rden, const float* carry,

@@ -102,6 +102,12 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   return r;
 }
 
+__device__ __forceinline__ float min_nan(float a, float b) {      // fminf that keeps a NaN
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
 // poly_exp2 of two values, NaN kept: 13 instructions for the pair at degree 4, where two single ones that keep a NaN take 20
 // and two that do not 18.  Degree 5 is as exact as the special-function unit (2.1e-7).
 template <int DEG>

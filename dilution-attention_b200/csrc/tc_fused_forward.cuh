@@ -39,8 +39,9 @@ static_assert(4 * 104 + 64 <= 5 * kFusedRegs, "setmaxnreg hands out what the blo
 // V[G] ones shares[G] | Q[4] (8 KB each) | staging (16 KB) | lse [4][64] | barriers
 template <int G> constexpr int kFusedSmem = (2 * G + 1) * kTileBytes + kFusedRing * kTileBytes / 2 + kTileBytes + 1024 + 256 + 1024;
 
-// G: compute warpgroups of 128 keys.  CR: query rows per checkpoint.
-template <int G, int CR, bool PAIR>
+// G: compute warpgroups of 128 keys.  CR: query rows per checkpoint.  BID: the softmax form (expshift has no row statistics: rmax is
+// null and every log-sum-exp the shift's logarithm) or the sigmoid's, with the inclusive share step.
+template <int G, int CR, bool PAIR, int BID = kBidSoftmax>
 __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_v,
     const __grid_constant__ CUtensorMap map_out, Geom g, const __nv_bfloat16* __restrict__ k,
@@ -70,6 +71,8 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
   const int h0 = k0 / 64, nh = (g.tq + 63) / 64;          // half tiles of queries; warpgroup w sees those from h0 + 2 w on
   const int groups = min(G, (g.tk - k0 + kTileRows - 1) / kTileRows);
   const int64_t row_base = (int64_t)n * g.tq;
+  // what a query's scores are added to: minus its log-sum-exp, or plus (the sigmoid's exponent is lse - z)
+  auto offset = [&](float lse) { return BID == kBidSigmoid ? lse : -lse; };
 
   if (tid == 0) {
     ctl->abort = 0;
@@ -81,9 +84,9 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
   __syncwarp();
   if (warp == 0) tmem_alloc(smem_u32(&ctl->tmem), kTmem);
   if (wg == G) {
-    sL[row] = -load_lse(rmax, rden, row_base, h0 * 64 + row, g.tq);         // of the first three half tiles
+    sL[row] = offset(load_lse<BID>(rmax, rden, row_base, h0 * 64 + row, g.tq, g.lshift));    // of the first three half tiles
   } else if (wg == 0) {
-    if (row < 64) sL[128 + row] = -load_lse(rmax, rden, row_base, h0 * 64 + 128 + row, g.tq);
+    if (row < 64) sL[128 + row] = offset(load_lse<BID>(rmax, rden, row_base, h0 * 64 + 128 + row, g.tq, g.lshift));
 #pragma unroll
     for (int c = 0; c < 8; ++c)
       reinterpret_cast<uint4*>(ones_ptr)[row * 8 + c] = make_uint4(c == (row & 7) ? 0x3f80u : 0u, 0u, 0u, 0u);
@@ -182,14 +185,18 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
         const int i3 = (h + 3) * 64 + row;
         const bool fetch = row < 64 && h + 3 < nh;
         if (fetch && i3 < g.tq) {
-          nx_max = rmax[row_base + i3];
-          nx_den = rden[row_base + i3];
+          if (BID == kBidSigmoid || rmax == nullptr) {
+            nx_max = g.lshift;
+          } else {
+            nx_max = rmax[row_base + i3];
+            nx_den = rden[row_base + i3];
+          }
         }
         const int u = h - h0, w4 = warp & 3;
         if (lane == 0) mbar_wait(ofull + 8 * (u & 1), (u >> 1) & 1, ctl, &g_status, kErrWaitMma);
         __syncwarp();
         tc_fence_after();
-        if (fetch) sL[64 * ((u + 3) & 3) + row] = -(nx_max + log2f(nx_den));
+        if (fetch) sL[64 * ((u + 3) & 3) + row] = offset(nx_max + log2f(nx_den));
         __syncwarp();
         const uint32_t tOb = tO + 64 * (u & 1) + lane_base;
         const uint32_t stage = sStage + HB * w4;
@@ -245,6 +252,7 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
     // committed + eps in front of a chunk of 32 queries, and what its sum has rounded off: the bids of a chunk are added up from
     // zero and folded in once, so that neither thousands of roundings nor bids under half an ulp of a large demand add up
     float base = g.eps, low = 0.f;
+    const float zscale = BID == kBidSigmoid ? -g.zscale : g.zscale;
     for (int h = h0 + 2 * wg; h < nh && wg < groups; ++h) {
       const int t = h - h0 - 2 * wg;
       float v0[32], v1[32];
@@ -267,17 +275,20 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
             float z[8], sh[8], dn[8];
 #pragma unroll
             for (int u = 0; u < 8; u += 2) {
-              const float2 z2 = fma2(make_float2(v[e8 * 8 + u], v[e8 * 8 + u + 1]), make_float2(g.zscale, g.zscale),
+              const float2 z2 = fma2(make_float2(v[e8 * 8 + u], v[e8 * 8 + u + 1]), make_float2(zscale, zscale),
                                      make_float2(ls[u], ls[u + 1]));
               z[u] = z2.x;
               z[u + 1] = z2.y;
             }
             // every fourth exponential is a polynomial on the FMA pipe (7.30 -> 7.08 ms when two warps shared a scheduler), of
             // degree 5: with degree 4 the demand, an output in fp32, is off by up to 4.6e-6 instead of 2.5e-6
-            const float2 fourth = poly_exp2_two<5>(make_float2(z[3], z[7]));
+            // (the sigmoid's exponents are of either sign: capped, where the bid is 1e-38 and less)
+            const float2 fourth = poly_exp2_two<5>(BID == kBidSigmoid ? make_float2(min_nan(z[3], 126.f), min_nan(z[7], 126.f))
+                                                                      : make_float2(z[3], z[7]));
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
               float p = (u & 3) != 3 ? fast_exp2(z[u]) : u == 3 ? fourth.x : fourth.y;
+              if (BID == kBidSigmoid) p = fast_rcp(1.f + p);
               if (MASK && (dead || ja > q0 + e8 * 8 + u)) p = 0.f;
               chunk_sum += p;
               sh[u] = p;
@@ -371,10 +382,10 @@ inline int forward_fused(const void* q, const void* k, const void* v, const Geom
   }
   const int64_t rows = g.n * g.tq;
   zero_sums_kernel<<<(unsigned)((rows * (kHeadDim / 4) + 255) / 256), 256, 0, st>>>(out, ssum, rows);
-  auto launch = [&](auto groups_c, auto cr_c, auto pair_c) -> int {
+  auto launch = [&](auto groups_c, auto cr_c, auto pair_c, auto bid_c) -> int {
     constexpr int G = decltype(groups_c)::value, smem = kFusedSmem<G>;
     static_assert(smem <= 232448 && (G > 1 || 2 * (smem + 1024) <= 233472), "one or two CTAs fit one SM's shared memory");
-    auto kern = forward_fused_kernel<G, decltype(cr_c)::value, decltype(pair_c)::value>;
+    auto kern = forward_fused_kernel<G, decltype(cr_c)::value, decltype(pair_c)::value, decltype(bid_c)::value>;
     if (int rc = set_smem_attr((const void*)kern, smem, err, errlen, G == 4 ? kFusedRegs : 0)) return rc;
     const int nsb = (g.tk + G * kTileRows - 1) / (G * kTileRows);
     kern<<<(unsigned)(g.n * nsb), 128 * (G + 1), smem, st>>>(mq, mv, mo, g, (const __nv_bfloat16*)k, rmax, rden, carry, total,
@@ -382,10 +393,16 @@ inline int forward_fused(const void* q, const void* k, const void* v, const Geom
     return 0;
   };
   using std::integral_constant;
+  using Softmax = integral_constant<int, kBidSoftmax>;
+  using Sigmoid = integral_constant<int, kBidSigmoid>;
   auto by_pair = [&](auto groups_c, auto cr_c) {
-    return pair_demands(g) ? launch(groups_c, cr_c, std::true_type{}) : launch(groups_c, cr_c, std::false_type{});
+    return pair_demands(g) ? launch(groups_c, cr_c, std::true_type{}, Softmax{}) : launch(groups_c, cr_c, std::false_type{}, Softmax{});
   };
   auto by_rows = [&](auto groups_c) {
+    if (g.bid == kBidSigmoid) {                             // (variants have checkpoints every 32 rows)
+      return pair_demands(g) ? launch(groups_c, integral_constant<int, 32>{}, std::true_type{}, Sigmoid{})
+                             : launch(groups_c, integral_constant<int, 32>{}, std::false_type{}, Sigmoid{});
+    }
     return g.carry_rows == 64 ? by_pair(groups_c, integral_constant<int, 64>{}) : by_pair(groups_c, integral_constant<int, 32>{});
   };
   if (int rc = fused_groups(g.n, g.tk) == 4 ? by_rows(integral_constant<int, 4>{}) : by_rows(integral_constant<int, 1>{})) return rc;

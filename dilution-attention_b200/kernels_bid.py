@@ -58,6 +58,9 @@ def _share_code(share_cumsum) -> int:
     return int(bool(share_cumsum))
 
 
+_SWEEP_BIDS = tuple(_lib.BID[b] for b in ("sigmoid", "expshift", "sigshift"))
+
+
 def _is_operator(bid: str, share_cumsum) -> bool:
     return bid == "softmax" and _share_code(share_cumsum) == 1
 
@@ -132,6 +135,17 @@ def dilution_attention_forward(
     return result
 
 
+def _takes_sweep(bid, share, code, prec, n, seq, head_dim):
+    """Training forwards that are one key-stationary sweep instead of the column-sum and main passes: the element-wise bids with the
+    inclusive share step, where rows are long or there are enough blocks of 512 keys for the SMs.  Sweep / two passes in us, sigmoid:
+    n = 32, T = 8192 783 / 1331; n = 30, T = 2048 79 / 110; n = 4, T = 4096 (32 blocks) 108 / 131; n = 200, T = 1024 160 / 183.
+    Expshift: n = 32, T = 8192 654 / 944; n = 4, T = 4096 98 / 111; n = 200, T = 1024 143 / 148, but n = 100, T = 1024 (200 blocks)
+    84 / 80 and n = 400, T = 512 105 / 104."""
+    return (share == 1 and bid in _SWEEP_BIDS and n * -(-seq // 512) >= (32 if seq >= 2048 else 256) and seq >= 1024
+            and K.TC_FUSED_FORWARD and _lib.tensor_core_path(code, prec, head_dim)
+            and not torch.are_deterministic_algorithms_enabled())
+
+
 class _VariantFn(torch.autograd.Function):
     """Autograd op of the variants (kernels_bid.py:731-815): fp32 output; dq, dk, dv in the
     input dtypes."""
@@ -153,9 +167,14 @@ class _VariantFn(torch.autograd.Function):
         ws, at = K._workspace(q.device, **parts)
         out = torch.empty(q.shape, device=q.device, dtype=torch.float32)
         rmax, rden, carry, total, ssum, pk = _parts(ws, at)
-        _lib.check(lib.dilution_variant_forward(
-            *(x.data_ptr() for x in ops), code, prec, n, seq, head_dim, 1.0 / math.sqrt(head_dim), EPS, bid, share,
-            float(shift), rmax, rden, carry, total, out.data_ptr(), ssum, pk, K._stream(q.device)), "dilution_variant_forward")
+        if _takes_sweep(bid, share, code, prec, n, seq, head_dim):
+            _lib.check(lib.dilution_variant_forward_fused(
+                *(x.data_ptr() for x in ops), code, prec, n, seq, head_dim, 1.0 / math.sqrt(head_dim), EPS, bid, float(shift),
+                carry, total, out.data_ptr(), ssum, K._stream(q.device)), "dilution_variant_forward_fused")
+        else:
+            _lib.check(lib.dilution_variant_forward(
+                *(x.data_ptr() for x in ops), code, prec, n, seq, head_dim, 1.0 / math.sqrt(head_dim), EPS, bid, share,
+                float(shift), rmax, rden, carry, total, out.data_ptr(), ssum, pk, K._stream(q.device)), "dilution_variant_forward")
         ctx.save_for_backward(q, k, v, out, ws)
         ctx.call = (dot_precision, bid, share, shift, at)
         return out

@@ -377,6 +377,12 @@ int dilution_variant_forward(const void* q, const void* k, const void* v, int dt
                              int64_t t, int d, float scale, float eps, int bid, int share, float shift, float* rmax,
                              float* rden, float* carry, float* total, float* out, float* ssum, float* pk,
                              void* stream);
+/* The same of an element-wise bid (sigmoid, expshift, sigshift) with the inclusive share step, bf16 inputs, BF16 precision and
+ * head_dim 64, as one key-stationary sweep in place of the column-sum and main passes: same outputs, added up in memory in no
+ * fixed order (dilution_forward_fused). */
+int dilution_variant_forward_fused(const void* q, const void* k, const void* v, int dtype, int precision, int64_t n, int64_t t,
+                                   int d, float scale, float eps, int bid, float shift, float* carry, float* total, float* out,
+                                   float* ssum, void* stream);
 int dilution_variant_backward(const void* q, const void* k, const void* v, int dtype, int precision, int64_t n,
                               int64_t t, int d, float scale, float eps, int bid, int share, float shift, const float* dout,
                               const float* out, const float* rmax, const float* rden, const float* carry,

@@ -1,0 +1,83 @@
+"""Element-wise bids with the inclusive share step as one key-stationary sweep, against the column-sum and main passes it replaces in
+training forwards (which the goldens and the oracle hold), on both block sizes and ragged lengths."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from conftest import load_package
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _run(pkg, q, k, v, bid, shift, eps, fused):
+    lib, L = pkg._lib.load(), pkg._lib
+    n, seq = q.shape[1], q.shape[2]
+    out, ssum, total = (torch.empty(n, seq, *s, device=DEV) for s in ((64,), (), ()))
+    carry = torch.zeros(n, (seq + 31) // 32, seq, device=DEV)
+    args = (*(x.data_ptr() for x in (q, k, v)), L.BF16, L.PREC["bf16"], n, seq, 64, 0.125, eps, L.BID[bid])
+    st = torch.cuda.current_stream().cuda_stream
+    if fused:
+        rc = lib.dilution_variant_forward_fused(*args, shift, carry.data_ptr(), total.data_ptr(), out.data_ptr(), ssum.data_ptr(), st)
+    else:
+        rc = lib.dilution_variant_forward(*args, 1, shift, None, None, carry.data_ptr(), total.data_ptr(), out.data_ptr(),
+                                          ssum.data_ptr(), None, st)
+    L.check(rc, "variant forward")
+    return out, ssum, total, carry
+
+
+def _inputs(rows, seq, std=1.0):
+    g = torch.Generator(device=DEV).manual_seed(rows * seq)
+    q, k, v = (torch.randn(1, rows, seq, 64, device=DEV, generator=g) for _ in range(3))
+    return (q * std).bfloat16(), k.bfloat16(), v.bfloat16()
+
+
+# 128 and 512 keys per block (200 blocks of 512), lengths around tiles, half tiles and checkpoints
+@pytest.mark.parametrize("rows,seq", [(1, 1), (2, 31), (1, 65), (3, 127), (2, 513), (1, 1777), (200, 129), (67, 1100), (100, 1024)])
+@pytest.mark.parametrize("bid,shift", [("sigmoid", 1.0), ("sigshift", 40.0), ("expshift", 1000.0)])
+@pytest.mark.parametrize("eps,std", [(1e-9, 1.0), (1e-30, 8.0)])
+def test_sweep_matches_the_two_passes(rows, seq, bid, shift, eps, std):
+    pkg = load_package()
+    x = _inputs(rows, seq, std)
+    (out, ssum, total, carry), (ref, rsum, rtotal, rcarry) = (_run(pkg, *x, bid, shift, eps, fused) for fused in (True, False))
+    # demands are fp32 sums of the same bids in another order; every fourth exponential is a polynomial (2e-7)
+    assert ((total - rtotal).abs() <= 2e-5 * rtotal.abs() + 1e-30).all()
+    block = torch.arange(carry.shape[1], device=DEV)[:, None] * 32
+    seen = torch.arange(seq, device=DEV)[None] < block         # what a backward reads: keys in front of a block's first query
+    assert ((carry - rcarry).abs() <= 2e-5 * rcarry.abs() + 1e-30)[:, seen].all()
+    # both round shares to 8 bits, at different values where the demands' last bits differ: 2^-8 of a share each
+    assert ((ssum - rsum).abs() <= 2.0 ** -7 * rsum.abs() + 1e-6).all()
+    assert (out - ref).abs().max().item() <= 2.0 ** -6 * ref.abs().max().item()
+
+
+def test_a_query_that_is_not_a_number_stays_in_its_rows_and_demands():
+    pkg = load_package()
+    q, k, v = _inputs(2, 700)
+    q[0, 0, 300] = float("nan")
+    out, _, total, _ = _run(pkg, q, k, v, "sigmoid", 1.0, 1e-9, True)
+    assert out[0, 300].isnan().all() and out[0, :300].isfinite().all() and out[1].isfinite().all()
+    assert total[0, :301].isnan().all() and total[0, 301:].isfinite().all()
+
+
+def test_training_calls_take_it():
+    pkg = load_package()
+    x, y = ([t.requires_grad_(True) for t in _inputs(rows, 2048)] for rows in (8, 7))
+    for share, name, x in ((True, "tc_forward_fused", x), ("exclusive", "tc_forward_main", x), (True, "tc_forward_main", y)):
+        pkg._lib.profile(True)
+        pkg._lib.profile_collect()
+        pkg.kernels_bid.dilution_attention(*x, dot_precision="bf16", bid="sigmoid", share_cumsum=share)
+        names = set(pkg._lib.profile_collect())
+        pkg._lib.profile(False)
+        assert name in names, names
+
+
+def test_other_calls_are_refused():
+    pkg = load_package()
+    lib, L = pkg._lib.load(), pkg._lib
+    one = 256                                                 # never dereferenced
+    for dtype, prec, d, bid in ((L.F32, L.PREC["tf32"], 64, "sigmoid"), (L.BF16, L.PREC["bf16"], 32, "sigmoid"),
+                                (L.BF16, L.PREC["bf16"], 64, "softmax"), (L.BF16, L.PREC["bf16"], 64, "relu")):
+        assert lib.dilution_variant_forward_fused(one, one, one, dtype, prec, 1, 8, d, 0.125, 1e-9, L.BID[bid], 1.0, one, one, one,
+                                                  one, None) == 2
