@@ -1754,6 +1754,413 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
   if (warp == 0) tmem_free(tmem, 512);
 }
 
+// The forward half of reverse_sweeps for a thread's 32 queries and the sigmoid's bid: scores become bids in vs, and inv takes
+// 1/(committed + p + eps) (the exclusive share step: 1/(committed + eps)).  incle is the key's demand (+ eps) in front of the queries.
+template <int SHARE, bool MASK>
+__device__ __forceinline__ void bids_and_inverses(float (&vs)[32], float (&inv)[32], float incle, const Geom& g, bool dead, int first_q) {
+  const float2 zs = make_float2(-g.zscale, -g.zscale), lse = make_float2(g.lshift, g.lshift);
+#pragma unroll
+  for (int e = 0; e < 32; e += 2) {
+    const float2 z2 = fma2(make_float2(vs[e], vs[e + 1]), zs, lse);
+    const float z[2] = {z2.x, z2.y};
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      float p = fast_rcp(1.f + fast_exp2(z[u]));
+      if (MASK && (dead || first_q > e + u)) p = 0.f;
+      if (SHARE == kShareInclusive) incle += p;
+      inv[e + u] = fast_rcp(incle);
+      if (SHARE == kShareExclusive) incle += p;
+      vs[e + u] = p;
+    }
+  }
+}
+
+// The backward half for 8 of them, last to first: vd holds their dO' . v, R the suffix of dk_share behind them and, afterwards, in
+// front of them.  shp takes their shares as bf16 pairs, p the Jacobian factor, inv that factor times dp.  The formulas stand in
+// reverse_sweeps.
+template <int SHARE>
+__device__ __forceinline__ void suffix_of_eight(float* p, float* inv, const float* vd, const float4* Dbar4, float& R, uint32_t* shp) {
+#pragma unroll
+  for (int c = 1; c >= 0; --c) {
+    const float4 d4 = Dbar4[c];
+    const float dbr[4] = {d4.x, d4.y, d4.z, d4.w};
+#pragma unroll
+    for (int h = 1; h >= 0; --h) {
+      const int e = 4 * c + 2 * h;
+      const float2 p2 = make_float2(p[e], p[e + 1]), i2 = make_float2(inv[e], inv[e + 1]);
+      const float2 w2 = mul2(sub2(make_float2(vd[e], vd[e + 1]), make_float2(dbr[2 * h], dbr[2 * h + 1])), i2), s2 = mul2(p2, i2);
+      const float r1 = fmaf(-w2.y, s2.y, R), r0 = fmaf(-w2.x, s2.x, r1);
+      const float2 jac2 = mul2(p2, sub2(make_float2(1.f, 1.f), p2));
+      const float2 pd2 = mul2(jac2, add2(w2, SHARE == kShareInclusive ? make_float2(r0, r1) : make_float2(r1, R)));
+      R = r0;
+      shp[2 * c + h] = pack_bf16(s2.x, s2.y);
+      p[e] = jac2.x;
+      p[e + 1] = jac2.y;
+      inv[e] = pd2.x;
+      inv[e + 1] = pd2.y;
+    }
+  }
+}
+
+// Main reverse pass (the reference's BA, kernels.py:677-775) of the sigmoid's bid with a share step.
+// grid = n * ceil(t/128), key blocks with the most queries first; one CTA per SM, five warpgroups: four of compute warps, and one
+// whose last warp issues every TMA copy and MMA while its first two move the finished dQ tiles out.
+//
+// The CTA keeps K and V of 128 keys (both as TMEM operands) and walks the queries from last to first in slices of 32, which the
+// compute warpgroups take in turn, one thread per key.  The demand of a key is stored every 32 query rows, so every slice starts
+// from a stored checkpoint; what a slice needs of the one behind it is the key's suffix of dk_share, one float per key, which is
+// handed from warp to warp (the four warps of a scheduler hold the same 32 keys): nothing in the loop waits for the whole CTA.  Per
+// slice:
+//   S^T, (dO' V^T)^T   [128 keys x 32 queries] each: 4 + 4 MMAs of N = 32, A = K, V in TMEM
+//   forwards           p and 1/(committed + p + eps), the demand accumulated from the checkpoint exactly as the forward pass did
+//   backwards          the suffix of dk_share from the slice's end in the reference's order (kernels.py:763-764); the suffix behind
+//                      the slice is added afterwards, dp being linear in it
+//   dV, dK             += share^T dO', pdp^T Q: shares and pdp go back into TMEM as bf16 pairs over the scores that were read, where
+//                      they are A operands (M = keys): 2 + 2 MMAs
+// and per 64 queries dQ^T = [K | 0]^T pdp, M = 64 features (and 64 rows of zeros), from the pdp that every thread also writes to
+// shared memory: 8 MMAs of N = 64 into one tile of 64 columns, moved out by TMA tensor reductions as in the fused forward.
+// TMEM: [S^T 32 | dOV^T 32] per warpgroup, dV 64, dK 64, V 32, K 32, dQ^T 64 = 512 columns.
+//
+// Against backward_main_kernel, whose eight compute warps go through a half-step together: whole backward, n = 32, T = 8192
+// 1673 -> 1437 us, n = 8, T = 4096 127 -> 107, n = 64, T = 2048 294 -> 271, n = 16, T = 1777 69.9 -> 65.7, but n = 384, T = 1024
+// 604 -> 609 and n = 256, T = 512 163 -> 168, where a block's start and end weigh more.  The three special-function operations of a
+// sigmoid score leave the card below its power limit; the softmax bid's passes of long rows run at it (1.72 GHz), and there this
+// form, which executes more instructions, gained nothing (14.5 / 14.6 ms at n = 64, T = 16384; n = 384, T = 1024 672 / 705 us).
+constexpr int kSliceRegs = 96;          // per thread at launch, by the launch bounds
+static_assert(4 * 104 + 64 <= 5 * kSliceRegs, "setmaxnreg hands out what the block was launched with");
+constexpr int kSliceThreads = 640;
+constexpr int kSliceRing = 6;                                     // half tiles (64 queries) of q and of do'
+constexpr int kSliceFrom = 1536;                                  // tokens of a row from which it is the faster one
+// K zeros | Q[6] dO'[6] (8 KB each) | pdp[2] | staging[2] (16 KB each) | dbar [4][64] | suffixes [4][128] | barriers
+constexpr int kSliceSmem = (2 + kSliceRing + 2 + 2) * kTileBytes + 1024 + 2048 + 512 + 1024;
+
+template <int SHARE>
+__global__ void __launch_bounds__(kSliceThreads, 1) backward_slices_kernel(
+    const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+    const __grid_constant__ CUtensorMap map_do, const __grid_constant__ CUtensorMap map_dq, Geom g,
+    const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
+    const float* __restrict__ dbarp, const float* __restrict__ carry, const float* __restrict__ total, float* __restrict__ dk_main,
+    __nv_bfloat16* __restrict__ dv) {
+  constexpr int R = kSliceRing;
+  constexpr uint32_t HB = kTileBytes / 2;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = align1024(smem_raw);
+  const uint32_t sK = smem_u32(smem), sZero = sK + kTileBytes;               // A of dQ^T: [K | 0], MN-major
+  const uint32_t sQ = sZero + kTileBytes, sD = sQ + R * HB, sPd = sD + R * HB;
+  const uint32_t sStage = sPd + 2 * kTileBytes;                              // [2][2 warps][64 queries][32 features] fp32
+  float* sDbar = reinterpret_cast<float*>(smem + (sStage - sK) + 2 * kTileBytes);   // [4][64] dbar' of a half tile's queries
+  float* sG = sDbar + 256;                                                   // [4][128] suffix in front of a warpgroup's slice
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sG + 512);
+  const uint32_t kfull = smem_u32(bars), fin = kfull + 8, qfull = fin + 8, sdone = qfull + 8 * R, dqdone = sdone + 32,
+                 tiles = dqdone + 16, dqfree = tiles + 32, chain = dqfree + 8;            // 1, 1, [R], [4], [2], [4], 1, [4][4]
+  Ctl* ctl = reinterpret_cast<Ctl*>(bars + 13 + R + 16);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wg = tid >> 7, row = tid & 127;
+  const int warp_u = uniform_warp();
+  const uint32_t lead = elect_one();
+  const int ncb = (g.tq + kCarryRows - 1) / kCarryRows;
+  const int n = (int)(blockIdx.x % g.n);
+  const int k0 = (int)(blockIdx.x / g.n) * kTileRows;
+  const int hl = (g.tq + 63) / 64 - 1, nh = hl - k0 / 64 + 1;   // half tiles hl .. k0 / 64 of queries: the u-th one is hl - u
+  const int64_t row_base = (int64_t)n * g.tq;
+  const int ja = k0 + row;
+  const bool dead = ja >= g.tk;
+
+  if (tid == 0) {
+    ctl->abort = 0;
+    for (int i = 0; i < 8 + R; ++i) mbar_init(kfull + 8 * i, 1);            // kfull, fin, qfull[R], sdone[4], dqdone[2]
+    for (int i = 0; i < 4; ++i) mbar_init(tiles + 8 * i, 4);
+    mbar_init(dqfree, 3);
+    for (int i = 0; i < 16; ++i) mbar_init(chain + 8 * i, 1);
+    fence_barrier_init();
+  }
+  __syncwarp();
+  if (warp == 0) tmem_alloc(smem_u32(&ctl->tmem), 512);
+  if (tid < 256) {
+    // of the first four half tiles (a negative row belongs to no half tile of this block)
+    const int i = (hl - (tid >> 6)) * 64 + (tid & 63);
+    sDbar[tid] = i >= 0 && i < g.tq ? dbarp[row_base + i] : 0.f;
+  } else if (wg == 2) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) reinterpret_cast<uint4*>(smem + kTileBytes)[row * 8 + c] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  fence_async_smem();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = uniform(ctl->tmem);
+  const uint32_t tS = tmem, tDV = tmem + 256, tDK = tmem + 320, tV = tmem + 384, tK = tmem + 416, tQ = tmem + 448;
+  const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+
+  if (wg < 2) {
+    // this key's row as an A operand: two head-dim elements per 32-bit column
+    uint32_t w[32];
+    const __nv_bfloat16* src = (wg == 0 ? v : k) + ((int64_t)n * g.tk + ja) * kHeadDim;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      uint4 x = make_uint4(0u, 0u, 0u, 0u);
+      if (!dead) x = reinterpret_cast<const uint4*>(src)[c];
+      w[4 * c] = x.x; w[4 * c + 1] = x.y; w[4 * c + 2] = x.z; w[4 * c + 3] = x.w;
+    }
+    __syncwarp();
+    tmem_st16(tV + 32 * wg + lane_base, w);
+    tmem_st16(tV + 32 * wg + lane_base + 16, w + 16);
+    tmem_st_wait();
+  } else if (wg < 4) {
+    // dV and dK start from zero, so that every MMA into them accumulates
+    uint32_t z[16];
+#pragma unroll
+    for (int c = 0; c < 16; ++c) z[c] = 0u;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) tmem_st16(tDV + 64 * (wg - 2) + lane_base + 16 * c, z);
+    tmem_st_wait();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+
+  if (wg == 4) {
+    // ------------------------------------------------------------ issue (its last warp), and the dQ read-out
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    if (warp_u == 19) {
+      constexpr uint32_t id_s = instr_desc(128, 32, 0, 0);     // scores: A from TMEM, B K-major
+      constexpr uint32_t id_kd = instr_desc(128, 64, 0, 1);    // dV, dK: A from TMEM (M = keys), B MN-major
+      constexpr uint32_t id_q = instr_desc(128, 64, 1, 1);     // dQ^T: A and B MN-major
+      const Desc dKm = make_desc(sK, sZero - sK, 1024), dPd = make_desc(sPd, kTileBytes, 1024);
+      const Desc dQk = make_desc(sQ, 16, 1024), dQm = make_desc(sQ, kTileBytes, 1024);
+      const Desc dDk = make_desc(sD, 16, 1024), dDm = make_desc(sD, kTileBytes, 1024);
+      auto load_rows = [&](int u) {
+        const int st = u % R;
+        if (!lead) return;
+        mbar_expect_tx(qfull + 8 * st, 2 * HB);
+        tma_load_tile(sQ + HB * st, &map_q, (hl - u) * 64, n, qfull + 8 * st);
+        tma_load_tile(sD + HB * st, &map_do, (hl - u) * 64, n, qfull + 8 * st);
+      };
+      // Place in the ring and warpgroup are compile-time (half tile u is the J-th of a round of the ring), so that an MMA's
+      // operands are constants away from uniform registers.
+      // scores of slice ODD of a half tile: queries 32..63 for ODD = 0, 0..31 for 1
+      auto issue_scores = [&](auto j_c, auto odd_c) {
+        constexpr int J = decltype(j_c)::value, ODD = decltype(odd_c)::value, W = (2 * J + ODD) & 3;
+        constexpr uint32_t off = (HB >> 4) * J + (ODD ? 0 : 256);
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) mma_ts(lead, tS + 64 * W, tK + 8 * kk, dQk, off + 2 * kk, id_s, kk > 0);
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) mma_ts(lead, tS + 64 * W + 32, tV + 8 * kk, dDk, off + 2 * kk, id_s, kk > 0);
+        mma_commit(lead, sdone + 8 * W);
+      };
+      using C0 = std::integral_constant<int, 0>;
+      using C1 = std::integral_constant<int, 1>;
+      if (lead) {
+        mbar_expect_tx(kfull, kTileBytes);
+        tma_load_tile(sK, &map_k, k0, n, kfull);
+      }
+      for (int u = 0; u < R && u < nh; ++u) load_rows(u);
+      mbar_wait_warp(qfull, 0, ctl, &g_status, kErrWaitTma);
+      tc_fence_after();
+      issue_scores(C0{}, C0{});
+      issue_scores(C0{}, C1{});
+      if (nh > 1) {
+        mbar_wait_warp(qfull + 8, 0, ctl, &g_status, kErrWaitTma);
+        tc_fence_after();
+        issue_scores(C1{}, C0{});
+        issue_scores(C1{}, C1{});
+      }
+      mbar_wait_warp(kfull, 0, ctl, &g_status, kErrWaitTma);
+      auto half = [&](auto j_c, int u) {
+        constexpr int J = decltype(j_c)::value, J2 = (J + 2) % R;
+        auto slice = [&](auto odd_c) {
+          constexpr int ODD = decltype(odd_c)::value, W = (2 * J + ODD) & 3;
+          constexpr uint32_t off = (HB >> 4) * J + (ODD ? 0 : 256);
+          mbar_wait_warp(tiles + 8 * W, (u >> 1) & 1, ctl, &g_status, kErrWaitTile);
+          tc_fence_after();
+#pragma unroll
+          for (int kk = 0; kk < 2; ++kk) {                     // contraction over the 32 queries
+            mma_ts(lead, tDV, tS + 64 * W + 8 * kk, dDm, off + 128 * kk, id_kd, 1);
+            mma_ts(lead, tDK, tS + 64 * W + 32 + 8 * kk, dQm, off + 128 * kk, id_kd, 1);
+          }
+          if (u + 2 < nh) {
+            if (!ODD) {
+              mbar_wait_warp(qfull + 8 * J2, ((u + 2) / R) & 1, ctl, &g_status, kErrWaitTma);
+              tc_fence_after();
+            }
+            issue_scores(std::integral_constant<int, J2>{}, odd_c);
+          }
+        };
+        slice(C0{});
+        slice(C1{});
+        // both slices of the half tile exist.  Once dQ^T of the one before is out, its queries' places in the ring are free, and
+        // dbar' of half tile u + 3 is in its place
+        if (u >= 1) {
+          mbar_wait_warp(dqfree, (u - 1) & 1, ctl, &g_status, kErrWaitDrain);
+          tc_fence_after();
+          if (u - 1 + R < nh) load_rows(u - 1 + R);
+        }
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)                         // contraction over the 128 keys
+          mma_ss(lead, tQ, dKm, 128 * kk, dPd, (kTileBytes >> 4) * (J & 1) + 128 * kk, id_q, kk > 0);
+        mma_commit(lead, dqdone + 8 * (J & 1));
+      };
+      static_assert(R == 6, "a round of the ring is six half tiles, an even number");
+      for (int u = 0; u < nh; u += R) {
+        half(C0{}, u);
+        if (u + 1 < nh) half(C1{}, u + 1);
+        if (u + 2 < nh) half(std::integral_constant<int, 2>{}, u + 2);
+        if (u + 3 < nh) half(std::integral_constant<int, 3>{}, u + 3);
+        if (u + 4 < nh) half(std::integral_constant<int, 4>{}, u + 4);
+        if (u + 5 < nh) half(std::integral_constant<int, 5>{}, u + 5);
+      }
+      mma_commit(lead, fin);
+      __syncwarp();
+    } else {
+      // dQ^T of half tile u to global memory by two warps, lane = feature (staging is doubled: a tile does not wait for the copy
+      // engine to have read the one before).  The third keeps dbar': that of half tile u + 4 takes the place of half tile u, whose
+      // last use lies in front of dqdone; the issuing warp has waited for the release of u before it issues scores of u + 3.
+      if (warp_u == 18) {
+        float next[2] = {0.f, 0.f};
+        auto fetch = [&](int u) {                              // (every row of an earlier half tile exists)
+          next[0] = dbarp[row_base + (hl - u) * 64 + lane];
+          next[1] = dbarp[row_base + (hl - u) * 64 + 32 + lane];
+        };
+        if (4 < nh) fetch(4);
+        for (int u = 0; u < nh; ++u) {
+          if (lane == 0) mbar_wait(dqdone + 8 * (u & 1), (u >> 1) & 1, ctl, &g_status, kErrWaitMma);
+          __syncwarp();
+          if (u + 4 < nh) {
+            sDbar[64 * (u & 3) + lane] = next[0];
+            sDbar[64 * (u & 3) + 32 + lane] = next[1];
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(dqfree);
+          if (u + 5 < nh) fetch(u + 5);
+        }
+      } else {
+        const uint32_t tile = tQ + lane_base;
+        for (int u = 0; u < nh; ++u) {
+          const uint32_t stage = sStage + kTileBytes * (u & 1) + HB * (warp & 1);
+          if (lane == 0) mbar_wait(dqdone + 8 * (u & 1), (u >> 1) & 1, ctl, &g_status, kErrWaitMma);
+          if (lane == 0) tma_wait_read_all_but_one();          // the last reduction but one has read this staging
+          __syncwarp();
+          tc_fence_after();
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            float o[32];
+            tmem_ld32(tile + 32 * c, o);
+            tmem_ld_wait(o);
+            if (c == 1) {
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(dqfree);              // this warp has read the tile
+            }
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+              asm volatile("st.shared.f32 [%0], %1;" ::"r"(stage + lane * 4 + (32 * c + e) * 128), "f"(o[e] * g.scale) : "memory");
+          }
+          fence_async_smem();
+          __syncwarp();
+          if (lane == 0) tma_reduce_add_tile(&map_dq, stage, 32 * (warp & 1), (hl - u) * 64, n);
+        }
+      }
+      if (lane == 0) tma_wait_read_all();
+      __syncwarp();
+    }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    // ------------------------------------------------------------ the compute warps: lane = key
+    const uint32_t tSw = tS + 64 * wg + lane_base, tDw = tSw + 32;
+    const uint32_t mine = chain + 8 * (4 * wg + (warp & 3)), behind = chain + 8 * (4 * ((wg + 3) & 3) + (warp & 3));
+    const float* sBehind = sG + 128 * ((wg + 3) & 3) + row;
+    // demand of the thread's key in front of slice i (exclusive of its first query): the stored checkpoint of that 32-row block
+    // (past the end: any value.  Queries behind the last one are rows of zeros in Q, dO' and dbar': their bids multiply zeros, and
+    // what they add to a demand no query in front of them sees)
+    const int rb = 2 * hl + 1 - wg;                            // of the warpgroup's first slice; four less for every other
+    const float* edge = carry + ((int64_t)n * ncb + rb) * g.tk + ja;
+    float incl = 0.f;
+    if (!dead && wg < 2 * nh) incl = rb < ncb ? *edge : total[(int64_t)n * g.tk + ja];
+    for (int i = wg; i < 2 * nh; i += 4) {
+      const int u = i >> 1, q0 = (hl - u) * 64 + ((i & 1) ? 0 : 32);
+      float incl_next = 0.f;                                   // read once, from a buffer far larger than L2
+      edge -= 4 * (int64_t)g.tk;
+      if (!dead && i + 4 < 2 * nh) incl_next = *edge;
+      const float4* Dbar4 = reinterpret_cast<const float4*>(sDbar + 64 * (u & 3) + ((i & 1) ? 0 : 32));
+      mbar_wait(sdone + 8 * wg, (i >> 2) & 1, ctl, &g_status, kErrWaitMma);
+      tc_fence_after();
+      float p[32], inv[32];
+      tmem_ld32(tSw, p);
+      tmem_ld_wait(p);
+      if (dead || q0 < k0 + kTileRows - 1) bids_and_inverses<SHARE, true>(p, inv, incl + g.eps, g, dead, ja - q0);
+      else bids_and_inverses<SHARE, false>(p, inv, incl + g.eps, g, dead, ja - q0);
+      __syncwarp();
+      float suffix = 0.f;                                      // of the slice alone
+#pragma unroll
+      for (int c = 1; c >= 0; --c) {
+        float vd[16];
+        uint32_t shp[8];
+        tmem_ld16(tDw + 16 * c, vd);
+        tmem_ld_wait16(vd);
+        suffix_of_eight<SHARE>(p + 16 * c + 8, inv + 16 * c + 8, vd + 8, Dbar4 + 4 * c + 2, suffix, shp + 4);
+        suffix_of_eight<SHARE>(p + 16 * c, inv + 16 * c, vd, Dbar4 + 4 * c, suffix, shp);
+        tmem_st8(tSw + 8 * c, shp);
+      }
+      float base = 0.f;                                        // the suffix behind the slice: dp is linear in it
+      if (i > 0) {
+        mbar_wait(behind, ((i - 1) >> 2) & 1, ctl, &g_status, kErrWaitTile);
+        base = *sBehind;
+      }
+      sG[128 * wg + row] = base + suffix;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(mine);
+      uint32_t pdt[16];
+#pragma unroll
+      for (int e = 0; e < 32; e += 2) {
+        const float2 pd2 = fma2(make_float2(p[e], p[e + 1]), make_float2(base, base), make_float2(inv[e], inv[e + 1]));
+        pdt[e >> 1] = pack_bf16(pd2.x, pd2.y);
+      }
+      // the products of half tile u - 2 have read the pdp buffer that is written next
+      if (u >= 2) mbar_wait(dqdone + 8 * (u & 1), ((u >> 1) - 1) & 1, ctl, &g_status, kErrWaitMma);
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sPd + kTileBytes * (u & 1) +
+                                                                      share_chunk_offset(row, ((i & 1) ? 0 : 32) + 8 * c)),
+                     "r"(pdt[4 * c]), "r"(pdt[4 * c + 1]), "r"(pdt[4 * c + 2]), "r"(pdt[4 * c + 3])
+                     : "memory");
+      tmem_st16(tDw, pdt);
+      incl = incl_next;
+      tmem_st_wait();
+      fence_async_smem();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(tiles + 8 * wg);
+    }
+  }
+  mbar_wait(fin, 0, ctl, &g_status, kErrWaitMma);
+  __syncwarp();
+  tc_fence_after();
+  if (wg < 4) {
+    // lane = key: each warpgroup stores 16 of the 64 columns of dk_main and dv
+    float a[16], b[16];
+    const int64_t o = ((int64_t)n * g.tk + ja) * kHeadDim + 16 * wg;
+    tmem_ld16(tDK + lane_base + 16 * wg, a);
+    tmem_ld16(tDV + lane_base + 16 * wg, b);
+    tmem_ld_wait16(a);
+    tmem_ld_wait16(b);
+    if (!dead) {
+#pragma unroll
+      for (int e = 0; e < 16; e += 4)
+        *reinterpret_cast<float4*>(dk_main + o + e) =
+            make_float4(a[e] * g.scale, a[e + 1] * g.scale, a[e + 2] * g.scale, a[e + 3] * g.scale);
+#pragma unroll
+      for (int e = 0; e < 16; e += 8)
+        *reinterpret_cast<uint4*>(dv + o + e) =
+            make_uint4(pack_bf16(b[e], b[e + 1]), pack_bf16(b[e + 2], b[e + 3]), pack_bf16(b[e + 4], b[e + 5]),
+                       pack_bf16(b[e + 6], b[e + 7]));
+    }
+  }
+  drain_if_aborted(ctl);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_free(tmem, 512);
+}
+
 // Barrier of the 128 threads of one warpgroup (named barriers 1 and 2).
 __device__ __forceinline__ void wg_barrier(int wg) {
   if (wg == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -2163,14 +2570,32 @@ inline int backward(const void* q, const void* k, const void* v, const Geom& g, 
   if (g.carry_rows == 32) {
     constexpr int smem_bwd = kBwdSmem;
     static_assert(smem_bwd <= 232448 && 2 * smem_bwd > 233472, "the backward main pass runs one CTA per SM");
-    mark("tc_backward_main", st, 0);
     const unsigned grid = (unsigned)(g.n * nkb);
-    DIL_TC_PLAIN_BID(g, DIL_TC_SHARE(g, {
-      if (int rc = set_smem_attr((const void*)backward_main_kernel<BID, SHARE>, smem_bwd, err, errlen, kBwdRegs)) return rc;
-      backward_main_kernel<BID, SHARE><<<grid, kBwdThreads, smem_bwd, st>>>(
-          mq, mk, md, mdq, g, (const __nv_bfloat16*)v, rmax, rden, dbarp, carry, total, dq_main, dk_main,
-          (__nv_bfloat16*)dv, ghat);
-    }))
+    const bool slices = g.bid == kBidSigmoid && g.share != kShareNone && g.tq >= kSliceFrom;
+    if (slices) {
+      CUtensorMap mq64, md64, mdq64;
+      if (int rc = make_map(&mq64, q, g.n, g.tq, err, errlen, kHeadDim, 64)) return rc;
+      if (int rc = make_map(&md64, dop, g.n, g.tq, err, errlen, kHeadDim, 64)) return rc;
+      if (int rc = make_map_f32(&mdq64, dq_main, g.n, g.tq, err, errlen, kHeadDim, 64, false)) return rc;
+      if (((uintptr_t)k | (uintptr_t)v) & 15) {
+        snprintf(err, errlen, "bf16 tensor-core path needs 16-byte aligned q/k/v");
+        return 1;
+      }
+      static_assert(kSliceSmem <= 232448 && 2 * kSliceSmem > 233472, "the main reverse pass runs one CTA per SM");
+      auto kern = g.share == kShareInclusive ? backward_slices_kernel<kShareInclusive> : backward_slices_kernel<kShareExclusive>;
+      if (int rc = set_smem_attr((const void*)kern, kSliceSmem, err, errlen, kSliceRegs)) return rc;
+      mark("tc_backward_main", st, 0);
+      kern<<<grid, kSliceThreads, kSliceSmem, st>>>(mq64, mk, md64, mdq64, g, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, dbarp,
+                                                    carry, total, dk_main, (__nv_bfloat16*)dv);
+    } else {
+      mark("tc_backward_main", st, 0);
+      DIL_TC_PLAIN_BID(g, DIL_TC_SHARE(g, {
+        if (int rc = set_smem_attr((const void*)backward_main_kernel<BID, SHARE>, smem_bwd, err, errlen, kBwdRegs)) return rc;
+        backward_main_kernel<BID, SHARE><<<grid, kBwdThreads, smem_bwd, st>>>(
+            mq, mk, md, mdq, g, (const __nv_bfloat16*)v, rmax, rden, dbarp, carry, total, dq_main, dk_main,
+            (__nv_bfloat16*)dv, ghat);
+      }))
+    }
     mark("tc_backward_main", st, 1);
   } else {
     snprintf(err, errlen, "the tensor-core backward needs checkpoints every 32 query rows (got %d)", g.carry_rows);
