@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) rowpass_product_ker
   if (warp == 0) tmem_free(tmem, kTmem);
 }
 
-// The same of bf16 heads of 64 where there are many blocks (kPairsFrom): two query tiles of 128 per CTA, one per compute warpgroup (lane
+// The same where there are long rows and many blocks (row_pairs; wide rows kWidePairsFrom): two query tiles of 128 per CTA, one per compute warpgroup (lane
 // = query, so that a row's sums and output need no merge), and a ninth warp that issues every TMA copy and MMA.  The keys come in
 // half tiles of 64: S = Q K^T (N = 64) and O take 128 TMEM columns of a warpgroup, P~ goes over the scores that were read, and two
 // CTAs give a scheduler four warps in four phases.  The issuing warp serves a warpgroup's P~ B and, behind it in the pipe, its next
@@ -336,20 +336,22 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) rowpass_product_ker
 // grid = n * ceil(tq/256), longest rows first.
 constexpr int kRowRing = 4;                           // half tiles of K (and V)
 constexpr int kRowThreads = 288;
-template <int MODE> constexpr int kRowSmem = 2 * (int)kTileBytes + kRowRing * MODE * (int)kTileBytes / 2 + 256 + 1024;
+template <int MODE, int W = kNarrow> constexpr int kRowSmem = (2 + kRowRing * MODE / 2) * (int)Rows<W>::kBytes + 256 + 1024;
 
-template <int MODE, typename TOut>
-__global__ void __launch_bounds__(kRowThreads, 2) rowpass_tiles_kernel(
+template <int MODE, typename TOut, int W = kNarrow>
+__global__ void __launch_bounds__(kRowThreads, W == kNarrow ? 2 : 1) rowpass_tiles_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, Geom g, float* __restrict__ rmax, float* __restrict__ rden,
     TOut* __restrict__ out) {
   static_assert(MODE == 1 || MODE == 2, "1: B = K (pk); 2: B = V (softmax attention)");
   constexpr int R = kRowRing;
-  constexpr uint32_t HB = kTileBytes / 2;
+  constexpr uint32_t TB = Rows<W>::kBytes, HB = TB / 2, HSub = kTileBytes / 2;    // a tile, half a tile, a sub-tile of that
+  constexpr int kAcc = Rows<W>::kCols, kWg = 64 + kAcc;                            // TMEM columns of O, and of a warpgroup
+  constexpr int kTmem = W == kNarrow ? 256 : 512;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
-  const uint32_t sQ = smem_u32(smem), sK = sQ + 2 * kTileBytes, sB = MODE == 2 ? sK + R * HB : sK;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 2 * kTileBytes + MODE * R * HB);
+  const uint32_t sQ = smem_u32(smem), sK = sQ + 2 * TB, sB = MODE == 2 ? sK + R * HB : sK;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 2 * TB + MODE * R * HB);
   const uint32_t qfull = smem_u32(bars), kfull = qfull + 8, kfree = kfull + 8 * R, sdone = kfree + 8 * R, pready = sdone + 16;
   Ctl* ctl = reinterpret_cast<Ctl*>(bars + 5 + 2 * R);
 
@@ -373,7 +375,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) rowpass_tiles_kernel(
     fence_barrier_init();
   }
   __syncwarp();
-  if (warp == 0) tmem_alloc(smem_u32(&ctl->tmem), 256);
+  if (warp == 0) tmem_alloc(smem_u32(&ctl->tmem), kTmem);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -381,18 +383,18 @@ __global__ void __launch_bounds__(kRowThreads, 2) rowpass_tiles_kernel(
 
   if (warp_u == 8) {
     // ------------------------------------------------------------ the issuing warp
-    constexpr uint32_t id_s = instr_desc(128, 64, 0, 0), id_p = instr_desc(128, 64, 0, 1);
-    const Desc dQ = make_desc(sQ, 16, 1024), dK = make_desc(sK, 16, 1024), dB = make_desc(sB, kTileBytes, 1024);
+    constexpr uint32_t id_s = instr_desc(128, 64, 0, 0), id_p = instr_desc(128, kAcc, 0, 1);
+    const Desc dQ = make_desc(sQ, 16, 1024), dK = make_desc(sK, 16, 1024), dB = make_desc(sB, HSub, 1024);
     auto load_keys = [&](int h) {
       const int st = h % R;
       if (!lead) return;
       mbar_expect_tx(kfull + 8 * st, MODE * HB);
-      tma_load_tile(sK + HB * st, &map_k, h * 64, n, kfull + 8 * st);
-      if (MODE == 2) tma_load_tile(sB + HB * st, &map_v, h * 64, n, kfull + 8 * st);
+      tma_load_rows<W>(sK + HB * st, &map_k, h * 64, n, kfull + 8 * st, HSub);
+      if (MODE == 2) tma_load_rows<W>(sB + HB * st, &map_v, h * 64, n, kfull + 8 * st, HSub);
     };
     if (lead) {
-      mbar_expect_tx(qfull, (nh1 > 0 ? 2 : 1) * kTileBytes);
-      for (int w = 0; w < (nh1 > 0 ? 2 : 1); ++w) tma_load_tile(sQ + kTileBytes * w, &map_q, (t0 + w) * kTileRows, n, qfull);
+      mbar_expect_tx(qfull, (nh1 > 0 ? 2 : 1) * TB);
+      for (int w = 0; w < (nh1 > 0 ? 2 : 1); ++w) tma_load_rows<W>(sQ + TB * w, &map_q, (t0 + w) * kTileRows, n, qfull);
     }
     for (int h = 0; h < R && h < nh; ++h) load_keys(h);
     mbar_wait_warp(qfull, 0, ctl, &g_status, kErrWaitTma);
@@ -401,18 +403,19 @@ __global__ void __launch_bounds__(kRowThreads, 2) rowpass_tiles_kernel(
       for (int w = 0; w < 2; ++w) {
         const int nw = w ? nh1 : nh0;
         if (h > nw || nw == 0) continue;
-        const uint32_t tS = tmem + 128 * w;
+        const uint32_t tS = tmem + kWg * w;
         if (h > 0) {
           mbar_wait_warp(pready + 8 * w, (h - 1) & 1, ctl, &g_status, kErrWaitTile);
           tc_fence_after();
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk)                          // 16 keys per instruction: 16 rows of 128 B = 128 units
-            mma_ts(lead, tS + 64, tS + 8 * kk, dB, (HB >> 4) * ((h - 1) % R) + 128 * kk, id_p, h > 1 || kk > 0);
+          for (int pl = 0; pl < Rows<W>::kPlanes; ++pl)
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)                        // 16 keys per instruction: 16 rows of 128 B = 128 units
+              mma_ts(lead, tS + 64, tS + 32 * pl + 8 * kk, dB, (HB >> 4) * ((h - 1) % R) + 128 * kk, id_p, h > 1 || pl > 0 || kk > 0);
         }
         if (h < nw) {
           tc_fence_after();
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk) mma_ss(lead, tS, dQ, 1024 * w + 2 * kk, dK, (HB >> 4) * (h % R) + 2 * kk, id_s, kk > 0);
+          mma_scores_wide<W>(lead, tS, Desc{dQ.lo + (TB >> 4) * w, dQ.hi}, kTileBytes, Desc{dK.lo + (HB >> 4) * (h % R), dK.hi}, HSub, id_s);
         }
         mma_commit(lead, sdone + 8 * w);                          // P~ B of h - 1 and the scores of h
       }
@@ -425,7 +428,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) rowpass_tiles_kernel(
     __syncwarp();
   } else {
     // ------------------------------------------------------------ the compute warps: lane = query
-    const uint32_t tS = tmem + 128 * wg + ((uint32_t)((warp & 3) * 32) << 16), tO = tS + 64;
+    const uint32_t tS = tmem + kWg * wg + ((uint32_t)((warp & 3) * 32) << 16), tO = tS + 64;
     const int nw = wg ? nh1 : nh0, i = (t0 + wg) * kTileRows + row, q0 = g.q_off + (t0 + wg) * kTileRows, ia = q0 + row;
     float m_ref = -INFINITY, s = 0.f;
     for (int h = 0; h < nw; ++h) {
@@ -437,7 +440,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) rowpass_tiles_kernel(
       tmem_ld32(tS + 32, v + 32);
       tmem_ld_wait(v);
       tmem_ld_wait(v + 32);
-      uint32_t pw[32];
+      uint32_t pw[32], pr[Rows<W>::kPlanes == 2 ? 32 : 1];
       float ps = 0.f;
       // P~ = 2^(z - reference) for the thread's 64 scores, two per instruction; their sum in ps
       auto exponentials = [&]() {
@@ -454,13 +457,18 @@ __global__ void __launch_bounds__(kRowThreads, 2) rowpass_tiles_kernel(
           acc1 = add2(acc1, p1);
           pw[e >> 1] = pack_bf16(p0.x, p0.y);
           pw[(e >> 1) + 1] = pack_bf16(p1.x, p1.y);
+          if (Rows<W>::kPlanes == 2) {
+            pr[e >> 1] = pack_bf16_rest(p0.x, p0.y, pw[e >> 1]);
+            pr[(e >> 1) + 1] = pack_bf16_rest(p1.x, p1.y, pw[(e >> 1) + 1]);
+          }
         }
         const float2 acc = add2(acc0, acc1);
         ps = acc.x + acc.y;
       };
       // (the reference, the common half tile and the slow path are those of rowpass_product_kernel)
       const bool edge = (h * 64 + 63 > q0) || ((h + 1) * 64 > g.tk);
-      bool slow = edge || __any_sync(0xffffffffu, m_ref == -INFINITY);
+      // (the first 128 keys set the reference, as there: the largest P~ is then 1 more often, which bf16 holds exactly)
+      bool slow = edge || h < 2 || __any_sync(0xffffffffu, m_ref == -INFINITY);
       if (!slow) {
         exponentials();
         slow = __any_sync(0xffffffffu, !(ps < kRefLimit));
@@ -485,7 +493,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) rowpass_tiles_kernel(
           const float f = fast_exp2(m_ref - (m_new == -INFINITY ? 0.f : m_new));
           if (!fresh && h > 0) {
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
+            for (int c = 0; c < kAcc / 16; ++c) {
               float o[16];
               tmem_ld16(tO + 16 * c, o);
               tmem_ld_wait16(o);
@@ -501,9 +509,13 @@ __global__ void __launch_bounds__(kRowThreads, 2) rowpass_tiles_kernel(
         exponentials();
       }
       s += ps;
-      // over the first 32 of the 64 scores: keys 2c, 2c+1 in column c
+      // over the first 32 of the 64 scores: keys 2c, 2c+1 in column c (the lo plane over the others)
       tmem_st16(tS, pw);
       tmem_st16(tS + 16, pw + 16);
+      if (Rows<W>::kPlanes == 2) {
+        tmem_st16(tS + 32, pr);
+        tmem_st16(tS + 48, pr + 16);
+      }
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -515,15 +527,23 @@ __global__ void __launch_bounds__(kRowThreads, 2) rowpass_tiles_kernel(
       __syncwarp();
       const float inv = (MODE == 1 ? g.scale : 1.f) / s;
       __syncwarp();                                           // (a division has paths of its own for NaN and the like)
-      TOut* dst = out + ((int64_t)n * g.tq + i) * kHeadDim;
+      const int d = W == kSplit ? g.d : Rows<W>::kHead;
+      TOut* dst = out + ((int64_t)n * g.tq + i) * d;
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
+      for (int c = 0; c < Rows<W>::kHead / 32; ++c) {
         float o[32];
         tmem_ld32(tO + 32 * c, o);
         tmem_ld_wait(o);
+        if (W == kSplit) {                                    // P~ K_hi + P~ K_lo
+          float lo[32];
+          tmem_ld32(tO + 64 + 32 * c, lo);
+          tmem_ld_wait(lo);
+#pragma unroll
+          for (int e = 0; e < 32; ++e) o[e] += lo[e];
+        }
 #pragma unroll
         for (int e = 0; e < 32; ++e) o[e] *= inv;
-        if (i < g.tq) store_row32<kNarrow>(dst + 32 * c, o, 32);
+        if (i < g.tq) store_row32<W>(dst + 32 * c, o, d - 32 * c);
       }
       if (i < g.tq && rmax != nullptr) {
         // the reference, not necessarily the row maximum (it lags behind it by design); every consumer uses the pair only as
@@ -536,7 +556,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) rowpass_tiles_kernel(
   drain_if_aborted(ctl);
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_free(tmem, 256);
+  if (warp == 0) tmem_free(tmem, kTmem);
 }
 
 // Key half of the softmax-Jacobian correction alone (the reference's BC, kernels.py:777-809),
@@ -749,14 +769,14 @@ __global__ void dq_from_pk_kernel(const float* __restrict__ dq_main, const float
 }
 
 // ---------------------------------------------------------------- host launchers
-// Pairs of query tiles from which a row pass takes rowpass_tiles_kernel.  Two CTAs of two tiles each want 296 of them at a time, and a
-// CTA takes twice the tiles of one of rowpass_product_kernel, whose warpgroups share a row's keys: on a chip that is not full that one
-// is done sooner.  Row pass with pk, one tile / pairs, in us: n = 64, T = 16384 (4096 pairs) 3134 / 2681; n = 128, T = 2048 (1024)
-// 131 / 125; n = 384, T = 1024 (1536) 128.7 / 128.2; n = 32, T = 4096 (512) 111.1 / 111.0; n = 16, T = 1777 (112) 24 / 36.
-// Softmax: n = 64, T = 8192 (2048) 805 / 732; n = 64, T = 4096 (1024) 211 / 197; n = 4, T = 32768 (512) 714 / 691; n = 64, T = 1024
-// (256) 27.5 / 28.8; n = 2, T = 3000 (24) 33 / 51.
-constexpr int64_t kPairsFrom = 512;
+// Which row passes take rowpass_tiles_kernel: long rows and many pairs of query tiles.  Two CTAs of two tiles each want 296 pairs at a
+// time, and a CTA takes twice the tiles of one of rowpass_product_kernel, whose warpgroups share a row's keys: on a chip that is not
+// full that one is done sooner, and short rows are mostly slow steps.  Row pass with pk, one tile / pairs, in us: n = 64, T = 16384
+// (4096 pairs) 3221 / 2858; n = 128, T = 2048 (1024) 130.8 / 129.1; n = 32, T = 4096 (512) 111 / 114; n = 384, T = 1024 (1536) 129 / 133;
+// n = 16, T = 1777 (112) 24 / 36.  Softmax: n = 64, T = 8192 (2048) 837 / 759; n = 64, T = 4096 (1024) 215 / 210; n = 128, T = 2048
+// (1024) 123 / 121; n = 64, T = 1024 (256) 27.5 / 28.8; n = 2, T = 3000 (24) 33 / 51.
 inline int64_t tile_pairs(const Geom& g) { return g.n * ((g.tq + 2 * kTileRows - 1) / (2 * kTileRows)); }
+inline bool row_pairs(const Geom& g) { return g.tq >= 2048 && tile_pairs(g) >= 1024; }
 
 // Pass 1 with the saved query correction: rmax, rden and pk = scale * softmax(q k^T) k.
 inline int rowstats_pk(const void* q, const void* k, const Geom& g, float* rmax, float* rden, float* pk,
@@ -764,8 +784,8 @@ inline int rowstats_pk(const void* q, const void* k, const Geom& g, float* rmax,
   CUtensorMap mq, mk;
   const int64_t pairs = tile_pairs(g);
   if (int rc = make_map(&mq, q, g.n, g.tq, err, errlen)) return rc;
-  if (int rc = make_map(&mk, k, g.n, g.tk, err, errlen, kHeadDim, pairs >= kPairsFrom ? 64 : kTileRows)) return rc;
-  if (pairs >= kPairsFrom) {
+  if (int rc = make_map(&mk, k, g.n, g.tk, err, errlen, kHeadDim, row_pairs(g) ? 64 : kTileRows)) return rc;
+  if (row_pairs(g)) {
     auto kern = rowpass_tiles_kernel<1, float>;
     constexpr int smem = kRowSmem<1> > kTwoPerSm ? kRowSmem<1> : kTwoPerSm;
     if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
@@ -791,11 +811,11 @@ inline int softmax_forward(const void* q, const void* k, const void* v, const Ge
                            float* rden, void* out, cudaStream_t st, char* err, size_t errlen) {
   CUtensorMap mq, mk, mv;
   const int64_t pairs = tile_pairs(g);
-  const int key_rows = pairs >= kPairsFrom ? 64 : kTileRows;
+  const int key_rows = row_pairs(g) ? 64 : kTileRows;
   if (int rc = make_map(&mq, q, g.n, g.tq, err, errlen)) return rc;
   if (int rc = make_map(&mk, k, g.n, g.tk, err, errlen, kHeadDim, key_rows)) return rc;
   if (int rc = make_map(&mv, v, g.n, g.tk, err, errlen, kHeadDim, key_rows)) return rc;
-  if (pairs >= kPairsFrom) {
+  if (row_pairs(g)) {
     auto kern = rowpass_tiles_kernel<2, __nv_bfloat16>;
     constexpr int smem = kRowSmem<2>;
     static_assert(2 * (smem + 1024) <= 233472 && 3 * (smem + 1024) > 233472, "two CTAs of the softmax pass fit one SM");

@@ -20,8 +20,8 @@ def _exact(q, k, v, row):
     return torch.softmax(z, -1), torch.logsumexp(z, -1)
 
 
-# rows x pairs of tiles: 512 of them and more; one less takes the kernel of single tiles
-@pytest.mark.parametrize("rows,seq", [(512, 1), (512, 64), (512, 127), (512, 129), (256, 257), (171, 513), (128, 1000), (511, 200)])
+# 1024 pairs of tiles and rows of 2048 tokens and more; one row less, or one token, takes the kernel of single tiles
+@pytest.mark.parametrize("rows,seq", [(128, 2048), (127, 2048), (128, 2047), (114, 2049), (114, 2111), (114, 2177), (103, 2433)])
 @pytest.mark.parametrize("std", [1.0, 24.0])
 def test_row_pass_against_64_bits(rows, seq, std):
     pkg = load_package()
@@ -46,3 +46,37 @@ def test_row_pass_against_64_bits(rows, seq, std):
         assert ((pk[row].double() - ref).abs() <= bound * size + 1e-6).all()
         got = (stats[0, row].double() + torch.log2(stats[1, row].double())) * math.log(2)
         assert ((got - lse).abs() <= 2e-6 * lse.abs().clamp(min=1.0) + 2e-6).all()
+
+
+# rows of 256 bytes: bf16 heads of 128, fp32 heads as hi + lo planes; 148 pairs of tiles and one less
+@pytest.mark.parametrize("rows,seq", [(148, 100), (74, 257), (148, 129), (50, 700), (147, 100)])
+@pytest.mark.parametrize("dtype,d", [(torch.bfloat16, 128), (torch.float32, 64), (torch.float32, 32)])
+@pytest.mark.parametrize("std", [1.0, 24.0])
+def test_wide_row_pass_against_64_bits(rows, seq, dtype, d, std):
+    pkg = load_package()
+    lib, L = pkg._lib.load(), pkg._lib
+    g = torch.Generator(device=DEV).manual_seed(rows + seq + d)
+    q, k, v = (torch.randn(rows, seq, d, device=DEV, generator=g) for _ in range(3))
+    q, k, v = (q * std).to(dtype), k.to(dtype), v.to(dtype)
+    st = torch.cuda.current_stream().cuda_stream
+    code, ops = L.BF16, (q, k, v)
+    if dtype == torch.float32:
+        code, ops = L.F32, tuple(torch.empty(rows, seq, 128, device=DEV, dtype=torch.bfloat16) for _ in range(3))
+        L.check(lib.dilution_split_operands(*(x.data_ptr() for x in (q, k, v)), rows * seq, d, *(x.data_ptr() for x in ops), st), "split")
+    f32 = dict(device=DEV, dtype=torch.float32)
+    rmax, rden, total, ssum = (torch.empty(rows, seq, **f32) for _ in range(4))
+    carry, out, pk = torch.empty(rows, (seq + 31) // 32, seq, **f32), torch.empty(rows, seq, d, **f32), torch.empty(rows, seq, d, **f32)
+    scale = d ** -0.5
+    L.check(lib.dilution_wide_forward(*(x.data_ptr() for x in ops), code, rows, seq, d, scale, 1e-9,
+                                      *(x.data_ptr() for x in (rmax, rden, carry, total, out, ssum, pk)), st), "wide forward")
+    for row in (0, rows - 1):
+        z = (q[row].double() @ k[row].double().T) * scale
+        size = (q[row].double().abs() @ k[row].double().abs().T) * scale
+        z = z.masked_fill(torch.ones_like(z, dtype=torch.bool).triu(1), float("-inf"))
+        p, lse = torch.softmax(z, -1), torch.logsumexp(z, -1)
+        # operands keep 16 bits as pairs (exact in bf16), so a score is off by 2^-16 of the sum of its terms' sizes, and P~ by that and 2^-16
+        off = (2.0 ** -16 * size).amax(-1) if dtype == torch.float32 else torch.zeros_like(lse)
+        got = (rmax[row].double() + torch.log2(rden[row].double())) * math.log(2)
+        assert ((got - lse).abs() <= off + 2e-6 * lse.abs().clamp(min=1.0) + 2e-6).all()
+        ref, width = scale * (p @ k[row].double()), scale * (p @ k[row].double().abs())
+        assert ((pk[row].double() - ref).abs() <= (2 * off[:, None] + 2.0 ** -14) * width + 1e-6).all()
