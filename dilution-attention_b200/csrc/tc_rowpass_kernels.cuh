@@ -31,30 +31,204 @@ namespace dil {
 namespace tc {
 
 constexpr float kRefLimit = 1099511627776.f;         // 2^40: a tile whose P~ sum to more moves the reference
-template <int MODE, int W = kNarrow> struct RowpassSmem {
+template <int MODE> struct RowpassSmem {
   // Q | K[stages] | (V[stages]) | stats [2][128] float4 | barriers + control.  Three stages when
   // K is the only streamed operand; two of K and two of V otherwise, so that two CTAs fit an SM.
   static constexpr int kStages = MODE == 2 ? 2 : 3;
   static constexpr int kTiles = 1 + kStages * (MODE == 2 ? 2 : 1);
-  static constexpr int kBytes = kTiles * (int)Rows<W>::kBytes + 4096 + 256 + 1024;
+  static constexpr int kBytes = kTiles * (int)kTileBytes + 4096 + 256 + 1024;
 };
 
+// One step of a warpgroup of a row pass (lane = query): the 64 scores of keys first_key and on at tS, of which it forms P~ over the
+// scores it has read (keys 2c, 2c+1 in column c, two planes: the lo plane over the other 32), and the sums.  tO: its accumulator;
+// ia: the lane's query; edge: some of the keys are masked for some of the tile's queries.
+template <int W>
+__device__ __forceinline__ void row_half_tile(uint32_t tS, uint32_t tO, const Geom& g, int first_key, int ia, bool edge, float& m_ref,
+                                              float& s) {
+  constexpr int kAcc = Rows<W>::kCols;
+  float v[64];
+  tmem_ld32(tS, v);
+  tmem_ld32(tS + 32, v + 32);
+  tmem_ld_wait(v);
+  tmem_ld_wait(v + 32);
+  uint32_t pw[32], pr[Rows<W>::kPlanes == 2 ? 32 : 1];
+  float ps = 0.f;
+  // P~ = 2^(z - reference) for the thread's 64 scores, two per instruction; their sum in ps
+  auto exponentials = [&]() {
+    const float mr = m_ref == -INFINITY ? 0.f : m_ref;
+    const float2 zs = make_float2(g.zscale, g.zscale), off = make_float2(-mr, -mr);
+    float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int e = 0; e < 64; e += 4) {
+      const float2 z0 = fma2(make_float2(v[e], v[e + 1]), zs, off);
+      const float2 z1 = fma2(make_float2(v[e + 2], v[e + 3]), zs, off);
+      const float2 p0 = make_float2(fast_exp2(z0.x), fast_exp2(z0.y));
+      const float2 p1 = make_float2(fast_exp2(z1.x), fast_exp2(z1.y));
+      acc0 = add2(acc0, p0);
+      acc1 = add2(acc1, p1);
+      pw[e >> 1] = pack_bf16(p0.x, p0.y);
+      pw[(e >> 1) + 1] = pack_bf16(p1.x, p1.y);
+      if (Rows<W>::kPlanes == 2) {
+        pr[e >> 1] = pack_bf16_rest(p0.x, p0.y, pw[e >> 1]);
+        pr[(e >> 1) + 1] = pack_bf16_rest(p1.x, p1.y, pw[(e >> 1) + 1]);
+      }
+    }
+    const float2 acc = add2(acc0, acc1);
+    ps = acc.x + acc.y;
+  };
+  // The common tile takes no maximum at all: the reference stays where it is as long as the
+  // tile's sum of P~ stays below 2^40 (then every P~ does, and nothing overflowed).
+  // Edge tiles (masking), rows that have not seen a score yet and tiles that outgrow the
+  // reference take the slow path: mask, take the tile's maximum, move the reference there,
+  // rescale what was accumulated under the old one, and form P~ again.
+  bool slow = edge || __any_sync(0xffffffffu, m_ref == -INFINITY);
+  if (!slow) {
+    exponentials();
+    slow = __any_sync(0xffffffffu, !(ps < kRefLimit));
+    if (slow) {                      // rare: the scores are still in TMEM, fetch them again
+      tmem_ld32(tS, v);
+      tmem_ld32(tS + 32, v + 32);
+      tmem_ld_wait(v);
+      tmem_ld_wait(v + 32);
+    }
+  }
+  if (slow) {
+    float cmax = -INFINITY;
+    if (edge) {
+#pragma unroll
+      for (int e = 0; e < 64; ++e) {
+        const int ja = first_key + e;
+        if (ja > ia || ja >= g.tk) v[e] = -INFINITY;
+        cmax = fmaxf(cmax, v[e]);
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 64; ++e) cmax = fmaxf(cmax, v[e]);
+    }
+    const float m_new = fmaxf(m_ref, cmax * g.zscale);
+    if (__any_sync(0xffffffffu, m_new != m_ref)) {
+      const bool fresh = __all_sync(0xffffffffu, m_ref == -INFINITY);   // nothing accumulated yet
+      // (no branch: the TMEM loads below are warp-wide; a row without a reference has nothing but zeros or NaN yet)
+      const float f = fast_exp2(m_ref - (m_new == -INFINITY ? 0.f : m_new));
+      if (!fresh) {
+#pragma unroll
+        for (int c = 0; c < kAcc / 16; ++c) {
+          float o[16];
+          tmem_ld16(tO + 16 * c, o);
+          tmem_ld_wait16(o);
+          uint32_t w[16];
+#pragma unroll
+          for (int e = 0; e < 16; ++e) w[e] = __float_as_uint(o[e] * f);
+          tmem_st16(tO + 16 * c, w);
+        }
+      }
+      s *= f;
+      m_ref = m_new;
+    }
+    exponentials();
+  }
+  s += ps;
+  tmem_st16(tS, pw);
+  tmem_st16(tS + 16, pw + 16);
+  if (Rows<W>::kPlanes == 2) {
+    tmem_st16(tS + 32, pr);
+    tmem_st16(tS + 48, pr + 16);
+  }
+  tmem_st_wait();
+}
+
+// The end of a row pass: the two warpgroups' halves of every row are merged.  Each finishes half of the output columns: it hands the
+// other half of its accumulator, with its statistics, to the other one through sX [2][128][half a row].  n, i: the lane's row and query;
+// sync: a barrier of the two.
+template <int MODE, int WG, int W, typename TOut, typename Sync>
+__device__ __forceinline__ void row_merge(uint32_t tO, const Geom& g, int n, int i, int row, float m_ref, float s, float4* sStat, float* sX,
+                                          float* __restrict__ rmax, float* __restrict__ rden, TOut* __restrict__ out, Sync sync) {
+  constexpr int kHalf = Rows<W>::kHead / 2;
+  // columns [base, base + 32) of this warpgroup's accumulator (kSplit: P K_hi + P K_lo)
+  auto fetch = [&](int base, float* o) {
+    __syncwarp();                                         // (rows behind the last query leave the loops below)
+    tmem_ld32(tO + base, o);
+    tmem_ld_wait(o);
+    if (W == kSplit) {
+      float lo[32];
+      tmem_ld32(tO + 64 + base, lo);
+      tmem_ld_wait(lo);
+#pragma unroll
+      for (int e = 0; e < 32; ++e) o[e] += lo[e];
+    }
+  };
+  sStat[WG * 128 + row] = make_float4(m_ref, s, 0.f, 0.f);
+  float* give = sX + ((1 - WG) * 128 + row) * kHalf;      // read by the other warpgroup
+#pragma unroll
+  for (int c0 = 0; c0 < kHalf; c0 += 32) {
+    float o[32];
+    fetch(kHalf * (1 - WG) + c0, o);
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      reinterpret_cast<float4*>(give + c0)[c ^ (row & 7)] = make_float4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
+  }
+  sync();
+  const float4 other = sStat[(1 - WG) * 128 + row];
+  const float m = fmaxf(m_ref, other.x);                  // finite: warpgroup 0 always sees key 0
+  const float ref = m == -INFINITY ? 0.f : m;
+  const float f_own = fast_exp2(m_ref - ref), f_oth = fast_exp2(other.x - ref);
+  const float den = s * f_own + other.y * f_oth;
+  const float inv = (MODE == 1 ? g.scale : 1.f) / den;
+  __syncwarp();                                           // (a division has paths of its own for NaN and the like)
+  const float a_own = f_own * inv, a_oth = f_oth * inv;
+  const float* take = sX + (WG * 128 + row) * kHalf;
+  const int d = W == kSplit ? g.d : Rows<W>::kHead;
+#pragma unroll
+  for (int c0 = 0; c0 < kHalf; c0 += 32) {
+    float r[32];
+    fetch(kHalf * WG + c0, r);
+    if (i >= g.tq) continue;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const float4 x = reinterpret_cast<const float4*>(take + c0)[c ^ (row & 7)];
+      r[4 * c] = r[4 * c] * a_own + x.x * a_oth;
+      r[4 * c + 1] = r[4 * c + 1] * a_own + x.y * a_oth;
+      r[4 * c + 2] = r[4 * c + 2] * a_own + x.z * a_oth;
+      r[4 * c + 3] = r[4 * c + 3] * a_own + x.w * a_oth;
+    }
+    TOut* dst = out + ((int64_t)n * g.tq + i) * d + kHalf * WG + c0;
+    if (std::is_same<TOut, float>::value) {
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        if (W != kSplit || kHalf * WG + c0 + 4 * c < d)
+          reinterpret_cast<float4*>(dst)[c] = make_float4(r[4 * c], r[4 * c + 1], r[4 * c + 2], r[4 * c + 3]);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        reinterpret_cast<uint4*>(dst)[c] =
+            make_uint4(pack_bf16(r[8 * c], r[8 * c + 1]), pack_bf16(r[8 * c + 2], r[8 * c + 3]),
+                       pack_bf16(r[8 * c + 4], r[8 * c + 5]), pack_bf16(r[8 * c + 6], r[8 * c + 7]));
+    }
+  }
+  if (WG == 0 && i < g.tq && rmax != nullptr) {
+    // the merged reference, not necessarily the row maximum (it lags behind it by design);
+    // every consumer uses the pair only as the log-sum-exp rmax + log2(rden)
+    rmax[(int64_t)n * g.tq + i] = m;
+    rden[(int64_t)n * g.tq + i] = den;
+  }
+}
+
 // ONE_POLLS: one lane of the issuing warp waits for the next tiles, the others behind it (kOnePollsAbove).
-template <int MODE, typename TOut, int W = kNarrow, bool ONE_POLLS = false>
-__global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) rowpass_product_kernel(
+template <int MODE, typename TOut, bool ONE_POLLS = false>
+__global__ void __launch_bounds__(256, 2) rowpass_product_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, Geom g, float* __restrict__ rmax, float* __restrict__ rden,
     TOut* __restrict__ out) {
   static_assert(MODE == 1 || MODE == 2, "1: B = K (pk); 2: B = V (softmax attention)");
-  constexpr uint32_t TB = Rows<W>::kBytes;
-  constexpr int kAcc = Rows<W>::kCols;               // accumulator columns of one warpgroup
-  constexpr int kTmem = W == kNarrow ? 256 : 512;
+  constexpr uint32_t TB = kTileBytes;
+  constexpr int kAcc = kHeadDim;                     // accumulator columns of one warpgroup
+  constexpr int kTmem = 256;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
   const uint32_t sQ = smem_u32(smem), sK0 = sQ + TB;
-  constexpr int kRowpassStages = RowpassSmem<MODE, W>::kStages;
+  constexpr int kRowpassStages = RowpassSmem<MODE>::kStages;
   const uint32_t sB0 = MODE == 2 ? sK0 + kRowpassStages * TB : sK0;
-  constexpr int kTiles = RowpassSmem<MODE, W>::kTiles;
+  constexpr int kTiles = RowpassSmem<MODE>::kTiles;
   float4* sStat = reinterpret_cast<float4*>(smem + kTiles * TB);            // [2][128]
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kTiles * TB + 4096);
   Ctl* ctl = reinterpret_cast<Ctl*>(bars + 8);
@@ -96,14 +270,14 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) rowpass_product_ker
   auto load_stage = [&](int jb) {          // thread 0: K (and V) tile jb into its ring slot
     const int st = jb % kRowpassStages;
     mbar_expect_tx(kfull + 8 * st, kStageTx);
-    tma_load_rows<W>(sK0 + TB * st, &map_k, jb * kTileRows, n, kfull + 8 * st);
-    if (MODE == 2) tma_load_rows<W>(sB0 + TB * st, &map_v, jb * kTileRows, n, kfull + 8 * st);
+    tma_load_tile(sK0 + TB * st, &map_k, jb * kTileRows, n, kfull + 8 * st);
+    if (MODE == 2) tma_load_tile(sB0 + TB * st, &map_v, jb * kTileRows, n, kfull + 8 * st);
   };
   if (tid == 0) {
     mbar_expect_tx(kfull, kStageTx + TB);
-    tma_load_rows<W>(sQ, &map_q, ib * kTileRows, n, kfull);
-    tma_load_rows<W>(sK0, &map_k, 0, n, kfull);
-    if (MODE == 2) tma_load_rows<W>(sB0, &map_v, 0, n, kfull);
+    tma_load_tile(sQ, &map_q, ib * kTileRows, n, kfull);
+    tma_load_tile(sK0, &map_k, 0, n, kfull);
+    if (MODE == 2) tma_load_tile(sB0, &map_v, 0, n, kfull);
     for (int jb = 1; jb < kRowpassStages && jb < njb; ++jb) load_stage(jb);
   }
   tc_fence_before();
@@ -112,14 +286,13 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) rowpass_product_ker
   if (warp_u == 0) {
     mbar_wait(kfull, 0, ctl, &g_status, kErrWaitTma);
     tc_fence_after();
-    mma_scores_w<W>(lead, tS, sQ, sK0, 128);
+    mma_scores_w<kNarrow>(lead, tS, sQ, sK0, 128);
     mma_commit(lead, sdone);
   }
   __syncwarp();
 
   float m_ref = -INFINITY, s = 0.f;
   const int ia = q0 + row;
-  const uint32_t taddr = tS + lane_base + 64 * wg;
   for (int jb = 0; jb < njb; ++jb) {
     const int st = jb % kRowpassStages;
     // scores of tile jb are ready, and the product of tile jb-1 has completed
@@ -128,98 +301,8 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) rowpass_product_ker
     if (tid == 0 && jb >= 1 && jb - 1 + kRowpassStages < njb)
       load_stage(jb - 1 + kRowpassStages);                          // the slot of tile jb-1 is free
     __syncwarp();
-    float v[64];
-    tmem_ld32(taddr, v);
-    tmem_ld32(taddr + 32, v + 32);
-    tmem_ld_wait(v);
-    tmem_ld_wait(v + 32);
-    uint32_t pw[32], pr[Rows<W>::kPlanes == 2 ? 32 : 1];
-    float ps = 0.f;
-    // P~ = 2^(z - reference) for the thread's 64 scores, two per instruction; their sum in ps
-    auto exponentials = [&]() {
-      const float mr = m_ref == -INFINITY ? 0.f : m_ref;
-      const float2 zs = make_float2(g.zscale, g.zscale), off = make_float2(-mr, -mr);
-      float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int e = 0; e < 64; e += 4) {
-        const float2 z0 = fma2(make_float2(v[e], v[e + 1]), zs, off);
-        const float2 z1 = fma2(make_float2(v[e + 2], v[e + 3]), zs, off);
-        const float2 p0 = make_float2(fast_exp2(z0.x), fast_exp2(z0.y));
-        const float2 p1 = make_float2(fast_exp2(z1.x), fast_exp2(z1.y));
-        acc0 = add2(acc0, p0);
-        acc1 = add2(acc1, p1);
-        pw[e >> 1] = pack_bf16(p0.x, p0.y);
-        pw[(e >> 1) + 1] = pack_bf16(p1.x, p1.y);
-        if (Rows<W>::kPlanes == 2) {
-          pr[e >> 1] = pack_bf16_rest(p0.x, p0.y, pw[e >> 1]);
-          pr[(e >> 1) + 1] = pack_bf16_rest(p1.x, p1.y, pw[(e >> 1) + 1]);
-        }
-      }
-      const float2 acc = add2(acc0, acc1);
-      ps = acc.x + acc.y;
-    };
-    // The common tile takes no maximum at all: the reference stays where it is as long as the
-    // tile's sum of P~ stays below 2^40 (then every P~ does, and nothing overflowed).
-    // Edge tiles (masking), rows that have not seen a score yet and tiles that outgrow the
-    // reference take the slow path: mask, take the tile's maximum, move the reference there,
-    // rescale what was accumulated under the old one, and form P~ again.
     const bool edge = (jb * kTileRows + kTileRows - 1 > q0) || ((jb + 1) * kTileRows > g.tk);
-    bool slow = edge || __any_sync(0xffffffffu, m_ref == -INFINITY);
-    if (!slow) {
-      exponentials();
-      slow = __any_sync(0xffffffffu, !(ps < kRefLimit));
-      if (slow) {                      // rare: the scores are still in TMEM, fetch them again
-        tmem_ld32(taddr, v);
-        tmem_ld32(taddr + 32, v + 32);
-        tmem_ld_wait(v);
-        tmem_ld_wait(v + 32);
-      }
-    }
-    if (slow) {
-      float cmax = -INFINITY;
-      if (edge) {
-#pragma unroll
-        for (int e = 0; e < 64; ++e) {
-          const int ja = jb * kTileRows + wg * 64 + e;
-          if (ja > ia || ja >= g.tk) v[e] = -INFINITY;
-          cmax = fmaxf(cmax, v[e]);
-        }
-      } else {
-#pragma unroll
-        for (int e = 0; e < 64; ++e) cmax = fmaxf(cmax, v[e]);
-      }
-      const float m_new = fmaxf(m_ref, cmax * g.zscale);
-      if (__any_sync(0xffffffffu, m_new != m_ref)) {
-        const bool fresh = __all_sync(0xffffffffu, m_ref == -INFINITY);   // nothing accumulated yet
-        // (no branch: the TMEM loads below are warp-wide; a row without a reference has nothing but zeros or NaN yet)
-        const float f = fast_exp2(m_ref - (m_new == -INFINITY ? 0.f : m_new));
-        if (!fresh) {
-#pragma unroll
-          for (int c = 0; c < kAcc / 16; ++c) {
-            float o[16];
-            tmem_ld16(tO + lane_base + 16 * c, o);
-            tmem_ld_wait16(o);
-            uint32_t w[16];
-#pragma unroll
-            for (int e = 0; e < 16; ++e) w[e] = __float_as_uint(o[e] * f);
-            tmem_st16(tO + lane_base + 16 * c, w);
-          }
-        }
-        s *= f;
-        m_ref = m_new;
-      }
-      exponentials();
-    }
-    s += ps;
-    // P~ goes over the first 32 of this thread's 64 consumed score columns: keys 2c, 2c+1 of the
-    // warpgroup's half in column c (two planes: the lo plane over the other 32)
-    tmem_st16(taddr, pw);
-    tmem_st16(taddr + 16, pw + 16);
-    if (Rows<W>::kPlanes == 2) {
-      tmem_st16(taddr + 32, pr);
-      tmem_st16(taddr + 48, pr + 16);
-    }
-    tmem_st_wait();
+    row_half_tile<kNarrow>(tS + lane_base + 64 * wg, tO + lane_base, g, jb * kTileRows + wg * 64, ia, edge, m_ref, s);
     tc_fence_before();
     __syncthreads();
     if (warp_u == 0) {
@@ -229,16 +312,14 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) rowpass_product_ker
 #pragma unroll
       for (int w = 0; w < 2; ++w)
 #pragma unroll
-        for (int pl = 0; pl < Rows<W>::kPlanes; ++pl)
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)      // 16 keys per instruction: 16 rows of 128 B = 128 units
-            mma_ts(lead, tmem + 128 + kAcc * w, tS + 64 * w + 32 * pl + 8 * kk, dB, 128 * (4 * w + kk), id_pv, 1);
+        for (int kk = 0; kk < 4; ++kk)        // 16 keys per instruction: 16 rows of 128 B = 128 units
+          mma_ts(lead, tmem + 128 + kAcc * w, tS + 64 * w + 8 * kk, dB, 128 * (4 * w + kk), id_pv, 1);
       if (jb + 1 < njb) {
         const int sn = (jb + 1) % kRowpassStages;
         if (!ONE_POLLS || (tid & 31) == 0) mbar_wait(kfull + 8 * sn, ((jb + 1) / kRowpassStages) & 1, ctl, &g_status, kErrWaitTma);
         if (ONE_POLLS) __syncwarp();
         tc_fence_after();
-        mma_scores_w<W>(lead, tS, sQ, sK0 + TB * sn, 128);
+        mma_scores_w<kNarrow>(lead, tS, sQ, sK0 + TB * sn, 128);
       }
       mma_commit(lead, sdone);
     }
@@ -246,132 +327,77 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 2 : 1) rowpass_product_ker
   }
   mbar_wait(sdone, njb & 1, ctl, &g_status, kErrWaitMma);
   tc_fence_after();
-  // merge the two halves of every row.  Each warpgroup finishes half of the output columns:
-  // it hands the other half of its accumulator, with its statistics, to the other warpgroup.
-  auto merge = [&](auto wg_c) {
-    constexpr int WG = decltype(wg_c)::value;
-    constexpr int kHalf = Rows<W>::kHead / 2;
-    // columns [base, base + 32) of this warpgroup's accumulator (kSplit: P K_hi + P K_lo)
-    auto fetch = [&](int base, float* o) {
-      tmem_ld32(tO + lane_base + base, o);
-      tmem_ld_wait(o);
-      if (W == kSplit) {
-        float lo[32];
-        tmem_ld32(tO + lane_base + 64 + base, lo);
-        tmem_ld_wait(lo);
-#pragma unroll
-        for (int e = 0; e < 32; ++e) o[e] += lo[e];
-      }
-    };
-    sStat[WG * 128 + row] = make_float4(m_ref, s, 0.f, 0.f);
-    float* give = sX + ((1 - WG) * 128 + row) * kHalf;      // read by the other warpgroup
-#pragma unroll
-    for (int c0 = 0; c0 < kHalf; c0 += 32) {
-      float o[32];
-      fetch(kHalf * (1 - WG) + c0, o);
-#pragma unroll
-      for (int c = 0; c < 8; ++c)
-        reinterpret_cast<float4*>(give + c0)[c ^ (row & 7)] = make_float4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
-    }
-    __syncthreads();
-    const float4 other = sStat[(1 - WG) * 128 + row];
-    const float m = fmaxf(m_ref, other.x);                  // finite: warpgroup 0 always sees key 0
-    const float ref = m == -INFINITY ? 0.f : m;
-    const float f_own = fast_exp2(m_ref - ref), f_oth = fast_exp2(other.x - ref);
-    const float den = s * f_own + other.y * f_oth;
-    const float inv = (MODE == 1 ? g.scale : 1.f) / den;
-    __syncwarp();                                           // (a division has paths of its own for NaN and the like)
-    const float a_own = f_own * inv, a_oth = f_oth * inv;
-    const float* take = sX + (WG * 128 + row) * kHalf;
-    const int i = ib * kTileRows + row;
-    const int d = W == kSplit ? g.d : Rows<W>::kHead;
-#pragma unroll
-    for (int c0 = 0; c0 < kHalf; c0 += 32) {
-      float r[32];
-      fetch(kHalf * WG + c0, r);
-      if (i >= g.tq) continue;
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const float4 x = reinterpret_cast<const float4*>(take + c0)[c ^ (row & 7)];
-        r[4 * c] = r[4 * c] * a_own + x.x * a_oth;
-        r[4 * c + 1] = r[4 * c + 1] * a_own + x.y * a_oth;
-        r[4 * c + 2] = r[4 * c + 2] * a_own + x.z * a_oth;
-        r[4 * c + 3] = r[4 * c + 3] * a_own + x.w * a_oth;
-      }
-      TOut* dst = out + ((int64_t)n * g.tq + i) * d + kHalf * WG + c0;
-      if (std::is_same<TOut, float>::value) {
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-          if (W != kSplit || kHalf * WG + c0 + 4 * c < d)
-            reinterpret_cast<float4*>(dst)[c] = make_float4(r[4 * c], r[4 * c + 1], r[4 * c + 2], r[4 * c + 3]);
-      } else {
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-          reinterpret_cast<uint4*>(dst)[c] =
-              make_uint4(pack_bf16(r[8 * c], r[8 * c + 1]), pack_bf16(r[8 * c + 2], r[8 * c + 3]),
-                         pack_bf16(r[8 * c + 4], r[8 * c + 5]), pack_bf16(r[8 * c + 6], r[8 * c + 7]));
-      }
-    }
-    if (WG == 0 && i < g.tq && rmax != nullptr) {
-      // the merged reference, not necessarily the row maximum (it lags behind it by design);
-      // every consumer uses the pair only as the log-sum-exp rmax + log2(rden)
-      rmax[(int64_t)n * g.tq + i] = m;
-      rden[(int64_t)n * g.tq + i] = den;
-    }
-  };
-  if (wg == 0) merge(std::integral_constant<int, 0>{}); else merge(std::integral_constant<int, 1>{});
+  auto sync = [] { __syncthreads(); };
+  const int i = ib * kTileRows + row;
+  if (wg == 0) row_merge<MODE, 0, kNarrow>(tO + lane_base, g, n, i, row, m_ref, s, sStat, sX, rmax, rden, out, sync);
+  else row_merge<MODE, 1, kNarrow>(tO + lane_base, g, n, i, row, m_ref, s, sStat, sX, rmax, rden, out, sync);
   drain_if_aborted(ctl);
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_free(tmem, kTmem);
 }
 
-// The same where there are long rows and many blocks (row_pairs; wide rows kWidePairsFrom): two query tiles of 128 per CTA, one per compute warpgroup (lane
-// = query, so that a row's sums and output need no merge), and a ninth warp that issues every TMA copy and MMA.  The keys come in
-// half tiles of 64: S = Q K^T (N = 64) and O take 128 TMEM columns of a warpgroup, P~ goes over the scores that were read, and two
-// CTAs give a scheduler four warps in four phases.  The issuing warp serves a warpgroup's P~ B and, behind it in the pipe, its next
-// scores as soon as its P~ is written; while those are on their way the other three warps of the scheduler compute.  A step of 64 keys
-// takes a warp 1240 cycles of arithmetic alone and 2150 in all with three others beside it (the special-function unit's floor: 2048);
-// continuous calls run at the card's power limit (1.72 GHz, 995 W), so that polynomials for some of the exponentials give nothing.
-// grid = n * ceil(tq/256), longest rows first.
-constexpr int kRowRing = 4;                           // half tiles of K (and V)
-constexpr int kRowThreads = 288;
-template <int MODE, int W = kNarrow> constexpr int kRowSmem = (2 + kRowRing * MODE / 2) * (int)Rows<W>::kBytes + 256 + 1024;
+// The same with a warp that issues every TMA copy and MMA.  Of each query tile's two warpgroups one takes the half tiles of 64 keys
+// 0, 2, 4, .., the other 1, 3, 5, ..: the keys that they have in rowpass_product_kernel, with scores of their own.  The issuing warp
+// serves a warpgroup's P~ B and, behind it in the pipe, its next scores as soon as its P~ is written, and nothing in the loop waits for
+// the whole CTA.  Keys, their order and every operation on them are those of rowpass_product_kernel, and so are the results, bit for bit.
+//
+// Wide rows: one query tile per CTA.  With one CTA per SM nothing else hides the round trip of a tile's scores.  Row pass with pk,
+// as rowpass_product_kernel / this, in us: d = 128 n = 32, T = 4096 263 / 209, n = 4, T = 4096 68 / 53, n = 100, T = 1024 91 / 81, n = 300,
+// T = 128 27.7 / 27.6, n = 20, T = 300 14.9 / 14.9; fp32 heads of 64 n = 32, T = 4096 281 / 223, n = 148, T = 256 21.2 / 21.2.  Two query
+// tiles per CTA, one per warpgroup, take 196 and 220 us at n = 32, T = 4096 and more than this with few blocks (n = 5, T = 8192 174,
+// here 123), but a row's accumulator then takes twice as many additions: the error of pk against 64 bits went from 1.71e-6 to 2.43e-6
+// (d = 128, n = 32, T = 2048), and that of dq of fp32 heads from 6.56e-6 to 6.57e-6.
+//
+// Narrow rows: two query tiles per CTA (kRowPairsFrom), so that each half tile of keys is copied once for 256 queries.  Long calls run at
+// the card's power limit, where one tile per CTA and two CTAs per SM gain nothing: softmax, n = 64, T = 8192, calls without a pause
+// 851 us as rowpass_product_kernel, 857 so, 800 with two tiles.
+// TMEM: [S 64 | O] per warpgroup.  grid = n * ceil(tq / queries of a CTA), longest rows first; one CTA per SM.
+template <int MODE, int W> struct RowIssuer {
+  static constexpr int kTiles = W == kNarrow ? 2 : 1;                    // query tiles
+  static constexpr int kThreads = 256 * kTiles + 32;
+  static constexpr int kRing = 8;                                        // half tiles of K (and V)
+  // Q[tiles] | K[ring] (V[ring]) | stats [tiles][2][128] float4 | barriers + control
+  static constexpr int kOperands = (2 * kTiles + kRing * MODE) * (int)Rows<W>::kBytes / 2;
+  static constexpr int kBytes = kOperands + 4096 * kTiles + 256 + 1024;
+};
 
-template <int MODE, typename TOut, int W = kNarrow>
-__global__ void __launch_bounds__(kRowThreads, W == kNarrow ? 2 : 1) rowpass_tiles_kernel(
+template <int MODE, typename TOut, int W>
+__global__ void __launch_bounds__(RowIssuer<MODE, W>::kThreads, 1) rowpass_issuer_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, Geom g, float* __restrict__ rmax, float* __restrict__ rden,
     TOut* __restrict__ out) {
   static_assert(MODE == 1 || MODE == 2, "1: B = K (pk); 2: B = V (softmax attention)");
-  constexpr int R = kRowRing;
+  using Form = RowIssuer<MODE, W>;
+  constexpr int R = Form::kRing, NT = Form::kTiles, kTmem = 512;
   constexpr uint32_t TB = Rows<W>::kBytes, HB = TB / 2, HSub = kTileBytes / 2;    // a tile, half a tile, a sub-tile of that
   constexpr int kAcc = Rows<W>::kCols, kWg = 64 + kAcc;                            // TMEM columns of O, and of a warpgroup
-  constexpr int kTmem = W == kNarrow ? 256 : 512;
+  static_assert(2 * NT * kWg <= kTmem, "the warpgroups' columns fit the allocation");
+  static_assert(NT * 128 * Rows<W>::kHead * 4 <= R * MODE * (int)HB, "the merge area fits the K stages");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
-  const uint32_t sQ = smem_u32(smem), sK = sQ + 2 * TB, sB = MODE == 2 ? sK + R * HB : sK;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 2 * TB + MODE * R * HB);
-  const uint32_t qfull = smem_u32(bars), kfull = qfull + 8, kfree = kfull + 8 * R, sdone = kfree + 8 * R, pready = sdone + 16;
-  Ctl* ctl = reinterpret_cast<Ctl*>(bars + 5 + 2 * R);
+  const uint32_t sQ = smem_u32(smem), sK = sQ + NT * TB, sB = MODE == 2 ? sK + R * HB : sK;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Form::kOperands + 4096 * NT);
+  const uint32_t qfull = smem_u32(bars), kfull = qfull + 8, kfree = kfull + 8 * R, sdone = kfree + 8 * R, pready = sdone + 16 * NT;
+  Ctl* ctl = reinterpret_cast<Ctl*>(bars + 1 + 2 * R + 4 * NT);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wg = tid >> 7, row = tid & 127;
   const int warp_u = uniform_warp();
   const uint32_t lead = elect_one();
-  const int npair = (g.tq + 2 * kTileRows - 1) / (2 * kTileRows);
+  const int nqb = (g.tq + NT * kTileRows - 1) / (NT * kTileRows);
   const int n = (int)(blockIdx.x % g.n);
-  const int t0 = (npair - 1 - (int)(blockIdx.x / g.n)) * 2;       // query tiles t0 and t0 + 1
+  const int ib = (nqb - 1 - (int)(blockIdx.x / g.n)) * NT;                  // (first) query tile
   // half tiles of keys that a tile's queries see; none for a tile behind the last query
-  auto half_tiles = [&](int w) {
-    return (t0 + w) * kTileRows < g.tq ? min(g.tk - 1, g.q_off + (t0 + w) * kTileRows + kTileRows - 1) / 64 + 1 : 0;
+  auto half_tiles = [&](int tile) {
+    const int i0 = (ib + tile) * kTileRows;
+    return i0 < g.tq ? min(g.tk - 1, g.q_off + i0 + kTileRows - 1) / 64 + 1 : 0;
   };
-  const int nh0 = half_tiles(0), nh1 = half_tiles(1), nh = max(nh0, nh1);
+  const int nh0 = half_tiles(0), nh1 = NT == 2 ? half_tiles(1) : 0, nh = max(nh0, nh1);
 
   if (tid == 0) {
     ctl->abort = 0;
-    for (int i = 0; i < 3 + 2 * R; ++i) mbar_init(qfull + 8 * i, 1);          // qfull, kfull[R], kfree[R], sdone[2]
-    mbar_init(pready, 4);
-    mbar_init(pready + 8, 4);
+    for (int i = 0; i < 1 + 2 * R + 2 * NT; ++i) mbar_init(qfull + 8 * i, 1);          // qfull, kfull[R], kfree[R], sdone[2 NT]
+    for (int i = 0; i < 2 * NT; ++i) mbar_init(pready + 8 * i, 4);
     fence_barrier_init();
   }
   __syncwarp();
@@ -381,7 +407,7 @@ __global__ void __launch_bounds__(kRowThreads, W == kNarrow ? 2 : 1) rowpass_til
   tc_fence_after();
   const uint32_t tmem = uniform(ctl->tmem);
 
-  if (warp_u == 8) {
+  if (warp_u == 8 * NT) {
     // ------------------------------------------------------------ the issuing warp
     constexpr uint32_t id_s = instr_desc(128, 64, 0, 0), id_p = instr_desc(128, kAcc, 0, 1);
     const Desc dQ = make_desc(sQ, 16, 1024), dK = make_desc(sK, 16, 1024), dB = make_desc(sB, HSub, 1024);
@@ -392,166 +418,80 @@ __global__ void __launch_bounds__(kRowThreads, W == kNarrow ? 2 : 1) rowpass_til
       tma_load_rows<W>(sK + HB * st, &map_k, h * 64, n, kfull + 8 * st, HSub);
       if (MODE == 2) tma_load_rows<W>(sB + HB * st, &map_v, h * 64, n, kfull + 8 * st, HSub);
     };
+    const int tiles = nh1 > 0 ? 2 : 1;
     if (lead) {
-      mbar_expect_tx(qfull, (nh1 > 0 ? 2 : 1) * TB);
-      for (int w = 0; w < (nh1 > 0 ? 2 : 1); ++w) tma_load_rows<W>(sQ + TB * w, &map_q, (t0 + w) * kTileRows, n, qfull);
+      mbar_expect_tx(qfull, tiles * TB);
+      for (int i = 0; i < tiles; ++i) tma_load_rows<W>(sQ + TB * i, &map_q, (ib + i) * kTileRows, n, qfull);
     }
     for (int h = 0; h < R && h < nh; ++h) load_keys(h);
     mbar_wait_warp(qfull, 0, ctl, &g_status, kErrWaitTma);
-    for (int h = 0; h <= nh; ++h) {
+    for (int h = 0; h < nh + 2; ++h) {
       if (h < nh) mbar_wait_warp(kfull + 8 * (h % R), (h / R) & 1, ctl, &g_status, kErrWaitTma);
-      for (int w = 0; w < 2; ++w) {
-        const int nw = w ? nh1 : nh0;
-        if (h > nw || nw == 0) continue;
+#pragma unroll
+      for (int i = 0; i < NT; ++i) {
+        const int w = 2 * i + (h & 1), nt = i ? nh1 : nh0;
         const uint32_t tS = tmem + kWg * w;
-        if (h > 0) {
-          mbar_wait_warp(pready + 8 * w, (h - 1) & 1, ctl, &g_status, kErrWaitTile);
+        if (nt == 0 || h >= nt + 2) continue;
+        if (h >= 2) {
+          mbar_wait_warp(pready + 8 * w, ((h >> 1) - 1) & 1, ctl, &g_status, kErrWaitTile);
           tc_fence_after();
 #pragma unroll
           for (int pl = 0; pl < Rows<W>::kPlanes; ++pl)
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)                        // 16 keys per instruction: 16 rows of 128 B = 128 units
-              mma_ts(lead, tS + 64, tS + 32 * pl + 8 * kk, dB, (HB >> 4) * ((h - 1) % R) + 128 * kk, id_p, h > 1 || pl > 0 || kk > 0);
+              mma_ts(lead, tS + 64, tS + 32 * pl + 8 * kk, dB, (HB >> 4) * ((h - 2) % R) + 128 * kk, id_p, 1);
         }
-        if (h < nw) {
+        if (h < nt) {
           tc_fence_after();
-          mma_scores_wide<W>(lead, tS, Desc{dQ.lo + (TB >> 4) * w, dQ.hi}, kTileBytes, Desc{dK.lo + (HB >> 4) * (h % R), dK.hi}, HSub, id_s);
+          mma_scores_wide<W>(lead, tS, Desc{dQ.lo + (TB >> 4) * i, dQ.hi}, kTileBytes, Desc{dK.lo + (HB >> 4) * (h % R), dK.hi}, HSub, id_s);
         }
-        mma_commit(lead, sdone + 8 * w);                          // P~ B of h - 1 and the scores of h
+        mma_commit(lead, sdone + 8 * w);                          // P~ B of h - 2 and the scores of h, one of them or none
       }
-      if (h > 0) mma_commit(lead, kfree + 8 * ((h - 1) % R));
-      if (h > 1 && h - 2 + R < nh) {
-        mbar_wait_warp(kfree + 8 * ((h - 2) % R), ((h - 2) / R) & 1, ctl, &g_status, kErrWaitMma);
-        load_keys(h - 2 + R);
+      if (h >= 2) mma_commit(lead, kfree + 8 * ((h - 2) % R));
+      // half tile h - 3, whose products were issued one round ago, makes room for h - 3 + R
+      if (h >= 3 && h - 3 + R < nh) {
+        mbar_wait_warp(kfree + 8 * ((h - 3) % R), ((h - 3) / R) & 1, ctl, &g_status, kErrWaitMma);
+        load_keys(h - 3 + R);
       }
     }
     __syncwarp();
   } else {
     // ------------------------------------------------------------ the compute warps: lane = query
     const uint32_t tS = tmem + kWg * wg + ((uint32_t)((warp & 3) * 32) << 16), tO = tS + 64;
-    const int nw = wg ? nh1 : nh0, i = (t0 + wg) * kTileRows + row, q0 = g.q_off + (t0 + wg) * kTileRows, ia = q0 + row;
-    float m_ref = -INFINITY, s = 0.f;
-    for (int h = 0; h < nw; ++h) {
-      mbar_wait(sdone + 8 * wg, h & 1, ctl, &g_status, kErrWaitMma);
-      tc_fence_after();
-      __syncwarp();
-      float v[64];
-      tmem_ld32(tS, v);
-      tmem_ld32(tS + 32, v + 32);
-      tmem_ld_wait(v);
-      tmem_ld_wait(v + 32);
-      uint32_t pw[32], pr[Rows<W>::kPlanes == 2 ? 32 : 1];
-      float ps = 0.f;
-      // P~ = 2^(z - reference) for the thread's 64 scores, two per instruction; their sum in ps
-      auto exponentials = [&]() {
-        const float mr = m_ref == -INFINITY ? 0.f : m_ref;
-        const float2 zs = make_float2(g.zscale, g.zscale), off = make_float2(-mr, -mr);
-        float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
+    {
+      uint32_t z[16];
 #pragma unroll
-        for (int e = 0; e < 64; e += 4) {
-          const float2 z0 = fma2(make_float2(v[e], v[e + 1]), zs, off);
-          const float2 z1 = fma2(make_float2(v[e + 2], v[e + 3]), zs, off);
-          const float2 p0 = make_float2(fast_exp2(z0.x), fast_exp2(z0.y));
-          const float2 p1 = make_float2(fast_exp2(z1.x), fast_exp2(z1.y));
-          acc0 = add2(acc0, p0);
-          acc1 = add2(acc1, p1);
-          pw[e >> 1] = pack_bf16(p0.x, p0.y);
-          pw[(e >> 1) + 1] = pack_bf16(p1.x, p1.y);
-          if (Rows<W>::kPlanes == 2) {
-            pr[e >> 1] = pack_bf16_rest(p0.x, p0.y, pw[e >> 1]);
-            pr[(e >> 1) + 1] = pack_bf16_rest(p1.x, p1.y, pw[(e >> 1) + 1]);
-          }
-        }
-        const float2 acc = add2(acc0, acc1);
-        ps = acc.x + acc.y;
-      };
-      // (the reference, the common half tile and the slow path are those of rowpass_product_kernel)
-      const bool edge = (h * 64 + 63 > q0) || ((h + 1) * 64 > g.tk);
-      // (the first 128 keys set the reference, as there: the largest P~ is then 1 more often, which bf16 holds exactly)
-      bool slow = edge || h < 2 || __any_sync(0xffffffffu, m_ref == -INFINITY);
-      if (!slow) {
-        exponentials();
-        slow = __any_sync(0xffffffffu, !(ps < kRefLimit));
-        if (slow) {                      // rare: the scores are still in TMEM, fetch them again
-          tmem_ld32(tS, v);
-          tmem_ld32(tS + 32, v + 32);
-          tmem_ld_wait(v);
-          tmem_ld_wait(v + 32);
-        }
-      }
-      if (slow) {
-        float cmax = -INFINITY;
+      for (int c = 0; c < 16; ++c) z[c] = 0u;
 #pragma unroll
-        for (int e = 0; e < 64; ++e) {
-          const int ja = h * 64 + e;
-          if (edge && (ja > ia || ja >= g.tk)) v[e] = -INFINITY;
-          cmax = fmaxf(cmax, v[e]);
-        }
-        const float m_new = fmaxf(m_ref, cmax * g.zscale);
-        if (__any_sync(0xffffffffu, m_new != m_ref)) {
-          const bool fresh = __all_sync(0xffffffffu, m_ref == -INFINITY);   // nothing accumulated yet
-          const float f = fast_exp2(m_ref - (m_new == -INFINITY ? 0.f : m_new));
-          if (!fresh && h > 0) {
-#pragma unroll
-            for (int c = 0; c < kAcc / 16; ++c) {
-              float o[16];
-              tmem_ld16(tO + 16 * c, o);
-              tmem_ld_wait16(o);
-              uint32_t w[16];
-#pragma unroll
-              for (int e = 0; e < 16; ++e) w[e] = __float_as_uint(o[e] * f);
-              tmem_st16(tO + 16 * c, w);
-            }
-          }
-          s *= f;
-          m_ref = m_new;
-        }
-        exponentials();
-      }
-      s += ps;
-      // over the first 32 of the 64 scores: keys 2c, 2c+1 in column c (the lo plane over the others)
-      tmem_st16(tS, pw);
-      tmem_st16(tS + 16, pw + 16);
-      if (Rows<W>::kPlanes == 2) {
-        tmem_st16(tS + 32, pr);
-        tmem_st16(tS + 48, pr + 16);
-      }
+      for (int c = 0; c < kAcc / 16; ++c) tmem_st16(tO + 16 * c, z);
       tmem_st_wait();
+    }
+    const int tile = NT == 2 ? wg >> 1 : 0, half = wg & 1, nt = tile ? nh1 : nh0;
+    const int i = (ib + tile) * kTileRows + row, q0 = g.q_off + (ib + tile) * kTileRows, ia = q0 + row;
+    float m_ref = -INFINITY, s = 0.f;
+    int t = 0;                                                // the warpgroup's own count of half tiles
+    for (int h = half; h < nt; h += 2, ++t) {
+      mbar_wait_warp(sdone + 8 * wg, t & 1, ctl, &g_status, kErrWaitMma);
+      tc_fence_after();
+      const bool edge = ((h | 1) * 64 + 63 > q0) || (((h | 1) + 1) * 64 > g.tk);      // (by whole tiles, as there)
+      row_half_tile<W>(tS, tO, g, h * 64, ia, edge, m_ref, s);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(pready + 8 * wg);
     }
-    if (nw > 0) {
-      mbar_wait(sdone + 8 * wg, nw & 1, ctl, &g_status, kErrWaitMma);
-      tc_fence_after();
-      __syncwarp();
-      const float inv = (MODE == 1 ? g.scale : 1.f) / s;
-      __syncwarp();                                           // (a division has paths of its own for NaN and the like)
-      const int d = W == kSplit ? g.d : Rows<W>::kHead;
-      TOut* dst = out + ((int64_t)n * g.tq + i) * d;
-#pragma unroll
-      for (int c = 0; c < Rows<W>::kHead / 32; ++c) {
-        float o[32];
-        tmem_ld32(tO + 32 * c, o);
-        tmem_ld_wait(o);
-        if (W == kSplit) {                                    // P~ K_hi + P~ K_lo
-          float lo[32];
-          tmem_ld32(tO + 64 + 32 * c, lo);
-          tmem_ld_wait(lo);
-#pragma unroll
-          for (int e = 0; e < 32; ++e) o[e] += lo[e];
-        }
-#pragma unroll
-        for (int e = 0; e < 32; ++e) o[e] *= inv;
-        if (i < g.tq) store_row32<W>(dst + 32 * c, o, d - 32 * c);
-      }
-      if (i < g.tq && rmax != nullptr) {
-        // the reference, not necessarily the row maximum (it lags behind it by design); every consumer uses the pair only as
-        // the log-sum-exp rmax + log2(rden)
-        rmax[(int64_t)n * g.tq + i] = m_ref;
-        rden[(int64_t)n * g.tq + i] = s;
-      }
-    }
+    if (nt > 0) mbar_wait_warp(sdone + 8 * wg, t & 1, ctl, &g_status, kErrWaitMma);
+    tc_fence_after();
+    // every product has read the K stages, which the merge goes over
+    asm volatile("bar.sync 1, %0;" ::"n"(256 * NT) : "memory");
+    // merge area [2][128][half a row] and statistics [2][128] of this tile
+    float* sX = reinterpret_cast<float*>(smem + NT * TB) + tile * 128 * Rows<W>::kHead;
+    float4* sStat = reinterpret_cast<float4*>(smem + Form::kOperands) + 256 * tile;
+    auto sync = [tile] {
+      if (NT == 1 || tile == 0) asm volatile("bar.sync 2, 256;" ::: "memory");
+      else asm volatile("bar.sync 3, 256;" ::: "memory");
+    };
+    if (nt > 0 && half == 0) row_merge<MODE, 0, W>(tO, g, n, i, row, m_ref, s, sStat, sX, rmax, rden, out, sync);
+    else if (nt > 0) row_merge<MODE, 1, W>(tO, g, n, i, row, m_ref, s, sStat, sX, rmax, rden, out, sync);
   }
   drain_if_aborted(ctl);
   tc_fence_before();
@@ -769,27 +709,29 @@ __global__ void dq_from_pk_kernel(const float* __restrict__ dq_main, const float
 }
 
 // ---------------------------------------------------------------- host launchers
-// Which row passes take rowpass_tiles_kernel: long rows and many pairs of query tiles.  Two CTAs of two tiles each want 296 pairs at a
-// time, and a CTA takes twice the tiles of one of rowpass_product_kernel, whose warpgroups share a row's keys: on a chip that is not
-// full that one is done sooner, and short rows are mostly slow steps.  Row pass with pk, one tile / pairs, in us: n = 64, T = 16384
-// (4096 pairs) 3221 / 2858; n = 128, T = 2048 (1024) 130.8 / 129.1; n = 32, T = 4096 (512) 111 / 114; n = 384, T = 1024 (1536) 129 / 133;
-// n = 16, T = 1777 (112) 24 / 36.  Softmax: n = 64, T = 8192 (2048) 837 / 759; n = 64, T = 4096 (1024) 215 / 210; n = 128, T = 2048
-// (1024) 123 / 121; n = 64, T = 1024 (256) 27.5 / 28.8; n = 2, T = 3000 (24) 33 / 51.
+// Narrow row passes that take rowpass_issuer_kernel: rows of kRowPairsFrom tokens in kRowPairs blocks of 256 queries.  Its CTAs have an
+// SM to themselves, with their start and end unhidden, and 96 registers.  Calls without a pause, rowpass_product_kernel / it, in us,
+// with pk: n = 64, T = 16384 3109 / 2901, n = 64, T = 8192 782 / 768, n = 8, T = 8192 (256 blocks) 115.5 / 97.1, n = 64, T = 6144
+// 455.6 / 454.5, n = 20, T = 6144 149.3 / 145.6, n = 64, T = 5120 326 / 328, n = 64, T = 4096 217 / 221, n = 128, T = 2048 131 / 143.
+// Softmax: n = 64, T = 16384 3409 / 3043, n = 64, T = 8192 851 / 800, n = 1, T = 131072 2915 / 2765, n = 8, T = 8192 106 / 99, n = 64,
+// T = 6144 479 / 470, n = 20, T = 6144 147.5 / 146.2, n = 64, T = 5120 338 / 335, n = 64, T = 4096 220.5 / 221.5, n = 128, T = 2048 130 / 137,
+// and with fewer blocks than SMs n = 2, T = 3000 32.8 / 40.4.
+constexpr int kRowPairsFrom = 6144, kRowPairs = 256;
 inline int64_t tile_pairs(const Geom& g) { return g.n * ((g.tq + 2 * kTileRows - 1) / (2 * kTileRows)); }
-inline bool row_pairs(const Geom& g) { return g.tq >= 2048 && tile_pairs(g) >= 1024; }
+inline bool row_issuer(const Geom& g) { return g.q_off + g.tq >= kRowPairsFrom && tile_pairs(g) >= kRowPairs; }
 
 // Pass 1 with the saved query correction: rmax, rden and pk = scale * softmax(q k^T) k.
 inline int rowstats_pk(const void* q, const void* k, const Geom& g, float* rmax, float* rden, float* pk,
                        cudaStream_t st, char* err, size_t errlen) {
   CUtensorMap mq, mk;
-  const int64_t pairs = tile_pairs(g);
+  const bool issuer = row_issuer(g);
   if (int rc = make_map(&mq, q, g.n, g.tq, err, errlen)) return rc;
-  if (int rc = make_map(&mk, k, g.n, g.tk, err, errlen, kHeadDim, row_pairs(g) ? 64 : kTileRows)) return rc;
-  if (row_pairs(g)) {
-    auto kern = rowpass_tiles_kernel<1, float>;
-    constexpr int smem = kRowSmem<1> > kTwoPerSm ? kRowSmem<1> : kTwoPerSm;
-    if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
-    kern<<<(unsigned)pairs, kRowThreads, smem, st>>>(mq, mk, mk, g, rmax, rden, pk);
+  if (int rc = make_map(&mk, k, g.n, g.tk, err, errlen, kHeadDim, issuer ? 64 : kTileRows)) return rc;
+  if (issuer) {
+    using Form = RowIssuer<1, kNarrow>;
+    auto kern = rowpass_issuer_kernel<1, float, kNarrow>;
+    if (int rc = set_smem_attr((const void*)kern, Form::kBytes, err, errlen)) return rc;
+    kern<<<(unsigned)tile_pairs(g), Form::kThreads, Form::kBytes, st>>>(mq, mk, mk, g, rmax, rden, pk);
     return launch_status("tc rowstats_pk", err, errlen);
   }
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
@@ -810,22 +752,22 @@ constexpr unsigned kOnePollsAbove = 2 * 148;
 inline int softmax_forward(const void* q, const void* k, const void* v, const Geom& g, float* rmax,
                            float* rden, void* out, cudaStream_t st, char* err, size_t errlen) {
   CUtensorMap mq, mk, mv;
-  const int64_t pairs = tile_pairs(g);
-  const int key_rows = row_pairs(g) ? 64 : kTileRows;
+  const bool issuer = row_issuer(g);
+  const int key_rows = issuer ? 64 : kTileRows;
   if (int rc = make_map(&mq, q, g.n, g.tq, err, errlen)) return rc;
   if (int rc = make_map(&mk, k, g.n, g.tk, err, errlen, kHeadDim, key_rows)) return rc;
   if (int rc = make_map(&mv, v, g.n, g.tk, err, errlen, kHeadDim, key_rows)) return rc;
-  if (row_pairs(g)) {
-    auto kern = rowpass_tiles_kernel<2, __nv_bfloat16>;
-    constexpr int smem = kRowSmem<2>;
-    static_assert(2 * (smem + 1024) <= 233472 && 3 * (smem + 1024) > 233472, "two CTAs of the softmax pass fit one SM");
-    if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
-    kern<<<(unsigned)pairs, kRowThreads, smem, st>>>(mq, mk, mv, g, rmax, rden, (__nv_bfloat16*)out);
+  if (issuer) {
+    using Form = RowIssuer<2, kNarrow>;
+    auto kern = rowpass_issuer_kernel<2, __nv_bfloat16, kNarrow>;
+    static_assert(Form::kBytes <= 232448, "fits an SM");
+    if (int rc = set_smem_attr((const void*)kern, Form::kBytes, err, errlen)) return rc;
+    kern<<<(unsigned)tile_pairs(g), Form::kThreads, Form::kBytes, st>>>(mq, mk, mv, g, rmax, rden, (__nv_bfloat16*)out);
     return launch_status("tc softmax_forward", err, errlen);
   }
   const int nqb = (g.tq + kTileRows - 1) / kTileRows;
   const unsigned grid = (unsigned)(g.n * nqb);
-  auto kern = grid > kOnePollsAbove ? rowpass_product_kernel<2, __nv_bfloat16, kNarrow, true>
+  auto kern = grid > kOnePollsAbove ? rowpass_product_kernel<2, __nv_bfloat16, true>
                                     : rowpass_product_kernel<2, __nv_bfloat16>;
   constexpr int smem = RowpassSmem<2>::kBytes;
   static_assert(2 * (smem + 1024) <= 233472 && 3 * (smem + 1024) > 233472, "two CTAs of the softmax pass fit one SM");

@@ -493,11 +493,6 @@ inline int wide_maps(WideMaps* m, const void* q, const void* k, const void* v, c
   return make_map(&m->v, v, g.n, g.tk, err, errlen, 128);
 }
 
-// Pairs of query tiles from which the row pass of wide rows takes rowpass_tiles_kernel, one CTA per SM.  Passes 1-3, one tile / pairs, in
-// us: d = 128 n = 32, T = 4096 (512 pairs) 631 / 551, n = 64, T = 1024 (256) 140 / 127, n = 128, T = 512 (256) 108 / 99; fp32 heads of
-// 64 n = 32, T = 4096 624 / 567.  With fewer pairs than SMs a block's two tiles would share one.
-constexpr int64_t kWidePairsFrom = 148;
-
 // Passes 1-3 on wide rows; pk (n, t, d) fp32 is written when it is not null.
 template <int W>
 inline int wide_forward(const void* q, const void* k, const void* v, const Geom& g, float* rmax, float* rden,
@@ -506,23 +501,15 @@ inline int wide_forward(const void* q, const void* k, const void* v, const Geom&
   WideMaps m;
   if (int rc = wide_maps(&m, q, k, v, g, err, errlen)) return rc;
   const unsigned grid = (unsigned)(g.n * ((g.tq + kTileRows - 1) / kTileRows));
-  if (pk != nullptr && tile_pairs(g) >= kWidePairsFrom) {
+  if (pk != nullptr) {
     CUtensorMap mk64;
     if (int rc = make_map(&mk64, k, g.n, g.tk, err, errlen, 128, 64)) return rc;
-    auto kern = rowpass_tiles_kernel<1, float, W>;
-    constexpr int smem = kRowSmem<1, W>;
+    auto kern = rowpass_issuer_kernel<1, float, W>;
+    constexpr int smem = RowIssuer<1, W>::kBytes;
     static_assert(smem <= 232448 && 2 * smem > 233472, "one CTA (512 TMEM columns) per SM");
     if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
     mark("tc_wide_rowstats_pk", st, 0);
-    kern<<<(unsigned)tile_pairs(g), kRowThreads, smem, st>>>(m.q, mk64, mk64, g, rmax, rden, pk);
-    mark("tc_wide_rowstats_pk", st, 1);
-  } else if (pk != nullptr) {
-    auto kern = rowpass_product_kernel<1, float, W>;
-    constexpr int smem = RowpassSmem<1, W>::kBytes;
-    static_assert(smem <= 232448 && 2 * smem > 233472, "one CTA (512 TMEM columns) per SM");
-    if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
-    mark("tc_wide_rowstats_pk", st, 0);
-    kern<<<grid, 256, smem, st>>>(m.q, m.k, m.k, g, rmax, rden, pk);
+    kern<<<grid, RowIssuer<1, W>::kThreads, smem, st>>>(m.q, mk64, mk64, g, rmax, rden, pk);
     mark("tc_wide_rowstats_pk", st, 1);
   } else {
     constexpr int smem = kRowstatsSmem<W>;

@@ -1,5 +1,4 @@
-"""Row passes of many blocks: pairs of query tiles with an issuing warp.  The route at its edge, ragged lengths around the tiles, and a
-reference exponent that has to move, against 64 bits."""
+"""Row passes of many blocks: ragged lengths around the tiles, and a reference exponent that has to move, against 64 bits."""
 
 from __future__ import annotations
 
@@ -20,7 +19,7 @@ def _exact(q, k, v, row):
     return torch.softmax(z, -1), torch.logsumexp(z, -1)
 
 
-# 1024 pairs of tiles and rows of 2048 tokens and more; one row less, or one token, takes the kernel of single tiles
+# 1024 blocks of 256 queries and more in rows of 2048 tokens and more, one row less, and one token
 @pytest.mark.parametrize("rows,seq", [(128, 2048), (127, 2048), (128, 2047), (114, 2049), (114, 2111), (114, 2177), (103, 2433)])
 @pytest.mark.parametrize("std", [1.0, 24.0])
 def test_row_pass_against_64_bits(rows, seq, std):
@@ -48,7 +47,7 @@ def test_row_pass_against_64_bits(rows, seq, std):
         assert ((got - lse).abs() <= 2e-6 * lse.abs().clamp(min=1.0) + 2e-6).all()
 
 
-# rows of 256 bytes: bf16 heads of 128, fp32 heads as hi + lo planes; 148 pairs of tiles and one less
+# rows of 256 bytes: bf16 heads of 128, fp32 heads as hi + lo planes; 148 blocks of 256 queries and one less
 @pytest.mark.parametrize("rows,seq", [(148, 100), (74, 257), (148, 129), (50, 700), (147, 100)])
 @pytest.mark.parametrize("dtype,d", [(torch.bfloat16, 128), (torch.float32, 64), (torch.float32, 32)])
 @pytest.mark.parametrize("std", [1.0, 24.0])
