@@ -39,8 +39,9 @@ static_assert(4 * 104 + 64 <= 5 * kFusedRegs, "setmaxnreg hands out what the blo
 // V[G] ones shares[G] | Q[4] (8 KB each) | staging (16 KB) | lse [4][64] | barriers
 template <int G> constexpr int kFusedSmem = (2 * G + 1) * kTileBytes + kFusedRing * kTileBytes / 2 + kTileBytes + 1024 + 256 + 1024;
 
-// G: compute warpgroups of 128 keys.  CR: query rows per checkpoint.  BID: the softmax form (expshift has no row statistics: rmax is
-// null and every log-sum-exp the shift's logarithm) or the sigmoid's, with the inclusive share step.
+// G: compute warpgroups of 128 keys.  CR: query rows per checkpoint.  BID, with the inclusive share step: softmax, the sigmoid's form, or
+// expshift, which has no row statistics (every log-sum-exp is the shift's logarithm) and whose bids have no upper end: an exponential may
+// overflow, and so may a demand, which then stays infinite while the rows behind it are finite.
 template <int G, int CR, bool PAIR, int BID = kBidSoftmax>
 __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_v,
@@ -185,7 +186,7 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
         const int i3 = (h + 3) * 64 + row;
         const bool fetch = row < 64 && h + 3 < nh;
         if (fetch && i3 < g.tq) {
-          if (BID == kBidSigmoid || rmax == nullptr) {
+          if (BID != kBidSoftmax) {
             nx_max = g.lshift;
           } else {
             nx_max = rmax[row_base + i3];
@@ -282,9 +283,15 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
             }
             // every fourth exponential is a polynomial on the FMA pipe (7.30 -> 7.08 ms when two warps shared a scheduler), of
             // degree 5: with degree 4 the demand, an output in fp32, is off by up to 4.6e-6 instead of 2.5e-6
-            // (the sigmoid's exponents are of either sign: capped, where the bid is 1e-38 and less)
-            const float2 fourth = poly_exp2_two<5>(BID == kBidSigmoid ? make_float2(min_nan(z[3], 126.f), min_nan(z[7], 126.f))
-                                                                      : make_float2(z[3], z[7]));
+            // (the sigmoid's exponents are of either sign: capped, where the bid is 1e-38 and less.  Expshift's go past 128, where the
+            // polynomial's scale would run into the sign: twice 2^(z - 1) up to the infinity at z = 129.  657 -> 665 us at n = 32,
+            // T = 8192, 686 with every exponential from the special-function unit)
+            float2 fourth;
+            if (BID == kBidExpshift) {
+              fourth = poly_exp2_two<5>(make_float2(min_nan(z[3] - 1.f, 128.f), min_nan(z[7] - 1.f, 128.f)));
+              fourth = add2(fourth, fourth);
+            } else if (BID == kBidSigmoid) fourth = poly_exp2_two<5>(make_float2(min_nan(z[3], 126.f), min_nan(z[7], 126.f)));
+            else fourth = poly_exp2_two<5>(make_float2(z[3], z[7]));
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
               float p = (u & 3) != 3 ? fast_exp2(z[u]) : u == 3 ? fourth.x : fourth.y;
@@ -304,7 +311,7 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
         };
         if (masked) chunk(std::true_type{}); else chunk(std::false_type{});
         const float add = chunk_sum - low, sum = base + add;
-        low = (sum - base) - add;
+        low = BID == kBidExpshift && !(sum < INFINITY) ? 0.f : (sum - base) - add;      // (inf - inf)
         base = sum;
         __syncwarp();
       };
@@ -395,6 +402,7 @@ inline int forward_fused(const void* q, const void* k, const void* v, const Geom
   using std::integral_constant;
   using Softmax = integral_constant<int, kBidSoftmax>;
   using Sigmoid = integral_constant<int, kBidSigmoid>;
+  using Expshift = integral_constant<int, kBidExpshift>;
   auto by_pair = [&](auto groups_c, auto cr_c) {
     return pair_demands(g) ? launch(groups_c, cr_c, std::true_type{}, Softmax{}) : launch(groups_c, cr_c, std::false_type{}, Softmax{});
   };
@@ -403,6 +411,7 @@ inline int forward_fused(const void* q, const void* k, const void* v, const Geom
       return pair_demands(g) ? launch(groups_c, integral_constant<int, 32>{}, std::true_type{}, Sigmoid{})
                              : launch(groups_c, integral_constant<int, 32>{}, std::false_type{}, Sigmoid{});
     }
+    if (!g.normalised) return launch(groups_c, integral_constant<int, 32>{}, std::false_type{}, Expshift{});
     return g.carry_rows == 64 ? by_pair(groups_c, integral_constant<int, 64>{}) : by_pair(groups_c, integral_constant<int, 32>{});
   };
   if (int rc = fused_groups(g.n, g.tk) == 4 ? by_rows(integral_constant<int, 4>{}) : by_rows(integral_constant<int, 1>{})) return rc;

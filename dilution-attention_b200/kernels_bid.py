@@ -139,7 +139,7 @@ def _takes_sweep(bid, share, code, prec, n, seq, head_dim):
     """Training forwards that are one key-stationary sweep instead of the column-sum and main passes: the element-wise bids with the
     inclusive share step, where rows are long or there are enough blocks of 512 keys for the SMs.  Sweep / two passes in us, sigmoid:
     n = 32, T = 8192 783 / 1331; n = 30, T = 2048 79 / 110; n = 4, T = 4096 (32 blocks) 108 / 131; n = 200, T = 1024 160 / 183.
-    Expshift: n = 32, T = 8192 654 / 944; n = 4, T = 4096 98 / 111; n = 200, T = 1024 143 / 148, but n = 100, T = 1024 (200 blocks)
+    Expshift: n = 32, T = 8192 665 / 944; n = 4, T = 4096 98 / 111; n = 200, T = 1024 144 / 148, but n = 100, T = 1024 (200 blocks)
     84 / 80 and n = 400, T = 512 105 / 104."""
     return (share == 1 and bid in _SWEEP_BIDS and n * -(-seq // 512) >= (32 if seq >= 2048 else 256) and seq >= 1024
             and K.TC_FUSED_FORWARD and _lib.tensor_core_path(code, prec, head_dim)

@@ -61,6 +61,38 @@ def test_a_query_that_is_not_a_number_stays_in_its_rows_and_demands():
     assert total[0, :301].isnan().all() and total[0, 301:].isfinite().all()
 
 
+def _one_large_score(rows, seq, row, key, score):
+    """q, k, v with one score of that size, of query `row` and key `key` of the first row; no other score of that key is above 0."""
+    q, k, v = _inputs(rows, seq, 0.5)
+    q[0, 0, :, 0], q[0, 0, row], k[0, 0, key] = 0.0, 0.0, 0.0
+    q[0, 0, row, 0], k[0, 0, key, 0] = score / 2, 16.0
+    return q, k, v
+
+
+# both block sizes; every position modulo four (one exponential in four is a polynomial), the first and the last of a chunk of 32
+@pytest.mark.parametrize("rows,seq", [(2, 200), (200, 600)])
+@pytest.mark.parametrize("row", [60, 61, 62, 63, 64, 67, 96])
+@pytest.mark.parametrize("score", [88.5, 89.5, 98.5, 150.0, 400.0])
+def test_an_expshift_bid_that_overflows_spoils_its_own_row(rows, seq, row, score):
+    """exp(88.5) is an fp32 number, exp(89.5) is not: its demand is infinite from there on and its own row is inf / inf, but later
+    rows are finite: nobody gets a share of that key any more."""
+    pkg = load_package()
+    key = 40
+    out, ssum, total, carry = _run(pkg, *_one_large_score(rows, seq, row, key, score), "expshift", 1.0, 1e-9, True)
+    over = score > 88.7
+    nan_rows = out[0].isnan().any(-1).nonzero().flatten().tolist()
+    assert nan_rows == ([row] if over else []), nan_rows
+    assert out[1:].isfinite().all() and not total.isnan().any()
+    if over:
+        assert total[0, key] == float("inf") and out[0, row].isnan().all() and ssum[0, row].isnan()
+        assert (carry[0, row // 32 + 1:, key] == float("inf")).all()
+    else:
+        assert abs(total[0, key].item() / 2.7230907e38 - 1) < 1e-4            # exp(88.5)
+    keep = torch.ones(seq, dtype=torch.bool, device=DEV)
+    keep[key] = False
+    assert total[0, keep].isfinite().all() and carry[0, :, :key].isfinite().all()
+
+
 def test_training_calls_take_it():
     pkg = load_package()
     x, y = ([t.requires_grad_(True) for t in _inputs(rows, 2048)] for rows in (8, 7))
