@@ -604,9 +604,9 @@ __global__ void __launch_bounds__(256, W != kNarrow ? 2 : row_sum_bid(BID) ? 3 :
 template <int W> constexpr int kMainSmem =
     4 * (int)Rows<W>::kBytes + (1 + 2 * Rows<W>::kPlanes) * (int)kTileBytes + 512 + 128;
 
-// The bids of softmax form: softmax, and expshift, whose log-sum-exp is a constant.  SHARE selects the ablations of
+// BID: softmax, or expshift, whose log-sum-exp is a constant and whose bids have no upper end.  SHARE selects the ablations of
 // kernels_bid.py (exclusive or absent share step, :254-262); the default instantiation is the operator.
-template <int SHARE = kShareInclusive, bool PAIR = true>
+template <int SHARE = kShareInclusive, bool PAIR = true, int BID = kBidSoftmax>
 __global__ void __launch_bounds__(256, 2) forward_main_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, Geom g, const float* __restrict__ rmax,
@@ -739,8 +739,13 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
         }
         // two special-function ops per score bind this pass: every fourth exponential of the
         // softmax bid is a polynomial on the FMA pipe (79.7 -> 75.3 ms at the 128K prefill shape)
-        const float2 fourth = poly_exp2_two<4>(make_float2(fmaf(v[e8 * 8 + 3], g.zscale, -lcur[0].w),
-                                                        fmaf(v[e8 * 8 + 7], g.zscale, -lcur[1].w)));
+        float2 fourth = make_float2(fmaf(v[e8 * 8 + 3], g.zscale, -lcur[0].w), fmaf(v[e8 * 8 + 7], g.zscale, -lcur[1].w));
+        if (BID == kBidExpshift) {                           // exponents past 128: as in the fused sweep
+          fourth = poly_exp2_two<4>(make_float2(min_nan(fourth.x - 1.f, 128.f), min_nan(fourth.y - 1.f, 128.f)));
+          fourth = add2(fourth, fourth);
+        } else {
+          fourth = poly_exp2_two<4>(fourth);
+        }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const float ls[4] = {lcur[h].x, lcur[h].y, lcur[h].z, lcur[h].w};
@@ -2528,7 +2533,7 @@ inline int forward_main(const void* q, const void* k, const void* v, const Geom&
       if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
       kern<<<grid, kMainThreads<kNarrow>, smem, st>>>(mq, mk, mv, g, rmax, rden, carry, carry_base, nullptr, out, ssum);
     } else {
-      auto kern = forward_main_kernel<SHARE, PAIR>;
+      auto kern = g.normalised ? forward_main_kernel<SHARE, PAIR> : forward_main_kernel<SHARE, SHARE != kShareInclusive, kBidExpshift>;
       if (int rc = set_smem_attr((const void*)kern, smem, err, errlen)) return rc;
       kern<<<grid, 256, smem, st>>>(mq, mk, mv, g, rmax, rden, carry, carry_base, out, ssum);
     }

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-def _run(pkg, q, k, v, bid, shift, eps, fused):
+def _run(pkg, q, k, v, bid, shift, eps, fused, share=1):
     lib, L = pkg._lib.load(), pkg._lib
     n, seq = q.shape[1], q.shape[2]
     out, ssum, total = (torch.empty(n, seq, *s, device=DEV) for s in ((64,), (), ()))
@@ -22,7 +22,7 @@ def _run(pkg, q, k, v, bid, shift, eps, fused):
     if fused:
         rc = lib.dilution_variant_forward_fused(*args, shift, carry.data_ptr(), total.data_ptr(), out.data_ptr(), ssum.data_ptr(), st)
     else:
-        rc = lib.dilution_variant_forward(*args, 1, shift, None, None, carry.data_ptr(), total.data_ptr(), out.data_ptr(),
+        rc = lib.dilution_variant_forward(*args, share, shift, None, None, carry.data_ptr(), total.data_ptr(), out.data_ptr(),
                                           ssum.data_ptr(), None, st)
     L.check(rc, "variant forward")
     return out, ssum, total, carry
@@ -73,12 +73,13 @@ def _one_large_score(rows, seq, row, key, score):
 @pytest.mark.parametrize("rows,seq", [(2, 200), (200, 600)])
 @pytest.mark.parametrize("row", [60, 61, 62, 63, 64, 67, 96])
 @pytest.mark.parametrize("score", [88.5, 89.5, 98.5, 150.0, 400.0])
-def test_an_expshift_bid_that_overflows_spoils_its_own_row(rows, seq, row, score):
+@pytest.mark.parametrize("fused", [True, False])
+def test_an_expshift_bid_that_overflows_spoils_its_own_row(rows, seq, row, score, fused):
     """exp(88.5) is an fp32 number, exp(89.5) is not: its demand is infinite from there on and its own row is inf / inf, but later
     rows are finite: nobody gets a share of that key any more."""
     pkg = load_package()
     key = 40
-    out, ssum, total, carry = _run(pkg, *_one_large_score(rows, seq, row, key, score), "expshift", 1.0, 1e-9, True)
+    out, ssum, total, carry = _run(pkg, *_one_large_score(rows, seq, row, key, score), "expshift", 1.0, 1e-9, fused)
     over = score > 88.7
     nan_rows = out[0].isnan().any(-1).nonzero().flatten().tolist()
     assert nan_rows == ([row] if over else []), nan_rows
@@ -91,6 +92,22 @@ def test_an_expshift_bid_that_overflows_spoils_its_own_row(rows, seq, row, score
     keep = torch.ones(seq, dtype=torch.bool, device=DEV)
     keep[key] = False
     assert total[0, keep].isfinite().all() and carry[0, :, :key].isfinite().all()
+
+
+@pytest.mark.parametrize("row", [60, 61, 62, 63, 67, 127])
+@pytest.mark.parametrize("share", [0, 2])
+@pytest.mark.parametrize("score", [88.5, 89.5, 150.0])
+def test_an_expshift_bid_that_overflows_without_the_inclusive_step(row, share, score):
+    """Its share, and the row's sum, are infinite; later shares of the key after the exclusive step are 0."""
+    pkg = load_package()
+    q, k, v = _one_large_score(2, 200, row, 40, score)
+    v = (v.float() * 0.1).bfloat16()                         # (the bid times a value, in fp32, is to be finite)
+    out, ssum, _, _ = _run(pkg, q, k, v, "expshift", 1.0, 1.0, False, share)
+    over = score > 88.7
+    assert out[0].isnan().any(-1).nonzero().flatten().tolist() == ([row] if over else [])
+    assert out[1].isfinite().all() and ssum[0, row].isinf().item() is over
+    if not over:                                             # all of the row's share
+        assert (out[0, row] - v[0, 0, 40].float()).abs().max().item() < 2e-3
 
 
 def test_training_calls_take_it():
