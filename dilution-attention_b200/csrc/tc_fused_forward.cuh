@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1) forward_fused_k
                        "r"(pk[4 * e8]), "r"(pk[4 * e8 + 1]), "r"(pk[4 * e8 + 2]), "r"(pk[4 * e8 + 3])
                        : "memory");
       };
-      mbar_wait(sdone + 8 * wg, t & 1, ctl, &g_status, kErrWaitMma);
+      mbar_wait_warp(sdone + 8 * wg, t & 1, ctl, &g_status, kErrWaitMma);
       tc_fence_after();
       tmem_ld32(tSw, v0);
       tmem_ld_wait(v0);

@@ -806,7 +806,7 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
     }
     __syncwarp();
   }
-  mbar_wait(sdone, njb & 1, ctl, &g_status, kErrWaitMma);
+  mbar_wait_warp(sdone, njb & 1, ctl, &g_status, kErrWaitMma);
   tc_fence_after();
   {
     // lane = query now: each warpgroup stores half of the output columns of row `row`, 32 at a time
@@ -1010,7 +1010,7 @@ __global__ void __launch_bounds__(kMainThreads<W>, W == kNarrow ? 2 : 1) forward
     if (jb + 1 < njb) den_next = load_den(jb + 1);   // lands while this tile is processed
     const bool dead = ja >= g.tk;
     const bool masked = dead || jb * kTileRows + kTileRows - 1 > qh;
-    mbar_wait(sdone, jb & 1, ctl, &g_status, kErrWaitMma);
+    mbar_wait_warp(sdone, jb & 1, ctl, &g_status, kErrWaitMma);
     tc_fence_after();
 #pragma unroll
     for (int c = 0; c < CW / 32; ++c) {
@@ -1076,7 +1076,7 @@ __global__ void __launch_bounds__(kMainThreads<W>, W == kNarrow ? 2 : 1) forward
         }
       };
       if (masked) chunk(std::true_type{}); else chunk(std::false_type{});
-      if (c == 0 && jb >= 1) mbar_wait(odone, (jb - 1) & 1, ctl, &g_status, kErrWaitMma);
+      if (c == 0 && jb >= 1) mbar_wait_warp(odone, (jb - 1) & 1, ctl, &g_status, kErrWaitMma);
 #pragma unroll
       for (int e8 = 0; e8 < 4; ++e8) {
         const uint32_t dst = sSh + share_chunk_offset(row, wg * CW + c * 32 + e8 * 8);
@@ -1093,7 +1093,7 @@ __global__ void __launch_bounds__(kMainThreads<W>, W == kNarrow ? 2 : 1) forward
     __syncwarp();
     if (lane == 0) mbar_arrive(shready);
   }
-  mbar_wait(odone, (njb - 1) & 1, ctl, &g_status, kErrWaitMma);
+  mbar_wait_warp(odone, (njb - 1) & 1, ctl, &g_status, kErrWaitMma);
   tc_fence_after();
   if (wg < 2) {
     // lane = query now: each of two warpgroups stores half of the output columns of row `row`, 32 at a time
@@ -1658,7 +1658,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
         }
         st_dbar = dbarp[row_base + i];
       }
-      mbar_wait(sdone + 8 * odd, s & 1, ctl, &g_status, kErrWaitMma);
+      mbar_wait_warp(sdone + 8 * odd, s & 1, ctl, &g_status, kErrWaitMma);
       tc_fence_after();
       float vs[32], vd[32];
       const uint32_t tcol = lane_base + 64 * odd + cw;
@@ -1697,7 +1697,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
         if (iq0 + lane < g.tq) atomicAdd(ghat + row_base + iq0 + lane, sum);
       } else {
         // the dQ MMAs of the previous 128 queries read the pdp buffer that is written next
-        if (!odd && s >= 1) mbar_wait(dqdone, (s - 1) & 1, ctl, &g_status, kErrWaitMma);
+        if (!odd && s >= 1) mbar_wait_warp(dqdone, (s - 1) & 1, ctl, &g_status, kErrWaitMma);
         uint32_t pdt[16];                              // 32 pdp values as bf16 pairs
 #pragma unroll
         for (int e8 = 0; e8 < 4; ++e8) {
@@ -1729,7 +1729,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) backward_main_kernel(
       if (lane == 0) mbar_arrive(tiles + 8 * odd);
     }
   }
-  mbar_wait(sdone + 8, nsteps & 1, ctl, &g_status, kErrWaitMma);
+  mbar_wait_warp(sdone + 8, nsteps & 1, ctl, &g_status, kErrWaitMma);
   tc_fence_after();
   if (PASS != 1 && warp < 8) {
     // lane = key: each warpgroup stores 32 of the 64 columns of dk_main and dv
@@ -2087,7 +2087,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) backward_slices_kernel(
       edge -= 4 * (int64_t)g.tk;
       if (!dead && i + 4 < 2 * nh) incl_next = *edge;
       const float4* Dbar4 = reinterpret_cast<const float4*>(sDbar + 64 * (u & 3) + ((i & 1) ? 0 : 32));
-      mbar_wait(sdone + 8 * wg, (i >> 2) & 1, ctl, &g_status, kErrWaitMma);
+      mbar_wait_warp(sdone + 8 * wg, (i >> 2) & 1, ctl, &g_status, kErrWaitMma);
       tc_fence_after();
       float p[32], inv[32];
       tmem_ld32(tSw, p);
@@ -2121,7 +2121,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) backward_slices_kernel(
         pdt[e >> 1] = pack_bf16(pd2.x, pd2.y);
       }
       // the products of half tile u - 2 have read the pdp buffer that is written next
-      if (u >= 2) mbar_wait(dqdone + 8 * (u & 1), ((u >> 1) - 1) & 1, ctl, &g_status, kErrWaitMma);
+      if (u >= 2) mbar_wait_warp(dqdone + 8 * (u & 1), ((u >> 1) - 1) & 1, ctl, &g_status, kErrWaitMma);
 #pragma unroll
       for (int c = 0; c < 4; ++c)
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sPd + kTileBytes * (u & 1) +
@@ -2346,7 +2346,7 @@ __global__ void __launch_bounds__(256, 2) backward_correction_kernel(
       mma_commit(lead, sdone);
     }
     __syncwarp();
-    mbar_wait(dqdone, t & 1, ctl, &g_status, kErrWaitMma);
+    mbar_wait_warp(dqdone, t & 1, ctl, &g_status, kErrWaitMma);
     tc_fence_after();
     {
       // lane = query: each warpgroup owns 32 of the 64 columns.  The fp32 tile is staged in
@@ -2371,7 +2371,7 @@ __global__ void __launch_bounds__(256, 2) backward_correction_kernel(
     tc_fence_before();
   }
   if (row == 0) tma_wait_read_all();
-  mbar_wait(sdone, nsteps & 1, ctl, &g_status, kErrWaitMma);
+  mbar_wait_warp(sdone, nsteps & 1, ctl, &g_status, kErrWaitMma);
   tc_fence_after();
   {
     // lane = key: each warpgroup finishes 32 of the 64 columns of dk

@@ -656,7 +656,7 @@ __global__ void __launch_bounds__(256, W == kNarrow ? 4 : 2) backward_key_correc
     }
     __syncwarp();
   }
-  mbar_wait(sdone, nhalf & 1, ctl, &g_status, kErrWaitMma);
+  mbar_wait_warp(sdone, nhalf & 1, ctl, &g_status, kErrWaitMma);
   tc_fence_after();
   // lane = key: each warpgroup finishes half of the columns of dk, 32 at a time
   constexpr int kHead = Rows<W>::kHead, kHalf = kHead / 2;

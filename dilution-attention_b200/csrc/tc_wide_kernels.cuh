@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
       // statistics go two half-steps ahead: one barrier of the compute warps lies between their store and their use
       const bool fetch = wg == 0 && row < 64 && h + 2 < nhalf;
       if (fetch) load_stats(hb - 2, &nx_lse, &nx_dbar, &nx_gh);
-      mbar_wait(sdone + (NS == 2 ? 8 * b : 0), (h / NS) & 1, ctl, &g_status, kErrWaitMma);
+      mbar_wait_warp(sdone + (NS == 2 ? 8 * b : 0), (h / NS) & 1, ctl, &g_status, kErrWaitMma);
       tc_fence_after();
       float vs[32], vd[32];
       tmem_ld32(tS + sc + tcol, vs);
@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
       const float fix = wg == 1 ? rother : 0.f;
       sigma = R + rother;                              // the suffix behind the next half-step
       // the dQ products of the previous half-step read the pdp buffer that is written next
-      if (h >= 1) mbar_wait(dqdone, (h - 1) & 1, ctl, &g_status, kErrWaitMma);
+      if (h >= 1) mbar_wait_warp(dqdone, (h - 1) & 1, ctl, &g_status, kErrWaitMma);
       {
         uint32_t pdt[16 * P];
 #pragma unroll
@@ -443,7 +443,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) wide_backward_main_kernel(
       }
     }
   }
-  mbar_wait(sdone + 8 * (NS - 1), (nhalf / NS) & 1, ctl, &g_status, kErrWaitMma);   // the last commit: every product
+  mbar_wait_warp(sdone + 8 * (NS - 1), (nhalf / NS) & 1, ctl, &g_status, kErrWaitMma);   // the last commit: every product
   tc_fence_after();
   if (warp < 8) {
     // lane = key: each warpgroup stores half of the columns of dk_main and dv, 32 at a time

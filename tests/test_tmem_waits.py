@@ -35,3 +35,18 @@ def test_cluster_barriers_do_not_take_whole_warps_for_granted():
     for path in glob.glob(os.path.join(ROOT, "dilution-attention_b200", "csrc", "*.cuh")):
         for line in open(path):
             assert not re.search(r'asm.*barrier\.cluster\..*\.aligned', line), (path, line)
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=os.path.basename)
+def test_lanes_meet_between_a_poll_and_a_warp_wide_instruction(path):
+    """Lanes may leave a polling loop in different turns; tcgen05.ld and .st and setmaxnreg want all 32 of them."""
+    lines = open(path).read().split("\n")
+    meets = re.compile(r"__sync(warp|threads)\(|mbar_wait_warp\(|wg_barrier\(|bar\.sync")
+    wants = re.compile(r"\btmem_(ld|st)\d+\(|setmaxnreg|row_half_tile<|row_merge<")
+    for at, line in enumerate(lines):
+        if not re.search(r"\bmbar_wait\(", line) or "== 0) mbar_wait(" in line or "bool mbar_wait(" in line or path.endswith("tc_common.cuh"):
+            continue
+        for after in lines[at + 1:]:
+            if meets.search(after) or after == "}":
+                break
+            assert not wants.search(after), (at + 1, line, after)
