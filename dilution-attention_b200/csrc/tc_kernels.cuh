@@ -784,7 +784,8 @@ __global__ void __launch_bounds__(256, 2) forward_main_kernel(
       }
     }
     };
-    if (diag || dead) tile(std::true_type{}); else tile(std::false_type{});
+    // (by whole warps: the TMEM loads are warp-wide, and the keys of a row may end in the middle of one)
+    if (__any_sync(0xffffffffu, diag || dead)) tile(std::true_type{}); else tile(std::false_type{});
     fence_async_smem();
     tc_fence_before();
     __syncthreads();

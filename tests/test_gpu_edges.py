@@ -94,3 +94,14 @@ def test_operands_off_a_16_byte_boundary_are_refused_and_upstream_gradients_copi
     ref = torch.autograd.grad(out, leaves, dout.clone())
     for a, b in zip(got, ref):
         assert torch.allclose(a.float(), b.float(), rtol=1e-2, atol=1e-3 * b.abs().max().item())
+
+
+@pytest.mark.parametrize("queries,keys", [(300, 200), (257, 130), (700, 129), (384, 33), (130, 1)])
+def test_more_queries_than_keys(kernels, queries, keys):
+    """The last key tile ends in the middle of a warp, for queries that see all of it: forward only, against the exact kernels on
+    the same operands."""
+    q, k, v, _ = make_inputs(1, 2, queries, 64, 21)
+    x = [t.bfloat16().to(DEV) for t in (q, k[:, :, :keys], v[:, :, :keys])]
+    out = kernels.dilution_attention_forward(*x, dot_precision="bf16")
+    ref = kernels.dilution_attention_forward(*(t.float() for t in x), dot_precision="ieee")
+    assert (out - ref).abs().max().item() < 2e-2
