@@ -59,6 +59,18 @@ def test_a_row_does_not_depend_on_how_many_there_are(rows, seq, few, d, dtype, s
         assert torch.equal(many[:few], one)
 
 
+@pytest.mark.parametrize("what", [0, 1, 2])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf")])
+@pytest.mark.parametrize("pos", [3, 70, 6143, 6199])
+def test_values_that_are_not_finite(what, value, pos):
+    """What such a value does is the same in a call of 264 blocks of 256 queries and in one of 240, bit for bit."""
+    x = _inputs(11, 6200, 64, 1.0)
+    x[what][1, pos, 5] = value
+    for many, one in zip(_narrow(*x), _narrow(*(t[:10].contiguous() for t in x))):
+        assert torch.equal(many[:10].isnan(), one.isnan()) and torch.equal(many[:10].nan_to_num(7.0), one.nan_to_num(7.0))
+        assert many[0].isfinite().all() and many[2:].isfinite().all()
+
+
 @pytest.mark.parametrize("std", [1.0, 24.0])
 def test_both_sides_of_the_line(std):
     x = _inputs(11, 6144, 64, std)

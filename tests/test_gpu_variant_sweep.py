@@ -122,6 +122,25 @@ def test_training_calls_take_it():
         assert name in names, names
 
 
+def test_deterministic_algorithms_keep_the_two_passes():
+    pkg = load_package()
+    x = [t.requires_grad_(True) for t in _inputs(8, 2048)]
+    call = lambda: pkg.kernels_bid.dilution_attention(*x, dot_precision="bf16", bid="sigmoid", share_cumsum=True)      # noqa: E731
+    sweep = call().detach()
+    torch.use_deterministic_algorithms(True)
+    try:
+        pkg._lib.profile(True)
+        pkg._lib.profile_collect()
+        got = [call().detach() for _ in range(3)]
+        names = set(pkg._lib.profile_collect())
+        pkg._lib.profile(False)
+    finally:
+        torch.use_deterministic_algorithms(False)
+    assert "tc_forward_main" in names and "tc_forward_fused" not in names, names
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+    assert (sweep - got[0]).abs().max().item() < 1e-2                      # both round their shares to bf16
+
+
 def test_other_calls_are_refused():
     pkg = load_package()
     lib, L = pkg._lib.load(), pkg._lib

@@ -22,6 +22,12 @@ KERNELS = [
 ]
 
 
+KERNELS += [
+    ("backward_slices_kernel", "tc_kernels.cuh", "if (wg == 4) {\n    // ---", "setmaxnreg.inc"),
+    ("rowpass_issuer_kernel", "tc_rowpass_kernels.cuh", "if (warp_u == 8 * NT) {", "drain_if_aborted"),
+]
+
+
 @pytest.mark.parametrize("kernel,name,begin,end", KERNELS, ids=[k[0] for k in KERNELS])
 def test_lanes_meet_behind_every_wait(kernel, name, begin, end):
     text = open(os.path.join(CSRC, name)).read()

@@ -73,3 +73,10 @@ def test_every_launch_of_a_split_asks():
     for name, launches in (("tc_fused_forward.cuh", 1), ("tc_kernels.cuh", 1), ("tc_wide_kernels.cuh", 3)):
         asks = re.findall(r"set_smem_attr\(\(const void\*\)\w[^;]*" + kernels[name] + r"[^;]*;", _text(name))
         assert len(asks) == launches, (name, asks)
+
+
+def test_the_reverse_pass_in_slices_asks_too():
+    """tc_kernels.cuh has a second kernel with a split, and one launch of it; no third."""
+    text = _text("tc_kernels.cuh")
+    assert len(re.findall(r"set_smem_attr\(\(const void\*\)\w[^;]*kSliceRegs[^;]*;", text)) == 1
+    assert text.count("setmaxnreg.inc") == 2 and "static_assert(4 * 104 + 64 <= 5 * kSliceRegs" in text
