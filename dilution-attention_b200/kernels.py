@@ -115,9 +115,10 @@ def _sweep_is_faster(n, seq, carry_rows):
     is zeroed, reduced into and divided once per row of few tiles: n = 48, T = 1536 74 / 74, n = 16, T = 1536 49 / 51, n = 64,
     T = 1024 57 / 55, n = 384, T = 512 107 / 103, n = 1024, T = 128 61 / 52; with 256 blocks of 512 keys it still wins from 1024
     tokens on: n = 384, T = 1024 251 / 271, n = 128, T = 1024 93 / 98, but n = 512, T = 768 236 / 233.  Training calls of fewer
-    than 74 blocks of 256 keys (half of the SMs) take it at any length, and those of up to 100 that are no longer than 2048 tokens
-    the two passes: within 5 us of each other, where a step's launches take the host 150.  Calls that no backward follows keep the
-    two passes up to 2048 tokens, where those repeat bit for bit."""
+    than 74 blocks of 256 keys (half of the SMs) take it at any length.  Those of 74 to 100 that are no longer than 2048 tokens keep the
+    two passes, as they have had them: 2 to 8 us more (n = 13, T = 1536 46 / 48, n = 16, T = 1536 46 / 50, n = 12, T = 2048 55 / 63), where
+    a step's launches take the host 150.  Calls that no backward follows keep the two passes up to 2048 tokens, where those repeat
+    bit for bit."""
     if carry_rows != 32:
         return seq > 2048
     blocks = n * -(-seq // 256)
@@ -126,15 +127,12 @@ def _sweep_is_faster(n, seq, carry_rows):
     return blocks > 100 if seq >= 1536 else seq >= 1024 and n * -(-seq // 512) >= 256
 
 
-def _two_passes(n, seq, carry_rows):
-    """Calls that keep the column-sum and main passes under torch.use_deterministic_algorithms, whose outputs and demands repeat bit
-    for bit; the sweep adds up outputs in memory in no fixed order.  Calls that no backward follows all do (_takes_sweep).  A
-    training call's gradients do not repeat either way, so it gives up the sweep only where the sweep does not fill the chip, or
-    rows are short, and the host's launches outlast neither."""
+def _two_passes(n, seq):
+    """Training calls that keep the column-sum and main passes under torch.use_deterministic_algorithms, whose outputs repeat bit for
+    bit; the sweep adds up outputs in memory in no fixed order.  Gradients do not repeat either way, so these are the calls that
+    have had repeatable outputs, not those where the two passes are the faster ones (_sweep_is_faster)."""
     if seq > 2048 and n * -(-seq // 512) >= 256:
         return False
-    if carry_rows != 32:
-        return True
     blocks = n * -(-seq // 256)
     return blocks >= 74 if seq <= 2048 else seq >= 2560 or blocks > 100
 
@@ -144,7 +142,7 @@ def _takes_sweep(code, prec, n, tq, tk, head_dim, carry_rows):
     if not (TC_FUSED_FORWARD and tq == tk and _lib.tensor_core_path(code, prec, head_dim)):
         return False
     if torch.are_deterministic_algorithms_enabled():
-        return carry_rows == 32 and not _two_passes(n, tq, carry_rows)
+        return carry_rows == 32 and not _two_passes(n, tq)
     return _sweep_is_faster(n, tq, carry_rows)
 
 
@@ -213,10 +211,10 @@ def dilution_attention_forward(
     order in which an output's partial sums are added (kernels pick their blocks by a
     slab's rows).
 
-    On the tensor-core path a call of 256 blocks of 512 keys or more adds up its output in
-    no fixed order and repeats to fp32 rounding only; under
-    torch.use_deterministic_algorithms(True) it takes kernels that repeat bit for bit
-    (unless a backward will follow), a sixth slower at 128K tokens.
+    On the tensor-core path a call of more than 2048 tokens adds up its output in no fixed
+    order and repeats to fp32 rounding only; under torch.use_deterministic_algorithms(True)
+    it takes kernels that repeat bit for bit (unless a backward will follow), about a third
+    slower at 128K tokens.
     """
     result, aux = _attention_forward(q, k, v, dot_precision, return_aux, _save_pk, scratch_budget_gib, _training)
     if return_aux:

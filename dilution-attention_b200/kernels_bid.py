@@ -223,7 +223,13 @@ def dilution_attention(
     shift: float = 1.0,
 ) -> torch.Tensor:
     """Differentiable fused attention under the selected bid and share step
-    (kernels_bid.py:818-849)."""
+    (kernels_bid.py:818-849).
+
+    On the tensor-core path the element-wise bids (sigmoid, expshift, sigshift) with the
+    inclusive share step add up the output of long calls (_takes_sweep) in no fixed order, which
+    repeats to fp32 rounding only; under torch.use_deterministic_algorithms(True), and in
+    dilution_attention_forward, it repeats bit for bit.
+    """
     code_b, code_s = _bid_code(bid), _share_code(share_cumsum)
     _resolve_precision(dot_precision)
     if _is_operator(bid, share_cumsum):

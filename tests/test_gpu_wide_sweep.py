@@ -51,11 +51,17 @@ def test_sweep_of_512_keys(rows, seq, training):
         assert (out[:, r:r + 1].cpu() - want).abs().max().item() < 2e-2
 
 
-@pytest.mark.parametrize("rows,seq,training,sweep", [(52, 2048, False, False), (52, 2049, False, True), (51, 2049, False, False),
-                                                     (10, 2559, True, True), (10, 2560, True, False), (32, 4096, True, True),
-                                                     (31, 4096, True, False)])
+def _route(rows, seq, training):
+    pkg = load_package()
+    return pkg.kernels._takes_sweep(pkg._lib.BF16, pkg._lib.PREC["bf16"], rows, seq, seq, 64, 32 if training else 64)
+
+
+@pytest.mark.parametrize("rows,seq,training,sweep", [(52, 2048, False, False), (52, 2049, False, True), (51, 2049, False, True),
+                                                     (1, 2049, False, True), (10, 2559, True, True), (10, 2560, True, True),
+                                                     (12, 2304, True, True), (32, 4096, True, True), (31, 4096, True, True),
+                                                     (12, 1536, True, True), (13, 1536, True, False), (16, 1600, True, True)])
 def test_route(rows, seq, training, sweep):
-    assert load_package().kernels._two_passes(rows, seq, 32 if training else 64) is not sweep
+    assert _route(rows, seq, training) is sweep
 
 
 def test_deterministic_algorithms_keep_the_two_passes():
@@ -78,8 +84,13 @@ def test_deterministic_algorithms_keep_the_two_passes():
     assert (sweep - got[0][0]).abs().max().item() < 1e-2                  # both round their shares to bf16
 
 
-@pytest.mark.parametrize("rows,seq,sweep", [(11, 2304, True), (12, 2304, False), (10, 2559, True), (11, 2559, False),
-                                            (51, 2559, False), (52, 2559, True)])
-def test_route_of_training_calls_a_little_longer_than_short_rows(rows, seq, sweep):
-    """Beyond 100 blocks of 256 keys the sweep of few blocks is slower than the two passes by more than the host hides."""
-    assert load_package().kernels._two_passes(rows, seq, 32) is not sweep
+@pytest.mark.parametrize("rows,seq,sweep", [(11, 2304, True), (12, 2304, False), (10, 2559, True), (10, 2560, False), (11, 2559, False),
+                                            (51, 2559, False), (52, 2559, True), (32, 4096, True), (31, 4096, False)])
+def test_route_under_deterministic_algorithms(rows, seq, sweep):
+    """Training calls keep the two passes, whose outputs repeat, beyond 100 blocks of 256 keys or 2559 tokens and up to 256 blocks of 512;
+    calls that no backward follows always do."""
+    torch.use_deterministic_algorithms(True)
+    try:
+        assert _route(rows, seq, True) is sweep and _route(rows, seq, False) is False
+    finally:
+        torch.use_deterministic_algorithms(False)
