@@ -113,9 +113,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, Ctl* ct
 }
 
 // The wait of a whole warp: its lanes meet behind it.  Every lane polls for itself and may leave in another turn than its
-// neighbours, but TMEM loads and stores and register hand-overs want the warp whole (.sync.aligned).  In a warp that issues only the elected lane's
-// MMAs, commits and copies make the barriers go on; a lane that was still polling when the phase after the next began
-// would wait for a parity that comes back no more.  No such lane can exist if nothing is issued before all have seen the phase.
+// neighbours, but TMEM loads and stores and register hand-overs want the warp whole (.sync.aligned).  In a warp that issues only
+// the elected lane's MMAs, commits and copies make the barriers go on; a lane that was still polling when the phase after the next
+// began would wait for a parity that comes back no more.  No such lane can exist if nothing is issued before all have seen the phase.
 __device__ __forceinline__ void mbar_wait_warp(uint32_t bar, uint32_t parity, Ctl* ctl, int* status, int code) {
   mbar_wait(bar, parity, ctl, status, code);
   __syncwarp();

@@ -1194,9 +1194,9 @@ __device__ __forceinline__ float mass_jac(float f, float l, const Geom& g) {
 
 // One thread's 32 queries of the main reverse pass: vs holds their raw scores against the thread's key, vd
 // dO' . v; incle is the key's demand (+ eps) in front of them, R the suffix of dk_share behind them, and query
-// e sees the key when e >= first_q and, under END, e < end_q (MASK; all of them do otherwise).  Afterwards shp holds the shares as bf16 pairs (SPLIT: their lo plane
-// behind them), vs the Jacobian factor, vd that factor times dp, and R the suffix in front of the queries.
-// Two sweeps.  Forwards: p and 1/(committed+p+eps), the demand
+// e sees the key when e >= first_q and, under END, e < end_q (MASK; all of them do otherwise).  Afterwards shp holds the shares as
+// bf16 pairs (SPLIT: their lo plane behind them), vs the Jacobian factor, vd that factor times dp, and R the suffix in front of the
+// queries.  Two sweeps.  Forwards: p and 1/(committed+p+eps), the demand
 // accumulated from the checkpoint in front exactly as the forward pass did.  Backwards: the
 // suffix of dk_share (kernels.py:763-764), accumulated from the last query to the first as
 // the reference does — its terms grow towards a key's first bidders, so the other order
@@ -1995,7 +1995,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) backward_slices_kernel(
         slice(C0{});
         slice(C1{});
         // both slices of the half tile exist.  Once dQ^T of the one before is out, its queries' places in the ring are free, and
-        // dbar' of half tile u + 3 is in its place
+        // dbar' of half tile u + 3 is in its place (its scores are issued in the turn for u + 1)
         if (u >= 1) {
           mbar_wait_warp(dqfree, (u - 1) & 1, ctl, &g_status, kErrWaitDrain);
           tc_fence_after();
@@ -2020,7 +2020,8 @@ __global__ void __launch_bounds__(kSliceThreads, 1) backward_slices_kernel(
     } else {
       // dQ^T of half tile u to global memory by two warps, lane = feature (staging is doubled: a tile does not wait for the copy
       // engine to have read the one before).  The third keeps dbar': that of half tile u + 4 takes the place of half tile u, whose
-      // last use lies in front of dqdone; the issuing warp has waited for the release of u before it issues scores of u + 3.
+      // last use lies in front of dqdone; the issuing warp waits for the release of u at the end of its turn for u + 1, in front of the
+      // scores of u + 4.
       if (warp_u == 18) {
         float next[2] = {0.f, 0.f};
         auto fetch = [&](int u) {                              // (every row of an earlier half tile exists)
